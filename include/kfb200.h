@@ -102,6 +102,13 @@ int kfb_dequantize(const void* packed, const void* scales, int N, int K, int gro
  * INT4 weight-only linear  y[M, N] = x[M, K] @ W_hat[N, K]^T,  x and y fp16.
  * ------------------------------------------------------------------------------------- */
 
+/* The dispatcher behind ops.int4_linear (kernelforge/ops.py:193-214, 286-302): any M >= 1, N >= 1, the kernel chosen by
+ * shape.  x, bias and y are of `dtype` (KFB_F16 or KFB_BF16); bias [N] or NULL is added to the rounded product and the
+ * sum rounded again, like `y + bias`.  Workspace: kfb_int4_linear_ws_bytes bytes, 16-byte aligned (0: none needed). */
+size_t kfb_int4_linear_ws_bytes(int M, int N, int K, int group, int dtype);
+int kfb_int4_linear(const void* x, const void* packed, const void* scales, const void* bias, void* y,
+                    int M, int N, int K, int group, int dtype, void* ws, size_t ws_bytes, void* stream);
+
 /* int4_gemv (csrc/gemm/dequant_gemv.cu:21-36, kernel csrc/gemm/dequant_gemv_kernel.cuh:38-109):
  * 1 <= M <= 8, any N >= 1, K % group == 0, group in {64,128}.  FP32 accumulation, one
  * rounding to fp16.  No workspace.  The weights are streamed by the TMA unit into shared

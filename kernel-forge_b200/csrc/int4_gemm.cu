@@ -17,6 +17,7 @@
 // Split-K partial sums are reduced in split order by a second kernel (deterministic).
 // Rows past N and batch rows past M are zero-filled by TMA and never stored.
 #include "common.cuh"
+#include "int4_gemm.cuh"
 #include "sm100.cuh"
 
 namespace kfb {
@@ -46,6 +47,7 @@ struct OutSpec {
   int ld;    // row stride of every buffer, in elements
   int col0;  // first column this rank writes
   int bf16;  // the buffers hold bf16 instead of fp16 (the 16-bit stores are the same)
+  const uint16_t* bias;  // [N] of the output type or nullptr: added to the rounded product, rounded again (as `y + bias`)
 };
 
 template <int MT>
@@ -108,6 +110,17 @@ __device__ __forceinline__ uint16_t round16(float v, bool bf16) {
   }
   const __half h = __float2half_rn(v);
   return *reinterpret_cast<const uint16_t*>(&h);
+}
+
+// round16(v), then + bias as a 16-bit addition: the two roundings of `y = product; y + bias`
+__device__ __forceinline__ uint16_t round16_bias(float v, uint16_t bias, bool bf16) {
+  const uint16_t r = round16(v, bf16);
+  if (bf16) {
+    const __nv_bfloat16 a = *reinterpret_cast<const __nv_bfloat16*>(&r), b = *reinterpret_cast<const __nv_bfloat16*>(&bias);
+    return round16(__bfloat162float(a) + __bfloat162float(b), true);
+  }
+  const __half a = *reinterpret_cast<const __half*>(&r), b = *reinterpret_cast<const __half*>(&bias);
+  return round16(__half2float(a) + __half2float(b), false);
 }
 
 // out: fp16 (bf16) y [M, N] when splits == 1, else FP32 partial [splits][M][N]
@@ -262,6 +275,8 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       uint8_t* tile = smem + wg * L::kStage;       // every stage is free once acc_done has completed
       const bool f32 = splits > 1;
       const int n_valid = min(kTileN, N - n0);     // columns of this tile that exist
+      const bool with_bias = !f32 && out.bias != nullptr;
+      const uint16_t bias = with_bias ? out.bias[min(row, N - 1)] : (uint16_t)0;
       constexpr int kCols = MT >= 32 ? 32 : MT;
       constexpr int kChunks = MT >= 32 ? MT / 32 : 1;
 #pragma unroll 1
@@ -281,7 +296,8 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         } else {
 #pragma unroll
           for (int c = 0; c < kCols; ++c)
-            reinterpret_cast<uint16_t*>(tile)[c * kTileN + r] = round16(__uint_as_float(acc[c]), kBf16);
+            reinterpret_cast<uint16_t*>(tile)[c * kTileN + r] =
+                with_bias ? round16_bias(__uint_as_float(acc[c]), bias, kBf16) : round16(__uint_as_float(acc[c]), kBf16);
         }
         asm volatile("bar.sync %0, 128;" ::"r"(1 + wg) : "memory");
         const int m_hi = min(kCols, M - (m0 + c0));  // batch rows of this chunk that exist
@@ -343,7 +359,7 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restr
     for (int s = 0; s < splits; ++s) acc += partial[(size_t)s * elems + i];
     const long long m = i / N;
     const int n = (int)(i - m * N);
-    const uint16_t v = round16(acc, out.bf16 != 0);
+    const uint16_t v = out.bias ? round16_bias(acc, out.bias[n], out.bf16 != 0) : round16(acc, out.bf16 != 0);
     for (int p = 0; p < out.count; ++p) reinterpret_cast<uint16_t*>(out.y[p])[m * out.ld + out.col0 + n] = v;
   }
 }
@@ -477,27 +493,29 @@ int gemm_common(const void* x, const void* packed, const void* scales, const gem
 
 }  // namespace
 
-extern "C" int kfb_int4_gemm(const void* x, const void* packed, const void* scales, void* y, int M, int N, int K,
-                             int group, void* ws, size_t ws_bytes, void* stream) {
-  gemm::OutSpec out = {};
+size_t kfb::gemm::ws_bytes(int M, int N, int K, int group) { return kfb_int4_gemm_ws_bytes(M, N, K, group); }
+
+int kfb::gemm::run(const void* x, const void* packed, const void* scales, const void* bias, void* y, int M, int N, int K, int group,
+                   bool bf16, void* ws, size_t ws_bytes, cudaStream_t stream) {
+  OutSpec out = {};
   out.y[0] = static_cast<__half*>(y);
   out.count = 1;
   out.ld = N;
-  out.col0 = 0;
-  if (!y) return fail(KFB_ERR_INVALID, "null pointer");
+  out.bf16 = bf16;
+  out.bias = static_cast<const uint16_t*>(bias);
   return gemm_common(x, packed, scales, out, M, N, K, group, ws, ws_bytes, stream);
+}
+
+extern "C" int kfb_int4_gemm(const void* x, const void* packed, const void* scales, void* y, int M, int N, int K,
+                             int group, void* ws, size_t ws_bytes, void* stream) {
+  if (!y) return fail(KFB_ERR_INVALID, "null pointer");
+  return gemm::run(x, packed, scales, nullptr, y, M, N, K, group, false, ws, ws_bytes, (cudaStream_t)stream);
 }
 
 extern "C" int kfb_int4_gemm_bf16(const void* x, const void* packed, const void* scales, void* y, int M, int N, int K,
                                   int group, void* ws, size_t ws_bytes, void* stream) {
-  gemm::OutSpec out = {};
-  out.y[0] = static_cast<__half*>(y);
-  out.count = 1;
-  out.ld = N;
-  out.col0 = 0;
-  out.bf16 = 1;
   if (!y) return fail(KFB_ERR_INVALID, "null pointer");
-  return gemm_common(x, packed, scales, out, M, N, K, group, ws, ws_bytes, stream);
+  return gemm::run(x, packed, scales, nullptr, y, M, N, K, group, true, ws, ws_bytes, (cudaStream_t)stream);
 }
 
 extern "C" int kfb_int4_gemm_allgather(const void* x, const void* packed, const void* scales, void* const* y_all,

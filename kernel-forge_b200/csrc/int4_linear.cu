@@ -1,0 +1,58 @@
+// The dispatcher of the INT4 linear: which kernel serves (M, N, K, dtype).  Host code only.
+//
+// The reference's dispatcher (kernelforge/ops.py:193-214) knows a GEMV up to M = 7 and a GEMM above; here:
+//   M = 1                 CUDA-core GEMV (int4_gemv.cu): one row of activations, nothing for an MMA to share
+//   fp16, N >= 75776      persistent streaming kernel (int4_gemv_mma.cuh) up to M = 16, where it has no bias to add
+//   M <= 32               small-batch kernel (int4_small.cu)
+//   otherwise             tcgen05 GEMM (int4_gemm.cu)
+#include "int4_gemm.cuh"
+#include "int4_small.cuh"
+
+using namespace kfb;
+
+namespace {
+
+enum class Route { kGemv, kStream, kSmall, kGemm };
+
+// Where the lines lie (graph of L2-cold calls, us):
+//   M = 1: GEMV / small-batch kernel 5632x2048 4.1/4.7, 1536x8960 5.2/6.2, 2560x2048 3.7/3.7, but 8960x1536 5.0/4.8,
+//     11264x2048 8.0/7.3: the GEMV's four or eight rows per warp leave it too few warps there.
+//   M = 32: small-batch kernel / GEMM 5632x2048 11.7/14.5, 2048x5632 8.7/11.9, 1536x8960 11.5/12.8, 8960x1536 10.7/16.0,
+//     11264x2048 17.4/17.9; the kernel's activation reads grow with M * N, the GEMM's time hardly with M.
+Route route(int M, int N, int K, int dtype, bool bias) {
+  const bool fp16 = dtype == KFB_F16;
+  if (fp16 && N >= 75776 && !bias && M <= 16) return M <= 8 ? Route::kGemv : Route::kStream;
+  if (fp16 && M == 1 && N < 8192) return Route::kGemv;
+  if (M <= 16 || (M <= 32 && (long long)N * K <= 24LL << 20)) return Route::kSmall;
+  return Route::kGemm;
+}
+
+}  // namespace
+
+extern "C" size_t kfb_int4_linear_ws_bytes(int M, int N, int K, int group, int dtype) {
+  return M <= 16 ? 0 : route(M, N, K, dtype, false) == Route::kGemm ? gemm::ws_bytes(M, N, K, group) : 0;
+}
+
+extern "C" int kfb_int4_linear(const void* x, const void* packed, const void* scales, const void* bias, void* y, int M, int N,
+                               int K, int group, int dtype, void* ws, size_t ws_bytes, void* stream) {
+  if (dtype != KFB_F16 && dtype != KFB_BF16) return fail(KFB_ERR_INVALID, "int4_linear takes fp16 or bf16 activations");
+  if (!x || !packed || !scales || !y) return fail(KFB_ERR_INVALID, "null pointer");
+  if (M < 1) return fail(KFB_ERR_INVALID, "int4_linear needs M >= 1, got M=%d", M);
+  switch (route(M, N, K, dtype, bias != nullptr)) {
+    case Route::kGemv:
+      if (bias) return kfb_int4_gemv_fused(x, packed, scales, y, M, N, K, group, 0, nullptr, 0.0f, bias, nullptr, 0, stream);
+      return kfb_int4_gemv(x, packed, scales, y, M, N, K, group, 0, stream);
+    case Route::kStream: return kfb_int4_small_batch(x, packed, scales, y, M, N, K, group, 0, stream);
+    case Route::kSmall: {
+      if (int rc = require_sm100()) return rc;
+      if (group != 64 && group != 128) return fail(KFB_ERR_INVALID, "group_size must be one of (64, 128), got %d", group);
+      if (N < 1 || K < group || K % group) return fail(KFB_ERR_INVALID, "K=%d is not a multiple of group_size=%d", K, group);
+      if (!aligned16(x) || !aligned16(packed)) return fail(KFB_ERR_ALIGNMENT, "x and packed must be 16-byte aligned");
+      gemv::Fusion fu = {};
+      fu.bias = static_cast<const __half*>(bias);
+      return small::run(x, packed, scales, y, M, N, K, group, dtype == KFB_BF16, /*weights_first=*/pdl_enabled(), pdl_enabled(),
+                        (cudaStream_t)stream, fu);
+    }
+    default: return gemm::run(x, packed, scales, bias, y, M, N, K, group, dtype == KFB_BF16, ws, ws_bytes, (cudaStream_t)stream);
+  }
+}

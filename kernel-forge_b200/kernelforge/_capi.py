@@ -44,6 +44,9 @@ _SIGNATURES = {
     "kfb_unpack_int4": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p]),
     "kfb_pack_int4": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p]),
     "kfb_dequantize": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_void_p]),
+    "kfb_int4_linear_ws_bytes": (c_size_t, [c_int, c_int, c_int, c_int, c_int]),
+    "kfb_int4_linear": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p,
+                                c_size_t, c_void_p]),
     "kfb_int4_gemv": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p]),
     "kfb_int4_gemv_fused": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_float,
                                     c_void_p, c_void_p, c_int, c_void_p]),
@@ -116,6 +119,23 @@ def lib() -> ctypes.CDLL:
                 f"libkfb200.so is not built or incomplete ({exc}). Run `python kernel-forge_b200/build.py`."
             ) from exc
     return _lib
+
+
+_host = None
+
+
+def host():
+    """kernelforge._host: the same library called with torch tensors from native code (csrc/host.cpp).  Raises ImportError
+    when it is not built."""
+    global _host
+    if _host is None:
+        lib()
+        try:
+            from . import _host as module
+        except ImportError as exc:
+            raise ImportError(f"kernelforge._host is not built or incomplete ({exc}). Run `python kernel-forge_b200/build.py`.") from exc
+        _host = module
+    return _host
 
 
 def check(rc: int) -> None:
