@@ -1,10 +1,11 @@
-"""Builds libkfb200.so (the C-ABI library) in-tree with nvcc for sm_100a.
+"""Builds libkfb200.so (the C-ABI library, nvcc for sm_100a) and kernelforge._host (its caller on torch tensors) in-tree.
 
     python kernel-forge_b200/build.py [--force] [--verbose]
 
 Each csrc/*.cu is compiled to build/<name>.o (in parallel, skipped when up to date) and the
 objects are linked into kernelforge/libkfb200.so.  ptxas resource usage (registers, spills,
-shared memory) of every kernel is kept in build/<name>.ptxas.txt.  No torch headers are used.
+shared memory) of every kernel is kept in build/<name>.ptxas.txt.  The library uses no torch headers;
+csrc/host.cpp does and becomes the CPython extension kernelforge/_host.so next to it.
 """
 
 from __future__ import annotations
@@ -21,6 +22,7 @@ PKG_ROOT = Path(__file__).resolve().parent
 CSRC = PKG_ROOT / "csrc"
 BUILD = PKG_ROOT / "build"
 LIB = PKG_ROOT / "kernelforge" / "libkfb200.so"
+HOST = PKG_ROOT / "kernelforge" / "_host.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
@@ -58,6 +60,28 @@ def _compile(src: Path, force: bool, verbose: bool) -> Path:
     return obj
 
 
+def _build_host(force: bool) -> Path:
+    """csrc/host.cpp -> kernelforge/_host.so, linked to libkfb200.so beside it and to the installed torch."""
+    src = CSRC / "host.cpp"
+    newest = max(src.stat().st_mtime, (PKG_ROOT.parent / "include" / "kfb200.h").stat().st_mtime, Path(__file__).stat().st_mtime)
+    if not force and HOST.exists() and HOST.stat().st_mtime >= newest:
+        return HOST
+    import sysconfig
+
+    import torch
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(_nvcc()).resolve().parent.parent
+    includes = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", cuda / "include", sysconfig.get_paths()["include"]]
+    cmd = [shutil.which("g++") or "c++", "-shared", "-fPIC", "-O2", "-std=c++17", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *(arg for i in includes for arg in ("-isystem", str(i))), str(src), "-o", str(HOST), f"-L{LIB.parent}", "-l:libkfb200.so",
+           f"-L{root / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python",
+           "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{root / 'lib'}"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed on {src.name}:\n{res.stdout}\n{res.stderr}")
+    return HOST
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
     BUILD.mkdir(exist_ok=True)
     sources = sorted(CSRC.glob("*.cu"))
@@ -69,6 +93,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         res = subprocess.run(cmd, capture_output=True, text=True)
         if res.returncode != 0:
             raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
+    _build_host(force)
     return LIB
 
 

@@ -5,8 +5,8 @@ reference's stable API (kernelforge/ops.py:171-302): `flash_attn`, `int4_linear`
 `int4_gemv`, `int4_gemm`, `GEMV_MAX_M`, and the two `torch.library` custom ops
 `kernelforge::flash_attn` / `kernelforge::int4_matmul` with their fake (meta) kernels, so the ops
 trace under torch.compile and capture in CUDA graphs.  Below the operator surface everything is
-new: tensors are handed as raw pointers to libkfb200.so (include/kfb200.h), hand-written sm_100a
-kernels.  Inference only: no backward pass is defined.  There is no CPU or PyTorch fallback.
+new: libkfb200.so (include/kfb200.h) holds hand-written sm_100a kernels, and plain calls reach it through
+native code (csrc/host.cpp) that checks and allocates; the validators here raise for the calls it declines.  Inference only: no backward pass is defined.  There is no CPU or PyTorch fallback.
 """
 
 from __future__ import annotations
@@ -311,12 +311,13 @@ SMALL_BATCH_MAX_M = 32
 # bench/sweep_int4_dispatch.py:47-57).  On B200 (CUDA graph, L2-cold weights, us, GEMV / GEMM):
 #   5632x2048  M=4 6.3/11.8  M=8 7.7/12.1    2048x2048  3.8/8.1  4.4/8.2    8960x1536  6.0/12.2  7.0/12.6
 #   1536x8960  8.6/12.1  11.8/12.2           11264x2048  10.5/18.0  12.3/17.9   32000x2048  15.2/24.3  18.3/24.3
-# so the GEMV keeps all of its range.
+# so the GEMV keeps all of its range (int4_matmul itself takes the small-batch kernel from M = 2 on).
 GEMV_MAX_M = 8
 
 
 def _small_batch_wins(m: int, n: int, k: int) -> bool:
-    """Where int4_small_batch measured faster than the tcgen05 GEMM for 8 < M <= 16 (same method as above, us):
+    """For callers that choose between the entry points int4_small_batch and int4_gemm themselves (int4_matmul has a
+    kernel of its own there): where int4_small_batch measured faster for 8 < M <= 16 (same method as above, us):
     M = 12: 5632x2048 10.1/12.3, 2048x2048 5.9/8.3, 8960x1536 9.1/13.1, 11264x2048 16.6/18.0, 128256x4096 128/153, but
     1536x8960 16.1/12.3, 2048x5632 12.1/11.4 and 32000x2048 26.8/24.4;  M = 16: 5632x2048 11.3/12.6, 2048x2048 6.5/8.3,
     8960x1536 9.6/13.3, 11264x2048 18.3/18.0, 128256x4096 133/153.  From M = 24 on the GEMM wins everywhere."""
@@ -343,29 +344,39 @@ def int4_gemm_ragged(x: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor
 
 
 def int4_matmul(x: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, group_size: int = 128) -> torch.Tensor:
-    """y = x @ W_hat^T for INT4 weights from kernelforge.quantize, choosing the kernel by M.
+    """y = x @ W_hat^T for INT4 weights from kernelforge.quantize, choosing the kernel by M (kfb_int4_linear).
 
-    M <= GEMV_MAX_M: the bandwidth-bound GEMV (FP32 accumulation); a little above it, where measured faster, the same
-    kernel with more batch columns (int4_small_batch).  Larger M: the tcgen05 GEMM.  bf16 activations (not in the
-    reference, README.md:103) take the GEMM at every M.
+    M = 1: the CUDA-core GEMV; M <= 32: the small-batch kernel (FP32 accumulation in both).  Larger M: the tcgen05 GEMM.
+    bf16 activations (not in the reference, README.md:103) take the same route.  A weight with a private prepacked copy
+    (prepack_weight_) runs batches of up to PREPACKED_GEMV_MAX_M rows on it.
     """
-    if x.dtype == torch.bfloat16:
-        _check_int4(x, packed, scales, group_size, allow_bf16=True)
-        _check_int4_storage(x, packed, scales, group_size)
-        return _gemm_launch(x, packed, scales, int(group_size))
-    if x.shape[0] <= PREPACKED_GEMV_MAX_M and x.dtype == torch.float16:
-        private = _prepacked_for(packed)          # set by prepack_weight_(packed)
-        if private is not None and _prepacked_wins(x.shape[0], packed.shape[0], x.shape[1]):
-            _check_int4(x, packed, scales, group_size)
-            _check_int4_storage(x, packed, scales, group_size)
-            return int4_gemv_prepacked(x, private, scales, group_size)
-    if x.shape[0] <= GEMV_MAX_M:
-        return int4_gemv(x, packed, scales, group_size)
-    if x.shape[0] <= 16 and _small_batch_wins(x.shape[0], packed.shape[0], x.shape[1]):
-        return int4_small_batch(x, packed, scales, group_size)
-    # the GEMM kernel takes any N; only the public int4_gemm wrapper keeps the reference's N % 64 rule,
-    # so an nn.Linear with an odd N that worked below the reference's crossover (M <= 7) keeps working
-    return int4_gemm_ragged(x, packed, scales, group_size)
+    y = _linear_launch(x, packed, scales, group_size, None) if isinstance(x, torch.Tensor) and x.dim() == 2 else None
+    if y is not None:
+        return y
+    _check_int4(x, packed, scales, group_size, allow_bf16=isinstance(x, torch.Tensor) and x.dtype == torch.bfloat16)
+    _check_int4_storage(x, packed, scales, group_size)
+    if x.shape[0] == 0 and x.dtype == torch.float16:
+        raise ValueError("int4_gemv handles M in [1, 8], got M=0")
+    if x.shape[0] == 0 or packed.shape[0] == 0:
+        return torch.empty(x.shape[0], packed.shape[0], dtype=x.dtype, device=x.device)
+    # tensor subclasses and the like: plain views of the same memory
+    return _linear_launch(x.as_subclass(torch.Tensor), packed.as_subclass(torch.Tensor), scales.as_subclass(torch.Tensor), group_size, None)
+
+
+def _linear_launch(x, packed, scales, group_size, bias):
+    """The native dispatcher, or the private prepacked copy of the weight where there is one; None for a call that is not
+    a plain one (the caller validates then)."""
+    if _PREPACKED and isinstance(x, torch.Tensor) and x.dtype == torch.float16 and x.is_contiguous() and x.dim() >= 1 and x.shape[-1] and (
+            bias is None or (bias.dtype == torch.float16 and bias.is_contiguous() and bias.shape == packed.shape[:1])):
+        m = x.numel() // x.shape[-1]
+        if 1 <= m <= PREPACKED_GEMV_MAX_M:
+            private = _prepacked_for(packed)          # set by prepack_weight_(packed)
+            if private is not None and _prepacked_wins(m, packed.shape[0], x.shape[-1]):
+                x2 = x.reshape(-1, x.shape[-1])
+                _check_int4(x2, packed, scales, group_size)
+                _check_int4_storage(x2, packed, scales, group_size)
+                return int4_gemv_prepacked(x2, private, scales, group_size, bias).reshape(*x.shape[:-1], packed.shape[0])
+    return _capi.host().int4_linear(x, packed, scales, group_size, bias)
 
 
 # ---------------------------------------------------------------------------
@@ -397,26 +408,18 @@ def _check_attn(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool,
         raise ValueError(f"causal attention needs Nq <= Nk (queries are the last Nq positions), got {nq} > {nk}")
 
 
-def _attn_launch(q, k, v, causal: bool, scale: float, kv_strides=None) -> torch.Tensor:
-    b, h, nq, d = q.shape
-    hk, nk = k.shape[1], k.shape[2]
-    o = torch.empty_like(q)
-    if q.numel() == 0:
+def _attn_launch(q, k, v, causal: bool, scale: float) -> torch.Tensor:
+    """The kernels on validated tensors (the body of the custom op)."""
+    o = _capi.host().flash_attn(q, k, v, causal, scale, True)
+    if o is not None:
         return o
-    if nk == 0:
+    if q.numel() == 0:
+        return torch.empty_like(q)
+    if k.shape[2] == 0:
         raise ValueError("attention needs at least one key (Nk >= 1)")
-    lib = _capi.lib()
-    ws_bytes = lib.kfb_flash_attn_ws_bytes(b, h, hk, nq, nk, d)
-    ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device) if ws_bytes else None
-    strides = None
-    if kv_strides is not None:
-        strides = (ctypes.c_int64 * 3)(*kv_strides)
-    with _capi.on_device(q.device):
-        _capi.check(lib.kfb_flash_attn_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(),
-                                           _capi.dtype_code(q.dtype), b, h, hk, nq, nk, d, int(causal), scale, strides,
-                                           ws.data_ptr() if ws is not None else None, ws_bytes,
-                                           _capi.stream_ptr(q.device)))
-    return o
+    # tensor subclasses, or K / V views that cannot be read in place
+    plain = lambda t: t.contiguous().as_subclass(torch.Tensor)
+    return _capi.host().flash_attn(plain(q), plain(k), plain(v), causal, scale, False)
 
 
 @torch.library.custom_op("kernelforge::flash_attn", mutates_args=())
@@ -439,16 +442,19 @@ def flash_attn(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool =
     treated as position Nk - Nq + i and sees keys 0 .. Nk - Nq + i.
     Returns [B, H, Nq, D] in the input dtype. Inference only (no backward).
     """
+    # Plain eager calls (CUDA-graph capture included) go straight to native code; the torch.library op, which costs
+    # ~15 us of dispatcher time, is for calls that are being traced and for tensor subclasses.
+    if not torch.compiler.is_compiling():
+        o = _capi.host().flash_attn(q, k, v, causal, scale, False)
+        if o is not None:
+            return o
     _check_attn(q, k, v, causal)
-    if _plain_eager(q):
-        return _attn_launch(q, k, v, bool(causal), _resolve_scale(scale, q.shape[-1]))
-    return _flash_attn_op(q, k, v, bool(causal), _resolve_scale(scale, q.shape[-1]))
+    scale = _resolve_scale(scale, q.shape[-1])
+    return _attn_launch(q, k, v, bool(causal), scale) if _plain_eager(q) else _flash_attn_op(q, k, v, bool(causal), scale)
 
 
 def _plain_eager(t: torch.Tensor) -> bool:
-    """True for an ordinary tensor outside torch.compile / export tracing.  The torch.library op costs ~15 us of
-    dispatcher time per call, which is as long as a small kernel; it is only needed when the call is being
-    traced (fake tensors, dynamo), so plain eager calls -- CUDA-graph capture included -- go straight to the library."""
+    """True for an ordinary tensor outside torch.compile / export tracing."""
     return type(t) is torch.Tensor and not torch.compiler.is_compiling()
 
 
@@ -458,14 +464,12 @@ def flash_attn_kv_view(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal
     [B, Hk, Lmax, D] buffer: the kernel reads the view in place (the reference copies it with
     .contiguous(), kernelforge/modules.py:95).  Views whose D axis is not dense, whose strides
     differ between k and v, or are not multiples of 8 elements, are copied first."""
+    if not torch.compiler.is_compiling():
+        o = _capi.host().flash_attn(q, k, v, causal, scale, True)
+        if o is not None:
+            return o
     _check_attn(q, k, v, causal, strided_kv=True)
-    if k.is_contiguous() and v.is_contiguous():
-        if _plain_eager(q):
-            return _attn_launch(q, k, v, bool(causal), _resolve_scale(scale, q.shape[-1]))
-        return _flash_attn_op(q, k, v, bool(causal), _resolve_scale(scale, q.shape[-1]))
-    if k.stride() != v.stride() or k.stride(3) != 1 or any(s % 8 for s in k.stride()[:3]):
-        return _flash_attn_op(q, k.contiguous(), v.contiguous(), bool(causal), _resolve_scale(scale, q.shape[-1]))
-    return _attn_launch(q, k, v, bool(causal), _resolve_scale(scale, q.shape[-1]), kv_strides=k.stride()[:3])
+    return _flash_attn_op(q, k.contiguous(), v.contiguous(), bool(causal), _resolve_scale(scale, q.shape[-1]))
 
 
 def flash_attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, kv_len: torch.Tensor,
@@ -477,6 +481,9 @@ def flash_attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
     written).  The length is read on the device, so the call can be captured once in a CUDA graph and
     replayed while the cache fills (the reference's graph-mode decode has to use SDPA instead,
     bench/e2e_model.py:91-92).  Returns [B, H, 1, D]."""
+    o = _capi.host().flash_attn_decode(q, k_cache, v_cache, kv_len, scale)
+    if o is not None:
+        return o
     _check_attn(q, k_cache, v_cache, False, strided_kv=True)
     if q.shape[2] != 1:
         raise ValueError(f"flash_attn_decode takes one query position per sequence, got Nq={q.shape[2]}")
@@ -484,18 +491,13 @@ def flash_attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
         raise TypeError("kv_len must be an int32 CUDA tensor with one entry per batch item")
     if k_cache.stride() != v_cache.stride() or k_cache.stride(3) != 1 or any(s % 8 for s in k_cache.stride()[:3]):
         raise ValueError("k_cache and v_cache must share strides, with a dense D axis and strides that are multiples of 8")
-    b, h, _, d = q.shape
-    hk, nk = k_cache.shape[1], k_cache.shape[2]
-    o = torch.empty_like(q)
-    lib = _capi.lib()
-    ws_bytes = lib.kfb_flash_attn_ws_bytes(b, h, hk, 1, nk, d)
-    ws = torch.empty(max(ws_bytes, 16), dtype=torch.uint8, device=q.device)
-    strides = (ctypes.c_int64 * 3)(*k_cache.stride()[:3])
-    with _capi.on_device(q.device):
-        _capi.check(lib.kfb_flash_attn_decode_kvlen(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), o.data_ptr(),
-                                                    _capi.dtype_code(q.dtype), b, h, hk, nk, d,
-                                                    _resolve_scale(scale, d), strides, kv_len.data_ptr(),
-                                                    ws.data_ptr(), ws_bytes, _capi.stream_ptr(q.device)))
+    scale = _resolve_scale(scale, q.shape[-1])
+    if q.numel() == 0:
+        return torch.empty_like(q)
+    plain = lambda t: t.as_subclass(torch.Tensor)
+    o = _capi.host().flash_attn_decode(plain(q), plain(k_cache), plain(v_cache), plain(kv_len), scale)
+    if o is None:
+        raise ValueError("q, k_cache, v_cache and kv_len must be non-empty and on one CUDA device")
     return o
 
 
@@ -554,19 +556,16 @@ def int4_linear(x: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, gro
     Leading dimensions are flattened into M, so [B, T, K] works like nn.Linear. The kernel is
     chosen by M (int4_matmul). Inference only (no backward).
     """
+    if not torch.compiler.is_compiling():
+        y = _linear_launch(x, packed, scales, group_size, bias)
+        if y is not None:
+            return y
     lead = x.shape[:-1]
     x2 = x.reshape(-1, x.shape[-1])
     if not x2.is_contiguous():
         x2 = x2.contiguous()
     _check_int4(x2, packed, scales, group_size, allow_bf16=True)
-    if _plain_eager(x2):
-        if bias is not None and x2.shape[0] <= FUSED_GEMV_MAX_M and bias.dtype == torch.float16 and bias.is_contiguous():
-            # decode-sized call: the bias goes into the GEMV epilogue (same two roundings as `y + bias`)
-            _check_int4_storage(x2, packed, scales, group_size)
-            return int4_gemv_fused(x2, packed, scales, int(group_size), bias=bias).reshape(*lead, packed.shape[0])
-        y = int4_matmul(x2, packed, scales, int(group_size))
-    else:
-        y = _int4_matmul_op(x2, packed, scales, int(group_size))
+    y = int4_matmul(x2, packed, scales, int(group_size)) if _plain_eager(x2) else _int4_matmul_op(x2, packed, scales, int(group_size))
     if bias is not None:
         y = y + bias
     return y.reshape(*lead, packed.shape[0])

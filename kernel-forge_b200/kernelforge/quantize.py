@@ -121,6 +121,9 @@ def unpack_int4(packed: torch.Tensor) -> torch.Tensor:
 
 def quantize_weight(weight: torch.Tensor, group_size: int = DEFAULT_GROUP_SIZE) -> QuantizedWeight:
     """Quantize and pack an nn.Linear weight [N, K] for the INT4 kernels."""
+    made = _capi.host().quantize_pack(weight, group_size) if isinstance(weight, torch.Tensor) and weight.is_cuda else None
+    if made is not None:
+        return QuantizedWeight(packed=made[0], scales=made[1], group_size=group_size, shape=tuple(weight.shape))
     n, k = _check_shape(weight, group_size)
     if weight.is_cuda:
         packed, scales = _cuda_quantize_pack(weight, group_size)
