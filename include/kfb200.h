@@ -348,6 +348,16 @@ int kfb_rope_kv_write(const void* qkv, const void* cos_table, const void* sin_ta
                       void* q_out, void* k_cache, void* v_cache, int B, int H, int Hk, int D, int Lmax,
                       void* stream);
 
+/* Rotary embedding + KV-cache write of a whole prompt: positions 0 .. T - 1 of B sequences.  qkv: [B, T, (H + 2 Hk) D];
+ * pairs != 0: rows of the q and k heads in the order of kfb_int4_gemv_rope_kv, 0: natural order.  q_out: [B, T, H, D]; rows
+ * 0 .. T - 1 of k_cache, v_cache [B, Hk, Lmax, D] are written.  The reference leaves this to Hugging Face (a dozen torch
+ * kernels and two copies per layer). */
+int kfb_rope_tokens(const void* qkv, const void* cos_table, const void* sin_table, void* q_out, void* k_cache,
+                    void* v_cache, int B, int T, int H, int Hk, int D, int Lmax, int pairs, void* stream);
+
+/* kfb_silu_mul for gate_up: [rows, 2 * inter] with gate and up of a feature side by side. */
+int kfb_silu_mul_pairs(const void* gate_up, void* out, int rows, int inter, void* stream);
+
 /* out[r, c] = fp16(fp16(silu(gate_up[r, c])) * gate_up[r, inter + c]); gate_up: [rows, 2 * inter]. */
 int kfb_silu_mul(const void* gate_up, void* out, int rows, int inter, void* stream);
 
@@ -366,6 +376,12 @@ int kfb_decode_finalize(void* best, void* tok, void* pos, void* kv_len, int M, v
  * weight with the rounding of kfb_add_rmsnorm.  embed: fp16 [vocab, hidden]. */
 int kfb_embed_rmsnorm(const void* tok, const void* embed, const void* weight, void* y, void* x_out, int rows,
                       int hidden, int vocab, float eps, void* stream);
+
+/* kfb_flash_attn_fwd for token-major q and o, [B, Nq, H, D]: what a projection writes and the next one reads, without
+ * the two transposes.  K, V, strides and workspace as there. */
+int kfb_flash_attn_fwd_tokens(const void* q, const void* k, const void* v, void* o, int dtype, int B, int H, int Hk,
+                              int Nq, int Nk, int D, int causal, float scale, const int64_t* kv_strides,
+                              void* ws, size_t ws_bytes, void* stream);
 
 /* Decode attention (Nq == 1, one query per head at the last cache position) for callers that
  * cannot allocate device memory: a server whose memory pool already owns the whole GPU, code

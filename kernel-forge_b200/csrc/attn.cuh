@@ -16,6 +16,9 @@ struct Problem {
   int causal;
   float scale;
   long long kv_stride_b, kv_stride_h, kv_stride_n;  // elements
+  // prefill only: strides of q and o in elements (D axis dense); n = 0 means dense [B, H, Nq, D]
+  long long q_stride_b = 0, q_stride_h = 0, q_stride_n = 0;
+  long long o_stride_b = 0, o_stride_h = 0, o_stride_n = 0;
   // decode only: device array of B valid lengths (<= Nk, the capacity of the cache); nullptr = all Nk keys
   const int* kv_len_dev = nullptr;
 };

@@ -93,6 +93,9 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 struct TileOrder {
   int q_index, bh;
 };
+struct Strides {   // of the output, in elements; the D axis is dense
+  long long b, h, n;
+};
 __device__ __forceinline__ TileOrder decode_tile_order(unsigned int block, int n_q, int bh_total, int heads_per_group) {
   const unsigned int per_group = (unsigned int)n_q * (unsigned int)heads_per_group;
   const int group = (int)(block / per_group);
@@ -184,7 +187,7 @@ __device__ __forceinline__ float exp_and_store(uint32_t s_tmem, uint32_t p_tmem,
 template <int D, bool kBf16>
 __global__ void __launch_bounds__(kThreads, 2)
 attn_prefill_serial_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                    const __grid_constant__ CUtensorMap tm_v, void* __restrict__ o_ptr, int H, int Hk, int Nq, int Nk,
+                    const __grid_constant__ CUtensorMap tm_v, void* __restrict__ o_ptr, const Strides o_st, int H, int Hk, int Nq, int Nk,
                     int causal, float scale_log2, int B, int n_q_tiles, int heads_per_group, unsigned int* status) {
   using L = Layout<D>;
   constexpr int S = L::kStages;
@@ -373,7 +376,7 @@ attn_prefill_serial_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
       tc_fence_after_sync();
       const float inv_l = 1.0f / l_run;
       const bool store = q0 + row < Nq;
-      uint8_t* dst = static_cast<uint8_t*>(o_ptr) + ((((size_t)b * H + h) * Nq + (size_t)(q0 + row)) * D) * 2;
+      uint8_t* dst = static_cast<uint8_t*>(o_ptr) + (b * o_st.b + h * o_st.h + (long long)(q0 + row) * o_st.n) * 2;
 #pragma unroll
       for (int c = 0; c < D / 32; ++c) {
         uint32_t o[32];
@@ -532,7 +535,7 @@ __device__ __forceinline__ float exp128(const uint32_t (&v)[4][32], uint32_t (&p
 template <int D, bool kBf16>
 __global__ void __launch_bounds__(kPairThreads, 1)
 attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                         const __grid_constant__ CUtensorMap tm_v, void* __restrict__ o_ptr, int B, int H, int Hk, int Nq,
+                         const __grid_constant__ CUtensorMap tm_v, void* __restrict__ o_ptr, const Strides o_st, int B, int H, int Hk, int Nq,
                          int Nk, int causal, float scale_log2, int n_pairs, int heads_per_group, unsigned int* status) {
   using L = PairLayout<D>;
   constexpr int S = L::kStages;
@@ -857,7 +860,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       tc_fence_after_sync();
       const float inv_l = 1.0f / l_run;
       const bool store = q0x + row < Nq;
-      uint8_t* dst = static_cast<uint8_t*>(o_ptr) + ((((size_t)b * H + h) * Nq + (size_t)(q0x + row)) * D) * 2;
+      uint8_t* dst = static_cast<uint8_t*>(o_ptr) + (b * o_st.b + h * o_st.h + (long long)(q0x + row) * o_st.n) * 2;
 #pragma unroll
       for (int c = 0; c < D / 32; ++c) {
         uint32_t o[32];
@@ -922,6 +925,7 @@ int launch(const Problem& p, const CUtensorMap& tq, const CUtensorMap& tk, const
     configured[dev] = true;
   }
   const float scale_log2 = p.scale * 1.4426950408889634f;
+  const Strides o_st{p.o_stride_b, p.o_stride_h, p.o_stride_n};
   const int q_tiles = ceil_div(p.Nq, kBlockM);
   const long long bh = (long long)p.B * p.H;
   // heads whose K and V (one KV head each at worst) fit in ~48 MB of L2 together
@@ -931,26 +935,29 @@ int launch(const Problem& p, const CUtensorMap& tq, const CUtensorMap& tk, const
     const int n_pairs = ceil_div(q_tiles, 2);
     if (bh * n_pairs > 0x7fffffffLL) return fail(KFB_ERR_INVALID, "too many query tiles for one launch");
     pair::attn_prefill_pair_kernel<D, kBf16><<<(unsigned)(bh * n_pairs), pair::kPairThreads, PL::kAlloc, stream>>>(
-        tq, tk, tv, p.o, p.B, p.H, p.Hk, p.Nq, p.Nk, p.causal, scale_log2, n_pairs, heads_per_group, status);
+        tq, tk, tv, p.o, o_st, p.B, p.H, p.Hk, p.Nq, p.Nk, p.causal, scale_log2, n_pairs, heads_per_group, status);
     KFB_LAUNCH_CHECK("attn_prefill_pair_kernel");
     return KFB_OK;
   }
   if (bh * q_tiles > 0x7fffffffLL) return fail(KFB_ERR_INVALID, "too many query tiles for one launch");
   serial::attn_prefill_serial_kernel<D, kBf16><<<(unsigned)(bh * q_tiles), kThreads, L::kAlloc, stream>>>(
-      tq, tk, tv, p.o, p.H, p.Hk, p.Nq, p.Nk, p.causal, scale_log2, p.B, q_tiles, heads_per_group, status);
+      tq, tk, tv, p.o, o_st, p.H, p.Hk, p.Nq, p.Nk, p.causal, scale_log2, p.B, q_tiles, heads_per_group, status);
   KFB_LAUNCH_CHECK("attn_prefill_serial_kernel");
   return KFB_OK;
 }
 
 }  // namespace
 
-int launch_prefill(const Problem& p, cudaStream_t stream) {
+int launch_prefill(const Problem& given, cudaStream_t stream) {
+  Problem p = given;
+  if (p.q_stride_n == 0) { p.q_stride_n = p.D; p.q_stride_h = (long long)p.Nq * p.D; p.q_stride_b = (long long)p.H * p.Nq * p.D; }
+  if (p.o_stride_n == 0) { p.o_stride_n = p.D; p.o_stride_h = (long long)p.Nq * p.D; p.o_stride_b = (long long)p.H * p.Nq * p.D; }
   unsigned int* status = device_status_word();
   if (!status) return fail(KFB_ERR_CUDA, "cannot resolve the device status word");
   CUtensorMap tq, tk, tv;
   const uint64_t D = p.D;
   const uint64_t qd[4] = {D, (uint64_t)p.Nq, (uint64_t)p.H, (uint64_t)p.B};
-  const uint64_t qs[3] = {D * 2, (uint64_t)p.Nq * D * 2, (uint64_t)p.H * p.Nq * D * 2};
+  const uint64_t qs[3] = {(uint64_t)p.q_stride_n * 2, (uint64_t)p.q_stride_h * 2, (uint64_t)p.q_stride_b * 2};
   const uint64_t kd[4] = {D, (uint64_t)p.Nk, (uint64_t)p.Hk, (uint64_t)p.B};
   const uint64_t ks[3] = {(uint64_t)p.kv_stride_n * 2, (uint64_t)p.kv_stride_h * 2, (uint64_t)p.kv_stride_b * 2};
   const uint32_t box[4] = {64, 128, 1, 1};

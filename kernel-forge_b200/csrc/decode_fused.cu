@@ -24,8 +24,10 @@ __device__ __forceinline__ float warp_sum(float v) {
 
 // One CTA (256 threads) per row.  hidden % 8 == 0, hidden <= 256 * 8 * kMaxVec.
 constexpr int kRmsThreads = 256;
-constexpr int kMaxVec = 4;  // 16-byte vectors per thread => hidden <= 8192
+constexpr int kRmsMaxVec = 16;  // most 16-byte vectors per thread => hidden <= 32768
 
+// kMaxVec: 16-byte vectors of the row a thread holds (1 for hidden <= 2048: no predicated copies of the loop body).
+template <int kMaxVec>
 __global__ void __launch_bounds__(kRmsThreads)
 add_rmsnorm_kernel(const __half* __restrict__ x, const __half* __restrict__ res, const __half* __restrict__ w,
                    __half* __restrict__ y, __half* __restrict__ sum_out, int hidden, float eps) {
@@ -143,6 +145,81 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const __half* __restrict_
   }
 }
 
+__device__ __forceinline__ __half silu_times(__half2 gate_up) {
+  const float g = __low2float(gate_up);
+  return __hmul(__float2half_rn(g / (1.0f + __expf(-g))), __high2half(gate_up));
+}
+
+// gu: gate and up of a feature side by side (the row order of int4_gemv_silu_pair), `total` features in all
+__global__ void __launch_bounds__(256) silu_mul_pairs_kernel(const __half2* __restrict__ gu, __half* __restrict__ out, long long total) {
+  const long long step = (long long)gridDim.x * blockDim.x, first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  for (long long i = first; i < total / 4; i += step) {
+    const uint4 v = reinterpret_cast<const uint4*>(gu)[i];
+    const __half2* h = reinterpret_cast<const __half2*>(&v);
+    __half o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[j] = silu_times(h[j]);
+    reinterpret_cast<uint2*>(out)[i] = *reinterpret_cast<const uint2*>(o);
+  }
+  if (first < total % 4) out[total / 4 * 4 + first] = silu_times(gu[total / 4 * 4 + first]);
+}
+
+// Rotary embedding and KV-cache write of T consecutive positions 0 .. T - 1 of B sequences.  A thread takes four rotation
+// pairs (16 bytes of qkv) or eight features of v.  kPairs: the q and k heads hold features (j, j + D / 2) side by side
+// (the row order of int4_gemv_rope_kv); otherwise the natural order.
+template <bool kPairs>
+__global__ void __launch_bounds__(256)
+rope_tokens_kernel(const __half* __restrict__ qkv, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+                   __half* __restrict__ q_out, __half* __restrict__ k_cache, __half* __restrict__ v_cache, int T, int H, int Hk,
+                   int D, int Lmax, long long items) {
+  const int per_head = D / 8, heads = H + 2 * Hk, per_token = heads * per_head, half = D / 2;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < items; i += (long long)gridDim.x * blockDim.x) {
+    const long long token = i / per_token;
+    const int r = (int)(i - token * per_token), head = r / per_head, c = r % per_head;
+    const int b = (int)(token / T), t = (int)(token - (long long)b * T);
+    const __half* src = qkv + (token * heads + head) * D;
+    if (head >= H + Hk) {
+      reinterpret_cast<uint4*>(v_cache + (((long long)b * Hk + (head - H - Hk)) * Lmax + t) * D)[c] = reinterpret_cast<const uint4*>(src)[c];
+      continue;
+    }
+    const int j = 4 * c;
+    float lo[4], hi[4];
+    if constexpr (kPairs) {
+      const uint4 v = reinterpret_cast<const uint4*>(src)[c];
+      const __half2* h = reinterpret_cast<const __half2*>(&v);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) { lo[e] = __low2float(h[e]); hi[e] = __high2float(h[e]); }
+    } else {
+      const uint2 a = reinterpret_cast<const uint2*>(src)[c], d = reinterpret_cast<const uint2*>(src + half)[c];
+      const __half2 *ah = reinterpret_cast<const __half2*>(&a), *dh = reinterpret_cast<const __half2*>(&d);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        lo[e] = e & 1 ? __high2float(ah[e >> 1]) : __low2float(ah[e >> 1]);
+        hi[e] = e & 1 ? __high2float(dh[e >> 1]) : __low2float(dh[e >> 1]);
+      }
+    }
+    const float* ct = cos_t + (long long)t * D + j;
+    const float* st = sin_t + (long long)t * D + j;
+    const float4 c0 = *reinterpret_cast<const float4*>(ct), c1 = *reinterpret_cast<const float4*>(ct + half);
+    const float4 s0 = *reinterpret_cast<const float4*>(st), s1 = *reinterpret_cast<const float4*>(st + half);
+    const float *c0p = &c0.x, *c1p = &c1.x, *s0p = &s0.x, *s1p = &s1.x;
+    __half rl[4], rh[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {   // both products and the sum rounded on their own, like the other RoPE kernels
+      rl[e] = __float2half_rn(__fsub_rn(__fmul_rn(lo[e], c0p[e]), __fmul_rn(hi[e], s0p[e])));
+      rh[e] = __float2half_rn(__fadd_rn(__fmul_rn(hi[e], c1p[e]), __fmul_rn(lo[e], s1p[e])));
+    }
+    __half* dst = head < H ? q_out + (token * H + head) * D : k_cache + (((long long)b * Hk + (head - H)) * Lmax + t) * D;
+    *reinterpret_cast<uint2*>(dst + j) = *reinterpret_cast<const uint2*>(rl);
+    *reinterpret_cast<uint2*>(dst + half + j) = *reinterpret_cast<const uint2*>(rh);
+  }
+}
+
+int blocks_for(long long items) {
+  const long long want = (items + 255) / 256, cap = (long long)sm_count() * 8;
+  return (int)(want < cap ? want : cap);
+}
+
 }  // namespace
 }  // namespace fused
 }  // namespace kfb
@@ -152,13 +229,16 @@ using namespace kfb;
 extern "C" int kfb_add_rmsnorm(const void* x, const void* residual, const void* weight, void* y, void* sum_out, int rows,
                                int hidden, float eps, void* stream) {
   if (int rc = require_sm100()) return rc;
-  if (rows < 1 || hidden < 8 || hidden % 8 || hidden > fused::kRmsThreads * 8 * fused::kMaxVec)
-    return fail(KFB_ERR_INVALID, "add_rmsnorm needs rows >= 1 and hidden a multiple of 8 up to %d, got %d x %d",
-                fused::kRmsThreads * 8 * fused::kMaxVec, rows, hidden);
+  constexpr int kWidest = fused::kRmsThreads * 8 * fused::kRmsMaxVec;
+  if (rows < 1 || hidden < 8 || hidden % 8 || hidden > kWidest)
+    return fail(KFB_ERR_INVALID, "add_rmsnorm needs rows >= 1 and hidden a multiple of 8 up to %d, got %d x %d", kWidest, rows, hidden);
   if (!x || !weight || !y) return fail(KFB_ERR_INVALID, "null pointer");
   if (!aligned16(x) || !aligned16(weight) || !aligned16(y) || (residual && !aligned16(residual)) || (sum_out && !aligned16(sum_out)))
     return fail(KFB_ERR_ALIGNMENT, "pointers must be 16-byte aligned");
-  return launch_kernel("add_rmsnorm_kernel", fused::add_rmsnorm_kernel, dim3(rows), dim3(fused::kRmsThreads), 0,
+  const int per_thread = ceil_div(hidden / 8, fused::kRmsThreads);
+  auto kernel = per_thread == 1 ? fused::add_rmsnorm_kernel<1> : per_thread == 2 ? fused::add_rmsnorm_kernel<2>
+                : per_thread <= 4 ? fused::add_rmsnorm_kernel<4> : fused::add_rmsnorm_kernel<fused::kRmsMaxVec>;
+  return launch_kernel("add_rmsnorm_kernel", kernel, dim3(rows), dim3(fused::kRmsThreads), 0,
                        (cudaStream_t)stream, pdl_enabled(), (const __half*)x, (const __half*)residual, (const __half*)weight,
                        (__half*)y, (__half*)sum_out, hidden, eps);
 }
@@ -189,4 +269,31 @@ extern "C" int kfb_silu_mul(const void* gate_up, void* out, int rows, int inter,
   if (blocks > cap) blocks = cap;
   return launch_kernel("silu_mul_kernel", fused::silu_mul_kernel, dim3((int)blocks), dim3(256), 0, (cudaStream_t)stream,
                        pdl_enabled(), (const __half*)gate_up, (__half*)out, rows, inter);
+}
+
+extern "C" int kfb_silu_mul_pairs(const void* gate_up, void* out, int rows, int inter, void* stream) {
+  if (int rc = require_sm100()) return rc;
+  if (rows < 1 || inter < 1) return fail(KFB_ERR_INVALID, "silu_mul_pairs needs rows, inter >= 1, got %d x %d", rows, inter);
+  if (!gate_up || !out) return fail(KFB_ERR_INVALID, "null pointer");
+  if (!aligned16(gate_up) || !aligned16(out)) return fail(KFB_ERR_ALIGNMENT, "pointers must be 16-byte aligned");
+  const long long total = (long long)rows * inter;
+  fused::silu_mul_pairs_kernel<<<fused::blocks_for((total + 3) / 4), 256, 0, (cudaStream_t)stream>>>((const __half2*)gate_up, (__half*)out, total);
+  KFB_LAUNCH_CHECK("silu_mul_pairs_kernel");
+  return KFB_OK;
+}
+
+extern "C" int kfb_rope_tokens(const void* qkv, const void* cos_table, const void* sin_table, void* q_out, void* k_cache,
+                               void* v_cache, int B, int T, int H, int Hk, int D, int Lmax, int pairs, void* stream) {
+  if (int rc = require_sm100()) return rc;
+  if (B < 1 || T < 1 || T > Lmax || H < 1 || Hk < 1 || (D != 64 && D != 128))
+    return fail(KFB_ERR_INVALID, "rope_tokens: bad shape B=%d T=%d H=%d Hk=%d D=%d Lmax=%d", B, T, H, Hk, D, Lmax);
+  if (!qkv || !cos_table || !sin_table || !q_out || !k_cache || !v_cache) return fail(KFB_ERR_INVALID, "null pointer");
+  if (!aligned16(qkv) || !aligned16(cos_table) || !aligned16(sin_table) || !aligned16(q_out) || !aligned16(k_cache) || !aligned16(v_cache))
+    return fail(KFB_ERR_ALIGNMENT, "pointers must be 16-byte aligned");
+  const long long items = (long long)B * T * (H + 2 * Hk) * (D / 8);
+  auto kernel = pairs ? fused::rope_tokens_kernel<true> : fused::rope_tokens_kernel<false>;
+  kernel<<<fused::blocks_for(items), 256, 0, (cudaStream_t)stream>>>((const __half*)qkv, (const float*)cos_table, (const float*)sin_table,
+                                                                     (__half*)q_out, (__half*)k_cache, (__half*)v_cache, T, H, Hk, D, Lmax, items);
+  KFB_LAUNCH_CHECK("rope_tokens_kernel");
+  return KFB_OK;
 }

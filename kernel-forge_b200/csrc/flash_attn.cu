@@ -16,6 +16,18 @@ int check_shape(int dtype, int B, int H, int Hk, int Nq, int Nk, int D, int caus
   return KFB_OK;
 }
 
+// K and V share their strides (elements); null: dense [B, Hk, Nk, D].
+int set_kv_strides(attn::Problem* p, const int64_t* st) {
+  if (!st) {
+    p->kv_stride_n = p->D; p->kv_stride_h = (long long)p->Nk * p->D; p->kv_stride_b = (long long)p->Hk * p->Nk * p->D;
+    return KFB_OK;
+  }
+  p->kv_stride_b = st[0]; p->kv_stride_h = st[1]; p->kv_stride_n = st[2];
+  if (st[2] < p->D || st[1] < 1 || st[0] < 1 || (st[0] % 8) || (st[1] % 8) || (st[2] % 8))
+    return fail(KFB_ERR_ALIGNMENT, "kv strides must be positive multiples of 8 elements with a row stride >= D");
+  return KFB_OK;
+}
+
 }  // namespace
 
 extern "C" size_t kfb_flash_attn_ws_bytes(int B, int H, int Hk, int Nq, int Nk, int D) {
@@ -37,17 +49,34 @@ extern "C" int kfb_flash_attn_fwd(const void* q, const void* k, const void* v, v
   p.dtype = dtype; p.B = B; p.H = H; p.Hk = Hk; p.Nq = Nq; p.Nk = Nk; p.D = D;
   p.causal = causal ? 1 : 0;
   p.scale = scale;
-  if (kv_strides) {
-    p.kv_stride_b = kv_strides[0]; p.kv_stride_h = kv_strides[1]; p.kv_stride_n = kv_strides[2];
-    if (p.kv_stride_n < D || p.kv_stride_h < 1 || p.kv_stride_b < 1 || (p.kv_stride_b % 8) || (p.kv_stride_h % 8) ||
-        (p.kv_stride_n % 8))
-      return fail(KFB_ERR_ALIGNMENT, "kv strides must be positive multiples of 8 elements with a row stride >= D");
-  } else {
-    p.kv_stride_n = D; p.kv_stride_h = (long long)Nk * D; p.kv_stride_b = (long long)Hk * Nk * D;
-  }
+  if (int rc = set_kv_strides(&p, kv_strides)) return rc;
   cudaStream_t s = (cudaStream_t)stream;
   if (Nq == 1) return attn::launch_decode(p, ws, ws_bytes, s);
   return attn::launch_prefill(p, s);
+}
+
+// The same for tensors in token-major layout (what a projection writes and the next one reads): q and o [B, Nq, H, D].
+extern "C" int kfb_flash_attn_fwd_tokens(const void* q, const void* k, const void* v, void* o, int dtype, int B, int H, int Hk,
+                                         int Nq, int Nk, int D, int causal, float scale, const int64_t* kv_strides, void* ws,
+                                         size_t ws_bytes, void* stream) {
+  if (Nq == 1)   // [B, 1, H, D] and [B, H, 1, D] are the same memory
+    return kfb_flash_attn_fwd(q, k, v, o, dtype, B, H, Hk, Nq, Nk, D, causal, scale, kv_strides, ws, ws_bytes, stream);
+  if (int rc = require_sm100()) return rc;
+  if (int rc = check_shape(dtype, B, H, Hk, Nq, Nk, D, causal)) return rc;
+  if (!(scale > 0.0f)) return fail(KFB_ERR_INVALID, "scale must be positive, got %g", (double)scale);
+  if (!q || !k || !v || !o) return fail(KFB_ERR_INVALID, "null pointer");
+  if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o))
+    return fail(KFB_ERR_ALIGNMENT, "q, k, v, o must be 16-byte aligned");
+  attn::Problem p;
+  p.q = q; p.k = k; p.v = v; p.o = o;
+  p.dtype = dtype; p.B = B; p.H = H; p.Hk = Hk; p.Nq = Nq; p.Nk = Nk; p.D = D;
+  p.causal = causal ? 1 : 0;
+  p.scale = scale;
+  if (int rc = set_kv_strides(&p, kv_strides)) return rc;
+  p.q_stride_h = p.o_stride_h = D;
+  p.q_stride_n = p.o_stride_n = (long long)H * D;
+  p.q_stride_b = p.o_stride_b = (long long)Nq * H * D;
+  return attn::launch_prefill(p, (cudaStream_t)stream);
 }
 
 // Decode attention against a static KV cache whose valid length lives on the device.
@@ -66,14 +95,7 @@ extern "C" int kfb_flash_attn_decode_kvlen(const void* q, const void* k, const v
   p.causal = 0;
   p.scale = scale;
   p.kv_len_dev = kv_len_dev;
-  if (kv_strides) {
-    p.kv_stride_b = kv_strides[0]; p.kv_stride_h = kv_strides[1]; p.kv_stride_n = kv_strides[2];
-    if (p.kv_stride_n < D || p.kv_stride_h < 1 || p.kv_stride_b < 1 || (p.kv_stride_b % 8) || (p.kv_stride_h % 8) ||
-        (p.kv_stride_n % 8))
-      return fail(KFB_ERR_ALIGNMENT, "kv strides must be positive multiples of 8 elements with a row stride >= D");
-  } else {
-    p.kv_stride_n = D; p.kv_stride_h = (long long)Nk * D; p.kv_stride_b = (long long)Hk * Nk * D;
-  }
+  if (int rc = set_kv_strides(&p, kv_strides)) return rc;
   return attn::launch_decode(p, ws, ws_bytes, (cudaStream_t)stream);
 }
 
@@ -102,14 +124,7 @@ extern "C" int kfb_flash_attn_decode_partial(const void* q, const void* k, const
   p.causal = 0;
   p.scale = scale;
   p.kv_len_dev = kv_len_dev;
-  if (kv_strides) {
-    p.kv_stride_b = kv_strides[0]; p.kv_stride_h = kv_strides[1]; p.kv_stride_n = kv_strides[2];
-    if (p.kv_stride_n < D || p.kv_stride_h < 1 || p.kv_stride_b < 1 || (p.kv_stride_b % 8) || (p.kv_stride_h % 8) ||
-        (p.kv_stride_n % 8))
-      return fail(KFB_ERR_ALIGNMENT, "kv strides must be positive multiples of 8 elements with a row stride >= D");
-  } else {
-    p.kv_stride_n = D; p.kv_stride_h = (long long)Nk * D; p.kv_stride_b = (long long)Hk * Nk * D;
-  }
+  if (int rc = set_kv_strides(&p, kv_strides)) return rc;
   return attn::launch_decode(p, partial, partial_bytes, (cudaStream_t)stream, /*partial_only=*/true);
 }
 

@@ -76,6 +76,14 @@ PyObject* guarded(F&& body) {
   }
 }
 
+PyObject* pair_of(at::Tensor first, PyObject* second /* new reference or null */) {
+  PyObject* f = second ? THPVariable_Wrap(std::move(first)) : nullptr;
+  PyObject* both = f ? PyTuple_Pack(2, f, second) : nullptr;
+  Py_XDECREF(f);
+  Py_XDECREF(second);
+  return both;
+}
+
 #define NOT_PLAIN Py_RETURN_NONE
 #define ARGS(count)                                                                         \
   if (n != (count)) {                                                                       \
@@ -233,12 +241,115 @@ PyObject* quantize_pack(PyObject*, PyObject* const* a, Py_ssize_t n) {
     rc = kfb_quantize_pack(w->data_ptr(), dtype_code(w->scalar_type()), (int)rows, (int)k, (int)group, packed.data_ptr(), scales.data_ptr(), stream);
     Py_END_ALLOW_THREADS
     if (rc) return raise_status(rc);
-    PyObject* p = THPVariable_Wrap(std::move(packed));
-    PyObject* s = p ? THPVariable_Wrap(std::move(scales)) : nullptr;
-    PyObject* both = s ? PyTuple_Pack(2, p, s) : nullptr;
-    Py_XDECREF(p);
-    Py_XDECREF(s);
-    return both;
+    return pair_of(std::move(packed), THPVariable_Wrap(std::move(scales)));
+  });
+}
+
+// fp16, contiguous, on x's device
+inline bool half_like(const at::Tensor* t, const at::Tensor& x) {
+  return t && t->scalar_type() == at::kHalf && t->is_contiguous() && t->device() == x.device();
+}
+
+// add_rmsnorm(x, weight, eps, residual or None) -> (y, s): x [rows, hidden]
+PyObject* add_rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  ARGS(4)
+  return guarded([&]() -> PyObject* {
+    const at::Tensor *x = plain(a[0]), *w = plain(a[1]), *res = nullptr;
+    const double eps = PyFloat_AsDouble(a[2]);
+    if (PyErr_Occurred()) return nullptr;
+    if (!x || x->dim() != 2 || !half_like(x, *x) || !half_like(w, *x) || w->numel() != x->size(1)) NOT_PLAIN;
+    if (a[3] != Py_None) {
+      res = plain(a[3]);
+      if (!half_like(res, *x) || res->sizes() != x->sizes()) NOT_PLAIN;
+    }
+    OnDevice dev(*x);
+    at::Tensor y = new_tensor(x->sizes(), at::kHalf, *x), s;
+    if (res) s = new_tensor(x->sizes(), at::kHalf, *x);
+    void* stream = stream_of(*x);
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = kfb_add_rmsnorm(x->data_ptr(), res ? res->data_ptr() : nullptr, w->data_ptr(), y.data_ptr(), res ? s.data_ptr() : nullptr,
+                         (int)x->size(0), (int)x->size(1), (float)eps, stream);
+    Py_END_ALLOW_THREADS
+    if (rc) return raise_status(rc);
+    if (res) return pair_of(std::move(y), THPVariable_Wrap(std::move(s)));
+    Py_INCREF(a[0]);
+    return pair_of(std::move(y), a[0]);
+  });
+}
+
+// rope_tokens(qkv, cos, sin, k_cache, v_cache, batch, heads, pairs) -> q [B, T, H, D]: qkv [B * T, (H + 2 Hk) D]
+PyObject* rope_tokens(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  ARGS(8)
+  return guarded([&]() -> PyObject* {
+    const at::Tensor *qkv = plain(a[0]), *cos = plain(a[1]), *sin = plain(a[2]), *kc = plain(a[3]), *vc = plain(a[4]);
+    long long b, h;
+    const int pairs = PyObject_IsTrue(a[7]);
+    if (!int_arg(a[5], &b) || !int_arg(a[6], &h) || pairs < 0) NOT_PLAIN;
+    if (!qkv || !half_like(qkv, *qkv) || !half_like(kc, *qkv) || !half_like(vc, *qkv) || !cos || !sin) NOT_PLAIN;
+    if (kc->dim() != 4 || kc->sizes() != vc->sizes() || kc->size(0) != b || b < 1 || qkv->dim() != 2 || qkv->size(0) % b) NOT_PLAIN;
+    const int64_t t = qkv->size(0) / b, hk = kc->size(1), lmax = kc->size(2), d = kc->size(3);
+    for (const at::Tensor* table : {cos, sin})
+      if (table->scalar_type() != at::kFloat || !table->is_contiguous() || table->dim() != 2 || table->size(0) < t || table->size(1) != d ||
+          table->device() != qkv->device())
+        NOT_PLAIN;
+    if (qkv->size(1) != (h + 2 * hk) * d) NOT_PLAIN;
+    OnDevice dev(*qkv);
+    at::Tensor q = new_tensor({b, t, h, d}, at::kHalf, *qkv);
+    void* stream = stream_of(*qkv);
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = kfb_rope_tokens(qkv->data_ptr(), cos->data_ptr(), sin->data_ptr(), q.data_ptr(), kc->data_ptr(), vc->data_ptr(), (int)b, (int)t, (int)h,
+                         (int)hk, (int)d, (int)lmax, pairs, stream);
+    Py_END_ALLOW_THREADS
+    return rc ? raise_status(rc) : THPVariable_Wrap(std::move(q));
+  });
+}
+
+// attention_tokens(q, k_cache, v_cache, kv_rows, causal) -> o: q and o [B, T, H, D], the first kv_rows rows of the caches
+PyObject* attention_tokens(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  ARGS(5)
+  return guarded([&]() -> PyObject* {
+    const at::Tensor *q = plain(a[0]), *kc = plain(a[1]), *vc = plain(a[2]);
+    long long nk;
+    const int causal = PyObject_IsTrue(a[4]);
+    if (!int_arg(a[3], &nk) || causal < 0) NOT_PLAIN;
+    if (!q || q->dim() != 4 || !half_like(q, *q) || !half_like(kc, *q) || !half_like(vc, *q) || kc->dim() != 4 || kc->sizes() != vc->sizes()) NOT_PLAIN;
+    const int64_t b = q->size(0), t = q->size(1), h = q->size(2), d = q->size(3), hk = kc->size(1), lmax = kc->size(2);
+    if (kc->size(0) != b || kc->size(3) != d || nk < 1 || nk > lmax || t < 1) NOT_PLAIN;
+    const int64_t strides[3] = {hk * lmax * d, lmax * d, d};
+    OnDevice dev(*q);
+    at::Tensor o = new_tensor(q->sizes(), at::kHalf, *q);
+    const size_t ws_bytes = kfb_flash_attn_ws_bytes((int)b, (int)h, (int)hk, (int)t, (int)nk, (int)d);
+    at::Tensor ws;
+    if (ws_bytes) ws = new_tensor({(int64_t)ws_bytes}, at::kByte, *q);
+    void* stream = stream_of(*q);
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = kfb_flash_attn_fwd_tokens(q->data_ptr(), kc->data_ptr(), vc->data_ptr(), o.data_ptr(), KFB_F16, (int)b, (int)h, (int)hk, (int)t, (int)nk,
+                                   (int)d, causal, (float)(1.0 / std::sqrt((double)d)), strides, ws_bytes ? ws.data_ptr() : nullptr, ws_bytes, stream);
+    Py_END_ALLOW_THREADS
+    return rc ? raise_status(rc) : THPVariable_Wrap(std::move(o));
+  });
+}
+
+// silu_mul(gate_up, pairs) -> act [rows, inter]: gate_up [rows, 2 * inter], gate | up or (pairs) side by side
+PyObject* silu_mul(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  ARGS(2)
+  return guarded([&]() -> PyObject* {
+    const at::Tensor* gu = plain(a[0]);
+    const int pairs = PyObject_IsTrue(a[1]);
+    if (pairs < 0 || !gu || gu->dim() != 2 || !half_like(gu, *gu) || gu->size(1) % 2) NOT_PLAIN;
+    const int64_t rows = gu->size(0), inter = gu->size(1) / 2;
+    OnDevice dev(*gu);
+    at::Tensor act = new_tensor({rows, inter}, at::kHalf, *gu);
+    void* stream = stream_of(*gu);
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = pairs ? kfb_silu_mul_pairs(gu->data_ptr(), act.data_ptr(), (int)rows, (int)inter, stream)
+               : kfb_silu_mul(gu->data_ptr(), act.data_ptr(), (int)rows, (int)inter, stream);
+    Py_END_ALLOW_THREADS
+    return rc ? raise_status(rc) : THPVariable_Wrap(std::move(act));
   });
 }
 
@@ -248,6 +359,10 @@ PyMethodDef methods[] = {
     METHOD(flash_attn, "flash_attn(q, k, v, causal, scale, views) -> o, or None when the call is not a plain one"),
     METHOD(flash_attn_decode, "flash_attn_decode(q, k_cache, v_cache, kv_len, scale) -> o, or None when the call is not a plain one"),
     METHOD(quantize_pack, "quantize_pack(weight, group_size) -> (packed, scales), or None when the call is not a plain one"),
+    METHOD(add_rmsnorm, "add_rmsnorm(x, weight, eps, residual) -> (y, s), or None"),
+    METHOD(rope_tokens, "rope_tokens(qkv, cos, sin, k_cache, v_cache, batch, heads, pairs) -> q [B, T, H, D], or None"),
+    METHOD(attention_tokens, "attention_tokens(q, k_cache, v_cache, kv_rows, causal) -> o [B, T, H, D], or None"),
+    METHOD(silu_mul, "silu_mul(gate_up, pairs) -> act, or None"),
     {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "Checked, allocating calls of libkfb200.so on torch tensors.", -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -148,7 +148,9 @@ __global__ void decode_finalize_kernel(unsigned long long* __restrict__ best, lo
 }
 
 // One CTA (256 threads) per token: x_out[row] = embed[tok[row]], y[row] = fp16(fp16(x * rsqrt(mean(x^2) + eps)) * w).
-constexpr int kMaxVec = 4;  // hidden <= 256 * 8 * 4
+constexpr int kWidestVec = 16;  // hidden <= 256 * 8 * 16
+// kMaxVec: 16-byte vectors of the row a thread holds
+template <int kMaxVec>
 __global__ void __launch_bounds__(kThreads)
 embed_rmsnorm_kernel(const long long* __restrict__ tok, const __half* __restrict__ embed, const __half* __restrict__ w,
                      __half* __restrict__ y, __half* __restrict__ x_out, int hidden, int vocab, float eps) {
@@ -243,13 +245,16 @@ extern "C" int kfb_decode_finalize(void* best, void* tok, void* pos, void* kv_le
 extern "C" int kfb_embed_rmsnorm(const void* tok, const void* embed, const void* weight, void* y, void* x_out, int rows,
                                  int hidden, int vocab, float eps, void* stream) {
   if (int rc = require_sm100()) return rc;
-  if (rows < 1 || vocab < 1 || hidden < 8 || hidden % 8 || hidden > lmhead::kThreads * 8 * lmhead::kMaxVec)
+  if (rows < 1 || vocab < 1 || hidden < 8 || hidden % 8 || hidden > lmhead::kThreads * 8 * lmhead::kWidestVec)
     return fail(KFB_ERR_INVALID, "embed_rmsnorm needs rows, vocab >= 1 and hidden a multiple of 8 up to %d, got %d x %d",
-                lmhead::kThreads * 8 * lmhead::kMaxVec, rows, hidden);
+                lmhead::kThreads * 8 * lmhead::kWidestVec, rows, hidden);
   if (!tok || !embed || !weight || !y || !x_out) return fail(KFB_ERR_INVALID, "null pointer");
   if (!aligned16(embed) || !aligned16(weight) || !aligned16(y) || !aligned16(x_out))
     return fail(KFB_ERR_ALIGNMENT, "pointers must be 16-byte aligned");
-  return launch_kernel("embed_rmsnorm_kernel", lmhead::embed_rmsnorm_kernel, dim3(rows), dim3(lmhead::kThreads), 0,
+  const int per_thread = ceil_div(hidden / 8, lmhead::kThreads);
+  auto kernel = per_thread == 1 ? lmhead::embed_rmsnorm_kernel<1> : per_thread <= 4 ? lmhead::embed_rmsnorm_kernel<4>
+                                                                                     : lmhead::embed_rmsnorm_kernel<lmhead::kWidestVec>;
+  return launch_kernel("embed_rmsnorm_kernel", kernel, dim3(rows), dim3(lmhead::kThreads), 0,
                        (cudaStream_t)stream, pdl_enabled(), static_cast<const long long*>(tok), static_cast<const __half*>(embed),
                        static_cast<const __half*>(weight), static_cast<__half*>(y), static_cast<__half*>(x_out), hidden, vocab, eps);
 }

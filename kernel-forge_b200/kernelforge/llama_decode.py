@@ -7,8 +7,9 @@ Here the step runs `ops.flash_attn_decode`, which reads the valid cache length f
 `ops.int4_linear` for the seven decoder linears of every layer; token ids, position and KV length all live
 on the device, so a step is a pure graph replay with no host synchronisation.
 
-Prefill uses torch for everything that is not one of the two hot paths (embedding, RMSNorm, RoPE, SiLU * up,
-residual adds, lm_head), as the reference does.  The decode step is launch-bound at batch 1, so there those
+Prefill runs nine kernels per layer (ops.add_rmsnorm, rope_tokens, attention_tokens, silu_mul and the four linears);
+written with torch for everything but the two hot paths, as the reference does, it was ~45 and bound by their launches.
+Only the lm_head over all prompt positions is torch's matmul.  The decode step is launch-bound at batch 1 too, so there the
 element-wise steps run as three fused kernels (ops.add_rmsnorm, ops.rope_kv_write, ops.silu_mul) and q/k/v and
 gate/up are stored as one quantised matrix each: 11 kernels per layer instead of ~48 (2.39 -> 0.85 ms per step
 on the TinyLlama-1.1B architecture).  The embedding lookup is fused into the first norm (ops.embed_rmsnorm), the fp16
@@ -270,32 +271,6 @@ class LlamaInt4Decoder:
                    "final_norm": sd["model.norm.weight"], "layers": layers}
         return cls(shape, weights, device, batch, max_len, tp_group=tp_group)
 
-    # ------------------------------------------------------------------ building blocks (torch)
-    def _rms(self, x, w):
-        xf = x.float()
-        return (xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + self.s.rms_eps)).to(torch.float16) * w
-
-    @staticmethod
-    def _rope(t, cos, sin):  # t [B, heads, T, D]; cos/sin broadcastable [T, D]
-        tf = t.float()
-        half = tf.shape[-1] // 2
-        rot = torch.cat([-tf[..., half:], tf[..., :half]], dim=-1)
-        return (tf * cos + rot * sin).to(torch.float16)
-
-    def _mlp(self, L, x):
-        h = self._rms(x, L["post_norm"])
-        gu = L["gate_up"](h)
-        inter = self.inter_loc
-        if self.pair_rows:
-            gu = gu.view(*gu.shape[:-1], inter, 2)
-            act = torch.nn.functional.silu(gu[..., 0]) * gu[..., 1]
-        else:
-            act = torch.nn.functional.silu(gu[..., :inter]) * gu[..., inter:]
-        lead = act.shape[:-1]
-        act = self._gather(act.reshape(-1, inter), "inter_bounds").reshape(*lead, self.s.intermediate)
-        down = L["down"](act)
-        return x + self._gather(down.reshape(-1, down.shape[-1]), "hidden_bounds").reshape(*lead, self.s.hidden)
-
     # ------------------------------------------------------------------ prefill
     @torch.no_grad()
     def prefill(self, ids: torch.Tensor) -> torch.Tensor:
@@ -304,30 +279,23 @@ class LlamaInt4Decoder:
         s, (b, t) = self.s, ids.shape
         if t >= self.max_len:
             raise ValueError(f"prompt of {t} tokens leaves no room in a cache of {self.max_len} rows for a decode step")
-        ids = ids.to(self.dev)
-        x = self.embed[ids]
-        cos, sin = self.cos[:t], self.sin[:t]
+        nq, rows = self.h_loc * s.head_dim, b * t
+        # nine kernels per layer and no copy in between: activations stay token-major [B * T, features], RoPE writes the
+        # cache and undoes the pair order of the rows, attention reads the cache in place
+        h, x = ops.embed_rmsnorm(ids.to(self.dev, torch.long).reshape(rows).contiguous(), self.embed, self.layers[0]["in_norm"], s.rms_eps)
+        res = None
         for li, L in enumerate(self.layers):
-            h = self._rms(x, L["in_norm"])
-            qkv = L["qkv"](h)
-            nq, nkv = self.h_loc * s.head_dim, self.hk_loc * s.head_dim
-            if self.pair_rows:   # features (j, j + D/2) sit side by side: back to the natural order
-                unpair = lambda z, heads: z.reshape(b, t, heads, s.head_dim // 2, 2).transpose(-1, -2).reshape(b, t, heads, s.head_dim)
-                q = unpair(qkv[..., :nq], self.h_loc).transpose(1, 2)
-                k = unpair(qkv[..., nq:nq + nkv], self.hk_loc).transpose(1, 2)
-            else:
-                q = qkv[..., :nq].reshape(b, t, self.h_loc, s.head_dim).transpose(1, 2)
-                k = qkv[..., nq:nq + nkv].reshape(b, t, self.hk_loc, s.head_dim).transpose(1, 2)
-            v = qkv[..., nq + nkv:].reshape(b, t, self.hk_loc, s.head_dim).transpose(1, 2)
-            q, k = self._rope(q, cos, sin), self._rope(k, cos, sin)
-            self.k_cache[li, :, :, :t] = k
-            self.v_cache[li, :, :, :t] = v
-            a = ops.flash_attn_kv_view(q.contiguous(), self.k_cache[li, :, :, :t], self.v_cache[li, :, :, :t], causal=True)
-            a = self._gather(a.transpose(1, 2).reshape(b * t, nq), "attn_bounds")
-            o = self._gather(L["o"](a), "hidden_bounds")
-            x = x + o.reshape(b, t, s.hidden)
-            x = self._mlp(L, x)
-        logits = self._rms(x, self.final_norm) @ self.lm_head.T
+            k_cache, v_cache = self.k_cache[li], self.v_cache[li]
+            if li:
+                h, x = ops.add_rmsnorm(x, L["in_norm"], s.rms_eps, res)
+            q = ops.rope_tokens(L["qkv"](h), self.cos, self.sin, k_cache, v_cache, b, self.h_loc, self.pair_rows)
+            a = ops.attention_tokens(q, k_cache, v_cache, t, True).view(rows, nq)
+            o = self._gather(L["o"](self._gather(a, "attn_bounds")), "hidden_bounds")
+            h, x = ops.add_rmsnorm(x, L["post_norm"], s.rms_eps, o)
+            act = self._gather(ops.silu_mul(L["gate_up"](h), self.pair_rows), "inter_bounds")
+            res = self._gather(L["down"](act), "hidden_bounds")
+        h, x = ops.add_rmsnorm(x, self.final_norm, s.rms_eps, res)
+        logits = (h @ self.lm_head.T).view(b, t, s.vocab)
         self.tok.copy_(logits[:, -1].float().argmax(-1))
         self.pos.fill_(t)
         self.kv_len.fill_(t + 1)

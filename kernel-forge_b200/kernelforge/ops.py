@@ -576,17 +576,29 @@ def int4_linear(x: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, gro
 # them to torch; used by kernelforge.llama_decode)
 # ---------------------------------------------------------------------------
 
+def _native(out, what: str):
+    if out is None:
+        raise ValueError(f"{what}: arguments must be non-empty contiguous fp16 CUDA tensors of matching shapes")
+    return out
+
+
 def add_rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float, residual: torch.Tensor | None = None):
     """(y, s): s = x + residual (x itself when residual is None), y = RMSNorm(s) * weight.  fp16 [rows, hidden]."""
-    rows, hidden = x.shape
-    y = torch.empty_like(x)
-    s = torch.empty_like(x) if residual is not None else x
-    with _capi.on_device(x.device):
-        _capi.check(_capi.lib().kfb_add_rmsnorm(x.data_ptr(), residual.data_ptr() if residual is not None else None,
-                                                weight.data_ptr(), y.data_ptr(),
-                                                s.data_ptr() if residual is not None else None, rows, hidden, eps,
-                                                _capi.stream_ptr(x.device)))
-    return y, s
+    return _native(_capi.host().add_rmsnorm(x, weight, eps, residual), "add_rmsnorm")
+
+
+def rope_tokens(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, batch: int,
+                heads: int, pairs: bool) -> torch.Tensor:
+    """Prefill's rope_kv_write: rotates q and k of positions 0 .. T - 1 of every sequence and writes k and v into those rows
+    of the caches [B, Hk, Lmax, D].  qkv: [B * T, (H + 2 Hk) D]; `pairs`: its q and k heads are in the row order of
+    interleave_qkv_for_rope.  Returns q [B, T, H, D]."""
+    return _native(_capi.host().rope_tokens(qkv, cos, sin, k_cache, v_cache, batch, heads, pairs), "rope_tokens")
+
+
+def attention_tokens(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, kv_rows: int, causal: bool) -> torch.Tensor:
+    """flash_attn with q and the result in token-major layout [B, T, H, D], against the first kv_rows rows of the caches
+    [B, Hk, Lmax, D]: the layout projections write and read, so nothing is transposed."""
+    return _native(_capi.host().attention_tokens(q, k_cache, v_cache, kv_rows, causal), "attention_tokens")
 
 
 def rope_kv_write(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, pos: torch.Tensor, k_cache: torch.Tensor,
@@ -602,13 +614,10 @@ def rope_kv_write(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, pos: 
     return q
 
 
-def silu_mul(gate_up: torch.Tensor) -> torch.Tensor:
-    """silu(gate) * up for gate_up = [rows, 2 * inter] (gate | up)."""
-    rows, two = gate_up.shape
-    out = torch.empty(rows, two // 2, dtype=torch.float16, device=gate_up.device)
-    with _capi.on_device(gate_up.device):
-        _capi.check(_capi.lib().kfb_silu_mul(gate_up.data_ptr(), out.data_ptr(), rows, two // 2, _capi.stream_ptr(gate_up.device)))
-    return out
+def silu_mul(gate_up: torch.Tensor, pairs: bool = False) -> torch.Tensor:
+    """silu(gate) * up for gate_up = [rows, 2 * inter]: gate | up, or (pairs) gate and up of a feature side by side, the row
+    order of interleave_gate_up."""
+    return _native(_capi.host().silu_mul(gate_up, pairs), "silu_mul")
 
 
 def lm_head_argmax(h: torch.Tensor, lm_head: torch.Tensor, logits: torch.Tensor | None = None,
