@@ -109,6 +109,12 @@ size_t kfb_int4_linear_ws_bytes(int M, int N, int K, int group, int dtype);
 int kfb_int4_linear(const void* x, const void* packed, const void* scales, const void* bias, void* y,
                     int M, int N, int K, int group, int dtype, void* ws, size_t ws_bytes, void* stream);
 
+/* The same for the gate / up projection of a SiLU MLP with gate and up rows interleaved (the row order of
+ * kfb_int4_gemv_silu_pair), any M, N % 4 == 0, fp16: act [M, N / 2] = fp16(fp16(silu(gate . x)) * (up . x)), without the
+ * [M, N] product going to memory and back.  Workspace as for kfb_int4_linear. */
+int kfb_int4_linear_silu_pairs(const void* x, const void* packed, const void* scales, void* act, int M, int N, int K, int group,
+                               void* ws, size_t ws_bytes, void* stream);
+
 /* int4_gemv (csrc/gemm/dequant_gemv.cu:21-36, kernel csrc/gemm/dequant_gemv_kernel.cuh:38-109):
  * 1 <= M <= 8, any N >= 1, K % group == 0, group in {64,128}.  FP32 accumulation, one
  * rounding to fp16.  No workspace.  The weights are streamed by the TMA unit into shared

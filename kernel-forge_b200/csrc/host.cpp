@@ -94,6 +94,7 @@ PyObject* pair_of(at::Tensor first, PyObject* second /* new reference or null */
 inline int dtype_code(at::ScalarType t) { return t == at::kHalf ? KFB_F16 : t == at::kBFloat16 ? KFB_BF16 : t == at::kFloat ? KFB_F32 : -1; }
 
 // int4_linear(x, packed, scales, group_size, bias or None) -> y
+// int4_linear(x, packed, scales, group_size, "silu_pairs") -> silu(gate) * up for gate / up-interleaved weight rows
 PyObject* int4_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   ARGS(5)
   return guarded([&]() -> PyObject* {
@@ -102,7 +103,8 @@ PyObject* int4_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (!x || !packed || !scales || !int_arg(a[3], &group)) NOT_PLAIN;
     const auto type = x->scalar_type();
     if ((type != at::kHalf && type != at::kBFloat16) || packed->scalar_type() != at::kInt || scales->scalar_type() != at::kHalf) NOT_PLAIN;
-    if (a[4] != Py_None) {
+    const bool silu = PyUnicode_Check(a[4]);
+    if (a[4] != Py_None && !silu) {
       bias = plain(a[4]);
       if (!bias || bias->scalar_type() != type || bias->dim() != 1 || !bias->is_contiguous() || bias->device() != x->device()) NOT_PLAIN;
     }
@@ -112,19 +114,22 @@ PyObject* int4_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if ((group != 64 && group != 128) || k < group || k % group || packed->size(1) * 8 != k || scales->size(0) != rows || scales->size(1) != k / group) NOT_PLAIN;
     const int64_t m = x->numel() / k;
     if (m < 1 || rows < 1 || m > INT32_MAX || rows > INT32_MAX || k > INT32_MAX || (bias && bias->size(0) != rows)) NOT_PLAIN;
+    if (silu && (type != at::kHalf || rows % 4)) NOT_PLAIN;
     OnDevice dev(*x);
     at::DimVector shape(x->sizes());
-    shape.back() = rows;
+    shape.back() = silu ? rows / 2 : rows;
     at::Tensor y = new_tensor(shape, type, *x);
     const int code = dtype_code(type);
     const size_t ws_bytes = kfb_int4_linear_ws_bytes((int)m, (int)rows, (int)k, (int)group, code);
     at::Tensor ws;
     if (ws_bytes) ws = new_tensor({(int64_t)ws_bytes}, at::kByte, *x);
-    void* stream = stream_of(*x);
+    void *stream = stream_of(*x), *wsp = ws_bytes ? ws.data_ptr() : nullptr;
     int rc;
     Py_BEGIN_ALLOW_THREADS
-    rc = kfb_int4_linear(x->data_ptr(), packed->data_ptr(), scales->data_ptr(), bias ? bias->data_ptr() : nullptr, y.data_ptr(), (int)m,
-                         (int)rows, (int)k, (int)group, code, ws_bytes ? ws.data_ptr() : nullptr, ws_bytes, stream);
+    if (silu) rc = kfb_int4_linear_silu_pairs(x->data_ptr(), packed->data_ptr(), scales->data_ptr(), y.data_ptr(), (int)m, (int)rows, (int)k,
+                                              (int)group, wsp, ws_bytes, stream);
+    else rc = kfb_int4_linear(x->data_ptr(), packed->data_ptr(), scales->data_ptr(), bias ? bias->data_ptr() : nullptr, y.data_ptr(), (int)m,
+                              (int)rows, (int)k, (int)group, code, wsp, ws_bytes, stream);
     Py_END_ALLOW_THREADS
     return rc ? raise_status(rc) : THPVariable_Wrap(std::move(y));
   });

@@ -3,17 +3,22 @@
 // Replaces dequant_gemm_tc_kernel + splitk_reduce of the reference
 // (csrc/gemm/dequant_gemm_tc_kernel.cuh:55-162: mma.sync, 64x64 tiles, cp.async, N % 64 == 0).
 //
-// The product is computed transposed, y^T = W_hat x^T, so the 128 weight rows of a tile fill the
-// M = 128 dimension of tcgen05.mma and the batch is the MMA N (16..256): small batches are not
-// padded up to a 128-row tile.  One CTA per (128 output features, batch tile, K split):
-//   warp 4  (1 thread)  TMA: the packed int32 tile (128 rows x 8 words = 64 k) and the fp16 x tile
-//                       (batch rows x 64 k, 128-byte swizzle) of each K block, mbarrier ring;
-//   warps 0-3 (128 thr) dequantise: thread r unpacks row r (magic-number nibble unpack, exact q,
-//                       one fp16 multiply by the group scale = the reference's fp16(q*s),
-//                       dequant_gemm_tc_kernel.cuh:100-112) and stores it as a K-major row of the
-//                       128-byte-swizzled A tile; fence.proxy.async; then, at the end, the epilogue:
-//                       TMEM -> registers -> fp16 y (or FP32 split-K partials), coalesced along N;
-//   warp 5  (1 thread)  tcgen05.mma.kind::f16 A[smem] x B[smem] -> FP32 accumulator in TMEM.
+// The product is computed transposed, y^T = W_hat x^T: weight rows are the M of tcgen05.mma, the batch is its N.  A
+// persistent kernel of CTA pairs (clusters of two, cta_group::2): a pair owns 256 weight rows x `mt` batch rows
+// (32 .. 256, chosen per call) of one K range.  Each CTA
+//   * brings its own 128 rows of packed words (TMA, two K blocks of 128 per copy) and HALF of the batch rows of the
+//     activation tile (TMA, 128-byte swizzle); the tensor cores of both read both halves;
+//   * dequantises its weight rows from registers straight into TENSOR MEMORY, the A operand of the MMA: one thread per
+//     row, exact q, one fp16 multiply by the group scale = the reference's fp16(q*s)
+//     (dequant_gemm_tc_kernel.cuh:100-112).  TMEM holds a ring of 4 K blocks (256 columns) next to the accumulator;
+//   * keeps 128 rows of the accumulator in its own TMEM and writes them: TMEM -> registers (which frees the accumulator
+//     for the next tile) -> pairs of neighbouring features exchanged between lanes -> rows of y.
+// What bounds it: the tensor pipe at large M (4 mt clocks per K block of 128), the dequantisation when mt is small.  Why pairs and TMEM operands: with one CTA per 128 x 256 tile and the dequantised
+// tile in shared memory, every 64 k moved 36 KB from L2 and wrote and re-read 16 KB of weights in shared memory; L2 ->
+// SM traffic was the limit at ~45 % of the tensor peak.  Here it is 20 KB per 64 k, and no dequantised weight
+// touches shared memory.
+//
+// Warps of a CTA: 0-7 dequantise, 8-15 epilogue, 16 TMA producer, 17 MMA issuer (leader CTA only).
 // Split-K partial sums are reduced in split order by a second kernel (deterministic).
 // Rows past N and batch rows past M are zero-filled by TMA and never stored.
 #include "common.cuh"
@@ -26,16 +31,38 @@ namespace {
 
 using namespace sm100;
 
-constexpr int kTileN = 128;   // output features per CTA (MMA M)
-constexpr int kBlockK = 64;   // k per pipeline stage (one 128-byte swizzle row of fp16)
-constexpr int kDequantWarps = 8;  // two threads per weight row: four packed words each
-constexpr int kThreads = (kDequantWarps + 2) * 32;
-constexpr int kProducerWarp = kDequantWarps;
-constexpr int kMmaWarp = kDequantWarps + 1;
+constexpr int kPairRows = 256;   // weight rows of a pair's tile (MMA M); 128 per CTA
+constexpr int kRows = 128;
+constexpr int kBlockK = 128;     // k per pipeline stage: two 64-wide (128-byte) swizzled activation tiles
+constexpr int kMaxTile = 256;    // most batch rows of a tile (MMA N)
+constexpr int kStages = 4;       // K blocks of dequantised weights in TMEM
+constexpr int kMaxXStages = 16;  // K blocks of activations in shared memory: as many as fit (4 at 256 batch rows per tile)
+constexpr int kWordStages = 4;   // copies of packed words in flight, two K blocks each
+constexpr int kDequantGroups = 2;  // warpgroups; they take the K blocks in turn
+constexpr int kDequantWarps = 4 * kDequantGroups, kEpilogueWarps = 8;
+constexpr int kProducerWarp = kDequantWarps + kEpilogueWarps;
+constexpr int kMmaWarp = kProducerWarp + 1;
+constexpr int kThreads = (kProducerWarp + 4) * 32;   // whole warpgroups: registers move between them
+// Registers per thread: 640 x 96 at launch; the epilogue keeps a row of the accumulator, rounded, in registers.
+constexpr int kRegsLaunch = 96, kRegsDequant = 88, kRegsEpilogue = 128, kRegsMisc = 40;
+static_assert(kDequantWarps * kRegsDequant + kEpilogueWarps * kRegsEpilogue + 4 * kRegsMisc <= kThreads / 32 * kRegsLaunch,
+              "setmaxnreg.inc only takes what the block was launched with");
+constexpr uint32_t kTmemCols = 512;
+constexpr uint32_t kColA = 256;  // 4 stages x 64 columns; the accumulator (or two of <= 128 columns) lies below
 
-enum WaitCode : uint32_t { kWaitFree = 0x301, kWaitLoaded, kWaitAReady, kWaitAcc };
+// shared memory
+constexpr int kWordBytes = kRows * 128;                       // 128 rows x 32 words
+constexpr int kXRing = 128 * 1024;                            // the activation ring; a K block takes mt / 2 rows x 256 bytes
+constexpr int kOffX = kWordStages * kWordBytes;
+constexpr int kOffBars = kOffX + kXRing;
+constexpr int kNumBars = 2 * kWordStages + 2 * kMaxXStages + 2 * kStages + 4;
+constexpr int kOffMisc = kOffBars + kNumBars * 8;
+constexpr int kSmem = kOffMisc + 16 + 1024;                   // + alignment of the tiles to 1024 bytes
+static_assert(kSmem <= 227 * 1024, "must fit in shared memory");
 
-// Where the fp16 result goes.  Plain call: one buffer [M, N].  Output-feature-sharded call (fused
+enum WaitCode : uint32_t { kWaitFree = 0x301, kWaitWords, kWaitX, kWaitAReady, kWaitAcc, kWaitAccFree, kWaitWordsFree, kWaitAFree };
+
+// Where the 16-bit result goes.  Plain call: one buffer [M, N].  Output-feature-sharded call (fused
 // all-gather): `count` buffers [M, ld], one per GPU of the group (peer-mapped device pointers, this
 // GPU's own buffer included); this rank's N columns are stored at column `col0` of EVERY buffer with
 // plain peer stores from the epilogue, so the gather overlaps the computation tile by tile and no
@@ -48,21 +75,22 @@ struct OutSpec {
   int col0;  // first column this rank writes
   int bf16;  // the buffers hold bf16 instead of fp16 (the 16-bit stores are the same)
   const uint16_t* bias;  // [N] of the output type or nullptr: added to the rounded product, rounded again (as `y + bias`)
+  int silu;  // fp16: features 2j, 2j + 1 are gate and up of one; the buffers hold [M, N / 2] = fp16(fp16(silu(gate)) * up)
 };
 
-template <int MT>
-struct Layout {
-  // TMA latency (~1400 clocks) + dequantisation + MMA of one K block must be covered by the other stages
-  static constexpr int kStages = MT <= 64 ? 4 : (MT == 128 ? 5 : 4);
-  static constexpr int kA = kTileN * kBlockK * 2;        // dequantised weights, 16 KB
-  static constexpr int kP = kTileN * (kBlockK / 8) * 4;  // packed words, 4 KB
-  static constexpr int kX = MT * kBlockK * 2;            // activations
-  static constexpr int kStage = kA + kP + kX;            // multiples of 1024
-  static constexpr int kBars = kStages * kStage;
-  static constexpr int kMisc = kBars + 3 * kStages * 8 + 8;
-  static constexpr int kBytes = kMisc + 16;
-  static constexpr int kAlloc = kBytes + 1024;
-  static constexpr uint32_t kTmemCols = MT < 32 ? 32 : MT;
+__device__ __forceinline__ uint16_t silu_pair(uint32_t gate_up) {
+  const __half2 h = *reinterpret_cast<const __half2*>(&gate_up);
+  const float g = __low2float(h);
+  const __half a = __hmul(__float2half_rn(g / (1.0f + __expf(-g))), __high2half(h));
+  return *reinterpret_cast<const uint16_t*>(&a);
+}
+
+
+struct Shape {
+  int M, N, K, group;
+  int mt;                          // batch rows per tile: a multiple of 32, <= 256
+  int m_tiles, n_tiles, splits;
+  int kblocks_per_split;           // a multiple of 2 (whole copies of packed words)
 };
 
 __device__ __forceinline__ uint32_t h2_as_u32(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
@@ -123,308 +151,475 @@ __device__ __forceinline__ uint16_t round16_bias(float v, uint16_t bias, bool bf
   return round16(__half2float(a) + __half2float(b), false);
 }
 
-// out: fp16 (bf16) y [M, N] when splits == 1, else FP32 partial [splits][M][N]
-template <int MT, bool kBf16>
-__global__ void __launch_bounds__(kThreads)
+// Pairs: one packed conversion (a single cvt.rn.f16.f32 runs at a quarter of the packed one's rate: draining an
+// accumulator took 3300 clocks with it), one packed addition.
+template <bool kBf16>
+__device__ __forceinline__ uint32_t round16x2(float lo, float hi) {
+  if constexpr (kBf16) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
+  }
+  const __half2 v = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+template <bool kBf16>
+__device__ __forceinline__ uint32_t add16x2(uint32_t a, uint32_t b) {
+  if constexpr (kBf16) {
+    const __nv_bfloat162 v = __hadd2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
+    return *reinterpret_cast<const uint32_t*>(&v);
+  }
+  const __half2 v = __hadd2(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+// out: 16-bit y [M, N] when splits == 1, else FP32 partial [splits][M][N]
+template <bool kBf16>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 int4_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
-                 const __half* __restrict__ scales, const OutSpec out, float* __restrict__ partial, int M, int N,
-                 int K, int group, int kblocks_per_split, unsigned int* status, unsigned long long* trace) {
-  using L = Layout<MT>;
-  constexpr int S = L::kStages;
+                 const __half* __restrict__ scales, const __grid_constant__ OutSpec out, float* __restrict__ partial,
+                 const __grid_constant__ Shape sh,
+                 unsigned int* status) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  uint64_t* loaded = reinterpret_cast<uint64_t*>(smem + L::kBars);  // TMA landed
-  uint64_t* a_ready = loaded + S;                                   // dequantised tile written
-  uint64_t* stage_free = a_ready + S;                               // MMAs of the stage retired
-  uint64_t* acc_done = stage_free + S;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::kMisc);
+  uint64_t* w_full = reinterpret_cast<uint64_t*>(smem + kOffBars);   // packed words landed
+  uint64_t* w_free = w_full + kWordStages;                           // ... and have been read
+  uint64_t* x_full = w_free + kWordStages;                           // activation tile landed
+  uint64_t* x_free = x_full + kMaxXStages;                           // the MMAs that read it have completed
+  uint64_t* a_ready = x_free + kMaxXStages;                             // leader: both CTAs' weights are in TMEM (and both x tiles landed)
+  uint64_t* a_free = a_ready + kStages;                              // the MMAs that read them have completed
+  uint64_t* acc_full = a_free + kStages;                         // [2] accumulator complete
+  uint64_t* acc_free = acc_full + 2;                                 // [2] leader: accumulator read by both CTAs
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kOffMisc);
   volatile uint32_t* abort_word = tmem_slot + 1;
   const AbortCtx ctx{abort_word, status};
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = blockIdx.x * kTileN;
-  const int m0 = blockIdx.y * MT;
-  const int split = blockIdx.z, splits = gridDim.z;
-  const int total_kblocks = K / kBlockK;
-  const int kb_begin = split * kblocks_per_split;
-  const int kb_end = min(total_kblocks, kb_begin + kblocks_per_split);
-  const int n_kb = kb_end - kb_begin;  // >= 1 by construction
+  const uint32_t rank = cluster_rank();
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const int items = sh.m_tiles * sh.n_tiles * sh.splits;
+  const int total_kb = (sh.K + kBlockK - 1) / kBlockK;   // a last half block: x is zero-filled past K
+  const bool two_acc = sh.mt <= 128;
+  const uint32_t x_half = (uint32_t)(sh.mt / 2) * 128u, x_bytes = 2 * x_half;   // this CTA's half of the batch rows x 64 / 128 k
+  const uint32_t x_stages = min((uint32_t)kMaxXStages, (uint32_t)kXRing / x_bytes);
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < S; ++s) {
-      mbar_init(&loaded[s], 1);
-      mbar_init(&a_ready[s], kDequantWarps);
-      mbar_init(&stage_free[s], 1);
-    }
-    mbar_init(acc_done, 1);
-    *abort_word = *reinterpret_cast<volatile unsigned int*>(status);
-    fence_mbar_init();
-  }
-  if (warp == kMmaWarp) {
-    tmem_alloc(tmem_slot, L::kTmemCols);
-    tmem_relinquish();
-  }
-  tc_fence_before_sync();
-  __syncthreads();
-  tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
-  const bool dead_on_arrival = *abort_word != 0;
-  // optional timeline of CTA (0,0,0) for tuning (builds with -DKFB_TRACE only): 8 clock stamps per K block
-#ifdef KFB_TRACE
-  const bool tracing = trace != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0;
-#else
-  constexpr bool tracing = false;
-#endif
-  auto stamp = [&](int i, int k) {
-    if (tracing && i < 64) trace[i * 8 + k] = clock64();
+  struct Item {
+    int m0, n0, kb_begin, n_kb, split;
+  };
+  auto item_at = [&](int it) {   // batch tiles fastest: the pairs running together share weight rows
+    Item w;
+    const int mt_i = it % sh.m_tiles, rest = it / sh.m_tiles;
+    w.split = rest / sh.n_tiles;
+    w.m0 = mt_i * sh.mt;
+    w.n0 = (rest - w.split * sh.n_tiles) * kPairRows + (int)rank * kRows;   // this CTA's weight rows
+    w.kb_begin = w.split * sh.kblocks_per_split;
+    w.n_kb = min(total_kb - w.kb_begin, sh.kblocks_per_split);
+    return w;
   };
 
-  if (dead_on_arrival) {
-    // fall through to the teardown
-  } else if (warp == kProducerWarp) {
+  // One pipeline step of the TMA producer: the words of K blocks i, i + 1 (even i) and the activations of K block i.
+  struct Ring {
+    uint32_t slot = 0, parity = 0;
+    __device__ void next(uint32_t stages) {
+      if (++slot == stages) { slot = 0; parity ^= 1u; }
+    }
+  };
+  Ring p_words, p_x;
+  auto load = [&](const Item& w, int i) -> bool {
+    if ((i & 1) == 0) {
+      if (!mbar_wait(&w_free[p_words.slot], p_words.parity ^ 1u, ctx, kWaitWordsFree)) return false;
+      mbar_arrive_expect_tx(&w_full[p_words.slot], kWordBytes);
+      tma_load_2d(smem + p_words.slot * kWordBytes, &tm_w, &w_full[p_words.slot], (w.kb_begin + i) * (kBlockK / 8), w.n0);
+      p_words.next(kWordStages);
+    }
+    if (!mbar_wait(&x_free[p_x.slot], p_x.parity ^ 1u, ctx, kWaitFree)) return false;
+    mbar_arrive_expect_tx(&x_full[p_x.slot], x_bytes);
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      tma_load_4d(smem + kOffX + p_x.slot * x_bytes + h * x_half, &tm_x, &x_full[p_x.slot], (w.kb_begin + i) * kBlockK + h * 64,
+                  w.m0 + (int)rank * (sh.mt / 2), 0, 0);
+    p_x.next(x_stages);
+    return true;
+  };
+  if (warp == kProducerWarp) {
     if (lane == 0) {
       tma_prefetch_desc(&tm_w);
       tma_prefetch_desc(&tm_x);
-      for (int i = 0; i < n_kb; ++i) {
-        const int s = i % S;
-        if (!mbar_wait(&stage_free[s], ((uint32_t)(i / S) & 1u) ^ 1u, ctx, kWaitFree)) break;
-        stamp(i, 0);
-        mbar_arrive_expect_tx(&loaded[s], L::kP + L::kX);
-        uint8_t* st = smem + s * L::kStage;
-        const int kb = kb_begin + i;
-        tma_load_2d(st + L::kA, &tm_w, &loaded[s], kb * (kBlockK / 8), n0);
-        tma_load_4d(st + L::kA + L::kP, &tm_x, &loaded[s], kb * kBlockK, m0, 0, 0);  // tm_x is a 4-D map
+      for (int s = 0; s < kWordStages; ++s) {
+        mbar_init(&w_full[s], 1);
+        mbar_init(&w_free[s], 8);   // the two groups that read a copy of words
       }
-    }
-  } else if (warp == kMmaWarp) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = idesc_f16(kTileN, MT, kBf16 ? 1 : 0, 0, 0);
-      for (int i = 0; i < n_kb; ++i) {
-        const int s = i % S;
-        const uint32_t ph = (uint32_t)(i / S) & 1u;
-        if (!mbar_wait(&a_ready[s], ph, ctx, kWaitAReady)) break;  // implies loaded[s]: the dequant warps waited on it
-        stamp(i, 4);
-        tc_fence_after_sync();
-        const uint32_t a_addr = smem_u32(smem + s * L::kStage);
-        const uint32_t b_addr = a_addr + L::kA + L::kP;
-#pragma unroll
-        for (int kk = 0; kk < kBlockK / 16; ++kk)
-          mma_ss(tmem_base, smem_desc_sw128(a_addr + kk * 32, 16, 1024), smem_desc_sw128(b_addr + kk * 32, 16, 1024),
-                 idesc, (i > 0 || kk > 0) ? 1u : 0u);
-        tc_commit(&stage_free[s]);
-        stamp(i, 5);
+      for (int s = 0; s < kMaxXStages; ++s) {
+        mbar_init(&x_full[s], 1);
+        mbar_init(&x_free[s], 1);
       }
-      tc_commit(acc_done);
+      for (int s = 0; s < kStages; ++s) {
+        mbar_init(&a_ready[s], 8);   // the four warps of a group, in both CTAs
+        mbar_init(&a_free[s], 1);
+      }
+      for (int i = 0; i < 2; ++i) {
+        mbar_init(&acc_full[i], 1);
+        mbar_init(&acc_free[i], 2 * kEpilogueWarps);
+      }
+      *abort_word = 0;
+      fence_mbar_init();
     }
+    __syncwarp();
+  }
+  if (warp == kMmaWarp) {
+    tmem_alloc_pair(tmem_slot, kTmemCols);
+    tmem_relinquish_pair();
+    tc_fence_before_sync();
+  }
+  // The producer only announces its part of the set-up and goes on to its first loads, which touch this CTA's barriers
+  // only; everybody else waits for this CTA here and for the other one (whose barriers it will arrive on, whose TMEM the
+  // MMAs will write) where it first needs it.
+  if (warp == kProducerWarp) {
+    asm volatile("bar.arrive 1, %0;" ::"n"(kThreads) : "memory");
   } else {
-    // ---------------------------------------------------------------- dequantise (two threads per weight row)
-    const int r = threadIdx.x & 127;   // weight row inside the tile; a warp covers 32 consecutive rows
-    const int half = threadIdx.x >> 7; // which four of the eight packed words of a K block
-    const int row = n0 + r;
-    const int groups = K / group;
-    const __half* srow = scales + (size_t)min(row, N - 1) * groups;
-    bool ok = true;
-    // The group scale of a K block comes from global memory (L2 latency of several hundred clocks): it is
-    // fetched two K blocks ahead so that the load never sits on the critical path of a pipeline stage.
-    __half sc_ring[3];
-    sc_ring[0] = srow[(kb_begin * kBlockK) / group];
-    sc_ring[1] = srow[(min(kb_begin + 1, kb_end - 1) * kBlockK) / group];
-    for (int i = 0; i < n_kb; ++i) {
-      const int s = i % S;
-      const uint32_t ph = (uint32_t)(i / S) & 1u;
-      sc_ring[2] = srow[(min(kb_begin + i + 2, kb_end - 1) * kBlockK) / group];
-      const __half sc = sc_ring[0];
-      sc_ring[0] = sc_ring[1];
-      sc_ring[1] = sc_ring[2];
-      ok = __all_sync(0xffffffffu, mbar_wait(&loaded[s], ph, ctx, kWaitLoaded));
-      if (!ok) break;
-      if (threadIdx.x == 0) stamp(i, 1);
-      uint8_t* st = smem + s * L::kStage;
-      const uint4 w = *reinterpret_cast<const uint4*>(st + L::kA + r * 32 + half * 16);
-      const __half2 s2 = __half2half2(sc);
-      uint8_t* arow = st + r * 128;
-      const int x = r & 7, c = half * 4;
-      if constexpr (kBf16) {
-        const float sf = __half2float(sc);
-        *reinterpret_cast<uint4*>(arow + (((c + 0) ^ x) << 4)) = dequant8_bf16(w.x, sf);
-        *reinterpret_cast<uint4*>(arow + (((c + 1) ^ x) << 4)) = dequant8_bf16(w.y, sf);
-        *reinterpret_cast<uint4*>(arow + (((c + 2) ^ x) << 4)) = dequant8_bf16(w.z, sf);
-        *reinterpret_cast<uint4*>(arow + (((c + 3) ^ x) << 4)) = dequant8_bf16(w.w, sf);
-      } else {
-        *reinterpret_cast<uint4*>(arow + (((c + 0) ^ x) << 4)) = dequant8(w.x, s2);
-        *reinterpret_cast<uint4*>(arow + (((c + 1) ^ x) << 4)) = dequant8(w.y, s2);
-        *reinterpret_cast<uint4*>(arow + (((c + 2) ^ x) << 4)) = dequant8(w.z, s2);
-        *reinterpret_cast<uint4*>(arow + (((c + 3) ^ x) << 4)) = dequant8(w.w, s2);
+    asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
+  }
+  cluster_arrive();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;   // (not used by the producer, which has not waited for it)
+
+  if (warp >= kProducerWarp) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsMisc));
+    if (warp == kProducerWarp) {
+    // ---------------------------------------------------------------- TMA
+    if (lane == 0) {
+      bool ok = true;
+      for (int it = pair; ok && it < items; it += pairs) {
+        const Item w = item_at(it);
+        for (int i = 0; ok && i < w.n_kb; ++i) ok = load(w, i);
       }
-      fence_proxy_async_smem();  // generic-proxy stores -> visible to tcgen05.mma
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&a_ready[s]);
-      if (threadIdx.x == 0) stamp(i, 2);
     }
-    // ---------------------------------------------------------------- epilogue
-    // TMEM lane = weight row n, column = batch row m, but y is [M, N]: going straight to global memory
-    // would be 2-byte stores with a stride of N (measured: 60 % of the kernel time).  Each warpgroup
-    // (warps 0-3 / 4-7, which own alternate 32-column chunks) transposes its chunk through a shared
-    // memory tile [32 m][128 n] and writes rows of 128 outputs with 16-byte stores.
-    if (ok) ok = __all_sync(0xffffffffu, mbar_wait(acc_done, 0, ctx, kWaitAcc));
-    if (threadIdx.x == 0) stamp(63, 6);
-    if (ok) {
-      tc_fence_after_sync();
-      const uint32_t lane_bits = (uint32_t)((warp & 3) * 32) << 16;
-      const int wg = warp >> 2;                    // 0 or 1
-      uint8_t* tile = smem + wg * L::kStage;       // every stage is free once acc_done has completed
-      const bool f32 = splits > 1;
-      const int n_valid = min(kTileN, N - n0);     // columns of this tile that exist
-      const bool with_bias = !f32 && out.bias != nullptr;
-      const uint16_t bias = with_bias ? out.bias[min(row, N - 1)] : (uint16_t)0;
-      constexpr int kCols = MT >= 32 ? 32 : MT;
-      constexpr int kChunks = MT >= 32 ? MT / 32 : 1;
-#pragma unroll 1
-      for (int ch = wg; ch < kChunks; ch += 2) {
-        const int c0 = ch * 32;
-        if (m0 + c0 >= M) break;  // uniform per warpgroup: batch rows that do not exist
-        uint32_t acc[32];
-        if constexpr (MT >= 32) {
-          tmem_ld_x32(tmem_base + lane_bits + c0, acc);
-        } else {
-          tmem_ld_x16(tmem_base + lane_bits + c0, acc);
-        }
-        tmem_wait_ld();
-        if (f32) {
+    __syncwarp();
+    cluster_wait();
+    } else if (warp == kMmaWarp) {
+    // ---------------------------------------------------------------- tcgen05.mma of the pair
+    // The whole warp walks the loop and one elected lane issues: addresses and descriptors then stay in uniform
+    // registers (inside `if (lane == 0)` every MMA costs ~95 clocks of moves into them, more than a small MMA takes).
+    cluster_wait();
+    if (rank == 0) {
+      const uint32_t idesc = idesc_f16(kPairRows, sh.mt, kBf16 ? 1 : 0, 0, 0);
+      const uint64_t desc0 = smem_desc_sw128(smem_u32(smem + kOffX), 16, 1024);
+      uint32_t kc = 0, ic = 0;
+      Ring x;
+      bool ok = true;
+      for (int it = pair; ok && it < items; it += pairs, ++ic) {
+        const int n_kb = item_at(it).n_kb;
+        const uint32_t buf = two_acc ? (ic & 1u) : 0u, use = two_acc ? (ic >> 1) : ic;
+        ok = __all_sync(0xffffffffu, mbar_wait(&acc_free[buf], (use & 1u) ^ 1u, ctx, kWaitAccFree));
+        if (!ok) break;
+        const uint32_t acc = tmem_base + buf * 128u;
+        for (int i = 0; i < n_kb; ++i, ++kc) {
+          const uint32_t s = kc % kStages;
+          ok = __all_sync(0xffffffffu, mbar_wait(&a_ready[s], (kc / kStages) & 1u, ctx, kWaitAReady));
+          if (!ok) break;
+          tc_fence_after_sync();
+          const uint32_t a = tmem_base + kColA + s * 64u;
+          const uint64_t b = desc0 + (uint64_t)(x.slot * (x_bytes >> 4));
+          if (elect_one()) {
 #pragma unroll
-          for (int c = 0; c < kCols; ++c) reinterpret_cast<float*>(tile)[c * kTileN + r] = __uint_as_float(acc[c]);
-        } else {
-#pragma unroll
-          for (int c = 0; c < kCols; ++c)
-            reinterpret_cast<uint16_t*>(tile)[c * kTileN + r] =
-                with_bias ? round16_bias(__uint_as_float(acc[c]), bias, kBf16) : round16(__uint_as_float(acc[c]), kBf16);
-        }
-        asm volatile("bar.sync %0, 128;" ::"r"(1 + wg) : "memory");
-        const int m_hi = min(kCols, M - (m0 + c0));  // batch rows of this chunk that exist
-        if (f32) {
-          float* dst = partial + ((size_t)split * M + m0 + c0) * N + n0;
-          if ((N & 3) == 0) {
-            for (int idx = r; idx < m_hi * 32; idx += 128) {
-              const int ml = idx >> 5, seg = idx & 31;
-              if (seg * 4 < n_valid)
-                *reinterpret_cast<uint4*>(dst + (size_t)ml * N + seg * 4) = reinterpret_cast<const uint4*>(tile)[ml * 32 + seg];
-            }
-          } else {
-            for (int ml = 0; ml < m_hi; ++ml)
-              if (r < n_valid) dst[(size_t)ml * N + r] = reinterpret_cast<const float*>(tile)[ml * kTileN + r];
+            for (int kk = 0; kk < kBlockK / 16; ++kk)
+              mma_ts_pair(acc, a + kk * 8, b + (uint64_t)((kk / 4) * (x_half >> 4) + (kk % 4) * 2), idesc, (i > 0 || kk > 0) ? 1u : 0u);
+            tc_commit_pair(&a_free[s]);
+            tc_commit_pair(&x_free[x.slot]);
+            if (i + 1 == n_kb) tc_commit_pair(&acc_full[buf]);
           }
-        } else {
-          const bool vec = ((out.ld | out.col0) & 7) == 0;  // every row segment starts on a 16-byte boundary
-          for (int p = 0; p < out.count; ++p) {
-            __half* dst = out.y[p] + (size_t)(m0 + c0) * out.ld + out.col0 + n0;
-            if (vec) {
-              for (int idx = r; idx < m_hi * 16; idx += 128) {
-                const int ml = idx >> 4, seg = idx & 15;
-                if (seg * 8 + 8 <= n_valid) {
-                  *reinterpret_cast<uint4*>(dst + (size_t)ml * out.ld + seg * 8) = reinterpret_cast<const uint4*>(tile)[ml * 16 + seg];
-                } else {
-                  for (int e = seg * 8; e < n_valid; ++e) dst[(size_t)ml * out.ld + e] = reinterpret_cast<const __half*>(tile)[ml * kTileN + e];
+          __syncwarp();
+          x.next(x_stages);
+        }
+      }
+    }
+    }
+  } else if (warp < kDequantWarps) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsDequant));
+    // ---------------------------------------------------------------- dequantise (thread = weight row)
+    // Two groups of four warps take the K blocks in turn: the mbarrier and TMEM round trips of one group pass while the
+    // other unpacks.  (All eight warps on every block, half a row each: 1200 clocks per block of 128; this: ~800.  Four
+    // groups are no faster: they saturate the issue slots, and the one warp that feeds the tensor cores suffers.)
+    const int r = (warp & 3) * 32 + lane;   // row inside the CTA's 128 = TMEM lane
+    const int turn = warp >> 2;             // which of the two K blocks of every copy of words
+    const int groups = sh.K / sh.group, gshift = sh.group == 128 ? 7 : 6;
+    const uint32_t a_base = tmem_base + kColA + ((uint32_t)((warp & 3) * 32) << 16);
+    uint32_t kc0 = 0, wc = 0;   // K blocks and copies of words before this item
+    bool ok = true, peer_ready = false;
+    for (int it = pair; ok && it < items; it += pairs) {
+      const Item w = item_at(it);
+      const __half* srow = scales + (size_t)min(w.n0 + r, sh.N - 1) * groups;
+      const int k_first = w.kb_begin * kBlockK;
+      auto scale_at = [&](int i, int half) { return srow[min((k_first + i * kBlockK + half * 64) >> gshift, groups - 1)]; };
+      __half nx[2] = {scale_at(turn, 0), scale_at(turn, 1)};   // scales of the two 64-wide halves, requested one block ahead
+      const int copies = (w.n_kb + 1) / 2;
+      uint32_t x_slot = (kc0 + turn) % x_stages, x_parity = ((kc0 + turn) / x_stages) & 1u;   // this group's K blocks in the x ring
+      for (int c = turn >> 1; c < copies; c += kDequantGroups / 2) {
+        const int i = 2 * c + (turn & 1);   // K block of this item
+        const __half sc[2] = {nx[0], nx[1]};
+        nx[0] = scale_at(i + kDequantGroups, 0);
+        nx[1] = scale_at(i + kDequantGroups, 1);
+        const uint32_t ws = (wc + c) % kWordStages;
+        ok = __all_sync(0xffffffffu, mbar_wait(&w_full[ws], ((wc + c) / kWordStages) & 1u, ctx, kWaitWords));
+        if (!ok) break;
+        const uint8_t* words = smem + ws * kWordBytes + r * 128;
+        const bool mine = i < w.n_kb;   // (not in the last copy of an odd number of blocks)
+        const uint32_t kc = kc0 + i, s = kc % kStages, ph = (kc / kStages) & 1u;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t pw[8];
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            *reinterpret_cast<uint4*>(&pw[4 * e]) = *reinterpret_cast<const uint4*>(words + (((4 * (turn & 1) + 2 * h + e) ^ (r & 7)) << 4));
+          if (h == 1) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&w_free[ws]);
+          }
+          uint32_t a[32];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            uint4 q;
+            if constexpr (kBf16) q = dequant8_bf16(pw[e], __half2float(sc[h]));
+            else q = dequant8(pw[e], __half2half2(sc[h]));
+            a[4 * e] = q.x; a[4 * e + 1] = q.y; a[4 * e + 2] = q.z; a[4 * e + 3] = q.w;
+          }
+          if (h == 0 && mine) {
+            ok = __all_sync(0xffffffffu, mbar_wait(&a_free[s], ph ^ 1u, ctx, kWaitAFree));
+            tc_fence_after_sync();
+          }
+          if (ok && mine) tmem_st_x32(a_base + s * 64u + h * 32u, a);
+        }
+        if (!ok || !mine) break;
+        ok = __all_sync(0xffffffffu, mbar_wait(&x_full[x_slot], x_parity, ctx, kWaitX));
+        if (!ok) break;
+        x_slot += kDequantGroups;
+        if (x_slot >= x_stages) { x_slot -= x_stages; x_parity ^= 1u; }   // x_stages >= kDequantGroups
+        if (!peer_ready) cluster_wait();
+        peer_ready = true;
+        tmem_wait_st();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_at(&a_ready[s], 0);
+      }
+      kc0 += w.n_kb;
+      wc += copies;
+    }
+    if (!peer_ready) cluster_wait();
+  } else {
+    // ---------------------------------------------------------------- epilogue
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsEpilogue));
+    // TMEM lane = weight row n, column = batch row m, but y is [M, N]: each of the two warpgroups (which own alternate
+    // 32-column chunks) rounds its chunks into registers and frees the accumulator.  Lanes 2j and 2j + 1 then exchange
+    // halves, so that each holds two neighbouring features of one batch row: 4-byte stores, 64 contiguous bytes of a
+    // row per half warp.  (A transpose through shared memory into 16-byte stores took 1700-2200 clocks per chunk.)
+    const int wg = (warp - kDequantWarps) >> 2, r = (warp & 3) * 32 + lane;
+    const uint32_t lane_bits = (uint32_t)((warp & 3) * 32) << 16;
+    const int chunks = sh.mt / 32;
+    // A wait expired earlier on this device: nothing is written (the read's latency passes during the products).
+    bool ok = __all_sync(0xffffffffu, *reinterpret_cast<volatile unsigned int*>(status) == 0);
+    cluster_wait();
+    uint32_t ic = 0;
+    for (int it = pair; ok && it < items; it += pairs, ++ic) {
+      const Item w = item_at(it);
+      const uint32_t buf = two_acc ? (ic & 1u) : 0u, use = two_acc ? (ic >> 1) : ic;
+      const int row = w.n0 + r;
+      const bool with_bias = sh.splits == 1 && out.bias != nullptr;
+      const uint32_t bias2 = with_bias ? out.bias[min(row, sh.N - 1)] * 0x10001u : 0u;
+      ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[buf], use & 1u, ctx, kWaitAcc));
+      if (!ok) break;
+      tc_fence_after_sync();
+      const uint32_t acc = tmem_base + buf * 128u + lane_bits;
+      if (sh.splits > 1) {   // FP32 partials: a warp's 32 rows are 128 contiguous bytes of every batch row
+        float* dst = partial + ((size_t)w.split * sh.M + w.m0) * sh.N + row;
+#pragma unroll 1
+        for (int ch = wg; ch < chunks; ch += 2) {
+          uint32_t v[32];
+          tmem_ld_x32(acc + ch * 32, v);
+          tmem_wait_ld_regs(v);
+          if (row < sh.N) {
+#pragma unroll
+            for (int c = 0; c < 32; ++c)
+              if (w.m0 + ch * 32 + c < sh.M) dst[(size_t)(ch * 32 + c) * sh.N] = __uint_as_float(v[c]);
+          }
+        }
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0 && it + (two_acc ? 2 : 1) * pairs < items) mbar_arrive_at(&acc_free[buf], 0);
+        continue;
+      }
+      uint32_t p[4][16];   // two batch rows per register
+#pragma unroll
+      for (int cc = 0; cc < 4; ++cc) {
+        const int ch = wg + 2 * cc;
+        if (ch < chunks) {
+          uint32_t v[32];
+          tmem_ld_x32(acc + ch * 32, v);
+          tmem_wait_ld_regs(v);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            p[cc][i] = round16x2<kBf16>(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
+            if (with_bias) p[cc][i] = add16x2<kBf16>(p[cc][i], bias2);
+          }
+        }
+      }
+      tc_fence_before_sync();
+      __syncwarp();
+      // the next tile may accumulate (the last arrivals would have nobody waiting: none is in flight when a CTA leaves)
+      if (lane == 0 && it + (two_acc ? 2 : 1) * pairs < items) mbar_arrive_at(&acc_free[buf], 0);
+      const int pair_n = (row & ~1) - w.n0;               // the two features this lane stores: n0 + pair_n, + 1
+      const int left = sh.N - (row & ~1);                 // how many of them (and beyond) exist
+      const bool vec = ((out.ld | out.col0) & 1) == 0;    // pairs are 4-byte aligned
+#pragma unroll
+      for (int cc = 0; cc < 4; ++cc) {
+        const int ch = wg + 2 * cc;
+        if (ch < chunks) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {   // this lane's batch row of the pair 2i, 2i + 1: the even one for even lanes
+            const uint32_t other = __shfl_xor_sync(0xffffffffu, p[cc][i], 1);
+            p[cc][i] = lane & 1 ? __byte_perm(p[cc][i], other, 0x3276) : __byte_perm(p[cc][i], other, 0x5410);
+          }
+          const int m_first = w.m0 + ch * 32 + (lane & 1);
+          const bool whole = vec && w.n0 + kRows <= sh.N && w.m0 + ch * 32 + 32 <= sh.M;   // uniform: no checks per store
+          if (out.silu) {   // (N is even: both features of a pair exist or neither does)
+            uint16_t* at = reinterpret_cast<uint16_t*>(out.y[0]) + (size_t)m_first * out.ld + ((w.n0 + pair_n) >> 1);
+#pragma unroll
+            for (int i = 0; i < 16; ++i, at += 2 * (size_t)out.ld)
+              if (left > 0 && m_first + 2 * i < sh.M) *at = silu_pair(p[cc][i]);
+            continue;
+          }
+          for (int o = 0; o < out.count; ++o) {
+            uint16_t* at = reinterpret_cast<uint16_t*>(out.y[o]) + (size_t)m_first * out.ld + out.col0 + w.n0 + pair_n;
+            const size_t two_rows = 2 * (size_t)out.ld;
+            if (whole) {
+#pragma unroll
+              for (int i = 0; i < 16; ++i, at += two_rows) *reinterpret_cast<uint32_t*>(at) = p[cc][i];
+            } else {
+#pragma unroll
+              for (int i = 0; i < 16; ++i, at += two_rows) {
+                const bool row_ok = m_first + 2 * i < sh.M;
+                if (row_ok && vec && left > 1) {
+                  *reinterpret_cast<uint32_t*>(at) = p[cc][i];
+                } else if (row_ok) {
+                  if (left > 0) at[0] = (uint16_t)p[cc][i];
+                  if (left > 1) at[1] = (uint16_t)(p[cc][i] >> 16);
                 }
               }
-            } else {
-              for (int ml = 0; ml < m_hi; ++ml)
-                if (r < n_valid) dst[(size_t)ml * out.ld + r] = reinterpret_cast<const __half*>(tile)[ml * kTileN + r];
             }
           }
         }
-        asm volatile("bar.sync %0, 128;" ::"r"(1 + wg) : "memory");  // tile is reused by the next chunk
       }
     }
   }
 
-  if (threadIdx.x == 0) stamp(63, 7);
-  if (!dead_on_arrival && *abort_word != 0) {
+  // teardown: every role of both CTAs falls through to here, also after an expired wait
+  if (*abort_word != 0) {
     const unsigned long long t0 = globaltimer_ns();
-    while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+    while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);  // let copies in flight land
   }
   tc_fence_before_sync();
   __syncthreads();
+  // Neither CTA leaves (or frees TMEM) while the other may still read its memory or arrive on its barriers.  Relaxed: the
+  // order of the output stores is not the barrier's business, and a release would wait for them (~1000 clocks).
+  cluster_arrive_relaxed();
+  cluster_wait();
   if (warp == kMmaWarp) {
     __syncwarp();
-    tmem_dealloc(tmem_base, L::kTmemCols);
+    tmem_dealloc_pair(tmem_base, kTmemCols);
   }
 }
 
-// y[m, col0 + n] = fp16(sum over splits, in split order, of partial[s][m][n]), in every output buffer
-__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restrict__ partial, const OutSpec out,
+// y[m, col0 + n] = 16-bit(sum over splits, in split order, of partial[s][m][n]) (+ bias), in every output buffer.  V: columns
+// per thread (4 where rows allow 16-byte loads).
+template <int V>
+__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restrict__ partial, const __grid_constant__ OutSpec out,
                                                             int M, int N, int splits) {
-  const long long elems = (long long)M * N;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < elems; i += (long long)gridDim.x * blockDim.x) {
-    float acc = 0.f;
-    for (int s = 0; s < splits; ++s) acc += partial[(size_t)s * elems + i];
-    const long long m = i / N;
-    const int n = (int)(i - m * N);
-    const uint16_t v = out.bias ? round16_bias(acc, out.bias[n], out.bf16 != 0) : round16(acc, out.bf16 != 0);
-    for (int p = 0; p < out.count; ++p) reinterpret_cast<uint16_t*>(out.y[p])[m * out.ld + out.col0 + n] = v;
+  const long long elems = (long long)M * N, vecs = elems / V;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < vecs; i += (long long)gridDim.x * blockDim.x) {
+    float acc[V];
+#pragma unroll
+    for (int e = 0; e < V; ++e) acc[e] = 0.f;
+    const float* p = partial + i * V;
+#pragma unroll 4
+    for (int s = 0; s < splits; ++s) {
+      if constexpr (V == 4) {
+        const float4 v = *reinterpret_cast<const float4*>(p + (size_t)s * elems);
+        acc[0] += v.x; acc[1] += v.y; acc[2] += v.z; acc[3] += v.w;
+      } else {
+        acc[0] += p[(size_t)s * elems];
+      }
+    }
+    const long long m = i * V / N;
+    const int n = (int)(i * V - m * N);
+    uint16_t v[V];
+#pragma unroll
+    for (int e = 0; e < V; ++e) v[e] = out.bias ? round16_bias(acc[e], out.bias[n + e], out.bf16 != 0) : round16(acc[e], out.bf16 != 0);
+    if constexpr (V == 4) {
+      if (out.silu) {
+        *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(out.y[0]) + m * out.ld + n / 2) =
+            silu_pair(v[0] | ((uint32_t)v[1] << 16)) | ((uint32_t)silu_pair(v[2] | ((uint32_t)v[3] << 16)) << 16);
+        continue;
+      }
+    }
+    for (int o = 0; o < out.count; ++o) {
+      uint16_t* dst = reinterpret_cast<uint16_t*>(out.y[o]) + m * out.ld + out.col0 + n;
+      if constexpr (V == 4) *reinterpret_cast<uint2*>(dst) = make_uint2(v[0] | ((uint32_t)v[1] << 16), v[2] | ((uint32_t)v[3] << 16));
+      else dst[0] = v[0];
+    }
   }
 }
 
-#ifdef KFB_TRACE
-unsigned long long* g_trace = nullptr;  // tuning aid, set through kfb_debug_set_gemm_trace
-#else
-constexpr unsigned long long* g_trace = nullptr;
-#endif
-
-struct Plan {
-  int mt, m_tiles, n_tiles, splits, kblocks_per_split;
-};
-
-Plan make_plan(int M, int N, int K) {
-  Plan p;
-  p.mt = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
-  p.m_tiles = ceil_div(M, p.mt);
-  p.n_tiles = ceil_div(N, kTileN);
-  const int kblocks = K / kBlockK;
-  const int tiles = p.m_tiles * p.n_tiles;
-  // Split K when that is cheaper than letting a grid smaller than the GPU walk all of K.  Cost model (us, fitted to
-  // measurements on B200): a CTA spends ~0.45 per K block plus ~2 of fill and drain; a split plan pays the reduce
-  // kernel, ~3 plus its traffic (splits FP32 partials read, fp16 written) at ~4 TB/s.  Measured examples: M = 128
-  // 8960 x 1536 unsplit 17.3 against 22.7 with 2 splits; M = 1024 256 x 1536 6 splits 15.3 against 19.2 unsplit.
-  const int sms = sm_count();
-  const int max_splits = kblocks / 4 > 0 ? kblocks / 4 : 1;  // at least 4 K blocks per split
-  int splits = 1;
+// Batch rows per tile and K splits, by a cost model fitted to measurements on B200 (us, graph of L2-cold calls, deviation
+// about 7 %): a K block of 128 takes 0.45 to dequantise (bf16: 0.55) and 2.3 per 1000 batch rows to multiply, whichever is
+// longer; a tile 0.6 plus 1.0 per 100 batch rows to drain (the last one also to store); 5.5 for launch, set-up and the
+// first block; a split plan 1.8 for the second kernel and its traffic at 5 TB/s.
+Shape make_plan(int M, int N, int K, int group, bool bf16) {
+  Shape best = {};
   double best_cost = 1e30;
-  for (int sp = 1; sp <= max_splits; ++sp) {
-    const int per = ceil_div(kblocks, sp);
-    const int real = ceil_div(kblocks, per);
-    if (real != sp) continue;
-    const int waves = ceil_div(tiles * real, sms);
-    double cost = waves * (0.45 * per + 2.0);
-    if (real > 1) cost += 3.0 + ((double)real * M * N * 4.0 + (double)M * N * 2.0) / 4.0e6;
-    if (cost < best_cost * 0.999) { best_cost = cost; splits = real; }
+  const int kblocks = ceil_div(K, kBlockK), n_tiles = ceil_div(N, kPairRows), pairs = sm_count() / 2;
+  for (int mt = 32; mt <= kMaxTile; mt += 32) {
+    const int m_tiles = ceil_div(M, mt);
+    if (mt > 32 && m_tiles == ceil_div(M, mt - 32)) continue;   // the same tiles, more padding
+    for (int sp = 1; sp <= 16; ++sp) {
+      const int per = ceil_div(ceil_div(kblocks, sp), 2) * 2;
+      const int splits = ceil_div(kblocks, per);
+      if (splits != sp) continue;
+      const long long items = (long long)m_tiles * n_tiles * splits;
+      const double waves = (double)((items + pairs - 1) / pairs);
+      const double unpack = bf16 ? 0.55 : 0.45, multiply = 0.0023 * mt;
+      double cost = 5.5 + waves * ((per < kblocks ? per : kblocks) * (multiply > unpack ? multiply : unpack) + 0.6) + 0.01 * mt;
+      if (splits > 1) cost += 1.8 + (double)splits * M * N * 8.0 / 5.0e6;
+      if (cost < best_cost) {
+        best_cost = cost;
+        best.mt = mt; best.m_tiles = m_tiles; best.n_tiles = n_tiles; best.splits = splits; best.kblocks_per_split = per;
+      }
+    }
   }
-  p.kblocks_per_split = ceil_div(kblocks, splits);
-  p.splits = ceil_div(kblocks, p.kblocks_per_split);  // no empty split
-  return p;
+  best.M = M; best.N = N; best.K = K; best.group = group;
+  return best;
 }
 
-template <int MT, bool kBf16>
-int launch(const Plan& p, const CUtensorMap& tw, const CUtensorMap& tx, const void* scales, const OutSpec& out, float* partial,
-           int M, int N, int K, int group, unsigned int* status, cudaStream_t stream) {
-  using L = Layout<MT>;
-  auto kernel = int4_gemm_kernel<MT, kBf16>;
+template <bool kBf16>
+int launch(const Shape& p, const CUtensorMap& tw, const CUtensorMap& tx, const void* scales, const OutSpec& out, float* partial,
+           unsigned int* status, cudaStream_t stream) {
+  auto kernel = int4_gemm_kernel<kBf16>;
   static bool configured[64] = {false};
   int dev = 0;
   KFB_CUDA_TRY(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    KFB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kAlloc));
+    KFB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
     configured[dev] = true;
   }
-  const dim3 grid(p.n_tiles, p.m_tiles, p.splits);
-  kernel<<<grid, kThreads, L::kAlloc, stream>>>(tw, tx, (const __half*)scales, out, partial, M, N, K, group,
-                                               p.kblocks_per_split, status, g_trace);
+  const long long items = (long long)p.m_tiles * p.n_tiles * p.splits;
+  const long long pairs = items < sm_count() / 2 ? items : sm_count() / 2;
+  kernel<<<dim3((unsigned)(2 * pairs)), kThreads, kSmem, stream>>>(tw, tx, (const __half*)scales, out, partial, p, status);
   KFB_LAUNCH_CHECK("int4_gemm_kernel");
   if (p.splits > 1) {
-    const long long elems = (long long)M * N;
-    long long blocks = (elems + 255) / 256;
+    const bool vec = ((p.N | out.col0) & 3) == 0 && (out.silu ? (out.ld & 1) == 0 : (out.ld & 3) == 0);
+    const long long work = (long long)p.M * p.N / (vec ? 4 : 1);
+    long long blocks = (work + 255) / 256;
     const long long cap = (long long)sm_count() * 8;
     if (blocks > cap) blocks = cap;
-    splitk_reduce_kernel<<<(int)blocks, 256, 0, stream>>>(partial, out, M, N, p.splits);
+    if (vec) splitk_reduce_kernel<4><<<(int)blocks, 256, 0, stream>>>(partial, out, p.M, p.N, p.splits);
+    else splitk_reduce_kernel<1><<<(int)blocks, 256, 0, stream>>>(partial, out, p.M, p.N, p.splits);
     KFB_LAUNCH_CHECK("splitk_reduce_kernel");
   }
   return KFB_OK;
@@ -436,10 +631,16 @@ int launch(const Plan& p, const CUtensorMap& tw, const CUtensorMap& tx, const vo
 
 using namespace kfb;
 
-extern "C" size_t kfb_int4_gemm_ws_bytes(int M, int N, int K, int group) {
+size_t kfb::gemm::ws_bytes(int M, int N, int K, int group, bool bf16) {
   if (M < 1 || N < 1 || K < 64 || (group != 64 && group != 128) || K % group) return 0;
-  const gemm::Plan p = gemm::make_plan(M, N, K);
+  const Shape p = make_plan(M, N, K, group, bf16);
   return p.splits > 1 ? (size_t)p.splits * M * N * sizeof(float) : 0;
+}
+
+// (fp16 and bf16 plans may split K differently: enough for both)
+extern "C" size_t kfb_int4_gemm_ws_bytes(int M, int N, int K, int group) {
+  const size_t a = gemm::ws_bytes(M, N, K, group, false), b = gemm::ws_bytes(M, N, K, group, true);
+  return a > b ? a : b;
 }
 
 namespace {
@@ -454,7 +655,8 @@ int gemm_common(const void* x, const void* packed, const void* scales, const gem
   for (int i = 0; i < out.count; ++i)
     if (!out.y[i] || !aligned16(out.y[i])) return fail(KFB_ERR_ALIGNMENT, "output buffers must be non-null and 16-byte aligned");
   if (!aligned16(x) || !aligned16(packed)) return fail(KFB_ERR_ALIGNMENT, "x and packed must be 16-byte aligned");
-  const gemm::Plan p = gemm::make_plan(M, N, K);
+  const gemm::Shape p = gemm::make_plan(M, N, K, group, out.bf16 != 0);
+  if ((long long)p.m_tiles * p.n_tiles * p.splits > 0x7fffffffLL) return fail(KFB_ERR_INVALID, "too many tiles for one launch");
   const size_t need = p.splits > 1 ? (size_t)p.splits * M * N * sizeof(float) : 0;
   if (need > 0 && (!ws || ws_bytes < need))
     return fail(KFB_ERR_WORKSPACE, "int4_gemm needs a %zu-byte workspace for %d K splits, got %zu", need, p.splits, ws_bytes);
@@ -463,59 +665,44 @@ int gemm_common(const void* x, const void* packed, const void* scales, const gem
   if (!status) return fail(KFB_ERR_CUDA, "cannot resolve the device status word");
 
   CUtensorMap tw, tx;
-  // packed int32 [N, K/8] seen as 32-bit elements, box 8 words x 128 rows, no swizzle
-  if (int rc = make_tmap_2d_plain(&tw, packed, /*elem_bytes=*/4, (uint64_t)K / 8, (uint64_t)N, (uint64_t)K / 2, 8, 128)) return rc;
-  // x fp16 [M, K], box 64 k x MT rows, 128-byte swizzle (reuse the 4-D helper with unit outer dims)
+  // packed int32 [N, K/8] as 32-bit elements, box 32 words (two K blocks) x 128 rows, 128-byte swizzle
+  if (int rc = make_tmap_2d_plain(&tw, packed, /*elem_bytes=*/4, (uint64_t)K / 8, (uint64_t)N, (uint64_t)K / 2, 32, gemm::kRows, true)) return rc;
+  // x [M, K], box 64 k x half a tile of rows, 128-byte swizzle (the 4-D helper with unit outer dims)
   const uint64_t xd[4] = {(uint64_t)K, (uint64_t)M, 1, 1};
   const uint64_t xs[3] = {(uint64_t)K * 2, (uint64_t)M * K * 2, (uint64_t)M * K * 2};
-  const uint32_t xb[4] = {64, (uint32_t)p.mt, 1, 1};
+  const uint32_t xb[4] = {64, (uint32_t)(p.mt / 2), 1, 1};
   if (int rc = make_tmap_4d_sw128(&tx, x, out.bf16 ? KFB_BF16 : KFB_F16, xd, xs, xb)) return rc;
 
   cudaStream_t s = (cudaStream_t)stream;
   float* partial = static_cast<float*>(ws);
-  if (out.bf16) {
-    switch (p.mt) {
-      case 16: return gemm::launch<16, true>(p, tw, tx, scales, out, partial, M, N, K, group, status, s);
-      case 32: return gemm::launch<32, true>(p, tw, tx, scales, out, partial, M, N, K, group, status, s);
-      case 64: return gemm::launch<64, true>(p, tw, tx, scales, out, partial, M, N, K, group, status, s);
-      case 128: return gemm::launch<128, true>(p, tw, tx, scales, out, partial, M, N, K, group, status, s);
-      default: return gemm::launch<256, true>(p, tw, tx, scales, out, partial, M, N, K, group, status, s);
-    }
-  }
-  switch (p.mt) {
-    case 16: return gemm::launch<16, false>(p, tw, tx, scales, out, partial, M, N, K, group, status, s);
-    case 32: return gemm::launch<32, false>(p, tw, tx, scales, out, partial, M, N, K, group, status, s);
-    case 64: return gemm::launch<64, false>(p, tw, tx, scales, out, partial, M, N, K, group, status, s);
-    case 128: return gemm::launch<128, false>(p, tw, tx, scales, out, partial, M, N, K, group, status, s);
-    default: return gemm::launch<256, false>(p, tw, tx, scales, out, partial, M, N, K, group, status, s);
-  }
+  return out.bf16 ? gemm::launch<true>(p, tw, tx, scales, out, partial, status, s) : gemm::launch<false>(p, tw, tx, scales, out, partial, status, s);
 }
 
 }  // namespace
 
-size_t kfb::gemm::ws_bytes(int M, int N, int K, int group) { return kfb_int4_gemm_ws_bytes(M, N, K, group); }
-
 int kfb::gemm::run(const void* x, const void* packed, const void* scales, const void* bias, void* y, int M, int N, int K, int group,
-                   bool bf16, void* ws, size_t ws_bytes, cudaStream_t stream) {
+                   bool bf16, bool silu, void* ws, size_t ws_bytes, cudaStream_t stream) {
+  if (silu && (bf16 || N % 4)) return fail(KFB_ERR_UNSUPPORTED, "the SiLU-pair epilogue is fp16 and needs N %% 4 == 0, got N=%d", N);
   OutSpec out = {};
   out.y[0] = static_cast<__half*>(y);
   out.count = 1;
-  out.ld = N;
+  out.ld = silu ? N / 2 : N;
   out.bf16 = bf16;
   out.bias = static_cast<const uint16_t*>(bias);
+  out.silu = silu;
   return gemm_common(x, packed, scales, out, M, N, K, group, ws, ws_bytes, stream);
 }
 
 extern "C" int kfb_int4_gemm(const void* x, const void* packed, const void* scales, void* y, int M, int N, int K,
                              int group, void* ws, size_t ws_bytes, void* stream) {
   if (!y) return fail(KFB_ERR_INVALID, "null pointer");
-  return gemm::run(x, packed, scales, nullptr, y, M, N, K, group, false, ws, ws_bytes, (cudaStream_t)stream);
+  return gemm::run(x, packed, scales, nullptr, y, M, N, K, group, false, false, ws, ws_bytes, (cudaStream_t)stream);
 }
 
 extern "C" int kfb_int4_gemm_bf16(const void* x, const void* packed, const void* scales, void* y, int M, int N, int K,
                                   int group, void* ws, size_t ws_bytes, void* stream) {
   if (!y) return fail(KFB_ERR_INVALID, "null pointer");
-  return gemm::run(x, packed, scales, nullptr, y, M, N, K, group, true, ws, ws_bytes, (cudaStream_t)stream);
+  return gemm::run(x, packed, scales, nullptr, y, M, N, K, group, true, false, ws, ws_bytes, (cudaStream_t)stream);
 }
 
 extern "C" int kfb_int4_gemm_allgather(const void* x, const void* packed, const void* scales, void* const* y_all,
@@ -533,11 +720,3 @@ extern "C" int kfb_int4_gemm_allgather(const void* x, const void* packed, const 
   out.col0 = col0;
   return gemm_common(x, packed, scales, out, M, N_local, K, group, ws, ws_bytes, stream);
 }
-
-#ifdef KFB_TRACE
-// Tuning aid of -DKFB_TRACE builds (not part of the public header): device buffer of 64 x 8 clock stamps written by
-// CTA (0,0,0).
-extern "C" void kfb_debug_set_gemm_trace(void* device_buffer) {
-  kfb::gemm::g_trace = static_cast<unsigned long long*>(device_buffer);
-}
-#endif

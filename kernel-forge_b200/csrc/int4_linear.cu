@@ -17,21 +17,33 @@ enum class Route { kGemv, kStream, kSmall, kGemm };
 // Where the lines lie (graph of L2-cold calls, us):
 //   M = 1: GEMV / small-batch kernel 5632x2048 4.1/4.7, 1536x8960 5.2/6.2, 2560x2048 3.7/3.7, but 8960x1536 5.0/4.8,
 //     11264x2048 8.0/7.3: the GEMV's four or eight rows per warp leave it too few warps there.
-//   M = 32: small-batch kernel / GEMM 5632x2048 11.7/14.5, 2048x5632 8.7/11.9, 1536x8960 11.5/12.8, 8960x1536 10.7/16.0,
-//     11264x2048 17.4/17.9; the kernel's activation reads grow with M * N, the GEMM's time hardly with M.
+//   M = 32: small-batch kernel / GEMM 2048x5632 8.7/12.3, 1536x8960 11.5/13.5, 8960x1536 10.7/11.6, 5632x2048 11.7/11.4,
+//     11264x2048 17.4/13.2; the kernel's activation reads grow with M * N, the GEMM's time hardly with M.
 Route route(int M, int N, int K, int dtype, bool bias) {
   const bool fp16 = dtype == KFB_F16;
   if (fp16 && N >= 75776 && !bias && M <= 16) return M <= 8 ? Route::kGemv : Route::kStream;
   if (fp16 && M == 1 && N < 8192) return Route::kGemv;
-  if (M <= 16 || (M <= 32 && (long long)N * K <= 24LL << 20)) return Route::kSmall;
+  if (M <= 16 || (M <= 32 && (long long)N * K <= 16LL << 20)) return Route::kSmall;
   return Route::kGemm;
 }
 
 }  // namespace
 
 extern "C" size_t kfb_int4_linear_ws_bytes(int M, int N, int K, int group, int dtype) {
-  return M <= 16 ? 0 : route(M, N, K, dtype, false) == Route::kGemm ? gemm::ws_bytes(M, N, K, group) : 0;
+  return M <= 16 ? 0 : route(M, N, K, dtype, false) == Route::kGemm ? gemm::ws_bytes(M, N, K, group, dtype == KFB_BF16) : 0;
 }
+
+namespace {
+
+int check_small(const void* x, const void* packed, int N, int K, int group) {
+  if (int rc = require_sm100()) return rc;
+  if (group != 64 && group != 128) return fail(KFB_ERR_INVALID, "group_size must be one of (64, 128), got %d", group);
+  if (N < 1 || K < group || K % group) return fail(KFB_ERR_INVALID, "K=%d is not a multiple of group_size=%d", K, group);
+  if (!aligned16(x) || !aligned16(packed)) return fail(KFB_ERR_ALIGNMENT, "x and packed must be 16-byte aligned");
+  return KFB_OK;
+}
+
+}  // namespace
 
 extern "C" int kfb_int4_linear(const void* x, const void* packed, const void* scales, const void* bias, void* y, int M, int N,
                                int K, int group, int dtype, void* ws, size_t ws_bytes, void* stream) {
@@ -44,15 +56,25 @@ extern "C" int kfb_int4_linear(const void* x, const void* packed, const void* sc
       return kfb_int4_gemv(x, packed, scales, y, M, N, K, group, 0, stream);
     case Route::kStream: return kfb_int4_small_batch(x, packed, scales, y, M, N, K, group, 0, stream);
     case Route::kSmall: {
-      if (int rc = require_sm100()) return rc;
-      if (group != 64 && group != 128) return fail(KFB_ERR_INVALID, "group_size must be one of (64, 128), got %d", group);
-      if (N < 1 || K < group || K % group) return fail(KFB_ERR_INVALID, "K=%d is not a multiple of group_size=%d", K, group);
-      if (!aligned16(x) || !aligned16(packed)) return fail(KFB_ERR_ALIGNMENT, "x and packed must be 16-byte aligned");
+      if (int rc = check_small(x, packed, N, K, group)) return rc;
       gemv::Fusion fu = {};
       fu.bias = static_cast<const __half*>(bias);
       return small::run(x, packed, scales, y, M, N, K, group, dtype == KFB_BF16, /*weights_first=*/pdl_enabled(), pdl_enabled(),
                         (cudaStream_t)stream, fu);
     }
-    default: return gemm::run(x, packed, scales, bias, y, M, N, K, group, dtype == KFB_BF16, ws, ws_bytes, (cudaStream_t)stream);
+    default: return gemm::run(x, packed, scales, bias, y, M, N, K, group, dtype == KFB_BF16, false, ws, ws_bytes, (cudaStream_t)stream);
   }
+}
+
+extern "C" int kfb_int4_linear_silu_pairs(const void* x, const void* packed, const void* scales, void* act, int M, int N, int K, int group,
+                                          void* ws, size_t ws_bytes, void* stream) {
+  if (!x || !packed || !scales || !act) return fail(KFB_ERR_INVALID, "null pointer");
+  if (M < 1 || N < 4 || N % 4) return fail(KFB_ERR_INVALID, "int4_linear_silu_pairs needs M >= 1 and N a multiple of 4, got M=%d N=%d", M, N);
+  const Route r = route(M, N, K, KFB_F16, true);
+  if (r == Route::kGemm) return gemm::run(x, packed, scales, nullptr, act, M, N, K, group, false, true, ws, ws_bytes, (cudaStream_t)stream);
+  if (r == Route::kGemv) return kfb_int4_gemv_silu_pair(x, packed, scales, act, M, N, K, group, 0, nullptr, 0.0f, 0, stream);
+  if (int rc = check_small(x, packed, N, K, group)) return rc;
+  gemv::Fusion fu = {};
+  fu.epi = gemv::kEpiSiluPair;
+  return small::run(x, packed, scales, act, M, N, K, group, false, /*weights_first=*/pdl_enabled(), pdl_enabled(), (cudaStream_t)stream, fu);
 }

@@ -47,6 +47,7 @@ _SIGNATURES = {
     "kfb_int4_linear_ws_bytes": (c_size_t, [c_int, c_int, c_int, c_int, c_int]),
     "kfb_int4_linear": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p,
                                 c_size_t, c_void_p]),
+    "kfb_int4_linear_silu_pairs": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]),
     "kfb_int4_gemv": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p]),
     "kfb_int4_gemv_fused": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_float,
                                     c_void_p, c_void_p, c_int, c_void_p]),

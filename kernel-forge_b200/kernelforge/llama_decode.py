@@ -280,7 +280,7 @@ class LlamaInt4Decoder:
         if t >= self.max_len:
             raise ValueError(f"prompt of {t} tokens leaves no room in a cache of {self.max_len} rows for a decode step")
         nq, rows = self.h_loc * s.head_dim, b * t
-        # nine kernels per layer and no copy in between: activations stay token-major [B * T, features], RoPE writes the
+        # eight or nine kernels per layer (SiLU * up sits in the epilogue of the gate / up projection when its rows are paired) and no copy in between: activations stay token-major [B * T, features], RoPE writes the
         # cache and undoes the pair order of the rows, attention reads the cache in place
         h, x = ops.embed_rmsnorm(ids.to(self.dev, torch.long).reshape(rows).contiguous(), self.embed, self.layers[0]["in_norm"], s.rms_eps)
         res = None
@@ -292,7 +292,11 @@ class LlamaInt4Decoder:
             a = ops.attention_tokens(q, k_cache, v_cache, t, True).view(rows, nq)
             o = self._gather(L["o"](self._gather(a, "attn_bounds")), "hidden_bounds")
             h, x = ops.add_rmsnorm(x, L["post_norm"], s.rms_eps, o)
-            act = self._gather(ops.silu_mul(L["gate_up"](h), self.pair_rows), "inter_bounds")
+            if self.pair_rows:
+                act = ops.int4_linear_silu_pairs(h, L["gate_up"].packed, L["gate_up"].scales, L["gate_up"].group)
+            else:
+                act = ops.silu_mul(L["gate_up"](h))
+            act = self._gather(act, "inter_bounds")
             res = self._gather(L["down"](act), "hidden_bounds")
         h, x = ops.add_rmsnorm(x, self.final_norm, s.rms_eps, res)
         logits = (h @ self.lm_head.T).view(b, t, s.vocab)

@@ -571,6 +571,15 @@ def int4_linear(x: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, gro
     return y.reshape(*lead, packed.shape[0])
 
 
+def int4_linear_silu_pairs(x: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, group_size: int = 128) -> torch.Tensor:
+    """act[..., N/2] = silu(gate . x) * (up . x) for a weight whose rows were interleaved with interleave_gate_up, any number
+    of rows of x: int4_linear and silu_mul(pairs=True) in one launch."""
+    act = _capi.host().int4_linear(x, packed, scales, group_size, "silu_pairs")
+    if act is None:
+        return silu_mul(int4_linear(x, packed, scales, group_size), pairs=True)
+    return act
+
+
 # ---------------------------------------------------------------------------
 # Fused element-wise steps of a decode step (not part of the reference's operator surface, which leaves
 # them to torch; used by kernelforge.llama_decode)

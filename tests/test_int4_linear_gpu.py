@@ -44,3 +44,28 @@ def test_small_batches(m, n, k, group, dtype):
 @pytest.mark.parametrize("m,n,k", [(1, 77, 256), (5, 1001, 256), (16, 192, 512), (33, 136, 256), (200, 72, 256), (64, 256, 4096)])
 def test_bias_in_the_epilogue(m, n, k, dtype):
     check(m, n, k, 128, dtype, True)
+
+
+# (M, N, K): tiles with remainders in every direction, one and several batch tiles, odd N (2-byte stores), a last half K
+# block of 64 (group 64), split K, two accumulators in flight (tiles of <= 128 batch rows) and one
+LARGE = [(33, 64, 128), (33, 257, 1024), (64, 1536, 4224), (96, 511, 640), (129, 130, 256), (257, 300, 2048), (300, 4096, 256),
+         (520, 1025, 704), (700, 2304, 1088), (2100, 512, 384)]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m,n,k", LARGE)
+def test_gemm_tiles(m, n, k, dtype):
+    check(m, n, k, 64, dtype, m % 2 == 0)
+    if k % 128 == 0:
+        check(m, n, k, 128, dtype, m % 2 == 1)
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 64, 256), (1, 11264, 256), (5, 36, 256), (31, 260, 512), (33, 132, 256), (70, 300, 4096), (300, 1028, 512)])
+def test_silu_pairs_epilogue(m, n, k):
+    _, x, packed, scales, _ = int4_case(m, n, k, 128, seed=n)
+    args = tuple(torch.from_numpy(a).cuda() for a in (x, packed, scales))
+    got = ops.int4_linear_silu_pairs(*args, 128)
+    gate, up = ops.int4_linear(*args, 128).view(m, n // 2, 2).unbind(-1)
+    want = torch.nn.functional.silu(gate) * up
+    assert got.shape == want.shape
+    assert (got.float() - want.float()).abs().max() <= 3e-3 * want.float().abs().max()
