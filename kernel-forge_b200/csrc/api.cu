@@ -249,7 +249,7 @@ namespace kfb {
 namespace {
 std::atomic<int> g_pdl{0};
 }
-bool pdl_enabled() { return g_pdl.load(std::memory_order_relaxed) != 0; }
+bool constants_are_old() { return g_pdl.load(std::memory_order_relaxed) != 0; }
 }  // namespace kfb
 
 extern "C" int kfb_set_programmatic_launch(int enable) { return kfb::g_pdl.exchange(enable ? 1 : 0); }

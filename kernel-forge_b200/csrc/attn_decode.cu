@@ -127,13 +127,6 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   const int b = blockIdx.z;
   const int h0 = hk * G + chunk * kRows;               // first query head of this CTA
   const int rows = min(kRows, G - chunk * kRows);      // real query heads
-  const int key_begin = split * keys_per_split;
-  // a static KV cache holds Nk rows of which only kv_len[b] are valid (read on the device, so the
-  // same launch can be replayed from a CUDA graph while the cache fills up)
-  const int valid = kv_len ? min(Nk, max(kv_len[b], 0)) : Nk;
-  const int key_end = min(valid, key_begin + keys_per_split);
-  const int n_tiles = key_end > key_begin ? (key_end - key_begin + kTileKeys - 1) / kTileKeys : 0;
-
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&full[s], 1);
@@ -143,8 +136,15 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     fence_mbar_init();
   }
   __syncthreads();
-  pdl_wait();               // q, the cache rows and kv_len may be the output of the kernel in front
+  pdl_wait(q, kv_len);      // q, the cache rows and kv_len may be the output of the kernel in front
   pdl_launch_dependents();
+  const int key_begin = split * keys_per_split;
+  // a static KV cache holds Nk rows of which only kv_len[b] are valid (read on the device, so the
+  // same launch can be replayed from a CUDA graph while the cache fills up)
+  const int valid = kv_len ? min(Nk, max(kv_len[b], 0)) : Nk;
+  const int key_end = min(valid, key_begin + keys_per_split);
+  const int n_tiles = key_end > key_begin ? (key_end - key_begin + kTileKeys - 1) / kTileKeys : 0;
+
   if (*abort_word != 0) return;  // uniform: written before the barrier, nothing has been issued yet
 
   float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
@@ -342,7 +342,7 @@ attn_decode_merge_kernel(const float* __restrict__ partial, uint16_t* __restrict
   constexpr int kPer = kRows * (D + 2);
   __shared__ float sm_m[kMergeLanes][D], sm_a[kMergeLanes][D], sm_l[kMergeLanes][D];
   const int h = blockIdx.x, b = blockIdx.y, d = threadIdx.x % D, j = threadIdx.x / D;
-  pdl_wait();
+  pdl_wait(partial);
   pdl_launch_dependents();
   const int G = H / Hk;
   const int chunks = (G + kRows - 1) / kRows;
@@ -436,10 +436,8 @@ int launch_merge_lanes(const float* partial, uint16_t* o, int B, int H, int Hk, 
                        cudaStream_t stream) {
   const dim3 grid(H, B);
   if ((long long)splits * sets >= 8)
-    return launch_kernel("attn_decode_merge_kernel", attn_decode_merge_kernel<D, kBf16, 8>, grid, dim3(D * 8), 0, stream, pdl_enabled(),
-                         partial, o, H, Hk, splits, sets, set_stride);
-  return launch_kernel("attn_decode_merge_kernel", attn_decode_merge_kernel<D, kBf16, 1>, grid, dim3(D), 0, stream, pdl_enabled(),
-                       partial, o, H, Hk, splits, sets, set_stride);
+    return launch_kernel("attn_decode_merge_kernel", attn_decode_merge_kernel<D, kBf16, 8>, grid, dim3(D * 8), 0, stream, partial, o, H, Hk, splits, sets, set_stride);
+  return launch_kernel("attn_decode_merge_kernel", attn_decode_merge_kernel<D, kBf16, 1>, grid, dim3(D), 0, stream, partial, o, H, Hk, splits, sets, set_stride);
 }
 
 template <int D, bool kBf16>
@@ -465,7 +463,7 @@ int launch_stages(const Problem& p, const SplitPlan& plan, const CUtensorMap& tk
     configured[dev] = true;
   }
   const dim3 grid(plan.splits, p.Hk * plan.chunks, p.B);
-  if (int rc = launch_kernel("attn_decode_kernel", kernel, grid, dim3(kThreads), L::kAlloc, stream, pdl_enabled(), tk, tv,
+  if (int rc = launch_kernel("attn_decode_kernel", kernel, grid, dim3(kThreads), L::kAlloc, stream, tk, tv,
                              (const uint16_t*)p.q, (uint16_t*)p.o, partial, p.H, p.Hk, p.Nk, plan.keys_per_split,
                              p.scale * 1.4426950408889634f, status, p.kv_len_dev, partial_only ? 1 : 0))
     return rc;

@@ -239,6 +239,8 @@ attn_prefill_serial_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  pdl_wait();   // every role: from here on memory of the kernel in front is read (and what it reads may be overwritten)
+  pdl_launch_dependents();
   const uint32_t tmem_base = *tmem_slot;
   const bool dead_on_arrival = *abort_word != 0;
 
@@ -602,6 +604,8 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  pdl_wait();   // every role: from here on memory of the kernel in front is read (and what it reads may be overwritten)
+  pdl_launch_dependents();
   const uint32_t tmem_base = *tmem_slot;
   const bool dead_on_arrival = *abort_word != 0;
 #ifdef KFB_TRACE
@@ -934,16 +938,13 @@ int launch(const Problem& p, const CUtensorMap& tq, const CUtensorMap& tk, const
   if (pair_kernel_for(D) && q_tiles >= 2) {
     const int n_pairs = ceil_div(q_tiles, 2);
     if (bh * n_pairs > 0x7fffffffLL) return fail(KFB_ERR_INVALID, "too many query tiles for one launch");
-    pair::attn_prefill_pair_kernel<D, kBf16><<<(unsigned)(bh * n_pairs), pair::kPairThreads, PL::kAlloc, stream>>>(
-        tq, tk, tv, p.o, o_st, p.B, p.H, p.Hk, p.Nq, p.Nk, p.causal, scale_log2, n_pairs, heads_per_group, status);
-    KFB_LAUNCH_CHECK("attn_prefill_pair_kernel");
-    return KFB_OK;
+    return launch_kernel("attn_prefill_pair_kernel", pair::attn_prefill_pair_kernel<D, kBf16>, dim3((unsigned)(bh * n_pairs)),
+                         dim3(pair::kPairThreads), PL::kAlloc, stream, tq, tk, tv, p.o, o_st, p.B, p.H, p.Hk, p.Nq, p.Nk, p.causal, scale_log2,
+                         n_pairs, heads_per_group, status);
   }
   if (bh * q_tiles > 0x7fffffffLL) return fail(KFB_ERR_INVALID, "too many query tiles for one launch");
-  serial::attn_prefill_serial_kernel<D, kBf16><<<(unsigned)(bh * q_tiles), kThreads, L::kAlloc, stream>>>(
-      tq, tk, tv, p.o, o_st, p.H, p.Hk, p.Nq, p.Nk, p.causal, scale_log2, p.B, q_tiles, heads_per_group, status);
-  KFB_LAUNCH_CHECK("attn_prefill_serial_kernel");
-  return KFB_OK;
+  return launch_kernel("attn_prefill_serial_kernel", serial::attn_prefill_serial_kernel<D, kBf16>, dim3((unsigned)(bh * q_tiles)), dim3(kThreads),
+                       L::kAlloc, stream, tq, tk, tv, p.o, o_st, p.H, p.Hk, p.Nq, p.Nk, p.causal, scale_log2, p.B, q_tiles, heads_per_group, status);
 }
 
 }  // namespace

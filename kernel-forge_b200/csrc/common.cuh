@@ -43,22 +43,32 @@ int require_sm100();
                          __FILE__, __LINE__);                                               \
   } while (0)
 
-// Programmatic dependent launch.  A kernel launched with the attribute may become resident while the kernel in front
-// of it in the stream is still running; it must call pdl_wait() before it touches anything that kernel wrote (or
-// still reads), and it releases its own successor with pdl_launch_dependents().  Every kernel of this library that
-// can be part of a decode step waits first and releases its successor right after, so at most two grids overlap and
-// the order of all memory operations is that of the plain stream.  Both instructions are no-ops in a kernel that
-// was launched without the attribute.
+// Programmatic dependent launch: every launch of this library carries the attribute.  Such a kernel may become resident
+// while the kernel in front of it in the stream is still running; it calls pdl_wait() before it touches anything that
+// kernel may have written (or still reads), and releases its own successor with pdl_launch_dependents() after that wait,
+// so at most two grids overlap and the order of all memory operations is that of the plain stream.  It hides launch and
+// set-up behind the predecessor's tail; and between plain launches the hardware was measured to start a kernel only at
+// multiples of 2.05 us after the one in front (a 3.0 us kernel costs 4.1 us, a 4.2 us one 6.1), with the attribute 0.5 us
+// after it.  Both instructions are no-ops without a predecessor.
+// A kernel may read CONSTANTS (weights, scales, norm weights) before its wait only where the caller knows that they are
+// older than the kernel in front: kfb_set_programmatic_launch (constants_are_old() below), used for decode steps.
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// `fresh`: pointers to what the kernel in front may have written.  Their values pass through the asm, so no load through
+// them can be moved above the wait (the compiler may move loads through `const T* __restrict__`, which it takes to be
+// invariant, across any memory clobber), nor become a non-coherent one.
+template <class... P>
+__device__ __forceinline__ void pdl_wait(P&... fresh) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  ((void)([](auto& p) { asm volatile("" : "+l"(p)::"memory"); }(fresh)), ...);
+}
 #endif
-// Whether launches carry the attribute (kfb_set_programmatic_launch; off by default).
-bool pdl_enabled();
+// kfb_set_programmatic_launch: constants may be read before pdl_wait() (off by default).
+bool constants_are_old();
 
 template <class... KArgs, class... Args>
 int launch_kernel(const char* what, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                  bool pdl, Args... args) {
+                  Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -68,7 +78,7 @@ int launch_kernel(const char* what, void (*kernel)(KArgs...), dim3 grid, dim3 bl
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
+  cfg.numAttrs = 1;
   cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
   if (e != cudaSuccess) return fail(KFB_ERR_CUDA, "launch of %s failed: %s", what, cudaGetErrorString(e));
   return KFB_OK;

@@ -30,18 +30,19 @@ constexpr int kRmsMaxVec = 16;  // most 16-byte vectors per thread => hidden <= 
 template <int kMaxVec>
 __global__ void __launch_bounds__(kRmsThreads)
 add_rmsnorm_kernel(const __half* __restrict__ x, const __half* __restrict__ res, const __half* __restrict__ w,
-                   __half* __restrict__ y, __half* __restrict__ sum_out, int hidden, float eps) {
+                   __half* __restrict__ y, __half* __restrict__ sum_out, int hidden, float eps, int early) {
   __shared__ float warp_part[kRmsThreads / 32];
   const int nvec = hidden / 8;
   // The norm weight is a constant of the model (and cold in HBM: every layer has its own): it is requested before the
   // wait for the kernel in front, so its round trip overlaps that kernel's tail instead of following the reduction.
+  if (!early) pdl_wait(x, res, w);   // unless it may have been written by that kernel
   uint4 wreg[kMaxVec];
 #pragma unroll
   for (int i = 0; i < kMaxVec; ++i) {
     const int v = threadIdx.x + i * kRmsThreads;
     if (v < nvec) wreg[i] = reinterpret_cast<const uint4*>(w)[v];
   }
-  pdl_wait();
+  pdl_wait(x, res);
   pdl_launch_dependents();
   const size_t base = (size_t)blockIdx.x * hidden;
   __half2 vals[kMaxVec][4];
@@ -99,7 +100,7 @@ __global__ void rope_kv_write_kernel(const __half* __restrict__ qkv, const float
                                      __half* __restrict__ q_out, __half* __restrict__ k_cache, __half* __restrict__ v_cache,
                                      int H, int Hk, int D, int Lmax, unsigned int* status) {
   const int head = blockIdx.x, b = blockIdx.y, d = threadIdx.x, half = D / 2;
-  pdl_wait();
+  pdl_wait(qkv, pos_ptr, cos_t, sin_t);
   pdl_launch_dependents();
   const long long pos = pos_ptr[0];
   // The position comes from device memory (a graph replay advances it), so it is checked here: a position outside
@@ -131,7 +132,7 @@ __global__ void rope_kv_write_kernel(const __half* __restrict__ qkv, const float
 // gu: [rows, 2 * inter] (gate | up) -> out [rows, inter]
 __global__ void __launch_bounds__(256) silu_mul_kernel(const __half* __restrict__ gu, __half* __restrict__ out, int rows, int inter) {
   const int per_row = inter / 2;  // half2 per row
-  pdl_wait();
+  pdl_wait(gu);
   pdl_launch_dependents();
   const long long total = (long long)rows * per_row;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -152,6 +153,8 @@ __device__ __forceinline__ __half silu_times(__half2 gate_up) {
 
 // gu: gate and up of a feature side by side (the row order of int4_gemv_silu_pair), `total` features in all
 __global__ void __launch_bounds__(256) silu_mul_pairs_kernel(const __half2* __restrict__ gu, __half* __restrict__ out, long long total) {
+  pdl_wait(gu);
+  pdl_launch_dependents();
   const long long step = (long long)gridDim.x * blockDim.x, first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   for (long long i = first; i < total / 4; i += step) {
     const uint4 v = reinterpret_cast<const uint4*>(gu)[i];
@@ -172,6 +175,8 @@ __global__ void __launch_bounds__(256)
 rope_tokens_kernel(const __half* __restrict__ qkv, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                    __half* __restrict__ q_out, __half* __restrict__ k_cache, __half* __restrict__ v_cache, int T, int H, int Hk,
                    int D, int Lmax, long long items) {
+  pdl_wait(qkv, cos_t, sin_t);
+  pdl_launch_dependents();
   const int per_head = D / 8, heads = H + 2 * Hk, per_token = heads * per_head, half = D / 2;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < items; i += (long long)gridDim.x * blockDim.x) {
     const long long token = i / per_token;
@@ -239,8 +244,8 @@ extern "C" int kfb_add_rmsnorm(const void* x, const void* residual, const void* 
   auto kernel = per_thread == 1 ? fused::add_rmsnorm_kernel<1> : per_thread == 2 ? fused::add_rmsnorm_kernel<2>
                 : per_thread <= 4 ? fused::add_rmsnorm_kernel<4> : fused::add_rmsnorm_kernel<fused::kRmsMaxVec>;
   return launch_kernel("add_rmsnorm_kernel", kernel, dim3(rows), dim3(fused::kRmsThreads), 0,
-                       (cudaStream_t)stream, pdl_enabled(), (const __half*)x, (const __half*)residual, (const __half*)weight,
-                       (__half*)y, (__half*)sum_out, hidden, eps);
+                       (cudaStream_t)stream, (const __half*)x, (const __half*)residual, (const __half*)weight,
+                       (__half*)y, (__half*)sum_out, hidden, eps, (int)constants_are_old());
 }
 
 extern "C" int kfb_rope_kv_write(const void* qkv, const void* cos_table, const void* sin_table, const void* pos_dev,
@@ -253,7 +258,7 @@ extern "C" int kfb_rope_kv_write(const void* qkv, const void* cos_table, const v
   unsigned int* status = device_status_word();
   if (!status) return fail(KFB_ERR_CUDA, "cannot resolve the device status word");
   return launch_kernel("rope_kv_write_kernel", fused::rope_kv_write_kernel, dim3(H + 2 * Hk, B), dim3(D / 2), 0,
-                       (cudaStream_t)stream, pdl_enabled(), (const __half*)qkv, (const float*)cos_table,
+                       (cudaStream_t)stream, (const __half*)qkv, (const float*)cos_table,
                        (const float*)sin_table, (const long long*)pos_dev, (__half*)q_out, (__half*)k_cache,
                        (__half*)v_cache, H, Hk, D, Lmax, status);
 }
@@ -268,7 +273,7 @@ extern "C" int kfb_silu_mul(const void* gate_up, void* out, int rows, int inter,
   const long long cap = (long long)sm_count() * 8;
   if (blocks > cap) blocks = cap;
   return launch_kernel("silu_mul_kernel", fused::silu_mul_kernel, dim3((int)blocks), dim3(256), 0, (cudaStream_t)stream,
-                       pdl_enabled(), (const __half*)gate_up, (__half*)out, rows, inter);
+                       (const __half*)gate_up, (__half*)out, rows, inter);
 }
 
 extern "C" int kfb_silu_mul_pairs(const void* gate_up, void* out, int rows, int inter, void* stream) {
@@ -277,9 +282,8 @@ extern "C" int kfb_silu_mul_pairs(const void* gate_up, void* out, int rows, int 
   if (!gate_up || !out) return fail(KFB_ERR_INVALID, "null pointer");
   if (!aligned16(gate_up) || !aligned16(out)) return fail(KFB_ERR_ALIGNMENT, "pointers must be 16-byte aligned");
   const long long total = (long long)rows * inter;
-  fused::silu_mul_pairs_kernel<<<fused::blocks_for((total + 3) / 4), 256, 0, (cudaStream_t)stream>>>((const __half2*)gate_up, (__half*)out, total);
-  KFB_LAUNCH_CHECK("silu_mul_pairs_kernel");
-  return KFB_OK;
+  return launch_kernel("silu_mul_pairs_kernel", fused::silu_mul_pairs_kernel, dim3(fused::blocks_for((total + 3) / 4)), dim3(256), 0,
+                       (cudaStream_t)stream, (const __half2*)gate_up, (__half*)out, total);
 }
 
 extern "C" int kfb_rope_tokens(const void* qkv, const void* cos_table, const void* sin_table, void* q_out, void* k_cache,
@@ -292,8 +296,6 @@ extern "C" int kfb_rope_tokens(const void* qkv, const void* cos_table, const voi
     return fail(KFB_ERR_ALIGNMENT, "pointers must be 16-byte aligned");
   const long long items = (long long)B * T * (H + 2 * Hk) * (D / 8);
   auto kernel = pairs ? fused::rope_tokens_kernel<true> : fused::rope_tokens_kernel<false>;
-  kernel<<<fused::blocks_for(items), 256, 0, (cudaStream_t)stream>>>((const __half*)qkv, (const float*)cos_table, (const float*)sin_table,
-                                                                     (__half*)q_out, (__half*)k_cache, (__half*)v_cache, T, H, Hk, D, Lmax, items);
-  KFB_LAUNCH_CHECK("rope_tokens_kernel");
-  return KFB_OK;
+  return launch_kernel("rope_tokens_kernel", kernel, dim3(fused::blocks_for(items)), dim3(256), 0, (cudaStream_t)stream, (const __half*)qkv,
+                       (const float*)cos_table, (const float*)sin_table, (__half*)q_out, (__half*)k_cache, (__half*)v_cache, T, H, Hk, D, Lmax, items);
 }

@@ -34,6 +34,7 @@ struct Fusion {
   const __half* bias;      // [N] or nullptr
   const __half* residual;  // [M, N] or nullptr
   int epi;                 // Epilogue
+  int early;               // weights and scales may be read before pdl_wait()
   RopeKv rope;
 };
 

@@ -13,54 +13,81 @@ namespace {
 // positions 0..7 hold offsets 0,2,4,6,1,3,5,7 (kernelforge/quantize.py:34).
 __device__ __forceinline__ int nibble_pos(int o) { return (o >> 1) + ((o & 1) << 2); }
 
-template <typename T>
-__device__ __forceinline__ float to_f32(T v);
-template <>
-__device__ __forceinline__ float to_f32<float>(float v) { return v; }
-template <>
-__device__ __forceinline__ float to_f32<__half>(__half v) { return __half2float(v); }
-template <>
-__device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
+// The 8 weights of one packed word as FP32.
+__device__ __forceinline__ void load8(const float* w, float (&v)[8]) {
+  const float4 a = __ldcs(reinterpret_cast<const float4*>(w)), b = __ldcs(reinterpret_cast<const float4*>(w) + 1);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+__device__ __forceinline__ void load8(const __half* w, float (&v)[8]) {
+  const uint4 a = __ldcs(reinterpret_cast<const uint4*>(w));
+  const __half2* h = reinterpret_cast<const __half2*>(&a);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) { const float2 f = __half22float2(h[i]); v[2 * i] = f.x; v[2 * i + 1] = f.y; }
+}
+__device__ __forceinline__ void load8(const __nv_bfloat16* w, float (&v)[8]) {
+  const uint4 a = __ldcs(reinterpret_cast<const uint4*>(w));
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&a);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(h[i]); v[2 * i] = f.x; v[2 * i + 1] = f.y; }
+}
 
-// One warp quantises 128 consecutive k of one row per step: lane l owns k = 4l .. 4l+3.
-// For G = 128 the warp is one group; for G = 64 each half-warp is one group.
-// Grid-stride over the N * K/128 warp-steps.
+// clamp(rint(v / s), -8, 7) + 8 with the quotient rounded to FP32 first, as the definition says.
+__device__ __noinline__ uint32_t quotient_exact(float v, float s) {
+  return (uint32_t)((int)fminf(fmaxf(rintf(__fdiv_rn(v, s)), -8.0f), 7.0f) + 8);
+}
+
+// One lane per packed word (8 consecutive k); G / 8 neighbouring lanes share a group.  Words and groups are contiguous
+// over the whole tensor, so the grid walks flat word indices and knows no rows.
+//
+// HBM-bound (2.5 bytes per fp16 weight).  What kept it from that was one IEEE division per weight (a dozen instructions)
+// and 8-byte loads: 11264 x 2048 fp16 42.8 us.  Now a weight is multiplied with the group's reciprocal, which is off by at
+// most 2e-6 for quotients below 8, and only where that could change the rounding (within 1e-5 of a half integer; or a
+// quotient outside +-7.4, infinity, NaN) is the division done.
 template <typename T, int G>
-__global__ void __launch_bounds__(256) quantize_pack_kernel(const T* __restrict__ w, int32_t* __restrict__ packed,
-                                                            __half* __restrict__ scales, int N, int K) {
+__global__ void __launch_bounds__(256) quantize_pack_kernel(const T* __restrict__ w, uint32_t* __restrict__ packed,
+                                                            __half* __restrict__ scales, long long words) {
+  constexpr int kLanes = G / 8, kUnroll = sizeof(T) == 4 ? 2 : 4;
+  pdl_wait(w);   // (the successor is not released early: it may read these weights before its own wait)
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  // (the loop runs by warps; a group's lanes all have a word or none, since `words` is a multiple of kLanes)
   const int lane = threadIdx.x & 31;
-  const long long steps_per_row = (K + 127) / 128;  // K % 128 == 64 is possible when G = 64
-  const long long total = (long long)N * steps_per_row;
-  const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-  for (long long step = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); step < total; step += warps) {
-    const long long row = step / steps_per_row;
-    const int k0 = (int)(step - row * steps_per_row) * 128;
-    const bool live = k0 + 4 * lane < K;  // a whole group is live or not (G divides K)
-    const T* src = w + row * K + k0 + 4 * lane;
-    float v[4];
+  for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; i0 - lane < words; i0 += kUnroll * stride) {
+    float v[kUnroll][8];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = live ? to_f32<T>(src[i]) : 0.0f;
-    float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
-    constexpr int kWidth = G / 4;  // lanes per group: 32 or 16
+    for (int u = 0; u < kUnroll; ++u)
+      if (i0 + u * stride < words) load8(w + (i0 + u * stride) * 8, v[u]);
 #pragma unroll
-    for (int off = kWidth / 2; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-    // scale = fp16(max(absmax / 7, smallest normal fp16)); exactly 1 for an all-zero group
-    float s = fmaxf(__fdiv_rn(amax, 7.0f), 6.103515625e-05f);
-    __half sh = __float2half_rn(s);
-    if (amax == 0.0f) sh = __float2half_rn(1.0f);
-    const float s32 = __half2float(sh);
-    uint32_t word = 0;
+    for (int u = 0; u < kUnroll; ++u) {
+      const long long i = i0 + u * stride;
+      const bool live = i < words;
+      float amax = 0.0f;
+      if (!live) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float q = rintf(__fdiv_rn(v[i], s32));
-      q = fminf(fmaxf(q, -8.0f), 7.0f);
-      const uint32_t u = (uint32_t)((int)q + 8) & 0xFu;
-      const int o = (lane & 1) * 4 + i;  // k offset inside the 8-weight word
-      word |= u << (4 * nibble_pos(o));
+        for (int j = 0; j < 8; ++j) v[u][j] = 0.0f;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(v[u][j]));
+#pragma unroll
+      for (int off = kLanes / 2; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+      // scale = fp16(max(absmax / 7, smallest normal fp16)); exactly 1 for an all-zero group
+      __half sh = __float2half_rn(fmaxf(__fdiv_rn(amax, 7.0f), 6.103515625e-05f));
+      if (amax == 0.0f) sh = __float2half_rn(1.0f);
+      const float s32 = __half2float(sh), inv = __fdiv_rn(1.0f, s32);
+      uint32_t word = 0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float r = v[u][j] * inv;
+        const float t = r + 12582920.0f;                 // 1.5 * 2^23 + 8: the low bits are rint(r) + 8 (ties to even)
+        const float frac = fabsf(r - (t - 12582920.0f));
+        uint32_t q = __float_as_uint(t) & 0xFu;
+        if (!(frac < 0.49999f && fabsf(r) < 7.4f)) q = quotient_exact(v[u][j], s32);
+        word |= q << (4 * nibble_pos(j));
+      }
+      if (live) {
+        packed[i] = word;
+        if ((lane & (kLanes - 1)) == 0) scales[i / kLanes] = sh;
+      }
     }
-    word |= __shfl_xor_sync(0xffffffffu, word, 1);
-    if (live && (lane & 1) == 0) packed[row * (K / 8) + k0 / 8 + (lane >> 1)] = (int32_t)word;
-    if (live && (lane & (kWidth - 1)) == 0) scales[row * (K / G) + k0 / G + lane / kWidth] = sh;
   }
 }
 
@@ -151,16 +178,16 @@ extern "C" int kfb_quantize_pack(const void* w, int w_dtype, int N, int K, int g
   if (!w || !packed || !scales) return fail(KFB_ERR_INVALID, "null pointer");
   if (!aligned16(w) || !aligned16(packed)) return fail(KFB_ERR_ALIGNMENT, "w and packed must be 16-byte aligned");
   cudaStream_t s = (cudaStream_t)stream;
-  const long long steps = (long long)N * ((K + 127) / 128);
-  const int grid = grid_for(steps, 8);
-#define KFB_Q(T, G) quantize_pack_kernel<T, G><<<grid, 256, 0, s>>>((const T*)w, (int32_t*)packed, (__half*)scales, N, K)
+  const long long words = (long long)N * (K / 8);
+  const int grid = grid_for(words, 256 * 2);
+#define KFB_Q(T, G)                                                                                                            \
+  return launch_kernel("quantize_pack_kernel", quantize_pack_kernel<T, G>, dim3(grid), dim3(256), 0, s, (const T*)w, (uint32_t*)packed, \
+                       (__half*)scales, words)
   if (w_dtype == KFB_F32) { if (group == 128) KFB_Q(float, 128); else KFB_Q(float, 64); }
-  else if (w_dtype == KFB_F16) { if (group == 128) KFB_Q(__half, 128); else KFB_Q(__half, 64); }
-  else if (w_dtype == KFB_BF16) { if (group == 128) KFB_Q(__nv_bfloat16, 128); else KFB_Q(__nv_bfloat16, 64); }
-  else return fail(KFB_ERR_INVALID, "w_dtype must be KFB_F16, KFB_BF16 or KFB_F32");
+  if (w_dtype == KFB_F16) { if (group == 128) KFB_Q(__half, 128); else KFB_Q(__half, 64); }
+  if (w_dtype == KFB_BF16) { if (group == 128) KFB_Q(__nv_bfloat16, 128); else KFB_Q(__nv_bfloat16, 64); }
 #undef KFB_Q
-  KFB_LAUNCH_CHECK("quantize_pack_kernel");
-  return KFB_OK;
+  return fail(KFB_ERR_INVALID, "w_dtype must be KFB_F16, KFB_BF16 or KFB_F32");
 }
 
 extern "C" int kfb_unpack_int4(const void* packed, int N, int K, void* q_out, void* stream) {

@@ -280,6 +280,8 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   }
   cluster_arrive();
   tc_fence_after_sync();
+  pdl_wait(scales);   // every role: from here on memory of the kernel in front is read (and what it reads may be overwritten)
+  pdl_launch_dependents();
   const uint32_t tmem_base = *tmem_slot;   // (not used by the producer, which has not waited for it)
 
   if (warp >= kProducerWarp) {
@@ -532,6 +534,8 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
 template <int V>
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restrict__ partial, const __grid_constant__ OutSpec out,
                                                             int M, int N, int splits) {
+  pdl_wait(partial);
+  pdl_launch_dependents();
   const long long elems = (long long)M * N, vecs = elems / V;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < vecs; i += (long long)gridDim.x * blockDim.x) {
     float acc[V];
@@ -610,17 +614,17 @@ int launch(const Shape& p, const CUtensorMap& tw, const CUtensorMap& tx, const v
   }
   const long long items = (long long)p.m_tiles * p.n_tiles * p.splits;
   const long long pairs = items < sm_count() / 2 ? items : sm_count() / 2;
-  kernel<<<dim3((unsigned)(2 * pairs)), kThreads, kSmem, stream>>>(tw, tx, (const __half*)scales, out, partial, p, status);
-  KFB_LAUNCH_CHECK("int4_gemm_kernel");
+  if (int rc = launch_kernel("int4_gemm_kernel", kernel, dim3((unsigned)(2 * pairs)), dim3(kThreads), kSmem, stream, tw, tx, (const __half*)scales,
+                             out, partial, p, status))
+    return rc;
   if (p.splits > 1) {
     const bool vec = ((p.N | out.col0) & 3) == 0 && (out.silu ? (out.ld & 1) == 0 : (out.ld & 3) == 0);
     const long long work = (long long)p.M * p.N / (vec ? 4 : 1);
     long long blocks = (work + 255) / 256;
     const long long cap = (long long)sm_count() * 8;
     if (blocks > cap) blocks = cap;
-    if (vec) splitk_reduce_kernel<4><<<(int)blocks, 256, 0, stream>>>(partial, out, p.M, p.N, p.splits);
-    else splitk_reduce_kernel<1><<<(int)blocks, 256, 0, stream>>>(partial, out, p.M, p.N, p.splits);
-    KFB_LAUNCH_CHECK("splitk_reduce_kernel");
+    return launch_kernel("splitk_reduce_kernel", vec ? splitk_reduce_kernel<4> : splitk_reduce_kernel<1>, dim3((unsigned)blocks), dim3(256), 0, stream,
+                         (const float*)partial, out, p.M, p.N, p.splits);
   }
   return KFB_OK;
 }

@@ -35,7 +35,7 @@ constexpr int kWarps = kThreads / 32;
 
 __device__ __forceinline__ uint4 ldg_stream(const uint4* p) {
   uint4 v;
-  asm("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+  asm("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
       : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
       : "l"(p));
   return v;
@@ -150,10 +150,10 @@ int4_gemv_kernel(const __half* __restrict__ x, const uint4* __restrict__ packed,
 #pragma unroll
     for (int r = 0; r < R; ++r) acc[m][r] = 0.f;
 
-  // Weights and scales are constants: the first two chunks of every lane are fetched BEFORE waiting for the kernel in
-  // front (programmatic dependent launch: this grid is already resident while that kernel finishes, so its launch
-  // latency and the first DRAM round trip are hidden); x (and y, in the epilogue) are touched only after the wait.
-  // The dependents of this grid are released right after its own wait has returned, so at most two grids overlap.
+  // The first two chunks of every lane are fetched BEFORE waiting for the kernel in front where they are known to be older
+  // than it (fu.early: this grid is already resident while that kernel finishes, so its launch latency and the first DRAM
+  // round trip are hidden); x (and y, in the epilogue) are touched only after the wait.
+  if (!fu.early) pdl_wait(x, packed, scales);
   const uint4* wrow[R];
   const __half* srow[R];
 #pragma unroll
@@ -176,9 +176,9 @@ int4_gemv_kernel(const __half* __restrict__ x, const uint4* __restrict__ packed,
   };
   fetch(0, c_first);
   fetch(1, c_first + stride);
-  if constexpr (XF == kXformNone) pdl_wait();   // (with a transform the wait opens the prologue below)
+  if constexpr (XF == kXformNone) pdl_wait(x);   // (with a transform the wait opens the prologue below)
   if constexpr (XF != kXformNone) {
-    pdl_wait();   // x is the previous kernel's output
+    pdl_wait(x);   // x is the previous kernel's output
     const int nvec = K / 8;
     if constexpr (XF == kXformRmsNorm) {
       __shared__ float part[M][kWarps];
@@ -377,12 +377,8 @@ int launch(const void* x, const void* packed, const void* scales, void* y, int N
            cudaStream_t stream, const Fusion& fu = Fusion{}) {
   const int tiles = ceil_div(N, R);
   const int grid = ceil_div(tiles, kWarps >> ksplit_log2);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = XF != kXformNone ? (size_t)M * K * sizeof(__half) : 0;
-  cfg.stream = stream;
-  if (cfg.dynamicSmemBytes > 48 * 1024) {
+  const size_t smem = XF != kXformNone ? (size_t)M * K * sizeof(__half) : 0;
+  if (smem > 48 * 1024) {
     static bool configured[64] = {false};
     int dev = 0;
     KFB_CUDA_TRY(cudaGetDevice(&dev));
@@ -391,14 +387,10 @@ int launch(const void* x, const void* packed, const void* scales, void* y, int N
       configured[dev] = true;
     }
   }
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = ((flags & 1) || pdl_enabled()) ? 1 : 0;
-  KFB_CUDA_TRY(cudaLaunchKernelEx(&cfg, int4_gemv_kernel<M, R, G, XF, EPI>, (const __half*)x, (const uint4*)packed,
-                                  (const __half*)scales, (__half*)y, N, K, ksplit_log2, fu));
-  return KFB_OK;
+  Fusion f = fu;
+  f.early = (flags & 1) || constants_are_old();
+  return launch_kernel("int4_gemv_kernel", int4_gemv_kernel<M, R, G, XF, EPI>, dim3(grid), dim3(kThreads), smem, stream, (const __half*)x,
+                       (const uint4*)packed, (const __half*)scales, (__half*)y, N, K, ksplit_log2, f);
 }
 
 template <int M, int G, int XF = kXformNone, int EPI = kEpiNone>

@@ -35,7 +35,7 @@ constexpr int kMaxBlocksPerWarp = 24;   // k blocks (of 64) one warp can keep in
 
 __device__ __forceinline__ uint4 ldg_stream(const uint4* p) {
   uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
 __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -52,6 +52,7 @@ __device__ __forceinline__ uint32_t pair_q(uint32_t w, int s) {
 
 // public packed words [N, K/8] -> fragment order (see the header comment).  One thread per 16-byte lane piece.
 __global__ void prepack_kernel(const uint32_t* __restrict__ packed, uint4* __restrict__ out, int N, int K) {
+  pdl_wait(packed);
   const int KB = K / 64, KW = K / 8;
   const long long total = (long long)(N / 16) * KB * 32;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -89,8 +90,9 @@ int4_gemv_frag_kernel(const __half* __restrict__ x, const uint4* __restrict__ wf
   const int kb0 = g0 * kBlocksPerGroup, kb1 = g1 * kBlocksPerGroup;
   const bool live = rb < n_rb;
 
-  // Weights are constants: every block of this warp is requested before the wait for the kernel in front (programmatic
-  // dependent launch), so the whole weight stream of the call is in flight while that kernel drains.
+  // Where the weights are older than the kernel in front (fu.early) every block of this warp is requested before the wait
+  // for it, so the whole weight stream of the call is in flight while that kernel drains.
+  if (!fu.early) pdl_wait(x, wf, scales);
   uint4 wbuf[NB];
   const uint4* wp = wf + ((size_t)(live ? rb : 0) * KB) * 32 + lane;
 #pragma unroll
@@ -106,7 +108,7 @@ int4_gemv_frag_kernel(const __half* __restrict__ x, const uint4* __restrict__ wf
     for (int i = 0; i < kMaxGroups; ++i)
       if (live && g0 + i < g1) { sc0[i] = srow0[g0 + i]; sc1[i] = srow1[g0 + i]; }
   }
-  pdl_wait();
+  pdl_wait(x);
   pdl_launch_dependents();
 
   float acc[MB][4];
@@ -181,7 +183,7 @@ int launch_mb(const void* x, const void* wf, const void* scales, void* y, int M,
   constexpr int RB = kWarps / KS;
   const int grid = ceil_div(N / 16, RB);
   return launch_kernel("int4_gemv_frag_kernel", int4_gemv_frag_kernel<KS, G, NB, EPI, MB>, dim3(grid), dim3(kThreads), 0, stream,
-                       pdl_enabled(), static_cast<const __half*>(x), static_cast<const uint4*>(wf),
+                       static_cast<const __half*>(x), static_cast<const uint4*>(wf),
                        static_cast<const __half*>(scales), static_cast<__half*>(y), M, N, K, fu);
 }
 
@@ -216,7 +218,7 @@ int pick(const void* x, const void* wf, const void* scales, void* y, int M, int 
 }
 
 int run(const char* what, const void* x, const void* prepacked, const void* scales, void* y, int M, int N, int K, int group,
-        void* stream, const gemv::Fusion& fu) {
+        void* stream, const gemv::Fusion& given) {
   if (int rc = require_sm100()) return rc;
   if (M < 1 || M > 32) return fail(KFB_ERR_INVALID, "%s handles M in [1, 32], got M=%d", what, M);
   if (group != 64 && group != 128) return fail(KFB_ERR_INVALID, "group_size must be one of (64, 128), got %d", group);
@@ -225,6 +227,8 @@ int run(const char* what, const void* x, const void* prepacked, const void* scal
   if (!x || !prepacked || !scales || !y) return fail(KFB_ERR_INVALID, "null pointer");
   if (!aligned16(x) || !aligned16(prepacked)) return fail(KFB_ERR_ALIGNMENT, "x and the prepacked weights must be 16-byte aligned");
   cudaStream_t s = (cudaStream_t)stream;
+  gemv::Fusion fu = given;
+  fu.early = constants_are_old();
   if (fu.epi == gemv::kEpiSiluPair)
     return group == 128 ? pick<128, gemv::kEpiSiluPair>(x, prepacked, scales, y, M, N, K, s, fu)
                         : pick<64, gemv::kEpiSiluPair>(x, prepacked, scales, y, M, N, K, s, fu);
@@ -253,9 +257,8 @@ extern "C" int kfb_int4_prepack(const void* packed, int N, int K, void* out, voi
   if (!aligned16(packed) || !aligned16(out)) return fail(KFB_ERR_ALIGNMENT, "packed and out must be 16-byte aligned");
   const long long total = (long long)(N / 16) * (K / 64) * 32;
   const int blocks = (int)((total + 255) / 256 < 4096 ? (total + 255) / 256 : 4096);
-  frag::prepack_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(static_cast<const uint32_t*>(packed), static_cast<uint4*>(out), N, K);
-  KFB_LAUNCH_CHECK("prepack_kernel");
-  return KFB_OK;
+  return launch_kernel("prepack_kernel", frag::prepack_kernel, dim3(blocks), dim3(256), 0, (cudaStream_t)stream, static_cast<const uint32_t*>(packed),
+                       static_cast<uint4*>(out), N, K);
 }
 
 extern "C" int kfb_int4_gemv_prepacked(const void* x, const void* prepacked, const void* scales, void* y, int M, int N, int K,

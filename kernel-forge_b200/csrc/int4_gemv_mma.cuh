@@ -622,7 +622,7 @@ int launch_ex(void (*kernel)(KArgs...), int grid, int threads, size_t smem, cuda
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = (pdl || pdl_enabled()) ? 1 : 0;
+  cfg.numAttrs = (pdl || constants_are_old()) ? 1 : 0;   // these kernels always read weights before their wait
   KFB_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...));
   return KFB_OK;
 }

@@ -59,8 +59,7 @@ extern "C" int kfb_int4_linear(const void* x, const void* packed, const void* sc
       if (int rc = check_small(x, packed, N, K, group)) return rc;
       gemv::Fusion fu = {};
       fu.bias = static_cast<const __half*>(bias);
-      return small::run(x, packed, scales, y, M, N, K, group, dtype == KFB_BF16, /*weights_first=*/pdl_enabled(), pdl_enabled(),
-                        (cudaStream_t)stream, fu);
+      return small::run(x, packed, scales, y, M, N, K, group, dtype == KFB_BF16, (cudaStream_t)stream, fu);
     }
     default: return gemm::run(x, packed, scales, bias, y, M, N, K, group, dtype == KFB_BF16, false, ws, ws_bytes, (cudaStream_t)stream);
   }
@@ -76,5 +75,5 @@ extern "C" int kfb_int4_linear_silu_pairs(const void* x, const void* packed, con
   if (int rc = check_small(x, packed, N, K, group)) return rc;
   gemv::Fusion fu = {};
   fu.epi = gemv::kEpiSiluPair;
-  return small::run(x, packed, scales, act, M, N, K, group, false, /*weights_first=*/pdl_enabled(), pdl_enabled(), (cudaStream_t)stream, fu);
+  return small::run(x, packed, scales, act, M, N, K, group, false, (cudaStream_t)stream, fu);
 }

@@ -37,11 +37,11 @@ struct Words {
   uint32_t w[W];
 };
 __device__ __forceinline__ void load_words(Words<4>& d, const uint32_t* p) {
-  asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(d.w[0]), "=r"(d.w[1]) : "l"(p));
-  asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(d.w[2]), "=r"(d.w[3]) : "l"(p + 8));
+  asm volatile("ld.global.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(d.w[0]), "=r"(d.w[1]) : "l"(p));
+  asm volatile("ld.global.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(d.w[2]), "=r"(d.w[3]) : "l"(p + 8));
 }
 __device__ __forceinline__ void load_words(Words<2>& d, const uint32_t* p) {
-  asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(d.w[0]), "=r"(d.w[1]) : "l"(p));
+  asm volatile("ld.global.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(d.w[0]), "=r"(d.w[1]) : "l"(p));
 }
 
 template <bool kBf16>
@@ -113,7 +113,7 @@ constexpr int min_blocks() { return KS == 16 ? 1 : RB * MB == 1 ? 4 : RB == 1 &&
 template <int G, int KS, int RB, int MB, bool kBf16>
 __global__ void __launch_bounds__(KS * 32, min_blocks<KS, RB, MB>())
 int4_small_kernel(const uint16_t* __restrict__ x, const uint32_t* __restrict__ packed, const __half* __restrict__ scales,
-                  uint16_t* __restrict__ y, int M, int N, int K, int weights_first, const gemv::Fusion fu) {
+                  uint16_t* __restrict__ y, int M, int N, int K, const gemv::Fusion fu) {
   constexpr int W = G / 32;                         // packed words per lane, row and group; and 16-byte pieces of x
   constexpr int kDepth = (KS == 16 && MB == 1 ? 4 : 2) * (128 / G);   // groups a warp keeps in flight
   constexpr int kRows = 16 * RB, kPad = kRows + 4;
@@ -126,6 +126,7 @@ int4_small_kernel(const uint16_t* __restrict__ x, const uint32_t* __restrict__ p
   const int SG = K / G, KW = K / 8;
   const int g0 = (int)((long long)SG * warp / warps), g1 = (int)((long long)SG * (warp + 1) / warps);
 
+  if (!fu.early) pdl_wait(x, packed, scales);   // (early: the weights are older than the kernel in front)
   const uint32_t* wrow[RB][2];
   const __half* srow[RB][2];
 #pragma unroll
@@ -149,10 +150,10 @@ int4_small_kernel(const uint16_t* __restrict__ x, const uint32_t* __restrict__ p
         }
     }
   };
-  if (!weights_first) pdl_wait();
+
 #pragma unroll
   for (int d = 0; d < kDepth; ++d) fetch(d, g0 + d);
-  if (weights_first) pdl_wait();
+  if (fu.early) pdl_wait(x);
   pdl_launch_dependents();
 
   float acc[RB][MB][4];
@@ -240,19 +241,21 @@ int4_small_kernel(const uint16_t* __restrict__ x, const uint32_t* __restrict__ p
 }
 
 template <int G, int KS, int RB, int MB, bool kBf16>
-int launch(const void* x, const void* packed, const void* scales, void* y, int M, int N, int K, bool weights_first,
-           bool pdl, cudaStream_t stream, const gemv::Fusion& fu) {
+int launch(const void* x, const void* packed, const void* scales, void* y, int M, int N, int K,
+           cudaStream_t stream, const gemv::Fusion& fu) {
   auto kernel = int4_small_kernel<G, KS, RB, MB, kBf16>;
   constexpr size_t smem = (size_t)KS * (8 * MB) * (16 * RB + 4) * sizeof(float);
   static_assert(smem <= 48 * 1024, "no opt-in for more shared memory is made");
-  return launch_kernel("int4_small_kernel", kernel, dim3(ceil_div(N, 16 * RB)), dim3(KS * 32), smem, stream, pdl,
-                       (const uint16_t*)x, (const uint32_t*)packed, (const __half*)scales, (uint16_t*)y, M, N, K, weights_first ? 1 : 0, fu);
+  return launch_kernel("int4_small_kernel", kernel, dim3(ceil_div(N, 16 * RB)), dim3(KS * 32), smem, stream,
+                       (const uint16_t*)x, (const uint32_t*)packed, (const __half*)scales, (uint16_t*)y, M, N, K, fu);
 }
 
 }  // namespace
 
-int run(const void* x, const void* packed, const void* scales, void* y, int M, int N, int K, int group, bool bf16, bool weights_first,
-        bool pdl, cudaStream_t stream, const gemv::Fusion& fu) {
+int run(const void* x, const void* packed, const void* scales, void* y, int M, int N, int K, int group, bool bf16, cudaStream_t stream,
+        const gemv::Fusion& given) {
+  gemv::Fusion fu = given;
+  fu.early = constants_are_old();
   // Few row blocks (at most one CTA per SM) and a long K: 16 shares of K instead of 8, so that a warp has half as many
   // groups one after the other (2048 x 5632, M = 8: 5.3 us against 6.1; at K = 2048 there is nothing to gain).
   // 9 <= M <= 16 and more row blocks than the three CTAs per SM hold: two row blocks per warp share the activations
@@ -260,7 +263,7 @@ int run(const void* x, const void* packed, const void* scales, void* y, int M, i
   const int row_blocks = ceil_div(N, 16), sms = sm_count();
   const bool long_k = row_blocks <= sms && K >= 4096;
   const bool two_rows = M > 8 && M <= 16 && row_blocks > 3 * sms;
-#define KFB_SMALL(G, KS, RB, MB, BF) return launch<G, KS, RB, MB, BF>(x, packed, scales, y, M, N, K, weights_first, pdl, stream, fu)
+#define KFB_SMALL(G, KS, RB, MB, BF) return launch<G, KS, RB, MB, BF>(x, packed, scales, y, M, N, K, stream, fu)
 #define KFB_SMALL_KS(G, BF)                                                            \
   {                                                                                    \
     if (two_rows) KFB_SMALL(G, 8, 2, 2, BF);                                           \

@@ -10,10 +10,9 @@ namespace small {
 constexpr int kMaxM = 32;
 
 // Arguments as checked by the caller: non-null, x and packed 16-byte aligned, K a multiple of `group` (64 or 128).
-// weights_first: packed and scales are older than the kernel in front of this one in the stream, so they may be read
-// before the programmatic-dependent-launch wait.  The pair epilogues of `fu` are fp16 only.
-int run(const void* x, const void* packed, const void* scales, void* y, int M, int N, int K, int group, bool bf16, bool weights_first,
-        bool pdl, cudaStream_t stream, const gemv::Fusion& fu);
+// The pair epilogues of `fu` are fp16 only.
+int run(const void* x, const void* packed, const void* scales, void* y, int M, int N, int K, int group, bool bf16, cudaStream_t stream,
+        const gemv::Fusion& fu);
 
 }  // namespace small
 }  // namespace kfb

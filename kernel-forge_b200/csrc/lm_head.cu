@@ -27,7 +27,7 @@ constexpr int kUnroll = 8;   // k chunks of 32 in flight per lane: 2 rows x 16 B
 
 __device__ __forceinline__ uint4 ldg_stream(const uint4* p) {
   uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
 __device__ __forceinline__ uint4 ldg_cached(const uint4* p) {
@@ -51,7 +51,7 @@ __device__ __forceinline__ uint32_t ordered_bits(float f) {
 template <int NB>
 __global__ void __launch_bounds__(kThreads)
 lm_head_gemv_kernel(const __half* __restrict__ x, const __half* __restrict__ w, __half* __restrict__ y,
-                    unsigned long long* __restrict__ best, int M, int N, int K) {
+                    unsigned long long* __restrict__ best, int M, int N, int K, int early) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
   const int row0 = (blockIdx.x * kWarps + warp) * kRowsPerWarp;
@@ -60,6 +60,7 @@ lm_head_gemv_kernel(const __half* __restrict__ x, const __half* __restrict__ w, 
     pdl_launch_dependents();
     return;
   }
+  if (!early) pdl_wait(x, w);   // the weights may be the work of the kernel in front
   const int ra = min(row0 + g, N - 1), rb = min(row0 + g + 8, N - 1);   // rows past N: a valid row, never stored
   const uint4* wa = reinterpret_cast<const uint4*>(w + (size_t)ra * K) + t;
   const uint4* wb = reinterpret_cast<const uint4*>(w + (size_t)rb * K) + t;
@@ -82,7 +83,7 @@ lm_head_gemv_kernel(const __half* __restrict__ x, const __half* __restrict__ w, 
       va[u] = ldg_stream(wa + c * 4);
       vb[u] = ldg_stream(wb + c * 4);
     }
-    if (c0 == 0) {   // the weights are constants: the first loads are in flight before the wait for the kernel in front
+    if (c0 == 0) {   // (early) the first loads are in flight before the wait for the kernel in front
       pdl_wait();
       pdl_launch_dependents();
     }
@@ -136,7 +137,7 @@ lm_head_gemv_kernel(const __half* __restrict__ x, const __half* __restrict__ w, 
 __global__ void decode_finalize_kernel(unsigned long long* __restrict__ best, long long* __restrict__ tok, long long* __restrict__ pos,
                                        int* __restrict__ kv_len, int M) {
   const int m = threadIdx.x;
-  pdl_wait();
+  pdl_wait(best);
   pdl_launch_dependents();
   if (m < M) {
     const unsigned long long key = best[m];
@@ -155,7 +156,7 @@ __global__ void __launch_bounds__(kThreads)
 embed_rmsnorm_kernel(const long long* __restrict__ tok, const __half* __restrict__ embed, const __half* __restrict__ w,
                      __half* __restrict__ y, __half* __restrict__ x_out, int hidden, int vocab, float eps) {
   __shared__ float warp_part[kWarps];
-  pdl_wait();
+  pdl_wait(tok, embed, w);
   pdl_launch_dependents();
   long long id = tok[blockIdx.x];
   id = id < 0 ? 0 : (id >= vocab ? vocab - 1 : id);   // an id outside the table reads a valid row instead of faulting
@@ -224,12 +225,12 @@ extern "C" int kfb_fp16_gemv_argmax(const void* x, const void* w, void* y, void*
   const auto* wp = static_cast<const __half*>(w);
   auto* yp = static_cast<__half*>(y);
   const dim3 gd(grid), bd(lmhead::kThreads);
-  const bool pdl = pdl_enabled();
+  const int early = constants_are_old();
   switch (ceil_div(M, 8)) {
-    case 1: return launch_kernel("lm_head_gemv_kernel", lmhead::lm_head_gemv_kernel<1>, gd, bd, 0, s, pdl, xp, wp, yp, b, M, N, K);
-    case 2: return launch_kernel("lm_head_gemv_kernel", lmhead::lm_head_gemv_kernel<2>, gd, bd, 0, s, pdl, xp, wp, yp, b, M, N, K);
-    case 3: return launch_kernel("lm_head_gemv_kernel", lmhead::lm_head_gemv_kernel<3>, gd, bd, 0, s, pdl, xp, wp, yp, b, M, N, K);
-    default: return launch_kernel("lm_head_gemv_kernel", lmhead::lm_head_gemv_kernel<4>, gd, bd, 0, s, pdl, xp, wp, yp, b, M, N, K);
+    case 1: return launch_kernel("lm_head_gemv_kernel", lmhead::lm_head_gemv_kernel<1>, gd, bd, 0, s, xp, wp, yp, b, M, N, K, early);
+    case 2: return launch_kernel("lm_head_gemv_kernel", lmhead::lm_head_gemv_kernel<2>, gd, bd, 0, s, xp, wp, yp, b, M, N, K, early);
+    case 3: return launch_kernel("lm_head_gemv_kernel", lmhead::lm_head_gemv_kernel<3>, gd, bd, 0, s, xp, wp, yp, b, M, N, K, early);
+    default: return launch_kernel("lm_head_gemv_kernel", lmhead::lm_head_gemv_kernel<4>, gd, bd, 0, s, xp, wp, yp, b, M, N, K, early);
   }
 }
 
@@ -238,7 +239,7 @@ extern "C" int kfb_decode_finalize(void* best, void* tok, void* pos, void* kv_le
   if (M < 1 || M > 1024) return fail(KFB_ERR_INVALID, "decode_finalize handles 1..1024 sequences, got %d", M);
   if (!best || !tok || !pos || !kv_len) return fail(KFB_ERR_INVALID, "null pointer");
   return launch_kernel("decode_finalize_kernel", lmhead::decode_finalize_kernel, dim3(1), dim3(((M + 31) / 32) * 32), 0,
-                       (cudaStream_t)stream, pdl_enabled(), static_cast<unsigned long long*>(best), static_cast<long long*>(tok),
+                       (cudaStream_t)stream, static_cast<unsigned long long*>(best), static_cast<long long*>(tok),
                        static_cast<long long*>(pos), static_cast<int*>(kv_len), M);
 }
 
@@ -255,6 +256,6 @@ extern "C" int kfb_embed_rmsnorm(const void* tok, const void* embed, const void*
   auto kernel = per_thread == 1 ? lmhead::embed_rmsnorm_kernel<1> : per_thread <= 4 ? lmhead::embed_rmsnorm_kernel<4>
                                                                                      : lmhead::embed_rmsnorm_kernel<lmhead::kWidestVec>;
   return launch_kernel("embed_rmsnorm_kernel", kernel, dim3(rows), dim3(lmhead::kThreads), 0,
-                       (cudaStream_t)stream, pdl_enabled(), static_cast<const long long*>(tok), static_cast<const __half*>(embed),
+                       (cudaStream_t)stream, static_cast<const long long*>(tok), static_cast<const __half*>(embed),
                        static_cast<const __half*>(weight), static_cast<__half*>(y), static_cast<__half*>(x_out), hidden, vocab, eps);
 }

@@ -1,0 +1,31 @@
+"""The GPU quantiser at the values where its reciprocal shortcut must hand over to the exact division, bit for bit against
+the torch formulation (kernelforge.quantize on a CPU tensor)."""
+
+import pytest
+import torch
+
+from kernelforge import quantize as kq
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("group", [64, 128])
+@pytest.mark.parametrize("n,k", [(1, 128), (3, 192), (129, 1152), (1000, 256)])
+def test_bits_at_half_integers_and_extremes(n, k, group, dtype):
+    if k % group:
+        pytest.skip("K is not a multiple of the group")
+    g = torch.Generator().manual_seed(n + k + group)
+    w = torch.randn(n, k, generator=g) * 0.02
+    ties = w[:, ::3].sign() * (torch.randint(0, 15, w[:, ::3].shape, generator=g) * 0.5)   # multiples of half a step
+    w[:, ::3] = ties * 0.015625
+    w[:, 5::7] = 0.109375                       # 7 steps of 2^-6: the scale is exactly 2^-6
+    w[0, :group] = 0.0                          # an all-zero group
+    if n > 1:
+        w[1] = torch.randn(k, generator=g) * 1e-6   # below the smallest scale
+    if n > 2:
+        w[2] = torch.randn(k, generator=g) * (1e4 if dtype == torch.float16 else 3e5)
+    w = w.to(dtype)
+    want, got = kq.quantize_weight(w, group), kq.quantize_weight(w.cuda(), group)
+    assert torch.equal(got.packed.cpu(), want.packed)
+    assert torch.equal(got.scales.cpu().view(torch.int16), want.scales.view(torch.int16))
