@@ -31,62 +31,88 @@ __device__ __forceinline__ void load8(const __nv_bfloat16* w, float (&v)[8]) {
   for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(h[i]); v[2 * i] = f.x; v[2 * i + 1] = f.y; }
 }
 
-// clamp(rint(v / s), -8, 7) + 8 with the quotient rounded to FP32 first, as the definition says.
-__device__ __noinline__ uint32_t quotient_exact(float v, float s) {
-  return (uint32_t)((int)fminf(fmaxf(rintf(__fdiv_rn(v, s)), -8.0f), 7.0f) + 8);
+// The packed word by definition: clamp(rint(v / s), -8, 7) + 8 with the quotient rounded to FP32 first.
+struct Eight {   // by value: an array whose address is taken would live in local memory for everybody
+  float v[8];
+};
+__device__ __noinline__ uint32_t pack_exact(Eight w, float s) {
+  uint32_t word = 0;
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    word |= (uint32_t)((int)fminf(fmaxf(rintf(__fdiv_rn(w.v[j], s)), -8.0f), 7.0f) + 8) << (4 * nibble_pos(j));
+  return word;
+}
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
 }
 
 // One lane per packed word (8 consecutive k); G / 8 neighbouring lanes share a group.  Words and groups are contiguous
-// over the whole tensor, so the grid walks flat word indices and knows no rows.
+// over the whole tensor, so a CTA takes a run of kUnroll * 256 flat word indices and knows no rows.
 //
-// HBM-bound (2.5 bytes per fp16 weight).  What kept it from that was one IEEE division per weight (a dozen instructions)
-// and 8-byte loads: 11264 x 2048 fp16 42.8 us.  Now a weight is multiplied with the group's reciprocal, which is off by at
-// most 2e-6 for quotients below 8, and only where that could change the rounding (within 1e-5 of a half integer; or a
-// quotient outside +-7.4, infinity, NaN) is the division done.
+// HBM-bound by design (2.5 bytes per fp16 weight), bound by issue slots in fact.  One IEEE division per weight (a dozen
+// instructions) and 8-byte loads took 42.8 us for 11264 x 2048 fp16; this kernel takes 15 us (3.9 TB/s).  A weight is
+// multiplied with the group's reciprocal and rounded by the magic-number addition of one FMA.  The product is off by at
+// most 2^-22 of itself, so the result can only differ from the definition's next to a half integer; a lane that sees such
+// a weight (or a quotient above 7.4, infinity, NaN) packs its word by the definition.
+constexpr int kQuantThreads = 256;
+constexpr int kQuantUnroll = 2;   // words per lane, requested at once (1 or 4: 5 % slower)
+
 template <typename T, int G>
-__global__ void __launch_bounds__(256) quantize_pack_kernel(const T* __restrict__ w, uint32_t* __restrict__ packed,
-                                                            __half* __restrict__ scales, long long words) {
-  constexpr int kLanes = G / 8, kUnroll = sizeof(T) == 4 ? 2 : 4;
+__global__ void __launch_bounds__(kQuantThreads, 8) quantize_pack_kernel(const T* __restrict__ w, uint32_t* __restrict__ packed,
+                                                                         __half* __restrict__ scales, long long words) {
+  constexpr int kLanes = G / 8;
   pdl_wait(w);   // (the successor is not released early: it may read these weights before its own wait)
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  // (the loop runs by warps; a group's lanes all have a word or none, since `words` is a multiple of kLanes)
-  const int lane = threadIdx.x & 31;
-  for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; i0 - lane < words; i0 += kUnroll * stride) {
-    float v[kUnroll][8];
+  // a group's lanes all have a word or none, since `words` is a multiple of kLanes
+  const long long first = (long long)blockIdx.x * (kQuantUnroll * kQuantThreads);
+  const int left = (int)min(words - first, (long long)(kQuantUnroll * kQuantThreads));
+  w += first * 8;
+  packed += first;
+  scales += first / kLanes;
+  float v[kQuantUnroll][8];
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u)
-      if (i0 + u * stride < words) load8(w + (i0 + u * stride) * 8, v[u]);
+  for (int u = 0; u < kQuantUnroll; ++u) {
+    const int i = u * kQuantThreads + threadIdx.x;
+    load8(w + 8 * min(i, left - 1), v[u]);   // past the end: the last word again, not stored
+  }
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
-      const long long i = i0 + u * stride;
-      const bool live = i < words;
-      float amax = 0.0f;
-      if (!live) {
+  for (int u = 0; u < kQuantUnroll; ++u) {
+    const int i = u * kQuantThreads + threadIdx.x;
+    float amax = fabsf(v[u][0]);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[u][j] = 0.0f;
-      }
+    for (int j = 1; j < 8; ++j) amax = fmaxf(amax, fabsf(v[u][j]));
 #pragma unroll
-      for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(v[u][j]));
+    for (int off = kLanes / 2; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+    // scale = fp16(max(absmax / 7, smallest normal fp16)); exactly 1 for an all-zero group
+    __half sh = __float2half_rn(fmaxf(__fdiv_rn(amax, 7.0f), 6.103515625e-05f));
+    if (amax == 0.0f) sh = __float2half_rn(1.0f);
+    const float s32 = __half2float(sh), inv = rcp_approx(s32);
+    // v * inv + 1.5 * 2^23 has rint(v / s) in its low bits (ties to even).  Rounding it with a slightly smaller and a
+    // slightly larger reciprocal tells whether the error of inv could matter.  The words of the sums are kBits + rint;
+    // the constant part, and the + 8 of every nibble, come in through kSum, so no masks are needed.
+    constexpr float kMagic = 12582912.0f;
+    constexpr uint32_t kBits = 0x4B400000u, kSum = 0u - (kBits - 8u) * 0x11111111u;
+    const float lo = inv * (1.0f - 1.0f / 1048576.0f), hi = inv * (1.0f + 1.0f / 1048576.0f);
+    uint32_t word = kSum, differ = 0;
+    float sum = 0.0f;   // not finite if any weight is (amax does not see NaN)
 #pragma unroll
-      for (int off = kLanes / 2; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-      // scale = fp16(max(absmax / 7, smallest normal fp16)); exactly 1 for an all-zero group
-      __half sh = __float2half_rn(fmaxf(__fdiv_rn(amax, 7.0f), 6.103515625e-05f));
-      if (amax == 0.0f) sh = __float2half_rn(1.0f);
-      const float s32 = __half2float(sh), inv = __fdiv_rn(1.0f, s32);
-      uint32_t word = 0;
+    for (int j = 0; j < 8; ++j) {
+      const float t = fmaf(v[u][j], lo, kMagic);
+      const uint32_t a = __float_as_uint(t), b = __float_as_uint(fmaf(v[u][j], hi, kMagic));
+      sum += t;
+      differ |= a ^ b;
+      word += a << (4 * nibble_pos(j));
+    }
+    if (!(differ == 0 && amax * inv < 7.4f && sum < 1e9f)) {
+      Eight w8;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float r = v[u][j] * inv;
-        const float t = r + 12582920.0f;                 // 1.5 * 2^23 + 8: the low bits are rint(r) + 8 (ties to even)
-        const float frac = fabsf(r - (t - 12582920.0f));
-        uint32_t q = __float_as_uint(t) & 0xFu;
-        if (!(frac < 0.49999f && fabsf(r) < 7.4f)) q = quotient_exact(v[u][j], s32);
-        word |= q << (4 * nibble_pos(j));
-      }
-      if (live) {
-        packed[i] = word;
-        if ((lane & (kLanes - 1)) == 0) scales[i / kLanes] = sh;
-      }
+      for (int j = 0; j < 8; ++j) w8.v[j] = v[u][j];
+      word = pack_exact(w8, s32);
+    }
+    if (i < left) {
+      packed[i] = word;
+      if ((threadIdx.x & (kLanes - 1)) == 0) scales[i / kLanes] = sh;
     }
   }
 }
@@ -179,10 +205,11 @@ extern "C" int kfb_quantize_pack(const void* w, int w_dtype, int N, int K, int g
   if (!aligned16(w) || !aligned16(packed)) return fail(KFB_ERR_ALIGNMENT, "w and packed must be 16-byte aligned");
   cudaStream_t s = (cudaStream_t)stream;
   const long long words = (long long)N * (K / 8);
-  const int grid = grid_for(words, 256 * 2);
-#define KFB_Q(T, G)                                                                                                            \
-  return launch_kernel("quantize_pack_kernel", quantize_pack_kernel<T, G>, dim3(grid), dim3(256), 0, s, (const T*)w, (uint32_t*)packed, \
-                       (__half*)scales, words)
+  constexpr int kPerCta = kQuantUnroll * kQuantThreads;
+  if (words > (1LL << 40)) return fail(KFB_ERR_INVALID, "weight too large");
+#define KFB_Q(T, G)                                                                                                          \
+  return launch_kernel("quantize_pack_kernel", quantize_pack_kernel<T, G>, dim3((unsigned)((words + kPerCta - 1) / kPerCta)), \
+                       dim3(kQuantThreads), 0, s, (const T*)w, (uint32_t*)packed, (__half*)scales, words)
   if (w_dtype == KFB_F32) { if (group == 128) KFB_Q(float, 128); else KFB_Q(float, 64); }
   if (w_dtype == KFB_F16) { if (group == 128) KFB_Q(__half, 128); else KFB_Q(__half, 64); }
   if (w_dtype == KFB_BF16) { if (group == 128) KFB_Q(__nv_bfloat16, 128); else KFB_Q(__nv_bfloat16, 64); }

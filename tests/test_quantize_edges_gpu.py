@@ -29,3 +29,14 @@ def test_bits_at_half_integers_and_extremes(n, k, group, dtype):
     want, got = kq.quantize_weight(w, group), kq.quantize_weight(w.cuda(), group)
     assert torch.equal(got.packed.cpu(), want.packed)
     assert torch.equal(got.scales.cpu().view(torch.int16), want.scales.view(torch.int16))
+
+
+def test_nan_and_infinity_take_the_definition():
+    """Not meaningful as weights, but the words stay what rint / clamp give: NaN and -inf the smallest code, in the lane only."""
+    w = torch.randn(2, 256, generator=torch.Generator().manual_seed(0)) * 0.02
+    clean = kq.quantize_weight(w.cuda(), 128)
+    bad = w.clone()
+    bad[0, 9] = float("nan")
+    got = kq.quantize_weight(bad.cuda(), 128)
+    q, q0 = kq.unpack_int4(got.packed).cpu(), kq.unpack_int4(clean.packed).cpu()
+    assert q[0, 9] == -8 and torch.equal(q[1], q0[1]) and torch.equal(q[0, 16:], q0[0, 16:])
