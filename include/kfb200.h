@@ -298,7 +298,8 @@ int kfb_peer_allgather(const void* src, void* const* dst_all, void* const* peer_
  *   kv_strides: NULL for contiguous k/v, else {batch, head, row} strides IN ELEMENTS shared by
  *   k and v (each a multiple of 8; the D axis must be dense), so a KV-cache view
  *   cache[:, :, :Nk] needs no copy.
- *   Prefill (Nq > 1): TMA-staged swizzled tiles, tcgen05 MMA, accumulators in TMEM.
+ *   Prefill (Nq > 1): TMA-staged swizzled tiles, tcgen05 MMA, accumulators in TMEM.  The workspace is optional there: with
+ *   kfb_flash_attn_ws_bytes bytes (16-byte aligned) a problem with few query tiles is split along the keys.
  *   Decode (Nq == 1): split-KV kernel; partial (o, m, l) per split go through `ws`.
  * ------------------------------------------------------------------------------------- */
 size_t kfb_flash_attn_ws_bytes(int B, int H, int Hk, int Nq, int Nk, int D);

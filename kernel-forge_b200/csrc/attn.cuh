@@ -23,8 +23,10 @@ struct Problem {
   const int* kv_len_dev = nullptr;
 };
 
-// Prefill / general path: one CTA per 128 query rows, TMA + tcgen05 + TMEM (attn_prefill.cu).
-int launch_prefill(const Problem& p, cudaStream_t stream);
+// Prefill / general path: tiles of 128 query rows, TMA + tcgen05 + TMEM (attn_prefill.cu).  The workspace is optional: a
+// problem with few tiles is split along the keys when it has prefill_ws_bytes bytes.
+size_t prefill_ws_bytes(int B, int H, int Hk, int Nq, int Nk, int D);
+int launch_prefill(const Problem& p, void* ws, size_t ws_bytes, cudaStream_t stream);
 
 // Decode path (Nq == 1): split-KV, one CTA per (batch, kv head, split) (attn_decode.cu).
 size_t decode_ws_bytes(int B, int H, int Hk, int Nk, int D);

@@ -4,12 +4,9 @@
 // mma.sync / ldmatrix / cp.async kernel.  Two kernels built on the Blackwell execution model (TMA into
 // 128-byte-swizzled shared-memory tiles, tcgen05.mma issued by one thread, accumulators in TMEM):
 //
-//   pair::attn_prefill_pair_kernel    one CTA per SM owns TWO adjacent query tiles of 128 rows of one
-//                                     (batch, head); steps of 128 keys.  All 512 TMEM columns: two S
-//                                     buffers, two O accumulators, two P buffers.  Two softmax
-//                                     warpgroups (one per tile) share the exponential unit of the SM
-//                                     in alternation while one thread feeds the tensor cores for both.
-//   serial::attn_prefill_serial_kernel one CTA per 128 query rows, two CTAs per SM (256 columns each).
+//   pair::attn_prefill_pair_kernel     one CTA per SM, two tiles of 128 query rows, key splits: nearly everything;
+//   serial::attn_prefill_serial_kernel one CTA per tile, two CTAs per SM (256 TMEM columns each): many heads that
+//                                      have a single tile each and no partner to share K / V with.
 //
 // Common to both: thread r of a softmax warpgroup owns query row r = TMEM lane r, so row maximum and
 // row sum need no shuffles; lazy rescale (the running base of a row only moves when the new maximum
@@ -21,7 +18,8 @@
 //
 // Numerics (as the reference, attn_v4_kernel.cuh:133-213): scores accumulate in FP32; x = s *
 // (scale * log2 e); masked = -inf; p = 2^(x - base); the row sum adds the unrounded p, the PV
-// product uses p rounded to fp16/bf16; O / l rounded once.  2^x is ex2.approx.ftz.f32.
+// product uses p rounded to fp16/bf16; O / l rounded once.  2^x is ex2.approx.ftz.f32 or a
+// polynomial of the same accuracy.
 #include "attn.cuh"
 #include "sm100.cuh"
 
@@ -108,9 +106,9 @@ __device__ __forceinline__ TileOrder decode_tile_order(unsigned int block, int n
 // ------------------------------------------------------------------------------------------------
 // Single-tile kernel: one CTA per 128 query rows, two CTAs resident per SM (256 TMEM columns each).
 // One S buffer of 128 keys, QK(j+1) issued behind PV(j), the softmax in two passes over S in TMEM
-// (maximum, then exponentials), P aliased on the S columns already consumed.  Used for head dim 128
-// and for problems with a single query tile (Nq <= 128: chunked prefill, short prompts), where a
-// CTA of the pair kernel below would run half empty.
+// (maximum, then exponentials), P aliased on the S columns already consumed.  Used for problems with
+// a single query tile per head, ungrouped heads and more of them than SMs, where a CTA of the pair
+// kernel below would run half empty.
 // ------------------------------------------------------------------------------------------------
 namespace serial {
 
@@ -414,67 +412,59 @@ attn_prefill_serial_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
 }  // namespace serial
 
 // ------------------------------------------------------------------------------------------------
-// Pair kernel: one CTA per SM, two query tiles (A = rows [q0, q0+128), B = the next 128) of one
-// (batch, head), steps of 128 keys.  384 threads (three warpgroups; warp 11 only takes part in barriers):
+// Pair kernel: one CTA per SM, two tiles (A and B) of 128 query rows that attend to one KV head, steps of 128 keys.  384
+// threads (three warpgroups; warp 11 only takes part in barriers):
 //   warps 0-3  softmax of tile A, warps 4-7 softmax of tile B (warp w touches TMEM lanes 32 (w % 4)..);
 //   warp 8     TMA producer: both Q tiles once, then K and V tiles of 128 keys through mbarrier rings;
-//   warps 9,10 one thread each issues the tcgen05.mma of tile A / tile B from an event loop: whichever
-//              of QK(j+1) and PV(j) of its tile has its inputs ready goes next.
+//   warps 9,10 issue the tcgen05.mma of tile A / tile B.  The warp stays uniform and one elected lane issues: addresses and
+//              descriptors are then uniform registers (inside `if (lane == 0)` every MMA costs ~95 clocks of moves into
+//              them); it sleeps in blocking waits, because polling takes issue slots from two of the softmax warps.
 // TMEM (all 512 columns), head dim 64:  S_X [128 X, +128)   O_X [256 + 64 X, +64)   P_X [384 + 64 X, +64)
 //                          head dim 128: S_X [128 X, +128)   O_X [256 + 128 X, +128), P_X aliased on S_X [.., +64)
-// A softmax thread loads the 128 scores of its row into registers in one go and releases the S buffer
-// at once (head dim 64), so QK(j+1) of that tile runs while the thread is still working on step j and
-// the softmax threads never wait for the tensor cores; P(j) goes to its own columns as soon as PV(j-1)
-// has finished reading them.  With head dim 128 the 512 columns leave no room for separate P buffers:
-// P(j) overwrites the first 64 columns of S(j) and QK(j+1) is queued behind PV(j) (tcgen05.mma
-// instructions of one thread execute in issue order).
 // Both tiles read the same K/V tiles, so each is brought into shared memory once for 256 query rows.
 //
-// What was measured on the way to this form (B=2 H=16 D=64 non-causal, TFLOP/s at N = 2048 / 8192, A/B on one box):
-//   one issuer thread for both tiles, softmax warpgroups unordered                          485 / 657
-//   one issuer thread per tile (issuing an MMA occupies the thread for about the MMA's duration and a commit for
-//     ~130 clocks: one thread feeding both tiles was the bottleneck; polled with mbarrier.test_wait, because a
-//     try_wait on a barrier that is not ready may suspend the thread)                        472 / 679
-//   + the two warpgroups take turns on the exponential units, baton passed after a block     491 / 695
-//   + baton passed half way through a block (this kernel)                                    534 / 765
-//   a baton per scheduler (32 threads) instead of per warpgroup                              459 / 621
-//   the first TMA loads issued before the set-up barrier                                     459 / 621
-//   two threads per query row (640 threads, maxima exchanged through shared memory)          403 / 618
-//   25 % of the exponentials as a degree-3 polynomial on the FMA pipe                        527 / 753
-// A 128 x 128 score tile costs 1024 clocks of the SM's exponential units; a step timeline of this kernel shows ~1460
-// clocks of exponentials per warp and step and ~1200 of everything else (score load, maxima, P store, barriers), the two
-// tiles alternating: ~1570 clocks per tile and step, 65 % of the unit's rate.  The polynomial does not help because a
-// warp's block of exponentials is bound by its own dependency chain (FMA -> ex2 -> add / convert), not by the unit.
+// What a tile's rows are.  Two or more query tiles per head: 128 consecutive queries of one head, tiles A and B neighbours.
+// At most 128 queries per head and grouped heads: `heads_per_tile` heads of a group x all Nq queries, so that a tile is as
+// full as it gets and K/V is read once for the group (16 queries of 8 heads are one tile, not eight).
+//
+// What bounds it: the exponentials (a 128 x 128 tile costs 1024 clocks of the SM's exponential units) and, at head dim
+// 128, equally the tensor pipe (1024 clocks per tile and step).  Either is reached only if a softmax warp never waits, so
+// its own chain -- scores, maximum, exponentials, P, PV, next QK -- is what counts:
+//   * a softmax thread loads the 128 scores of its row into registers in one go.  Head dim 64 then releases the S buffer,
+//     and QK(j+1) runs under step j; P has columns of its own;
+//   * head dim 128: P(j) overwrites half of S(j), so QK(j+1) can only follow PV(j).  P is handed over in two halves, and
+//     PV starts on the first 64 keys while the exponentials of the others run;
+//   * the two tiles take turns on the exponential units (a "baton"): one tile's exponentials run under the other's score
+//     load, maxima, P store and products.  Left alone the tiles fall into step and compete for the same unit;
+//   * head dim 64 computes some exponentials on the FMA pipe (exp_pair_fma), which is idle otherwise.
+// Measured (TFLOP/s, graph of calls; the kernels before: event-loop issuers at head dim 64, one tile per CTA and two passes
+// over S at head dim 128): B=2 H=16 N=2048 D=64 582 -> 610, causal 479 -> 521; N=8192 D=128 causal 1009 -> 1083;
+// 509 queries on 4093 keys, 12 heads, D=128: 59 us -> 30 (key splits).
+// Also measured at D=64, N=2048 (us; this kernel 56.4): scores of step j+1 loaded chunk by chunk under the exponentials of
+// step j 64; no baton 64; baton passed after all exponentials 66; polynomial for 4 of 16 pairs 58.6, for 5 59.2.
+//
+// Split over keys: a problem with few tiles (short chunks against a long cache) is cut along the keys too; a CTA then
+// writes its unnormalised O and (m, l) per row and attn_prefill_merge_kernel puts the pieces together in order.
 // ------------------------------------------------------------------------------------------------
 namespace pair {
-
-#ifdef KFB_TRACE
-// Tuning aid of -DKFB_TRACE builds: CTA 0 writes clock stamps [role][step < 32][8] (roles: 0 softmax thread of
-// tile A, 1 of tile B, 2 issuer, 3 producer) into a buffer set through kfb_debug_set_attn_trace.
-__device__ unsigned long long* g_trace_buf = nullptr;
-#define KFB_STAMP(role, j, k)                                                                        \
-  do {                                                                                               \
-    if (trace_ptr != nullptr && (j) < 32) trace_ptr[((role) * 32 + (j)) * 8 + (k)] = clock64();   \
-  } while (0)
-#else
-#define KFB_STAMP(role, j, k) do { } while (0)
-#endif
 
 constexpr int kPairThreads = 384;   // three warpgroups
 constexpr int kPairProducerWarp = 8;
 constexpr int kPairMmaWarp = 9;
 constexpr uint32_t kPairTmemCols = 512;
+constexpr int kPolyPairs = 3;       // head dim 64: of 16 pairs of scores, this many take exp_pair_fma
 
 template <int D>
 struct PairLayout {
   static constexpr bool kAliasP = D == 128;
+  static constexpr int kHalves = kAliasP ? 2 : 1;     // pieces in which P is handed to the tensor cores
   static constexpr int kStages = D == 64 ? 4 : 2;
   static constexpr int kTile = kBlockN * D * 2;       // bytes of one 128-row tile (Q, K or V)
   static constexpr int kQ = 0;                        // Q_A, Q_B
   static constexpr int kK = 2 * kTile;
   static constexpr int kV = kK + kStages * kTile;
   static constexpr int kBars = kV + kStages * kTile;
-  static constexpr int kNumBars = 1 + 4 * kStages + 10;
+  static constexpr int kNumBars = 1 + 4 * kStages + 12;
   static constexpr int kMisc = kBars + kNumBars * 8;
   static constexpr int kBytes = kMisc + 16;
   static constexpr int kAlloc = kBytes + 1024;
@@ -486,65 +476,74 @@ struct PairLayout {
   static constexpr uint32_t kStrideP = kAliasP ? 128u : 64u;
 };
 
-// Maximum of the 128 scores of this thread's row (in registers); sixteen independent chains of
-// three-input maxima.  kMask: columns past `limit` count as -inf.
-template <bool kMask>
-__device__ __forceinline__ float row_max128(const uint32_t (&v)[4][32], int limit) {
-  float mx[16];
+struct Params {
+  int B, H, Hk, Nq, Nk, causal;
+  float scale_log2;
+  int heads_per_tile;    // 0: a tile is 128 queries of one head; else that many heads x all Nq queries
+  int tiles;             // tiles of a unit: a (batch, head), or a (batch, KV head) with heads_per_tile
+  int units_per_group;   // launch order, see decode_tile_order
+  int splits;            // pieces of the key range
+  float* partial;        // splits > 1: [split][B H Nq][D] floats, then [split][B H Nq][2] (m in log2 units, l)
+};
+
+// Columns c0 .. c0 + 31 past `limit` (causal diagonal / ragged end) become -inf.
+__device__ __forceinline__ void mask32(uint32_t (&v)[32], int c0, int limit) {
 #pragma unroll
-  for (int i = 0; i < 16; ++i) mx[i] = -INFINITY;
-#pragma unroll
-  for (int c = 0; c < 4; ++c)
-#pragma unroll
-    for (int i = 0; i < 32; i += 2) {
-      float x0 = __uint_as_float(v[c][i]), x1 = __uint_as_float(v[c][i + 1]);
-      if (kMask && c * 32 + i > limit) x0 = -INFINITY;
-      if (kMask && c * 32 + i + 1 > limit) x1 = -INFINITY;
-      mx[i >> 1] = max3(mx[i >> 1], x0, x1);
-    }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) mx[i] = fmaxf(max3(mx[i], mx[i + 4], mx[i + 8]), mx[i + 12]);
-  return fmaxf(max3(mx[0], mx[1], mx[2]), mx[3]);
+  for (int i = 0; i < 32; ++i)
+    if (c0 + i > limit) v[i] = 0xFF800000u;
 }
 
-// p = 2^(x * scale - base) for the 128 scores of the row, rounded to the I/O type into `p` (two per
-// register).  Returns the FP32 row sum of the unrounded p.  Scale-and-subtract and the row sum use the
-// two-wide FP32 instructions of sm_100 (one issue slot per two elements); results per element are
-// those of the scalar forms.
-template <bool kMask, bool kBf16>
-__device__ __forceinline__ float exp128(const uint32_t (&v)[4][32], uint32_t (&p)[4][16], int limit, float scale_log2,
-                                       float base, uint64_t* pass_baton) {
-  float2 sum[4] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
-  const float2 sc2 = make_float2(scale_log2, scale_log2), nb2 = make_float2(-base, -base);
+// Running maxima of 32 scores: four independent chains of three-input maxima.
+__device__ __forceinline__ void max32(const uint32_t (&v)[32], float (&mx)[4]) {
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      float2 x = make_float2(__uint_as_float(v[c][2 * i]), __uint_as_float(v[c][2 * i + 1]));
-      if (kMask && c * 32 + 2 * i > limit) x.x = -INFINITY;
-      if (kMask && c * 32 + 2 * i + 1 > limit) x.y = -INFINITY;
-      x = __ffma2_rn(x, sc2, nb2);
-      const float2 e = make_float2(ex2(x.x), ex2(x.y));
-      sum[i & 3] = __fadd2_rn(sum[i & 3], e);
-      p[c][i] = pack2<kBf16>(e.x, e.y);
-    }
-    if (c == 1) mbar_arrive(pass_baton);   // half way: the other warp's first exponentials fill the gaps of the last ones here
-  }
-  const float2 t = __fadd2_rn(__fadd2_rn(sum[0], sum[1]), __fadd2_rn(sum[2], sum[3]));
-  return t.x + t.y;
+  for (int i = 0; i < 32; i += 2) mx[(i >> 1) & 3] = max3(mx[(i >> 1) & 3], __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
+}
+__device__ __forceinline__ float max_of(const float (&mx)[4]) { return fmaxf(max3(mx[0], mx[1], mx[2]), mx[3]); }
+
+// Two scores, p = 2^(x * scale - base), rounded to the I/O type into one register; the unrounded p are added to `sum`.
+// Scale-and-subtract and the sums use the two-wide FP32 instructions of sm_100 (results per element are those of the scalar
+// forms).
+template <bool kBf16>
+__device__ __forceinline__ uint32_t exp_pair(uint32_t v0, uint32_t v1, float2 sc2, float2 nb2, float2& sum) {
+  const float2 x = __ffma2_rn(make_float2(__uint_as_float(v0), __uint_as_float(v1)), sc2, nb2);
+  const float2 e = make_float2(ex2(x.x), ex2(x.y));
+  sum = __fadd2_rn(sum, e);
+  return pack2<kBf16>(e.x, e.y);
+}
+
+constexpr float kExp2C1 = 0.693146944f, kExp2C2 = 0.240221202f, kExp2C3 = 0.0555071346f, kExp2C4 = 0.00967554096f,
+                kExp2C5 = 0.00132764538f;
+
+// The same on the FMA pipe instead of the exponential unit: 2^x = 2^r 2^f with r = rint(x), f in [-1/2, 1/2] (Cody and
+// Waite's reduction), 2^f by a degree-5 polynomial fitted for least relative error there (2^-22, like ex2.approx), r added
+// to the exponent.  x below -125 counts as -125: far below the last bit of any sum it enters.
+template <bool kBf16>
+__device__ __forceinline__ uint32_t exp_pair_fma(uint32_t v0, uint32_t v1, float2 sc2, float2 nb2, float2& sum) {
+  float2 x = __ffma2_rn(make_float2(__uint_as_float(v0), __uint_as_float(v1)), sc2, nb2);
+  x.x = fmaxf(x.x, -125.0f);
+  x.y = fmaxf(x.y, -125.0f);
+  auto both = [](float c) { return make_float2(c, c); };
+  const float2 t = __fadd2_rn(x, both(12582912.0f));   // 1.5 * 2^23: the low bits are rint(x)
+  const float2 f = __ffma2_rn(__fadd2_rn(t, both(-12582912.0f)), both(-1.0f), x);
+  float2 y = __ffma2_rn(both(kExp2C5), f, both(kExp2C4));
+  y = __ffma2_rn(y, f, both(kExp2C3));
+  y = __ffma2_rn(y, f, both(kExp2C2));
+  y = __ffma2_rn(y, f, both(kExp2C1));
+  y = __ffma2_rn(y, f, both(1.0f));
+  y.x = __uint_as_float(__float_as_uint(y.x) + (__float_as_uint(t.x) << 23));
+  y.y = __uint_as_float(__float_as_uint(y.y) + (__float_as_uint(t.y) << 23));
+  sum = __fadd2_rn(sum, y);
+  return pack2<kBf16>(y.x, y.y);
 }
 
 template <int D, bool kBf16>
 __global__ void __launch_bounds__(kPairThreads, 1)
 attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                         const __grid_constant__ CUtensorMap tm_v, void* __restrict__ o_ptr, const Strides o_st, int B, int H, int Hk, int Nq,
-                         int Nk, int causal, float scale_log2, int n_pairs, int heads_per_group, unsigned int* status) {
+                         const __grid_constant__ CUtensorMap tm_v, void* __restrict__ o_ptr, const Strides o_st,
+                         const __grid_constant__ Params pr, unsigned int* status) {
   using L = PairLayout<D>;
-  constexpr int S = L::kStages;
+  constexpr int S = L::kStages, kHalves = L::kHalves;
   constexpr bool kAliasP = L::kAliasP;
-#ifdef KFB_TRACE
-  const unsigned long long t_entry = clock64();
-#endif
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBars);
@@ -555,42 +554,54 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   uint64_t* v_empty = v_full + S;
   uint64_t* s_full = v_empty + S;    // [X]: S_X written by QK
   uint64_t* s_free = s_full + 2;     // [X]: all 128 threads of tile X hold their scores in registers
-  uint64_t* p_ready = s_free + 2;    // [X]: P_X stored by all 128 threads
-  uint64_t* pv_done = p_ready + 2;   // [X]: the PV product that read P_X has completed (O_X updated)
-  uint64_t* turn = pv_done + 2;      // [X]: the other tile's warpgroup is half way through its exponentials: X may start
+  uint64_t* p_ready = s_free + 2;    // [X][half]: P_X stored by all 128 threads
+  uint64_t* pv_done = p_ready + 4;   // [X]: the PV product that read P_X has completed (O_X updated)
+  uint64_t* turn = pv_done + 2;      // [X]: the baton: X may start its exponentials
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::kMisc);
   volatile uint32_t* abort_word = tmem_slot + 1;
   const AbortCtx ctx{abort_word, status};
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const TileOrder ord = decode_tile_order(blockIdx.x, n_pairs, H * B, heads_per_group);
-  const int pair_idx = ord.q_index;
-  const int h = ord.bh % H, b = ord.bh / H;
-  const int hk = h / (H / Hk);
-  const int q0 = pair_idx * 2 * kBlockM;
+  const int H = pr.H, Hk = pr.Hk, Nq = pr.Nq, Nk = pr.Nk, causal = pr.causal, hpt = pr.heads_per_tile;
+  const int per_batch = hpt ? Hk : H;   // units of a batch item
+  const TileOrder ord = decode_tile_order(blockIdx.x, (pr.tiles + 1) >> 1, pr.B * per_batch, pr.units_per_group);
+  const int tile0 = 2 * ord.q_index;
+  const int b = ord.bh / per_batch, within = ord.bh - b * per_batch;
+  const int hk = hpt ? within : within / (H / Hk);
   const int causal_off = Nk - Nq;
+  const bool has_b = tile0 + 1 < pr.tiles;
+  // first head and first query of tile X
+  auto head_of = [&](int X) { return hpt ? hk * (H / Hk) + (tile0 + X) * hpt : within; };
+  auto query_of = [&](int X) { return hpt ? 0 : (tile0 + X) * kBlockM; };
   int n_steps[2];
 #pragma unroll
   for (int X = 0; X < 2; ++X) {
-    const int q0x = q0 + X * kBlockM;
     int kv_end = Nk;
-    if (causal) kv_end = min(Nk, min(q0x + kBlockM, Nq) + causal_off);
-    n_steps[X] = q0x < Nq ? (kv_end + kBlockN - 1) / kBlockN : 0;   // tile B may not exist
+    if (causal && !hpt) kv_end = min(Nk, min(query_of(X) + kBlockM, Nq) + causal_off);
+    n_steps[X] = X == 0 || has_b ? (kv_end + kBlockN - 1) / kBlockN : 0;
   }
-  const int n_max = max(n_steps[0], n_steps[1]);
+  // this CTA's steps [j0, j0 + n_max) of the key range; tile X takes part in the first n_of(X) of them
+  int j0 = 0, n_max = max(n_steps[0], n_steps[1]);
+  if (pr.splits > 1) {
+    const int per = (n_max + pr.splits - 1) / pr.splits;
+    j0 = blockIdx.y * per;
+    n_max = max(0, min(n_max - j0, per));
+  }
+  auto n_of = [&](int X) { return max(0, min(n_steps[X] - j0, n_max)); };
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     for (int s = 0; s < S; ++s) {
       mbar_init(&k_full[s], 1);
-      mbar_init(&k_empty[s], 2);   // one arrival per issuer thread
+      mbar_init(&k_empty[s], 2);   // one arrival per issuer
       mbar_init(&v_full[s], 1);
       mbar_init(&v_empty[s], 2);
     }
     for (int X = 0; X < 2; ++X) {
       mbar_init(&s_full[X], 1);
       mbar_init(&s_free[X], 128);
-      mbar_init(&p_ready[X], 128);
+      mbar_init(&p_ready[2 * X], 128);
+      mbar_init(&p_ready[2 * X + 1], 128);
       mbar_init(&pv_done[X], 1);
       mbar_init(&turn[X], 128);
     }
@@ -601,6 +612,11 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     tmem_alloc(tmem_slot, kPairTmemCols);
     tmem_relinquish();
   }
+  if (warp == kPairProducerWarp && lane == 0) {
+    tma_prefetch_desc(&tm_q);
+    tma_prefetch_desc(&tm_k);
+    tma_prefetch_desc(&tm_v);
+  }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -608,277 +624,279 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   pdl_launch_dependents();
   const uint32_t tmem_base = *tmem_slot;
   const bool dead_on_arrival = *abort_word != 0;
-#ifdef KFB_TRACE
-  unsigned long long* const trace_ptr = blockIdx.x == 0 ? g_trace_buf : nullptr;
-  if (threadIdx.x == 0 && trace_ptr) { trace_ptr[31 * 8 + 0] = t_entry; trace_ptr[31 * 8 + 1] = clock64(); }
-#endif
 
-  // Registers move from the warpgroup of the two single-thread roles to the softmax warpgroups, which keep
+  // Registers move from the warpgroup of the three single-warp roles to the softmax warpgroups, which keep
   // the 128 scores of a row in registers (2 x 128 x 208 + 128 x 88 = 64512 of 65536).  Each role branch
   // starts with its setmaxnreg, executed by all four warps of its warpgroup.
   if (dead_on_arrival) {
     // fall through to the teardown
   } else if (warp >= kPairProducerWarp) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
-  if (warp == kPairProducerWarp) {
-    // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      tma_prefetch_desc(&tm_q);
-      tma_prefetch_desc(&tm_k);
-      tma_prefetch_desc(&tm_v);
-      const int tiles = n_steps[1] > 0 ? 2 : 1;
-      mbar_arrive_expect_tx(q_full, (uint32_t)(tiles * L::kTile));
-      for (int X = 0; X < tiles; ++X)
+    if (warp == kPairProducerWarp) {
+      // ---------------------------------------------------------------- TMA producer
+      if (lane == 0 && n_max > 0) {
+        const int tiles = has_b ? 2 : 1;
+        const int q_rows = hpt ? hpt * Nq : kBlockM;   // rows a Q copy brings (hpt: the box is hpt heads x Nq queries)
+        mbar_arrive_expect_tx(q_full, (uint32_t)(tiles * q_rows * D * 2));
+        for (int X = 0; X < tiles; ++X)
 #pragma unroll
-        for (int half = 0; half < D / 64; ++half)
-          tma_load_4d(smem + L::kQ + X * L::kTile + half * kHalfBytes, &tm_q, q_full, half * 64, q0 + X * kBlockM, h, b);
-      for (int j = 0; j < n_max; ++j) {
-        const int s = j % S;
-        const uint32_t ph = (uint32_t)(j / S) & 1u;
-        if (!mbar_wait(&k_empty[s], ph ^ 1u, ctx, kWaitKEmpty)) break;
-        mbar_arrive_expect_tx(&k_full[s], L::kTile);
+          for (int half = 0; half < D / 64; ++half)
+            tma_load_4d(smem + L::kQ + X * L::kTile + half * kHalfBytes, &tm_q, q_full, half * 64, query_of(X), head_of(X), b);
+        for (int i = 0; i < n_max; ++i) {
+          const int s = i % S, key0 = (j0 + i) * kBlockN;
+          const uint32_t ph = (uint32_t)(i / S) & 1u;
+          if (!mbar_wait(&k_empty[s], ph ^ 1u, ctx, kWaitKEmpty)) break;
+          mbar_arrive_expect_tx(&k_full[s], L::kTile);
 #pragma unroll
-        for (int half = 0; half < D / 64; ++half)
-          tma_load_4d(smem + L::kK + s * L::kTile + half * kHalfBytes, &tm_k, &k_full[s], half * 64, j * kBlockN, hk, b);
-        if (!mbar_wait(&v_empty[s], ph ^ 1u, ctx, kWaitVEmpty)) break;
-        mbar_arrive_expect_tx(&v_full[s], L::kTile);
+          for (int half = 0; half < D / 64; ++half)
+            tma_load_4d(smem + L::kK + s * L::kTile + half * kHalfBytes, &tm_k, &k_full[s], half * 64, key0, hk, b);
+          if (!mbar_wait(&v_empty[s], ph ^ 1u, ctx, kWaitVEmpty)) break;
+          mbar_arrive_expect_tx(&v_full[s], L::kTile);
 #pragma unroll
-        for (int half = 0; half < D / 64; ++half)
-          tma_load_4d(smem + L::kV + s * L::kTile + half * kHalfBytes, &tm_v, &v_full[s], half * 64, j * kBlockN, hk, b);
+          for (int half = 0; half < D / 64; ++half)
+            tma_load_4d(smem + L::kV + s * L::kTile + half * kHalfBytes, &tm_v, &v_full[s], half * 64, key0, hk, b);
+        }
       }
-    }
-  } else if (warp == kPairMmaWarp || warp == kPairMmaWarp + 1) {
-    // ------------------------------------------------------------------ tcgen05.mma issuers (one thread per tile)
-    // Issuing an MMA occupies the issuing thread for about as long as the MMA runs, and a commit for ~130 clocks,
-    // so one thread feeding both tiles is the bottleneck of the CTA; with one issuer per tile the commits of one
-    // overlap the MMAs of the other.  The two threads never touch each other's TMEM columns.  A K / V stage goes
-    // back to the producer when BOTH have arrived on its `empty` barrier (count 2): a tile that does not need a
-    // key tile (no tile B, or one step less under a causal mask) still arrives for it once it has been loaded.
-    if (lane == 0) {
+    } else if (warp == kPairMmaWarp || warp == kPairMmaWarp + 1) {
+      // ---------------------------------------------------------------- tcgen05.mma issuers (one warp per tile)
+      // The two warps never touch each other's TMEM columns.  A K / V stage goes back to the producer when BOTH have
+      // arrived on its `empty` barrier (count 2): a tile that does not need a key tile (no tile B, or one step less under
+      // a causal mask) still arrives for it once it has been loaded.
       const int X = warp - kPairMmaWarp;
       constexpr uint32_t idesc_qk = idesc_f16(kBlockM, kBlockN, kBf16 ? 1 : 0, 0, 0);
       constexpr uint32_t idesc_pv = idesc_f16(kBlockM, D, kBf16 ? 1 : 0, 0, 1);
-      const uint32_t qa = smem_u32(smem + L::kQ) + (uint32_t)X * L::kTile;
-      const uint32_t k_addr0 = smem_u32(smem + L::kK), v_addr0 = smem_u32(smem + L::kV);
+      const uint64_t q_desc = smem_desc_sw128(smem_u32(smem + L::kQ) + (uint32_t)X * L::kTile, 16, 1024);
+      const uint64_t k_desc = smem_desc_sw128(smem_u32(smem + L::kK), 16, 1024);
+      const uint64_t v_desc = smem_desc_sw128(smem_u32(smem + L::kV), kHalfBytes, 1024);
       const uint32_t s_col = tmem_base + L::kColS + 128u * X, o_col = tmem_base + L::kColO + (uint32_t)D * X;
       const uint32_t p_col = tmem_base + L::kColP + L::kStrideP * X;
-      const int n = n_steps[X];
-      int qk_next = 0, pv_next = 0;   // steps handled so far (issued, or passed on for a tile that has no such step)
-      bool ok = n == 0 || mbar_wait(q_full, 0, ctx, kWaitQ);
-      tc_fence_after_sync();
-      uint32_t idle = 0;
-      unsigned long long idle_since = 0;
-      while (ok && (qk_next < n_max || pv_next < n_max)) {
-        bool progress = false;
-        // ---- S(j) = Q K(j)^T: needs the S buffer (scores of step j-1 in registers; with aliased P: PV(j-1)
-        //      issued, which executes first) and the K tile
-        if (qk_next < n_max) {
-          const int j = qk_next, s = j % S;
-          if (j >= n) {   // not a step of this tile: hand the stage on as soon as it has been filled
-            if (mbar_test_wait(&k_full[s], (uint32_t)(j / S) & 1u)) {
-              mbar_arrive(&k_empty[s]);
-              qk_next = j + 1;
-              progress = true;
-            }
-          } else {
-            const bool buffer_free = kAliasP ? (pv_next >= j) : (j == 0 || mbar_test_wait(&s_free[X], (uint32_t)(j - 1) & 1u));
-            if (buffer_free && mbar_test_wait(&k_full[s], (uint32_t)(j / S) & 1u)) {
-              KFB_STAMP(2 + X, j, 0);
-              tc_fence_after_sync();
-              const uint32_t ka = k_addr0 + (uint32_t)s * L::kTile;
+      const int n = n_of(X);
+      bool ok = true;
+      auto wait_for = [&](uint64_t* bar, uint32_t parity, uint32_t code) {
+        ok = ok && __all_sync(0xffffffffu, mbar_wait(bar, parity, ctx, code));
+        return ok;
+      };
+      // S(j) = Q K(j)^T
+      auto qk = [&](int j) {
+        const int s = j % S;
+        if (!wait_for(&k_full[s], (uint32_t)(j / S) & 1u, kWaitKFull)) return;
+        tc_fence_after_sync();
+        const uint64_t kd = k_desc + (uint64_t)(s * (L::kTile >> 4));
+        if (elect_one()) {
 #pragma unroll
-              for (int kk = 0; kk < D / 16; ++kk) {
-                const uint32_t off = (uint32_t)(kk / 4) * kHalfBytes + (uint32_t)(kk % 4) * 32u;
-                mma_ss(s_col, smem_desc_sw128(qa + off, 16, 1024), smem_desc_sw128(ka + off, 16, 1024), idesc_qk,
-                       kk > 0 ? 1u : 0u);
-              }
-              KFB_STAMP(2 + X, j, 1);
-              tc_commit(&s_full[X]);
-              tc_commit(&k_empty[s]);
-              KFB_STAMP(2 + X, j, 2);
-              qk_next = j + 1;
-              progress = true;
-            }
+          for (int kk = 0; kk < D / 16; ++kk) {
+            const uint64_t off = (uint64_t)(((kk / 4) * kHalfBytes + (kk % 4) * 32) >> 4);
+            mma_ss(s_col, q_desc + off, kd + off, idesc_qk, kk > 0 ? 1u : 0u);
           }
+          tc_commit(&s_full[X]);
         }
-        // ---- O += P(j) V(j): needs P (stored by the 128 softmax threads of the tile) and the V tile
-        if (pv_next < n_max && pv_next < qk_next) {
-          const int j = pv_next, s = j % S;
-          if (j >= n) {
-            if (mbar_test_wait(&v_full[s], (uint32_t)(j / S) & 1u)) {
-              mbar_arrive(&v_empty[s]);
-              pv_next = j + 1;
-              progress = true;
-            }
-          } else if (mbar_test_wait(&p_ready[X], (uint32_t)j & 1u) && mbar_test_wait(&v_full[s], (uint32_t)(j / S) & 1u)) {
-            KFB_STAMP(2 + X, j, 3);
-            tc_fence_after_sync();
-            const uint32_t va = v_addr0 + (uint32_t)s * L::kTile;
+        __syncwarp();
+      };
+      // O += P(j) V(j), in kHalves pieces of the 128 keys
+      auto pv = [&](int j) {
+        const int s = j % S;
+        constexpr int kPer = kBlockN / 16 / kHalves;
+        if (!wait_for(&v_full[s], (uint32_t)(j / S) & 1u, kWaitVFull)) return;
+        const uint64_t vd = v_desc + (uint64_t)(s * (L::kTile >> 4));
 #pragma unroll
-            for (int kk = 0; kk < kBlockN / 16; ++kk) {
+        for (int half = 0; half < kHalves; ++half) {
+          if (!wait_for(&p_ready[2 * X + half], (uint32_t)j & 1u, kWaitPReady)) return;
+          tc_fence_after_sync();
+          if (elect_one()) {
+#pragma unroll
+            for (int kk = 0; kk < kPer; ++kk) {
               // 16 keys per MMA: 16 rows of 128 bytes; the second 64-column block of V is kHalfBytes away
-              mma_ts(o_col, p_col + (uint32_t)kk * 8u, smem_desc_sw128(va + kk * 2048, kHalfBytes, 1024), idesc_pv,
-                     (j > 0 || kk > 0) ? 1u : 0u);
+              const int k = half * kPer + kk;
+              mma_ts(o_col, p_col + (uint32_t)k * 8u, vd + (uint64_t)(k * (2048 >> 4)), idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
             }
-            KFB_STAMP(2 + X, j, 4);
-            tc_commit(&pv_done[X]);
-            tc_commit(&v_empty[s]);
-            KFB_STAMP(2 + X, j, 5);
-            pv_next = j + 1;
-            progress = true;
+            // (aliased P: S(j + 1) complete implies PV(j) complete, so only the last step needs a commit of its own)
+            if (half + 1 == kHalves && (!kAliasP || j + 1 == n)) tc_commit(&pv_done[X]);
           }
+          __syncwarp();
         }
-        if (progress) {
-          idle = 0;
-          idle_since = 0;
-        } else if ((++idle & 63u) == 0) {   // bounded like every other wait of the library
-          if (*abort_word != 0) break;
-          const unsigned long long now = globaltimer_ns();
-          if (idle_since == 0) {
-            idle_since = now;
-          } else if (now - idle_since > ctx.timeout_ns) {
-            *abort_word = kWaitIssuer;
-            atomicCAS(status, 0u, (unsigned int)kWaitIssuer);
-            break;
+      };
+      auto release = [&](uint64_t* bar) {
+        if (ok && elect_one()) tc_commit(bar);
+        __syncwarp();
+      };
+      // A commit keeps the issuing thread for some 50-130 clocks, so the ones that only return a stage come last.
+      if (n > 0) {
+        wait_for(q_full, 0, kWaitQ);
+        qk(0);
+        release(&k_empty[0]);
+        for (int j = 0; ok && j < n; ++j) {
+          const int next = j + 1;
+          if (!kAliasP && next < n) {   // S(j + 1) as soon as the scores of step j are in registers
+            wait_for(&s_free[X], (uint32_t)j & 1u, kWaitSFull);
+            qk(next);
           }
+          pv(j);
+          if (kAliasP && next < n) qk(next);   // tcgen05.mma instructions of one thread execute in issue order
+          release(&v_empty[j % S]);
+          if (next < n) release(&k_empty[next % S]);
         }
       }
+      for (int j = n; ok && j < n_max; ++j) {   // steps that only the other tile has: hand the stages on once filled
+        const int s = j % S;
+        const uint32_t ph = (uint32_t)(j / S) & 1u;
+        if (wait_for(&k_full[s], ph, kWaitKFull) && elect_one()) mbar_arrive(&k_empty[s]);
+        __syncwarp();
+        if (wait_for(&v_full[s], ph, kWaitVFull) && elect_one()) mbar_arrive(&v_empty[s]);
+        __syncwarp();
+      }
     }
-  }
   } else {
     // ------------------------------------------------------------------ softmax + epilogue (warps 0-7)
     asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
     const int X = warp >> 2;                      // which tile
     const int row = threadIdx.x & 127;            // query row inside the tile == TMEM lane
-    const int q0x = q0 + X * kBlockM;
-    const int n = n_steps[X];
+    const int head = head_of(X) + (hpt ? row / Nq : 0);
+    const int query = hpt ? row % Nq : query_of(X) + row;
+    const bool real = (X == 0 || has_b) && (hpt ? row < hpt * Nq : query < Nq);
+    const int n = n_of(X);
     const uint32_t lane_bits = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t s_tmem = tmem_base + L::kColS + 128u * X + lane_bits;
     const uint32_t p_tmem = tmem_base + L::kColP + L::kStrideP * X + lane_bits;
     const uint32_t o_tmem = tmem_base + L::kColO + (uint32_t)D * X + lane_bits;
+    const int row_limit = causal ? min(Nk - 1, query + causal_off) : Nk - 1;   // last visible key of this row
+    const int tile_limit = causal ? min(Nk - 1, query_of(X) + causal_off) : Nk - 1;   // ... of the tile's first row
+    const float2 sc2 = make_float2(pr.scale_log2, pr.scale_log2);
     float m_base = -INFINITY;  // the base O and l are currently expressed in (log2 units)
     float l_run = 0.f;
     bool ok = true;
-    for (int j = 0; j < n_max; ++j) {
-      const uint32_t ph = (uint32_t)j & 1u;
-      if (j >= n) {
-        // no such step for this tile (no tile B, or one step less under a causal mask): only pass the baton on
-        if (X == 1 || j > 0) {
-          ok = __all_sync(0xffffffffu, mbar_wait(&turn[X], (X == 1 ? ph : ph ^ 1u), ctx, kWaitTurn));
-          if (!ok) break;
-        }
-        mbar_arrive(&turn[X ^ 1]);
-        continue;
-      }
-      // every lane polls: measured faster than one polling lane plus a shuffle
-      ok = __all_sync(0xffffffffu, mbar_wait(&s_full[X], ph, ctx, kWaitSFull));
-      if (!ok) break;
-      if ((threadIdx.x & 127) == 0) KFB_STAMP(X, j, 0);
+    auto wait_all = [&](uint64_t* bar, uint32_t parity, uint32_t code) {   // every lane polls: faster than one and a shuffle
+      ok = __all_sync(0xffffffffu, mbar_wait(bar, parity, ctx, code));
+      return ok;
+    };
+    auto wait_turn = [&](int i) { return wait_all(&turn[X], (X == 1 ? (uint32_t)i : (uint32_t)i + 1u) & 1u, kWaitTurn); };
+    for (int i = 0; ok && i < n; ++i) {
+      const uint32_t ph = (uint32_t)i & 1u;
+      if (!wait_all(&s_full[X], ph, kWaitSFull)) break;
       tc_fence_after_sync();
-      uint32_t v[4][32];   // the 128 scores of this row, loaded once
-#pragma unroll
-      for (int c = 0; c < 4; ++c) tmem_ld_x32(s_tmem + c * 32, v[c]);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) tmem_wait_ld_regs(v[c]);
+      uint32_t v[4][32];         // the 128 scores of this row
+      float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+      const int k0 = (j0 + i) * kBlockN;
+      const bool masked = k0 + kBlockN - 1 > tile_limit;
+      auto fetch = [&](int c) { tmem_ld_x32(s_tmem + c * 32, v[c]); };
+      auto scan = [&](int c) {
+        if (masked) mask32(v[c], c * 32, row_limit - k0);
+        max32(v[c], mx);
+      };
+      fetch(0);
+      fetch(1);
+      tmem_wait_ld_regs(v[0]);
+      tmem_wait_ld_regs(v[1]);
+      fetch(2);
+      fetch(3);
+      scan(0);
+      scan(1);
+      tmem_wait_ld_regs(v[2]);
+      tmem_wait_ld_regs(v[3]);
       if constexpr (!kAliasP) {   // the S buffer can take the next product already
         tc_fence_before_sync();
         mbar_arrive(&s_free[X]);
       }
-      if ((threadIdx.x & 127) == 0) KFB_STAMP(X, j, 1);
-      const int k0 = j * kBlockN;
-      const bool need_mask = (k0 + kBlockN > Nk) || (causal && (k0 + kBlockN - 1 > q0x + causal_off));
-      int limit = Nk - 1;
-      if (causal) limit = min(limit, q0x + row + causal_off);
-      limit -= k0;  // last visible column of this step for this row
-
-      const float m_step = (need_mask ? row_max128<true>(v, limit) : row_max128<false>(v, limit)) * scale_log2;
+      scan(2);
+      scan(3);
+      const float m_step = max_of(mx) * pr.scale_log2;
       // lazy rescale: move the base only when the maximum outgrew it by more than the threshold
-      const bool grow = m_step > m_base + kRescaleThreshold || m_base == -INFINITY;
-      float alpha = 1.0f;
-      if (grow && m_step != -INFINITY) {
-        alpha = ex2(m_base - m_step);  // 0 when m_base is still -inf
-        m_base = m_step;
-      }
+      const bool grow = m_step > m_base + kRescaleThreshold;   // (-inf + 8 = -inf: the first finite maximum counts)
+      const float alpha = grow ? ex2(m_base - m_step) : 1.0f;  // 0 when m_base is still -inf
+      m_base = grow ? m_step : m_base;
       const float base = (m_base == -INFINITY) ? 0.f : m_base;
-      if ((threadIdx.x & 127) == 0) KFB_STAMP(X, j, 2);
-      bool rescaled = false;
-      if (j > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) {
+      bool pv_waited = kAliasP || i == 0;   // (with aliased P, S(j) complete implies PV(j-1) complete)
+      if (i > 0 && __any_sync(0xffffffffu, grow)) {
         // O is rescaled between PV(j-1), which must have finished accumulating, and PV(j), which cannot have
         // started (it waits for this step's P).  Rare after the first steps.
-        rescaled = true;
-        if constexpr (!kAliasP) {
-          ok = __all_sync(0xffffffffu, mbar_wait(&pv_done[X], (uint32_t)(j - 1) & 1u, ctx, kWaitPvDone));
-          if (!ok) break;
-          tc_fence_after_sync();
-        }
-        {
+        if (!pv_waited && !wait_all(&pv_done[X], ph ^ 1u, kWaitPvDone)) break;
+        pv_waited = true;
+        tc_fence_after_sync();
 #pragma unroll
-          for (int c = 0; c < D / 32; ++c) {
-            uint32_t o[32];
-            tmem_ld_x32(o_tmem + c * 32, o);
-            tmem_wait_ld();
+        for (int c = 0; c < D / 32; ++c) {
+          uint32_t o[32];
+          tmem_ld_x32(o_tmem + c * 32, o);
+          tmem_wait_ld();
 #pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-            tmem_st_x32(o_tmem + c * 32, o);
-          }
+          for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
+          tmem_st_x32(o_tmem + c * 32, o);
         }
       }
-      // The two warpgroups take turns on the exponential units: A(0), B(0), A(1), B(1), ...  Left alone they drift into
-      // phase: both load scores and take maxima at the same time (units idle), then both want the units.  With the
-      // baton one runs its exponentials while the other loads, takes maxima, stores P and synchronises.  The baton is
-      // passed half way through, so the tail of one block overlaps the head of the next.  A waits for B(j-1), B for
-      // A(j).  (A baton per scheduler -- 32 threads instead of 128 -- measured 15 % slower: 74 against 64 us at
-      // B=2 H=16 N=2048; so did issuing the first TMA loads before the set-up barrier.)
-      if (X == 1 || j > 0) {
-        ok = __all_sync(0xffffffffu, mbar_wait(&turn[X], (X == 1 ? ph : ph ^ 1u), ctx, kWaitTurn));
-        if (!ok) break;
-      }
-      if ((threadIdx.x & 127) == 0) KFB_STAMP(X, j, 6);
-      uint32_t p16[4][16];
-      const float step_sum = need_mask ? exp128<true, kBf16>(v, p16, limit, scale_log2, base, &turn[X ^ 1])
-                                       : exp128<false, kBf16>(v, p16, limit, scale_log2, base, &turn[X ^ 1]);
-      l_run = fmaf(l_run, alpha, step_sum);
-      if ((threadIdx.x & 127) == 0) KFB_STAMP(X, j, 3);
-      if constexpr (!kAliasP) {
-        // PV(j-1) must have finished reading the P columns before they are overwritten.  By now it has: the
-        // exponentials above take longer than the product.  (With aliased P it finished before S(j) was
-        // written, which this thread has already waited for.)
-        if (j > 0 && !rescaled) {
-          ok = __all_sync(0xffffffffu, mbar_wait(&pv_done[X], (uint32_t)(j - 1) & 1u, ctx, kWaitPvDone));
-          if (!ok) break;
-          tc_fence_after_sync();
-        }
-      }
-      if ((threadIdx.x & 127) == 0) KFB_STAMP(X, j, 4);
+      if ((X == 1 || i > 0) && !wait_turn(i)) break;
+      const float2 nb2 = make_float2(-base, -base);
+      float2 sum[2] = {{0.f, 0.f}, {0.f, 0.f}};
+      uint32_t p[4][16];
+      auto expo = [&](int c, int e) {
+        if (!kAliasP && e < kPolyPairs) p[c][e] = exp_pair_fma<kBf16>(v[c][2 * e], v[c][2 * e + 1], sc2, nb2, sum[e & 1]);
+        else p[c][e] = exp_pair<kBf16>(v[c][2 * e], v[c][2 * e + 1], sc2, nb2, sum[e & 1]);
+      };
+      auto chunk = [&](int c) {   // (the order spreads the polynomials among the others)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) tmem_st_x16(p_tmem + c * 16, p16[c]);
+        for (int e = 0; e < 16; ++e) expo(c, (e * 5) & 15);
+      };
+      auto pass_baton = [&]() {   // (the operands keep the exponentials summed so far in front of it)
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0]; // %1 %2" ::"r"(smem_u32(&turn[X ^ 1])), "f"(sum[0].x), "f"(sum[1].x) : "memory");
+      };
+      chunk(0);
+      chunk(1);
+      if (!kAliasP) pass_baton();
+      if constexpr (kHalves == 2) {
+        tmem_st_x16(p_tmem, p[0]);
+        tmem_st_x16(p_tmem + 16, p[1]);
+        tmem_wait_st();
+        tc_fence_before_sync();
+        mbar_arrive(&p_ready[2 * X]);
+      }
+      chunk(2);
+      if (kAliasP) pass_baton();
+      chunk(3);
+      const float2 t = __fadd2_rn(sum[0], sum[1]);
+      l_run = fmaf(l_run, alpha, t.x + t.y);
+      if (!pv_waited) {   // PV(j-1) must have finished reading the P columns before they are overwritten: by now it has
+        if (!wait_all(&pv_done[X], ph ^ 1u, kWaitPvDone)) break;
+        tc_fence_after_sync();
+      }
+#pragma unroll
+      for (int c = kHalves == 2 ? 2 : 0; c < 4; ++c) tmem_st_x16(p_tmem + 16 * c, p[c]);
       tmem_wait_st();
       tc_fence_before_sync();
-      mbar_arrive(&p_ready[X]);
-      if ((threadIdx.x & 127) == 0) KFB_STAMP(X, j, 5);
+      mbar_arrive(&p_ready[2 * X + kHalves - 1]);
+    }
+    for (int i = n; ok && i < n_max; ++i) {   // steps that only the other tile has: pass the baton on
+      if ((X == 1 || i > 0) && !wait_turn(i)) break;
+      mbar_arrive(&turn[X ^ 1]);
     }
     // PVs complete in issue order: the last one done means all are
-    if (ok && n > 0) ok = __all_sync(0xffffffffu, mbar_wait(&pv_done[X], (uint32_t)(n - 1) & 1u, ctx, kWaitPvDone));
-    if (ok && n > 0) {
-      if (threadIdx.x == 0) KFB_STAMP(0, 31, 2);
+    if (ok && n > 0) wait_all(&pv_done[X], kAliasP ? 0u : (uint32_t)(n - 1) & 1u, kWaitPvDone);
+    if (ok) {
       tc_fence_after_sync();
-      const float inv_l = 1.0f / l_run;
-      const bool store = q0x + row < Nq;
-      uint8_t* dst = static_cast<uint8_t*>(o_ptr) + (b * o_st.b + h * o_st.h + (long long)(q0x + row) * o_st.n) * 2;
+      const long long grow_row = ((long long)b * H + head) * Nq + query;   // row of the dense [B H Nq] order of the partials
+      const long long rows = (long long)pr.B * H * Nq;
+      const bool part = pr.splits > 1;
+      float* o32 = part ? pr.partial + ((long long)blockIdx.y * rows + grow_row) * D : nullptr;
+      uint8_t* dst = static_cast<uint8_t*>(o_ptr) + (b * o_st.b + head * o_st.h + query * o_st.n) * 2;
+      if (part && real)
+        reinterpret_cast<float2*>(pr.partial + pr.splits * rows * D)[(long long)blockIdx.y * rows + grow_row] = make_float2(m_base, l_run);
+      if (n > 0) {
+        const float inv_l = 1.0f / l_run;
 #pragma unroll
-      for (int c = 0; c < D / 32; ++c) {
-        uint32_t o[32];
-        tmem_ld_x32(o_tmem + c * 32, o);
-        tmem_wait_ld();
-        if (store) {
-          uint32_t packed[16];
+        for (int c = 0; c < D / 32; ++c) {
+          uint32_t o[32];
+          tmem_ld_x32(o_tmem + c * 32, o);
+          tmem_wait_ld_regs(o);
+          if (real && part) {
 #pragma unroll
-          for (int i = 0; i < 16; ++i)
-            packed[i] = pack2<kBf16>(__uint_as_float(o[2 * i]) * inv_l, __uint_as_float(o[2 * i + 1]) * inv_l);
+            for (int e = 0; e < 8; ++e)
+              reinterpret_cast<uint4*>(o32 + c * 32)[e] = make_uint4(o[4 * e], o[4 * e + 1], o[4 * e + 2], o[4 * e + 3]);
+          } else if (real) {
+            uint32_t packed[16];
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            reinterpret_cast<uint4*>(dst + c * 64)[i] =
-                make_uint4(packed[4 * i], packed[4 * i + 1], packed[4 * i + 2], packed[4 * i + 3]);
+            for (int e = 0; e < 16; ++e)
+              packed[e] = pack2<kBf16>(__uint_as_float(o[2 * e]) * inv_l, __uint_as_float(o[2 * e + 1]) * inv_l);
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              reinterpret_cast<uint4*>(dst + c * 64)[e] =
+                  make_uint4(packed[4 * e], packed[4 * e + 1], packed[4 * e + 2], packed[4 * e + 3]);
+          }
         }
       }
     }
@@ -889,31 +907,87 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     const unsigned long long t0 = globaltimer_ns();
     while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);  // let copies in flight land
   }
-  if (threadIdx.x == 0) KFB_STAMP(0, 31, 3);
   tc_fence_before_sync();
   __syncthreads();
-  if (threadIdx.x == 0) KFB_STAMP(0, 31, 4);
   if (warp == kPairMmaWarp) {
     __syncwarp();
     tmem_dealloc(tmem_base, kPairTmemCols);
   }
-  if (threadIdx.x == kPairMmaWarp * 32) KFB_STAMP(0, 31, 5);
+}
+
+// o[row] = sum over splits of 2^(m_s - m) O_s[row] / sum of 2^(m_s - m) l_s, in split order.  A row per D / 4 threads.
+template <int D, bool kBf16>
+__global__ void __launch_bounds__(256) attn_prefill_merge_kernel(const float* __restrict__ partial, void* __restrict__ o_ptr, const Strides o_st,
+                                                                 int H, int Nq, long long rows, int splits) {
+  pdl_wait(partial);
+  pdl_launch_dependents();
+  constexpr int kPerRow = D / 4;
+  const long long idx = (long long)blockIdx.x * 256 + threadIdx.x, row = idx / kPerRow;
+  const int c = (int)(idx % kPerRow) * 4;
+  if (row >= rows) return;
+  const float2* ml = reinterpret_cast<const float2*>(partial + splits * rows * D);
+  float m = -INFINITY;
+  for (int s = 0; s < splits; ++s) m = fmaxf(m, ml[s * rows + row].x);
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  float l = 0.f;
+#pragma unroll 4
+  for (int s = 0; s < splits; ++s) {
+    const float2 w = ml[s * rows + row];
+    if (w.x == -INFINITY) continue;   // no step of this split reached the row (its O was not written)
+    const float f = ex2(w.x - m);
+    const float4 v = *reinterpret_cast<const float4*>(partial + (s * rows + row) * D + c);
+    acc.x = fmaf(f, v.x, acc.x); acc.y = fmaf(f, v.y, acc.y); acc.z = fmaf(f, v.z, acc.z); acc.w = fmaf(f, v.w, acc.w);
+    l = fmaf(f, w.y, l);
+  }
+  const float inv = 1.0f / l;
+  const long long bh = row / Nq;
+  uint8_t* dst = static_cast<uint8_t*>(o_ptr) + (bh / H * o_st.b + bh % H * o_st.h + (row - bh * Nq) * o_st.n + c) * 2;
+  *reinterpret_cast<uint2*>(dst) = make_uint2(pack2<kBf16>(acc.x * inv, acc.y * inv), pack2<kBf16>(acc.z * inv, acc.w * inv));
 }
 
 }  // namespace pair
 
-// Head dims the pair kernel serves (the others, and single-tile problems, take the single-tile kernel).
-constexpr bool pair_kernel_for(int D) {
-#ifdef KFB_PAIR_D128
-  return D == 64 || D == 128;
-#else
-  return D == 64;
-#endif
+// How a problem is cut (see the header of the pair kernel).
+struct PrefillPlan {
+  bool serial;
+  int heads_per_tile, tiles, units, splits;
+};
+
+PrefillPlan plan_prefill(const Problem& p) {
+  PrefillPlan c;
+  const int G = p.H / p.Hk, q_tiles = ceil_div(p.Nq, kBlockM), sms = sm_count();
+  c.heads_per_tile = 0;
+  c.tiles = q_tiles;
+  c.units = p.B * p.H;
+  if (q_tiles == 1 && G > 1) {
+    c.heads_per_tile = 1;
+    for (int d = 2; d <= G; ++d)
+      if (G % d == 0 && d * p.Nq <= kBlockM) c.heads_per_tile = d;
+    c.tiles = G / c.heads_per_tile;
+    c.units = p.B * p.Hk;
+  }
+  const long long ctas = (long long)c.units * ((c.tiles + 1) / 2);
+  // One tile per unit, ungrouped heads and more of them than SMs: the single-tile kernel keeps two tiles on an SM.
+  c.serial = c.tiles == 1 && c.heads_per_tile == 0 && ctas > sms;
+  // Key splits, by time in key steps (~1.5 us): set-up and drain of a CTA cost about two, the merge kernel two plus its
+  // traffic (partials written and read at ~4 TB/s).  Only grids smaller than the GPU gain.
+  c.splits = 1;
+  if (!c.serial) {
+    const int steps = ceil_div(p.Nk, kBlockN);
+    const double rows_mb = (double)p.B * p.H * p.Nq * p.D * 8.0 / 6.0e6;
+    double best = 1e30;
+    for (int s = 1; s <= steps && s <= 32 && (s == 1 || ctas * s <= sms); ++s) {
+      if (ceil_div(steps, ceil_div(steps, s)) != s) continue;   // an empty split
+      const double cost = (double)((ctas * s + sms - 1) / sms) * (ceil_div(steps, s) + 2.0) + (s > 1 ? 2.0 + s * rows_mb : 0.0);
+      if (cost < best) { best = cost; c.splits = s; }
+    }
+  }
+  return c;
 }
 
 template <int D, bool kBf16>
-int launch(const Problem& p, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, unsigned int* status,
-           cudaStream_t stream) {
+int launch(const Problem& p, const PrefillPlan& plan, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, float* partial,
+           unsigned int* status, cudaStream_t stream) {
   using L = Layout<D>;
   using PL = pair::PairLayout<D>;
   static bool configured[64] = {false};
@@ -930,31 +1004,45 @@ int launch(const Problem& p, const CUtensorMap& tq, const CUtensorMap& tk, const
   }
   const float scale_log2 = p.scale * 1.4426950408889634f;
   const Strides o_st{p.o_stride_b, p.o_stride_h, p.o_stride_n};
-  const int q_tiles = ceil_div(p.Nq, kBlockM);
-  const long long bh = (long long)p.B * p.H;
-  // heads whose K and V (one KV head each at worst) fit in ~48 MB of L2 together
-  const long long kv_bytes_per_head = 4LL * p.Nk * p.D;
-  const int heads_per_group = (int)std::min<long long>(bh, std::max<long long>(1, (48LL << 20) / kv_bytes_per_head));
-  if (pair_kernel_for(D) && q_tiles >= 2) {
-    const int n_pairs = ceil_div(q_tiles, 2);
-    if (bh * n_pairs > 0x7fffffffLL) return fail(KFB_ERR_INVALID, "too many query tiles for one launch");
-    return launch_kernel("attn_prefill_pair_kernel", pair::attn_prefill_pair_kernel<D, kBf16>, dim3((unsigned)(bh * n_pairs)),
-                         dim3(pair::kPairThreads), PL::kAlloc, stream, tq, tk, tv, p.o, o_st, p.B, p.H, p.Hk, p.Nq, p.Nk, p.causal, scale_log2,
-                         n_pairs, heads_per_group, status);
-  }
-  if (bh * q_tiles > 0x7fffffffLL) return fail(KFB_ERR_INVALID, "too many query tiles for one launch");
-  return launch_kernel("attn_prefill_serial_kernel", serial::attn_prefill_serial_kernel<D, kBf16>, dim3((unsigned)(bh * q_tiles)), dim3(kThreads),
-                       L::kAlloc, stream, tq, tk, tv, p.o, o_st, p.H, p.Hk, p.Nq, p.Nk, p.causal, scale_log2, p.B, q_tiles, heads_per_group, status);
+  // units whose K and V (one KV head each at worst) fit in ~48 MB of L2 together
+  const long long kv_bytes_per_unit = 4LL * p.Nk * p.D;
+  const int units_per_group = (int)std::min<long long>(plan.units, std::max<long long>(1, (48LL << 20) / kv_bytes_per_unit));
+  const long long ctas = (long long)plan.units * (plan.serial ? plan.tiles : (plan.tiles + 1) / 2);
+  if (ctas > 0x7fffffffLL) return fail(KFB_ERR_INVALID, "too many query tiles for one launch");
+  if (plan.serial)
+    return launch_kernel("attn_prefill_serial_kernel", serial::attn_prefill_serial_kernel<D, kBf16>, dim3((unsigned)ctas), dim3(kThreads),
+                         L::kAlloc, stream, tq, tk, tv, p.o, o_st, p.H, p.Hk, p.Nq, p.Nk, p.causal, scale_log2, p.B, plan.tiles,
+                         units_per_group, status);
+  pair::Params pr = {p.B, p.H, p.Hk, p.Nq, p.Nk, p.causal, scale_log2, plan.heads_per_tile, plan.tiles, units_per_group, plan.splits, partial};
+  if (int rc = launch_kernel("attn_prefill_pair_kernel", pair::attn_prefill_pair_kernel<D, kBf16>, dim3((unsigned)ctas, plan.splits),
+                             dim3(pair::kPairThreads), PL::kAlloc, stream, tq, tk, tv, p.o, o_st, pr, status))
+    return rc;
+  if (plan.splits == 1) return KFB_OK;
+  const long long rows = (long long)p.B * p.H * p.Nq, blocks = (rows * (D / 4) + 255) / 256;
+  return launch_kernel("attn_prefill_merge_kernel", pair::attn_prefill_merge_kernel<D, kBf16>, dim3((unsigned)blocks), dim3(256), 0, stream,
+                       (const float*)partial, p.o, o_st, p.H, p.Nq, rows, plan.splits);
+}
+
+size_t partial_bytes(const Problem& p, const PrefillPlan& plan) {
+  return plan.splits > 1 ? (size_t)plan.splits * p.B * p.H * p.Nq * (p.D + 2) * sizeof(float) : 0;
 }
 
 }  // namespace
 
-int launch_prefill(const Problem& given, cudaStream_t stream) {
+size_t prefill_ws_bytes(int B, int H, int Hk, int Nq, int Nk, int D) {
+  Problem p = {};
+  p.B = B; p.H = H; p.Hk = Hk; p.Nq = Nq; p.Nk = Nk; p.D = D;
+  return partial_bytes(p, plan_prefill(p));
+}
+
+int launch_prefill(const Problem& given, void* ws, size_t ws_bytes, cudaStream_t stream) {
   Problem p = given;
   if (p.q_stride_n == 0) { p.q_stride_n = p.D; p.q_stride_h = (long long)p.Nq * p.D; p.q_stride_b = (long long)p.H * p.Nq * p.D; }
   if (p.o_stride_n == 0) { p.o_stride_n = p.D; p.o_stride_h = (long long)p.Nq * p.D; p.o_stride_b = (long long)p.H * p.Nq * p.D; }
   unsigned int* status = device_status_word();
   if (!status) return fail(KFB_ERR_CUDA, "cannot resolve the device status word");
+  PrefillPlan plan = plan_prefill(p);
+  if (!ws || !aligned16(ws) || ws_bytes < partial_bytes(p, plan)) plan.splits = 1;   // the workspace is optional
   CUtensorMap tq, tk, tv;
   const uint64_t D = p.D;
   const uint64_t qd[4] = {D, (uint64_t)p.Nq, (uint64_t)p.H, (uint64_t)p.B};
@@ -962,19 +1050,16 @@ int launch_prefill(const Problem& given, cudaStream_t stream) {
   const uint64_t kd[4] = {D, (uint64_t)p.Nk, (uint64_t)p.Hk, (uint64_t)p.B};
   const uint64_t ks[3] = {(uint64_t)p.kv_stride_n * 2, (uint64_t)p.kv_stride_h * 2, (uint64_t)p.kv_stride_b * 2};
   const uint32_t box[4] = {64, 128, 1, 1};
-  if (int rc = make_tmap_4d_sw128(&tq, p.q, p.dtype, qd, qs, box)) return rc;
+  const uint32_t qbox[4] = {64, plan.heads_per_tile ? (uint32_t)p.Nq : 128u, plan.heads_per_tile ? (uint32_t)plan.heads_per_tile : 1u, 1};
+  if (int rc = make_tmap_4d_sw128(&tq, p.q, p.dtype, qd, qs, qbox)) return rc;
   if (int rc = make_tmap_4d_sw128(&tk, p.k, p.dtype, kd, ks, box)) return rc;
   if (int rc = make_tmap_4d_sw128(&tv, p.v, p.dtype, kd, ks, box)) return rc;
   const bool bf16 = p.dtype == KFB_BF16;
-  if (p.D == 64) return bf16 ? launch<64, true>(p, tq, tk, tv, status, stream) : launch<64, false>(p, tq, tk, tv, status, stream);
-  return bf16 ? launch<128, true>(p, tq, tk, tv, status, stream) : launch<128, false>(p, tq, tk, tv, status, stream);
+  float* partial = static_cast<float*>(ws);
+  if (p.D == 64)
+    return bf16 ? launch<64, true>(p, plan, tq, tk, tv, partial, status, stream) : launch<64, false>(p, plan, tq, tk, tv, partial, status, stream);
+  return bf16 ? launch<128, true>(p, plan, tq, tk, tv, partial, status, stream) : launch<128, false>(p, plan, tq, tk, tv, partial, status, stream);
 }
 
 }  // namespace attn
 }  // namespace kfb
-
-#ifdef KFB_TRACE
-extern "C" void kfb_debug_set_attn_trace(void* device_buffer) {
-  cudaMemcpyToSymbol(kfb::attn::pair::g_trace_buf, &device_buffer, sizeof(void*));
-}
-#endif

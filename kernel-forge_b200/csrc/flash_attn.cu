@@ -31,7 +31,8 @@ int set_kv_strides(attn::Problem* p, const int64_t* st) {
 }  // namespace
 
 extern "C" size_t kfb_flash_attn_ws_bytes(int B, int H, int Hk, int Nq, int Nk, int D) {
-  if (B < 1 || H < 1 || Hk < 1 || Nq != 1 || Nk < 1 || (D != 64 && D != 128) || H % Hk) return 0;
+  if (B < 1 || H < 1 || Hk < 1 || Nq < 1 || Nk < 1 || (D != 64 && D != 128) || H % Hk) return 0;
+  if (Nq > 1) return attn::prefill_ws_bytes(B, H, Hk, Nq, Nk, D);
   return attn::decode_ws_bytes(B, H, Hk, Nk, D);
 }
 
@@ -52,7 +53,7 @@ extern "C" int kfb_flash_attn_fwd(const void* q, const void* k, const void* v, v
   if (int rc = set_kv_strides(&p, kv_strides)) return rc;
   cudaStream_t s = (cudaStream_t)stream;
   if (Nq == 1) return attn::launch_decode(p, ws, ws_bytes, s);
-  return attn::launch_prefill(p, s);
+  return attn::launch_prefill(p, ws, ws_bytes, s);
 }
 
 // The same for tensors in token-major layout (what a projection writes and the next one reads): q and o [B, Nq, H, D].
@@ -76,7 +77,7 @@ extern "C" int kfb_flash_attn_fwd_tokens(const void* q, const void* k, const voi
   p.q_stride_h = p.o_stride_h = D;
   p.q_stride_n = p.o_stride_n = (long long)H * D;
   p.q_stride_b = p.o_stride_b = (long long)Nq * H * D;
-  return attn::launch_prefill(p, (cudaStream_t)stream);
+  return attn::launch_prefill(p, ws, ws_bytes, (cudaStream_t)stream);
 }
 
 // Decode attention against a static KV cache whose valid length lives on the device.
