@@ -1,14 +1,11 @@
 // Fused attention forward for sm_100a, general path (any Nq, Nk; GQA; bottom-right causal mask).
 //
 // Replaces attn_v4_kernel of the reference (csrc/attention/attn_v4_kernel.cuh:43-214), which is an
-// mma.sync / ldmatrix / cp.async kernel.  Two kernels built on the Blackwell execution model (TMA into
-// 128-byte-swizzled shared-memory tiles, tcgen05.mma issued by one thread, accumulators in TMEM):
+// mma.sync / ldmatrix / cp.async kernel.  One kernel built on the Blackwell execution model (TMA into
+// 128-byte-swizzled shared-memory tiles, tcgen05.mma issued by one thread, accumulators in TMEM), with two
+// tiles of 128 query rows per CTA or one, and a merge kernel for key splits.
 //
-//   pair::attn_prefill_pair_kernel     one CTA per SM, two tiles of 128 query rows, key splits: nearly everything;
-//   serial::attn_prefill_serial_kernel one CTA per tile, two CTAs per SM (256 TMEM columns each): many heads that
-//                                      have a single tile each and no partner to share K / V with.
-//
-// Common to both: thread r of a softmax warpgroup owns query row r = TMEM lane r, so row maximum and
+// Thread r of a softmax warpgroup owns query row r = TMEM lane r, so row maximum and
 // row sum need no shuffles; lazy rescale (the running base of a row only moves when the new maximum
 // exceeds it by more than 8 in log2 units -- a factor 256, far inside fp32 range -- and only then is
 // O in TMEM rescaled; O and l always share one base, so O / l is unaffected); causal: key steps above
@@ -33,30 +30,11 @@ using namespace sm100;
 
 constexpr int kBlockM = 128;
 constexpr int kBlockN = 128;   // keys per TMA tile and per step
-constexpr int kThreads = 192;  // single-tile kernel
-constexpr int kProducerWarp = 4;
-constexpr int kMmaWarp = 5;
-constexpr uint32_t kTmemCols = 256;
 constexpr int kHalfBytes = kBlockN * 128;  // one 64-column half of a tile: 128 rows x 128 bytes
 constexpr float kRescaleThreshold = 8.0f;  // log2 units
 
 enum WaitCode : uint32_t {
   kWaitQ = 0x101, kWaitKEmpty, kWaitKFull, kWaitVEmpty, kWaitVFull, kWaitSFull, kWaitPReady, kWaitPvDone, kWaitIssuer, kWaitTurn
-};
-
-template <int D>
-struct Layout {
-  static constexpr int kStages = D == 64 ? 2 : 1;
-  static constexpr int kTile = kBlockN * D * 2;
-  static constexpr int kQ = 0;
-  static constexpr int kK = kTile;
-  static constexpr int kV = kK + kStages * kTile;
-  static constexpr int kBars = kV + kStages * kTile;
-  static constexpr int kNumBars = 4 * kStages + 7;
-  static constexpr int kMisc = kBars + kNumBars * 8;
-  static constexpr int kBytes = kMisc + 16;
-  static constexpr int kAlloc = kBytes + 1024;  // room to align the tiles to 1024 bytes
-  static_assert(2 * kAlloc <= 227 * 1024, "two CTAs must fit on one SM");
 };
 
 __device__ __forceinline__ float ex2(float x) {
@@ -104,322 +82,16 @@ __device__ __forceinline__ TileOrder decode_tile_order(unsigned int block, int n
 }
 
 // ------------------------------------------------------------------------------------------------
-// Single-tile kernel: one CTA per 128 query rows, two CTAs resident per SM (256 TMEM columns each).
-// One S buffer of 128 keys, QK(j+1) issued behind PV(j), the softmax in two passes over S in TMEM
-// (maximum, then exponentials), P aliased on the S columns already consumed.  Used for problems with
-// a single query tile per head, ungrouped heads and more of them than SMs, where a CTA of the pair
-// kernel below would run half empty.
-// ------------------------------------------------------------------------------------------------
-namespace serial {
-
-constexpr uint32_t kSerialColS = 0, kSerialColP = 0, kSerialColO = 128;
-
-// Row maximum of the 128 scores of this thread's row.  The four 32-column TMEM loads are issued
-// back to back (the data of chunk c+1 is in flight while chunk c is reduced); eight independent
-// max chains.  kMask: columns past `limit` (causal diagonal / ragged tile) count as -inf.
-template <bool kMask>
-__device__ __forceinline__ float row_max(uint32_t s_tmem, int limit) {
-  float mx[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) mx[i] = -INFINITY;
-  uint32_t v[2][32];
-  tmem_ld_x32(s_tmem, v[0]);
-  tmem_wait_ld_regs(v[0]);
-#pragma unroll
-  for (int c = 0; c < kBlockN / 32; ++c) {
-    if (c + 1 < kBlockN / 32) tmem_ld_x32(s_tmem + (c + 1) * 32, v[(c + 1) & 1]);  // in flight during chunk c
-#pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      float x = __uint_as_float(v[c & 1][i]);
-      if (kMask && c * 32 + i > limit) x = -INFINITY;
-      mx[i & 7] = fmaxf(mx[i & 7], x);
-    }
-    if (c + 1 < kBlockN / 32) tmem_wait_ld_regs(v[(c + 1) & 1]);
-  }
-  return fmaxf(fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])), fmaxf(fmaxf(mx[4], mx[5]), fmaxf(mx[6], mx[7])));
-}
-
-// p = 2^(x * scale - base) for the 128 scores of the row, rounded to the I/O type and stored to
-// TMEM columns [16c, 16c+16) of `p_tmem` (which may alias the S columns: chunk c of P only covers
-// columns that chunk <= c of S has already been read from).  Returns the FP32 row sum.
-// ex2.approx.f32 per element; the sum adds the unrounded p (the reference's rule).  (ex2.approx.f16x2 on
-// pairs was tried: no faster on B200 -- 409 vs 433 TFLOP/s -- and less accurate, so it is not used.)
-// After the first half of the row (64 keys) has been stored, `half_ready` is signalled so the
-// issuer can start the first four PV MMAs while the second half is computed.
-template <bool kMask, bool kBf16>
-__device__ __forceinline__ float exp_and_store(uint32_t s_tmem, uint32_t p_tmem, int limit, float scale_log2, float base,
-                                              uint64_t* half_ready) {
-  float sum[4] = {0.f, 0.f, 0.f, 0.f};
-  uint32_t v[2][32];
-  tmem_ld_x32(s_tmem, v[0]);
-  tmem_wait_ld_regs(v[0]);
-#pragma unroll
-  for (int c = 0; c < kBlockN / 32; ++c) {
-    if (c + 1 < kBlockN / 32) tmem_ld_x32(s_tmem + (c + 1) * 32, v[(c + 1) & 1]);  // in flight during chunk c
-    uint32_t p16[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      float x0 = __uint_as_float(v[c & 1][2 * i]), x1 = __uint_as_float(v[c & 1][2 * i + 1]);
-      if (kMask && c * 32 + 2 * i > limit) x0 = -INFINITY;
-      if (kMask && c * 32 + 2 * i + 1 > limit) x1 = -INFINITY;
-      x0 = fmaf(x0, scale_log2, -base);
-      x1 = fmaf(x1, scale_log2, -base);
-      const float p0 = ex2(x0), p1 = ex2(x1);
-      sum[i & 3] += p0 + p1;
-      p16[i] = pack2<kBf16>(p0, p1);
-    }
-    tmem_st_x16(p_tmem + c * 16, p16);
-    if (c == 1) {
-      tmem_wait_st();
-      tc_fence_before_sync();
-      mbar_arrive(half_ready);
-    }
-    if (c + 1 < kBlockN / 32) tmem_wait_ld_regs(v[(c + 1) & 1]);
-  }
-  return (sum[0] + sum[1]) + (sum[2] + sum[3]);
-}
-
-// Two CTAs are resident per SM (168 registers x 192 threads x 2 = 64512 <= 65536; 83 / 99 KB of
-// shared memory each; 256 TMEM columns each): the softmax of one runs under the MMAs of the other.
-// Measured at B=2 H=16 N=2048 D=64: 402 TFLOP/s with two resident CTAs, 206 with one.
-template <int D, bool kBf16>
-__global__ void __launch_bounds__(kThreads, 2)
-attn_prefill_serial_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                    const __grid_constant__ CUtensorMap tm_v, void* __restrict__ o_ptr, const Strides o_st, int H, int Hk, int Nq, int Nk,
-                    int causal, float scale_log2, int B, int n_q_tiles, int heads_per_group, unsigned int* status) {
-  using L = Layout<D>;
-  constexpr int S = L::kStages;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBars);
-  uint64_t* q_full = bars;
-  uint64_t* k_full = bars + 1;
-  uint64_t* k_empty = k_full + S;
-  uint64_t* v_full = k_empty + S;
-  uint64_t* v_empty = v_full + S;
-  uint64_t* s_full = v_empty + S;
-  uint64_t* p_ready = s_full + 1;   // [0]: keys 0-63 of P stored, [1]: keys 64-127
-  uint64_t* pv_done = p_ready + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::kMisc);
-  volatile uint32_t* abort_word = tmem_slot + 1;
-  const AbortCtx ctx{abort_word, status};
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const TileOrder ord = decode_tile_order(blockIdx.x, n_q_tiles, H * B, heads_per_group);
-  const int q_tile = ord.q_index;
-  const int h = ord.bh % H, b = ord.bh / H;
-  const int hk = h / (H / Hk);
-  const int q0 = q_tile * kBlockM;
-  const int causal_off = Nk - Nq;
-  int kv_end = Nk;
-  if (causal) kv_end = min(Nk, min(q0 + kBlockM, Nq) + causal_off);
-  const int n_tiles = (kv_end + kBlockN - 1) / kBlockN;
-
-  if (threadIdx.x == 0) {
-    mbar_init(q_full, 1);
-    for (int s = 0; s < S; ++s) {
-      mbar_init(&k_full[s], 1);
-      mbar_init(&k_empty[s], 1);
-      mbar_init(&v_full[s], 1);
-      mbar_init(&v_empty[s], 1);
-    }
-    mbar_init(s_full, 1);
-    mbar_init(&p_ready[0], 128);
-    mbar_init(&p_ready[1], 128);
-    mbar_init(pv_done, 1);
-    *abort_word = *reinterpret_cast<volatile unsigned int*>(status);  // a wait expired earlier on this device:
-    fence_mbar_init();                                                // do no work, return at once
-  }
-  if (warp == kMmaWarp) {
-    tmem_alloc(tmem_slot, kTmemCols);
-    tmem_relinquish();
-  }
-  tc_fence_before_sync();
-  __syncthreads();
-  tc_fence_after_sync();
-  pdl_wait();   // every role: from here on memory of the kernel in front is read (and what it reads may be overwritten)
-  pdl_launch_dependents();
-  const uint32_t tmem_base = *tmem_slot;
-  const bool dead_on_arrival = *abort_word != 0;
-
-  if (dead_on_arrival) {
-    // fall through to the teardown
-  } else if (warp == kProducerWarp) {
-    // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      tma_prefetch_desc(&tm_q);
-      tma_prefetch_desc(&tm_k);
-      tma_prefetch_desc(&tm_v);
-      mbar_arrive_expect_tx(q_full, L::kTile);
-#pragma unroll
-      for (int half = 0; half < D / 64; ++half)
-        tma_load_4d(smem + L::kQ + half * kHalfBytes, &tm_q, q_full, half * 64, q0, h, b);
-      for (int j = 0; j < n_tiles; ++j) {
-        const int s = j % S;
-        const uint32_t ph = (uint32_t)(j / S) & 1u;
-        if (!mbar_wait(&k_empty[s], ph ^ 1u, ctx, kWaitKEmpty)) break;
-        mbar_arrive_expect_tx(&k_full[s], L::kTile);
-#pragma unroll
-        for (int half = 0; half < D / 64; ++half)
-          tma_load_4d(smem + L::kK + s * L::kTile + half * kHalfBytes, &tm_k, &k_full[s], half * 64, j * kBlockN, hk, b);
-        if (!mbar_wait(&v_empty[s], ph ^ 1u, ctx, kWaitVEmpty)) break;
-        mbar_arrive_expect_tx(&v_full[s], L::kTile);
-#pragma unroll
-        for (int half = 0; half < D / 64; ++half)
-          tma_load_4d(smem + L::kV + s * L::kTile + half * kHalfBytes, &tm_v, &v_full[s], half * 64, j * kBlockN, hk, b);
-      }
-    }
-  } else if (warp == kMmaWarp) {
-    // ------------------------------------------------------------------ tcgen05.mma issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc_qk = idesc_f16(kBlockM, kBlockN, kBf16 ? 1 : 0, 0, 0);
-      constexpr uint32_t idesc_pv = idesc_f16(kBlockM, D, kBf16 ? 1 : 0, 0, 1);
-      const uint32_t q_addr = smem_u32(smem + L::kQ);
-      auto issue_qk = [&](int j) -> bool {
-        const int s = j % S;
-        if (!mbar_wait(&k_full[s], (uint32_t)(j / S) & 1u, ctx, kWaitKFull)) return false;
-        tc_fence_after_sync();
-        const uint32_t k_addr = smem_u32(smem + L::kK + s * L::kTile);
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off = (uint32_t)(kk / 4) * kHalfBytes + (uint32_t)(kk % 4) * 32u;
-          mma_ss(tmem_base + kSerialColS, smem_desc_sw128(q_addr + off, 16, 1024), smem_desc_sw128(k_addr + off, 16, 1024),
-                 idesc_qk, kk > 0 ? 1u : 0u);
-        }
-        tc_commit(&k_empty[s]);
-        tc_commit(s_full);
-        return true;
-      };
-      bool ok = mbar_wait(q_full, 0, ctx, kWaitQ);
-      ok = ok && issue_qk(0);
-      for (int j = 0; ok && j < n_tiles; ++j) {
-        if (!mbar_wait(&p_ready[0], (uint32_t)j & 1u, ctx, kWaitPReady)) break;
-        const int s = j % S;
-        if (!mbar_wait(&v_full[s], (uint32_t)(j / S) & 1u, ctx, kWaitVFull)) break;
-        tc_fence_after_sync();
-        const uint32_t v_addr = smem_u32(smem + L::kV + s * L::kTile);
-        bool halves_ok = true;
-#pragma unroll
-        for (int kk = 0; kk < kBlockN / 16; ++kk) {
-          if (kk == kBlockN / 32) {  // second half of the keys: wait for the rest of P
-            halves_ok = mbar_wait(&p_ready[1], (uint32_t)j & 1u, ctx, kWaitPReady);
-            if (!halves_ok) break;
-            tc_fence_after_sync();
-          }
-          // 16 keys per step: 16 rows of 128 bytes; the second 64-column block of V is kHalfBytes away
-          mma_ts(tmem_base + kSerialColO, tmem_base + kSerialColP + (uint32_t)kk * 8u,
-                 smem_desc_sw128(v_addr + kk * 2048, kHalfBytes, 1024), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
-        }
-        if (!halves_ok) break;
-        tc_commit(&v_empty[s]);
-        tc_commit(pv_done);
-        if (j + 1 < n_tiles) {
-          // S(j+1) overwrites the columns P(j) lives in.  tcgen05.mma instructions of one thread execute in
-          // issue order, so PV(j) has read P before QK(j+1) writes.
-          if (!issue_qk(j + 1)) break;
-        }
-      }
-    }
-  } else {
-    // ------------------------------------------------------------------ softmax + epilogue (warps 0-3)
-    const int row = threadIdx.x;  // query row inside the tile == TMEM lane
-    const uint32_t lane_bits = (uint32_t)(warp * 32) << 16;
-    const uint32_t s_tmem = tmem_base + kSerialColS + lane_bits;
-    const uint32_t o_tmem = tmem_base + kSerialColO + lane_bits;
-    float m_base = -INFINITY;  // the base O and l are currently expressed in (log2 units)
-    float l_run = 0.f;
-    bool ok = true;
-    for (int j = 0; j < n_tiles; ++j) {
-      // every lane polls: measured faster than one polling lane plus a shuffle (416 vs 346 TFLOP/s)
-      ok = __all_sync(0xffffffffu, mbar_wait(s_full, (uint32_t)j & 1u, ctx, kWaitSFull));
-      if (!ok) break;
-      tc_fence_after_sync();
-      // S(j) complete implies PV(j-1) complete (the issuer orders them), so O may be touched here.
-      const int k0 = j * kBlockN;
-      const bool need_mask = (k0 + kBlockN > Nk) || (causal && (k0 + kBlockN - 1 > q0 + causal_off));
-      int limit = Nk - 1;
-      if (causal) limit = min(limit, q0 + row + causal_off);
-      limit -= k0;  // last visible column of this tile for this row
-
-      // ---- pass 1: row maximum
-      const float m_tile = (need_mask ? row_max<true>(s_tmem, limit) : row_max<false>(s_tmem, limit)) * scale_log2;
-      // lazy rescale: move the base only when the maximum outgrew it by more than the threshold
-      const bool grow = m_tile > m_base + kRescaleThreshold || m_base == -INFINITY;
-      float alpha = 1.0f;
-      if (grow && m_tile != -INFINITY) {
-        alpha = ex2(m_base - m_tile);  // 0 when m_base is still -inf
-        m_base = m_tile;
-      }
-      const float base = (m_base == -INFINITY) ? 0.f : m_base;
-      if (j > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) {
-#pragma unroll
-        for (int c = 0; c < D / 32; ++c) {
-          uint32_t o[32];
-          tmem_ld_x32(o_tmem + c * 32, o);
-          tmem_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-          tmem_st_x32(o_tmem + c * 32, o);
-        }
-      }
-      // ---- pass 2: p = 2^(x - base), row sum, P written over the S columns already consumed
-      const uint32_t p_tmem = tmem_base + kSerialColP + lane_bits;
-      const float tile_sum = need_mask ? exp_and_store<true, kBf16>(s_tmem, p_tmem, limit, scale_log2, base, &p_ready[0])
-                                       : exp_and_store<false, kBf16>(s_tmem, p_tmem, limit, scale_log2, base, &p_ready[0]);
-      l_run = fmaf(l_run, alpha, tile_sum);
-      tmem_wait_st();
-      tc_fence_before_sync();
-      mbar_arrive(&p_ready[1]);
-    }
-    if (ok) ok = __all_sync(0xffffffffu, mbar_wait(pv_done, (uint32_t)(n_tiles - 1) & 1u, ctx, kWaitPvDone));
-    if (ok) {
-      tc_fence_after_sync();
-      const float inv_l = 1.0f / l_run;
-      const bool store = q0 + row < Nq;
-      uint8_t* dst = static_cast<uint8_t*>(o_ptr) + (b * o_st.b + h * o_st.h + (long long)(q0 + row) * o_st.n) * 2;
-#pragma unroll
-      for (int c = 0; c < D / 32; ++c) {
-        uint32_t o[32];
-        tmem_ld_x32(o_tmem + c * 32, o);
-        tmem_wait_ld();
-        if (store) {
-          uint32_t packed[16];
-#pragma unroll
-          for (int i = 0; i < 16; ++i)
-            packed[i] = pack2<kBf16>(__uint_as_float(o[2 * i]) * inv_l, __uint_as_float(o[2 * i + 1]) * inv_l);
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            reinterpret_cast<uint4*>(dst + c * 64)[i] =
-                make_uint4(packed[4 * i], packed[4 * i + 1], packed[4 * i + 2], packed[4 * i + 3]);
-        }
-      }
-    }
-  }
-
-  // teardown: every role falls through to here, also after an expired wait
-  if (!dead_on_arrival && *abort_word != 0) {
-    const unsigned long long t0 = globaltimer_ns();
-    while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);  // let copies in flight land
-  }
-  tc_fence_before_sync();
-  __syncthreads();
-  if (warp == kMmaWarp) {
-    __syncwarp();
-    tmem_dealloc(tmem_base, kTmemCols);
-  }
-}
-
-}  // namespace serial
-
-// ------------------------------------------------------------------------------------------------
-// Pair kernel: one CTA per SM, two tiles (A and B) of 128 query rows that attend to one KV head, steps of 128 keys.  384
+// NT = 2: one CTA per SM owns two tiles (A and B) of 128 query rows that attend to one KV head, steps of 128 keys.  384
 // threads (three warpgroups; warp 11 only takes part in barriers):
 //   warps 0-3  softmax of tile A, warps 4-7 softmax of tile B (warp w touches TMEM lanes 32 (w % 4)..);
 //   warp 8     TMA producer: both Q tiles once, then K and V tiles of 128 keys through mbarrier rings;
 //   warps 9,10 issue the tcgen05.mma of tile A / tile B.  The warp stays uniform and one elected lane issues: addresses and
 //              descriptors are then uniform registers (inside `if (lane == 0)` every MMA costs ~95 clocks of moves into
 //              them); it sleeps in blocking waits, because polling takes issue slots from two of the softmax warps.
-// TMEM (all 512 columns), head dim 64:  S_X [128 X, +128)   O_X [256 + 64 X, +64)   P_X [384 + 64 X, +64)
+// NT = 1: one tile, 192 threads (warps 0-3, 4, 5), half of the TMEM columns, two CTAs per SM: smaller pieces, for grids
+// that would leave SMs idle (plan_prefill).
+// TMEM (NT = 2: all 512 columns), head dim 64:  S_X [128 X, +128)   O_X [256 + 64 X, +64)   P_X [384 + 64 X, +64)
 //                          head dim 128: S_X [128 X, +128)   O_X [256 + 128 X, +128), P_X aliased on S_X [.., +64)
 // Both tiles read the same K/V tiles, so each is brought into shared memory once for 256 query rows.
 //
@@ -446,33 +118,32 @@ attn_prefill_serial_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
 // Split over keys: a problem with few tiles (short chunks against a long cache) is cut along the keys too; a CTA then
 // writes its unnormalised O and (m, l) per row and attn_prefill_merge_kernel puts the pieces together in order.
 // ------------------------------------------------------------------------------------------------
-namespace pair {
+namespace tiles {
 
-constexpr int kPairThreads = 384;   // three warpgroups
-constexpr int kPairProducerWarp = 8;
-constexpr int kPairMmaWarp = 9;
-constexpr uint32_t kPairTmemCols = 512;
 constexpr int kPolyPairs = 3;       // head dim 64: of 16 pairs of scores, this many take exp_pair_fma
 
-template <int D>
-struct PairLayout {
+template <int D, int NT>
+struct TileLayout {
+  static constexpr int kProducerWarp = 4 * NT, kMmaWarp = 4 * NT + 1;   // (then one issuer warp per tile)
+  static constexpr int kThreads = NT == 2 ? 384 : 192;
+  static constexpr uint32_t kTmemCols = 256u * NT;
   static constexpr bool kAliasP = D == 128;
   static constexpr int kHalves = kAliasP ? 2 : 1;     // pieces in which P is handed to the tensor cores
-  static constexpr int kStages = D == 64 ? 4 : 2;
+  static constexpr int kStages = (D == 64 ? 2 : 1) * NT;
   static constexpr int kTile = kBlockN * D * 2;       // bytes of one 128-row tile (Q, K or V)
   static constexpr int kQ = 0;                        // Q_A, Q_B
-  static constexpr int kK = 2 * kTile;
+  static constexpr int kK = NT * kTile;
   static constexpr int kV = kK + kStages * kTile;
   static constexpr int kBars = kV + kStages * kTile;
   static constexpr int kNumBars = 1 + 4 * kStages + 12;
   static constexpr int kMisc = kBars + kNumBars * 8;
   static constexpr int kBytes = kMisc + 16;
-  static constexpr int kAlloc = kBytes + 1024;
-  static_assert(kAlloc <= 227 * 1024, "must fit in shared memory");
-  static_assert(2 * kAlloc > 228 * 1024, "one CTA per SM: a CTA allocates all 512 TMEM columns");
-  static constexpr uint32_t kColS = 0;                       // + 128 X
-  static constexpr uint32_t kColO = 256;                     // + D X
-  static constexpr uint32_t kColP = kAliasP ? 0u : 384u;     // + (kAliasP ? 128 : 64) X
+  static constexpr int kAlloc = kBytes + 1024;        // room to align the tiles to 1024 bytes
+  static_assert((NT == 1 ? 2 : 1) * kAlloc <= 227 * 1024, "two one-tile CTAs, or a two-tile CTA, must fit on an SM");
+  static_assert(NT == 1 || 2 * kAlloc > 228 * 1024, "one two-tile CTA per SM: it allocates all 512 TMEM columns");
+  static constexpr uint32_t kColS = 0;                              // + 128 X
+  static constexpr uint32_t kColO = 128 * NT;                       // + D X
+  static constexpr uint32_t kColP = kAliasP ? 0u : 192u * NT;       // + (kAliasP ? 128 : 64) X
   static constexpr uint32_t kStrideP = kAliasP ? 128u : 64u;
 };
 
@@ -536,12 +207,12 @@ __device__ __forceinline__ uint32_t exp_pair_fma(uint32_t v0, uint32_t v1, float
   return pack2<kBf16>(y.x, y.y);
 }
 
-template <int D, bool kBf16>
-__global__ void __launch_bounds__(kPairThreads, 1)
-attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+template <int D, bool kBf16, int NT>
+__global__ void __launch_bounds__(TileLayout<D, NT>::kThreads, NT == 2 ? 1 : 2)
+attn_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                          const __grid_constant__ CUtensorMap tm_v, void* __restrict__ o_ptr, const Strides o_st,
                          const __grid_constant__ Params pr, unsigned int* status) {
-  using L = PairLayout<D>;
+  using L = TileLayout<D, NT>;
   constexpr int S = L::kStages, kHalves = L::kHalves;
   constexpr bool kAliasP = L::kAliasP;
   extern __shared__ uint8_t smem_raw[];
@@ -564,12 +235,12 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int H = pr.H, Hk = pr.Hk, Nq = pr.Nq, Nk = pr.Nk, causal = pr.causal, hpt = pr.heads_per_tile;
   const int per_batch = hpt ? Hk : H;   // units of a batch item
-  const TileOrder ord = decode_tile_order(blockIdx.x, (pr.tiles + 1) >> 1, pr.B * per_batch, pr.units_per_group);
-  const int tile0 = 2 * ord.q_index;
+  const TileOrder ord = decode_tile_order(blockIdx.x, (pr.tiles + NT - 1) / NT, pr.B * per_batch, pr.units_per_group);
+  const int tile0 = NT * ord.q_index;
   const int b = ord.bh / per_batch, within = ord.bh - b * per_batch;
   const int hk = hpt ? within : within / (H / Hk);
   const int causal_off = Nk - Nq;
-  const bool has_b = tile0 + 1 < pr.tiles;
+  const bool has_b = NT == 2 && tile0 + 1 < pr.tiles;
   // first head and first query of tile X
   auto head_of = [&](int X) { return hpt ? hk * (H / Hk) + (tile0 + X) * hpt : within; };
   auto query_of = [&](int X) { return hpt ? 0 : (tile0 + X) * kBlockM; };
@@ -593,9 +264,9 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     mbar_init(q_full, 1);
     for (int s = 0; s < S; ++s) {
       mbar_init(&k_full[s], 1);
-      mbar_init(&k_empty[s], 2);   // one arrival per issuer
+      mbar_init(&k_empty[s], NT);   // one arrival per issuer
       mbar_init(&v_full[s], 1);
-      mbar_init(&v_empty[s], 2);
+      mbar_init(&v_empty[s], NT);
     }
     for (int X = 0; X < 2; ++X) {
       mbar_init(&s_full[X], 1);
@@ -608,11 +279,11 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     *abort_word = *reinterpret_cast<volatile unsigned int*>(status);  // a wait expired earlier on this device:
     fence_mbar_init();                                                // do no work, return at once
   }
-  if (warp == kPairMmaWarp) {   // the first issuer warp also owns the TMEM allocation
-    tmem_alloc(tmem_slot, kPairTmemCols);
+  if (warp == L::kMmaWarp) {   // the first issuer warp also owns the TMEM allocation
+    tmem_alloc(tmem_slot, L::kTmemCols);
     tmem_relinquish();
   }
-  if (warp == kPairProducerWarp && lane == 0) {
+  if (warp == L::kProducerWarp && lane == 0) {
     tma_prefetch_desc(&tm_q);
     tma_prefetch_desc(&tm_k);
     tma_prefetch_desc(&tm_v);
@@ -625,14 +296,14 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   const uint32_t tmem_base = *tmem_slot;
   const bool dead_on_arrival = *abort_word != 0;
 
-  // Registers move from the warpgroup of the three single-warp roles to the softmax warpgroups, which keep
+  // Two tiles: registers move from the warpgroup of the three single-warp roles to the softmax warpgroups, which keep
   // the 128 scores of a row in registers (2 x 128 x 208 + 128 x 88 = 64512 of 65536).  Each role branch
   // starts with its setmaxnreg, executed by all four warps of its warpgroup.
   if (dead_on_arrival) {
     // fall through to the teardown
-  } else if (warp >= kPairProducerWarp) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
-    if (warp == kPairProducerWarp) {
+  } else if (warp >= L::kProducerWarp) {
+    if constexpr (NT == 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+    if (warp == L::kProducerWarp) {
       // ---------------------------------------------------------------- TMA producer
       if (lane == 0 && n_max > 0) {
         const int tiles = has_b ? 2 : 1;
@@ -657,12 +328,12 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
             tma_load_4d(smem + L::kV + s * L::kTile + half * kHalfBytes, &tm_v, &v_full[s], half * 64, key0, hk, b);
         }
       }
-    } else if (warp == kPairMmaWarp || warp == kPairMmaWarp + 1) {
+    } else if (warp < L::kMmaWarp + NT) {
       // ---------------------------------------------------------------- tcgen05.mma issuers (one warp per tile)
       // The two warps never touch each other's TMEM columns.  A K / V stage goes back to the producer when BOTH have
       // arrived on its `empty` barrier (count 2): a tile that does not need a key tile (no tile B, or one step less under
       // a causal mask) still arrives for it once it has been loaded.
-      const int X = warp - kPairMmaWarp;
+      const int X = warp - L::kMmaWarp;
       constexpr uint32_t idesc_qk = idesc_f16(kBlockM, kBlockN, kBf16 ? 1 : 0, 0, 0);
       constexpr uint32_t idesc_pv = idesc_f16(kBlockM, D, kBf16 ? 1 : 0, 0, 1);
       const uint64_t q_desc = smem_desc_sw128(smem_u32(smem + L::kQ) + (uint32_t)X * L::kTile, 16, 1024);
@@ -747,7 +418,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     }
   } else {
     // ------------------------------------------------------------------ softmax + epilogue (warps 0-7)
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
+    if constexpr (NT == 2) asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
     const int X = warp >> 2;                      // which tile
     const int row = threadIdx.x & 127;            // query row inside the tile == TMEM lane
     const int head = head_of(X) + (hpt ? row / Nq : 0);
@@ -792,7 +463,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       scan(1);
       tmem_wait_ld_regs(v[2]);
       tmem_wait_ld_regs(v[3]);
-      if constexpr (!kAliasP) {   // the S buffer can take the next product already
+      if constexpr (!kAliasP && NT == 2) {   // the S buffer can take the next product already
         tc_fence_before_sync();
         mbar_arrive(&s_free[X]);
       }
@@ -821,7 +492,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
           tmem_st_x32(o_tmem + c * 32, o);
         }
       }
-      if ((X == 1 || i > 0) && !wait_turn(i)) break;
+      if (NT == 2 && (X == 1 || i > 0) && !wait_turn(i)) break;
       const float2 nb2 = make_float2(-base, -base);
       float2 sum[2] = {{0.f, 0.f}, {0.f, 0.f}};
       uint32_t p[4][16];
@@ -837,8 +508,10 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
         asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0]; // %1 %2" ::"r"(smem_u32(&turn[X ^ 1])), "f"(sum[0].x), "f"(sum[1].x) : "memory");
       };
       chunk(0);
+      // One-tile CTAs have 168 registers a thread: the last chunk is read once more instead of being kept.
+      if constexpr (NT == 1) fetch(3);
       chunk(1);
-      if (!kAliasP) pass_baton();
+      if (NT == 2 && !kAliasP) pass_baton();
       if constexpr (kHalves == 2) {
         tmem_st_x16(p_tmem, p[0]);
         tmem_st_x16(p_tmem + 16, p[1]);
@@ -847,7 +520,15 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
         mbar_arrive(&p_ready[2 * X]);
       }
       chunk(2);
-      if (kAliasP) pass_baton();
+      if (NT == 2 && kAliasP) pass_baton();
+      if constexpr (NT == 1) {
+        tmem_wait_ld_regs(v[3]);
+        if (masked) mask32(v[3], 96, row_limit - k0);
+        if constexpr (!kAliasP) {
+          tc_fence_before_sync();
+          mbar_arrive(&s_free[X]);
+        }
+      }
       chunk(3);
       const float2 t = __fadd2_rn(sum[0], sum[1]);
       l_run = fmaf(l_run, alpha, t.x + t.y);
@@ -861,7 +542,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       tc_fence_before_sync();
       mbar_arrive(&p_ready[2 * X + kHalves - 1]);
     }
-    for (int i = n; ok && i < n_max; ++i) {   // steps that only the other tile has: pass the baton on
+    for (int i = n; NT == 2 && ok && i < n_max; ++i) {   // steps that only the other tile has: pass the baton on
       if ((X == 1 || i > 0) && !wait_turn(i)) break;
       mbar_arrive(&turn[X ^ 1]);
     }
@@ -909,9 +590,9 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == kPairMmaWarp) {
+  if (warp == L::kMmaWarp) {
     __syncwarp();
-    tmem_dealloc(tmem_base, kPairTmemCols);
+    tmem_dealloc(tmem_base, L::kTmemCols);
   }
 }
 
@@ -945,12 +626,11 @@ __global__ void __launch_bounds__(256) attn_prefill_merge_kernel(const float* __
   *reinterpret_cast<uint2*>(dst) = make_uint2(pack2<kBf16>(acc.x * inv, acc.y * inv), pack2<kBf16>(acc.z * inv, acc.w * inv));
 }
 
-}  // namespace pair
+}  // namespace tiles
 
-// How a problem is cut (see the header of the pair kernel).
+// How a problem is cut (see the header of the kernel).
 struct PrefillPlan {
-  bool serial;
-  int heads_per_tile, tiles, units, splits;
+  int heads_per_tile, tiles, units, per_cta, splits;
 };
 
 PrefillPlan plan_prefill(const Problem& p) {
@@ -966,61 +646,71 @@ PrefillPlan plan_prefill(const Problem& p) {
     c.tiles = G / c.heads_per_tile;
     c.units = p.B * p.Hk;
   }
-  const long long ctas = (long long)c.units * ((c.tiles + 1) / 2);
-  // One tile per unit, ungrouped heads and more of them than SMs: the single-tile kernel keeps two tiles on an SM.
-  c.serial = c.tiles == 1 && c.heads_per_tile == 0 && ctas > sms;
-  // Key splits, by time in key steps (~1.5 us): set-up and drain of a CTA cost about two, the merge kernel two plus its
-  // traffic (partials written and read at ~4 TB/s).  Only grids smaller than the GPU gain.
+  // Tiles per CTA and key splits, by a cost model in us fitted to measurements on B200: a key step takes a two-tile CTA
+  // 2.05 (head dim 64: 1.44), a one-tile CTA 1.7 (1.1) alone on its SM and 2.085 (1.65) beside another one; set-up and drain
+  // 5.3 and 4.6; the merge kernel 2.5 and its traffic at ~4 TB/s.  So a grid smaller than the GPU takes one tile per CTA
+  // (1 x 16 x 1093 queries D = 128: 20.1 us against 23.6) and splits the keys; long ones share K / V between two tiles
+  // (2 x 16 x 8192 D = 128 causal: 514 against 542).
+  const int steps = ceil_div(p.Nk, kBlockN);
+  const bool wide = p.D == 128;
+  const double merge_mb = (double)p.B * p.H * p.Nq * p.D * 8.0 / 4.0e6;
+  double best = 1e30;
+  c.per_cta = 1;
   c.splits = 1;
-  if (!c.serial) {
-    const int steps = ceil_div(p.Nk, kBlockN);
-    const double rows_mb = (double)p.B * p.H * p.Nq * p.D * 8.0 / 6.0e6;
-    double best = 1e30;
-    for (int s = 1; s <= steps && s <= 32 && (s == 1 || ctas * s <= sms); ++s) {
-      if (ceil_div(steps, ceil_div(steps, s)) != s) continue;   // an empty split
-      const double cost = (double)((ctas * s + sms - 1) / sms) * (ceil_div(steps, s) + 2.0) + (s > 1 ? 2.0 + s * rows_mb : 0.0);
-      if (cost < best) { best = cost; c.splits = s; }
+  for (int per_cta = 1; per_cta <= 2; ++per_cta)
+    for (int s = 1; s <= steps && s <= 32; ++s) {
+      const int per = ceil_div(steps, s);
+      if (ceil_div(steps, per) != s) continue;   // an empty split
+      const long long ctas = (long long)c.units * ceil_div(c.tiles, per_cta) * s;
+      if (s > 1 && ctas > 2 * sms) break;
+      // Waves of CTAs; a causal grid has CTAs of all lengths, longest first, and fills its last wave.
+      const long long slots = per_cta == 2 ? sms : 2 * sms;
+      const double waves = p.causal && p.Nq > p.Nk / 2 ? (double)ctas / slots : (double)((ctas + slots - 1) / slots);
+      const double len = p.causal && ctas > slots ? per * (1.0 - 0.5 * p.Nq / p.Nk) + 0.5 : per;
+      double cost = 0.0;
+      if (per_cta == 2) cost = (ctas <= sms ? 1.0 : waves) * (len * (wide ? 2.05 : 1.44) + 5.3);
+      else if (ctas <= sms) cost = per * (wide ? 1.7 : 1.1) + 4.6;
+      else cost = (ctas <= slots ? 1.0 : waves) * (len * (wide ? 2.085 : 1.65) + 4.6);
+      if (s > 1) cost += 2.5 + s * merge_mb;
+      if (cost < best) { best = cost; c.per_cta = per_cta; c.splits = s; }
     }
-  }
   return c;
+}
+
+template <int D, bool kBf16, int NT>
+int launch_tiles(const Problem& p, const PrefillPlan& plan, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, float* partial,
+                 unsigned int* status, cudaStream_t stream) {
+  using L = tiles::TileLayout<D, NT>;
+  auto kernel = tiles::attn_prefill_kernel<D, kBf16, NT>;
+  static bool configured[64] = {false};
+  int dev = 0;
+  KFB_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev >= 0 && dev < 64 && !configured[dev]) {
+    KFB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kAlloc));
+    configured[dev] = true;
+  }
+  const Strides o_st{p.o_stride_b, p.o_stride_h, p.o_stride_n};
+  // units whose K and V (one KV head each at worst) fit in ~48 MB of L2 together
+  const long long kv_bytes_per_unit = 4LL * p.Nk * p.D;
+  const int units_per_group = (int)std::min<long long>(plan.units, std::max<long long>(1, (48LL << 20) / kv_bytes_per_unit));
+  const long long ctas = (long long)plan.units * ceil_div(plan.tiles, NT);
+  if (ctas > 0x7fffffffLL) return fail(KFB_ERR_INVALID, "too many query tiles for one launch");
+  tiles::Params pr = {p.B, p.H, p.Hk, p.Nq, p.Nk, p.causal, p.scale * 1.4426950408889634f, plan.heads_per_tile, plan.tiles, units_per_group,
+                     plan.splits, partial};
+  if (int rc = launch_kernel("attn_prefill_kernel", kernel, dim3((unsigned)ctas, plan.splits), dim3(L::kThreads), L::kAlloc, stream, tq, tk, tv,
+                             p.o, o_st, pr, status))
+    return rc;
+  if (plan.splits == 1) return KFB_OK;
+  const long long rows = (long long)p.B * p.H * p.Nq, blocks = (rows * (D / 4) + 255) / 256;
+  return launch_kernel("attn_prefill_merge_kernel", tiles::attn_prefill_merge_kernel<D, kBf16>, dim3((unsigned)blocks), dim3(256), 0, stream,
+                       (const float*)partial, p.o, o_st, p.H, p.Nq, rows, plan.splits);
 }
 
 template <int D, bool kBf16>
 int launch(const Problem& p, const PrefillPlan& plan, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, float* partial,
            unsigned int* status, cudaStream_t stream) {
-  using L = Layout<D>;
-  using PL = pair::PairLayout<D>;
-  static bool configured[64] = {false};
-  int dev = 0;
-  KFB_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev >= 0 && dev < 64 && !configured[dev]) {
-    KFB_CUDA_TRY(cudaFuncSetAttribute(serial::attn_prefill_serial_kernel<D, kBf16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      L::kAlloc));
-    KFB_CUDA_TRY(cudaFuncSetAttribute(serial::attn_prefill_serial_kernel<D, kBf16>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                      cudaSharedmemCarveoutMaxShared));
-    KFB_CUDA_TRY(cudaFuncSetAttribute(pair::attn_prefill_pair_kernel<D, kBf16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      PL::kAlloc));
-    configured[dev] = true;
-  }
-  const float scale_log2 = p.scale * 1.4426950408889634f;
-  const Strides o_st{p.o_stride_b, p.o_stride_h, p.o_stride_n};
-  // units whose K and V (one KV head each at worst) fit in ~48 MB of L2 together
-  const long long kv_bytes_per_unit = 4LL * p.Nk * p.D;
-  const int units_per_group = (int)std::min<long long>(plan.units, std::max<long long>(1, (48LL << 20) / kv_bytes_per_unit));
-  const long long ctas = (long long)plan.units * (plan.serial ? plan.tiles : (plan.tiles + 1) / 2);
-  if (ctas > 0x7fffffffLL) return fail(KFB_ERR_INVALID, "too many query tiles for one launch");
-  if (plan.serial)
-    return launch_kernel("attn_prefill_serial_kernel", serial::attn_prefill_serial_kernel<D, kBf16>, dim3((unsigned)ctas), dim3(kThreads),
-                         L::kAlloc, stream, tq, tk, tv, p.o, o_st, p.H, p.Hk, p.Nq, p.Nk, p.causal, scale_log2, p.B, plan.tiles,
-                         units_per_group, status);
-  pair::Params pr = {p.B, p.H, p.Hk, p.Nq, p.Nk, p.causal, scale_log2, plan.heads_per_tile, plan.tiles, units_per_group, plan.splits, partial};
-  if (int rc = launch_kernel("attn_prefill_pair_kernel", pair::attn_prefill_pair_kernel<D, kBf16>, dim3((unsigned)ctas, plan.splits),
-                             dim3(pair::kPairThreads), PL::kAlloc, stream, tq, tk, tv, p.o, o_st, pr, status))
-    return rc;
-  if (plan.splits == 1) return KFB_OK;
-  const long long rows = (long long)p.B * p.H * p.Nq, blocks = (rows * (D / 4) + 255) / 256;
-  return launch_kernel("attn_prefill_merge_kernel", pair::attn_prefill_merge_kernel<D, kBf16>, dim3((unsigned)blocks), dim3(256), 0, stream,
-                       (const float*)partial, p.o, o_st, p.H, p.Nq, rows, plan.splits);
+  return plan.per_cta == 2 ? launch_tiles<D, kBf16, 2>(p, plan, tq, tk, tv, partial, status, stream)
+                           : launch_tiles<D, kBf16, 1>(p, plan, tq, tk, tv, partial, status, stream);
 }
 
 size_t partial_bytes(const Problem& p, const PrefillPlan& plan) {
