@@ -7,13 +7,19 @@
 //     CTAs so that even B = 1, Hk = 4 fills the 148 SMs;
 //   * the G = H / Hk query heads of a KV head are the M rows of the MMA (chunks of 16), so every K/V
 //     byte is read from HBM ONCE per group instead of once per query head;
-//   * a producer warp streams 64-key K and V tiles with TMA (128-byte swizzle) through a 4-stage
-//     mbarrier ring; four consumer warps each take 16 keys of a tile: S = Q K^T and O += P V on
-//     mma.sync.m16n8k16 (FP32 accumulate) -- the kernel is bandwidth-bound (8 FLOP per K/V byte at
-//     G = 8), tensor cores only keep the ALU cost below the HBM time;
-//   * per-warp online softmax (base 2, FP32), warps merged in shared memory in fixed order, one
-//     partial (O, m, l) per split written to the caller's workspace and combined in split order by
-//     a second small kernel => deterministic.  With one split the result is written directly.
+//   * a producer warp streams 64-key K and V tiles with TMA (128-byte swizzle) through an mbarrier
+//     ring; each consumer warp takes whole tiles in turn: S = Q K^T and O += P V on mma.sync.m16n8k16
+//     (FP32 accumulate) -- the kernel is bandwidth-bound (8 FLOP per K/V byte at G = 8), tensor cores
+//     only keep the ALU cost below the HBM time.  (Four warps sharing every tile, 16 keys each, walked
+//     through as many dependent softmax steps as there are tiles; a warp per tile has a quarter or a
+//     sixth of them, each with four times the independent work.)
+//   * the key range of a split is cut on the device from the valid length, so the splits of a short
+//     sequence in a long cache are as even as those of a full one;
+//   * per-warp online softmax (base 2, FP32), warps merged in shared memory in fixed order.  Up to
+//     eight splits form a thread-block cluster and are merged through distributed shared memory, in
+//     split order, every CTA a share of the output: one launch, nothing goes through global memory.
+//     More splits write one partial (O, m, l) each to the caller's workspace, combined in split order
+//     by a second small kernel.  Both are deterministic; with one split the result is written directly.
 #include "attn.cuh"
 #include "sm100.cuh"
 
@@ -24,19 +30,24 @@ namespace {
 using namespace sm100;
 
 constexpr int kTileKeys = 64;
-constexpr int kConsumerWarps = 4;
-constexpr int kThreads = (kConsumerWarps + 1) * 32;
-// Depth of the K/V tile ring.  A grid that fills the SMs (large batches) runs 3 CTAs per SM with 4 stages each; a grid
-// smaller than the GPU (decode at batch 1-8: B * Hk CTAs) is bound by the bytes ONE SM keeps in flight, so there the ring
-// takes (nearly) the whole shared memory and every tile of a short cache is requested at once.
-constexpr int kStagesShallow = 4;
+// Depth of the K/V tile ring and consumer warps.  A grid larger than the GPU runs several CTAs per SM with a shallow ring
+// each: three of 4 tiles at D = 64, two of 3 tiles at D = 128.  A grid of at most one CTA per SM (decode at batch 1-8:
+// B * Hk * splits CTAs) is bound by the bytes ONE SM keeps in flight, so there the ring takes (nearly) the whole shared
+// memory and every tile of a short cache is requested at once.
+template <int D> constexpr int shallow_stages() { return D == 64 ? 4 : 3; }
 template <int D> constexpr int deep_stages() { return D == 64 ? 12 : 6; }
+template <int D, int kStages> constexpr int consumer_warps() { return kStages == shallow_stages<D>() ? kStages : 6; }
 constexpr int kRows = 16;  // query heads per CTA (MMA M)
 
 enum WaitCode : uint32_t { kWaitFull = 0x201, kWaitEmpty };
 
 template <int D, int kStages>
 struct Layout {
+  static constexpr int kWarps = consumer_warps<D, kStages>();
+  static constexpr int kThreads = (kWarps + 1) * 32;
+  // a stage always holds tiles of the same warp: with another warp's tile in between, a wait for the round after next could
+  // be taken for the round before (copies may complete out of order)
+  static_assert(kStages % kWarps == 0, "");
   static constexpr int kHalf = kTileKeys * 128;       // 64 keys x 64 columns
   static constexpr int kTile = kTileKeys * D * 2;     // one K or V tile
   static constexpr int kStage = 2 * kTile;            // K then V
@@ -45,7 +56,7 @@ struct Layout {
   static constexpr int kBytes = kMisc + 16;
   static constexpr int kAlloc = kBytes + 1024;
   // the cross-warp merge reuses the tile ring: per warp O[16][D] + m[16] + l[16] floats
-  static constexpr int kMergeBytes = kConsumerWarps * kRows * (D + 2) * 4;
+  static constexpr int kMergeBytes = (kWarps + 1) * kRows * (D + 2) * 4;
   static_assert(kMergeBytes <= kBars, "merge scratch must fit in the tile ring");
 };
 
@@ -98,6 +109,13 @@ __device__ __forceinline__ uint16_t pack1(float x) {
   }
 }
 
+__device__ __forceinline__ float ld_cluster(uint32_t local_addr, uint32_t rank) {
+  float v;
+  asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %1, %2;\n\tld.shared::cluster.f32 %0, [ra];\n\t}"
+               : "=f"(v) : "r"(local_addr), "r"(rank) : "memory");
+  return v;
+}
+
 // byte offset of (key row r, 16-byte chunk c of the 128-byte row) inside a 128B-swizzled 64-key half tile
 __device__ __forceinline__ uint32_t swz(int r, int c) { return (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)); }
 
@@ -106,12 +124,13 @@ template <int D>
 __host__ __device__ constexpr int partial_floats() { return kRows * (D + 2); }
 
 template <int D, bool kBf16, int kStages>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__((consumer_warps<D, kStages>() + 1) * 32)
 attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                    const uint16_t* __restrict__ q, uint16_t* __restrict__ o, float* __restrict__ partial, int H, int Hk,
-                   int Nk, int keys_per_split, float scale_log2, unsigned int* status, const int* __restrict__ kv_len,
-                   int force_partial) {
+                   int Nk, float scale_log2, unsigned int* status, const int* __restrict__ kv_len,
+                   int force_partial, int clustered) {
   using L = Layout<D, kStages>;
+  constexpr int kConsumerWarps = L::kWarps, kThreads = L::kThreads;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + L::kBars);
@@ -130,7 +149,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&full[s], 1);
-      mbar_init(&empty[s], kConsumerWarps);
+      mbar_init(&empty[s], 1);
     }
     *abort_word = *reinterpret_cast<volatile unsigned int*>(status);  // non-zero: an earlier wait expired
     fence_mbar_init();
@@ -138,14 +157,15 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   __syncthreads();
   pdl_wait(q, kv_len);      // q, the cache rows and kv_len may be the output of the kernel in front
   pdl_launch_dependents();
-  const int key_begin = split * keys_per_split;
   // a static KV cache holds Nk rows of which only kv_len[b] are valid (read on the device, so the
   // same launch can be replayed from a CUDA graph while the cache fills up)
   const int valid = kv_len ? min(Nk, max(kv_len[b], 0)) : Nk;
-  const int key_end = min(valid, key_begin + keys_per_split);
+  const int tiles_valid = (valid + kTileKeys - 1) / kTileKeys, per_split = (tiles_valid + splits - 1) / splits;
+  const int key_begin = split * per_split * kTileKeys;
+  const int key_end = min(valid, key_begin + per_split * kTileKeys);
   const int n_tiles = key_end > key_begin ? (key_end - key_begin + kTileKeys - 1) / kTileKeys : 0;
-
-  if (*abort_word != 0) return;  // uniform: written before the barrier, nothing has been issued yet
+  const bool aborted = *abort_word != 0;   // uniform: written before the barrier, nothing has been issued yet
+  if (aborted && !clustered) return;
 
   float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
   float oacc[D / 8][4];
@@ -154,7 +174,9 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
 #pragma unroll
     for (int e = 0; e < 4; ++e) oacc[i][e] = 0.f;
 
-  if (warp == kConsumerWarps) {
+  if (aborted) {
+    // a cluster's CTAs leave together
+  } else if (warp == kConsumerWarps) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
       tma_prefetch_desc(&tm_k);
@@ -190,52 +212,65 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       }
     }
     const int mat = lane >> 3, mrow = lane & 7;
-    for (int t = 0; t < n_tiles; ++t) {
+    for (int t = warp; t < n_tiles; t += kConsumerWarps) {
       const int s = t % kStages;
       const bool ok = __all_sync(0xffffffffu, mbar_wait(&full[s], (uint32_t)(t / kStages) & 1u, ctx, kWaitFull));
       if (!ok) break;
       const uint32_t k_base = smem_u32(smem + s * L::kStage);
       const uint32_t v_base = k_base + L::kTile;
-      const int kw = warp * 16;  // this warp's 16 keys inside the tile
+      constexpr int kBlocks = kTileKeys / 16;   // blocks of 16 keys
 
-      // S[16 heads x 16 keys]: two n-tiles of 8 keys
-      float sacc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+      // S[16 heads x 64 keys]: eight n-tiles of 8 keys
+      float sacc[2 * kBlocks][4];
 #pragma unroll
-      for (int kk = 0; kk < D / 16; ++kk) {
-        // matrices: (keys 0-7, d 0-7) (keys 0-7, d 8-15) (keys 8-15, d 0-7) (keys 8-15, d 8-15)
-        const int key = kw + (mat >> 1) * 8 + mrow;
-        const int dchunk = kk * 2 + (mat & 1);
-        uint32_t r0, r1, r2, r3;
-        ldmatrix_x4(k_base + (dchunk >> 3) * L::kHalf + swz(key, dchunk & 7), r0, r1, r2, r3);
-        mma16816<kBf16>(sacc[0], qa[kk], r0, r1);
-        mma16816<kBf16>(sacc[1], qa[kk], r2, r3);
-      }
+      for (int i = 0; i < 2 * kBlocks; ++i) sacc[i][0] = sacc[i][1] = sacc[i][2] = sacc[i][3] = 0.f;
+#pragma unroll
+      for (int kk = 0; kk < D / 16; ++kk)
+#pragma unroll
+        for (int kb = 0; kb < kBlocks; ++kb) {
+          // matrices: (keys 0-7, d 0-7) (keys 0-7, d 8-15) (keys 8-15, d 0-7) (keys 8-15, d 8-15)
+          const int key = kb * 16 + (mat >> 1) * 8 + mrow;
+          const int dchunk = kk * 2 + (mat & 1);
+          uint32_t r0, r1, r2, r3;
+          ldmatrix_x4(k_base + (dchunk >> 3) * L::kHalf + swz(key, dchunk & 7), r0, r1, r2, r3);
+          mma16816<kBf16>(sacc[2 * kb], qa[kk], r0, r1);
+          mma16816<kBf16>(sacc[2 * kb + 1], qa[kk], r2, r3);
+        }
       // mask keys past this split's range (TMA zero-fills past Nk; keys of the next split are real data)
-      const int key_abs = key_begin + t * kTileKeys + kw + 2 * t4;
+      const int left = key_end - (key_begin + t * kTileKeys);   // keys of this tile that count
+      if (left < kTileKeys) {
 #pragma unroll
-      for (int nt = 0; nt < 2; ++nt)
+        for (int nt = 0; nt < 2 * kBlocks; ++nt)
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (key_abs + nt * 8 + (e & 1) >= key_end) sacc[nt][e] = -INFINITY;
+          for (int e = 0; e < 4; ++e)
+            if (nt * 8 + 2 * t4 + (e & 1) >= left) sacc[nt][e] = -INFINITY;
+      }
 
       // online softmax for rows g (e = 0,1) and g + 8 (e = 2,3)
-      uint32_t pa[4];
+      uint32_t pa[kBlocks][4];
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
-        float mx = fmaxf(fmaxf(sacc[0][2 * r], sacc[0][2 * r + 1]), fmaxf(sacc[1][2 * r], sacc[1][2 * r + 1]));
+        float mx = sacc[0][2 * r];
+#pragma unroll
+        for (int nt = 0; nt < 2 * kBlocks; ++nt) mx = fmaxf(mx, fmaxf(sacc[nt][2 * r], sacc[nt][2 * r + 1]));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
         const float m_new = fmaxf(m_run[r], mx * scale_log2);
         const float base = (m_new == -INFINITY) ? 0.f : m_new;
         const float alpha = ex2(m_run[r] - base);
-        const float p00 = ex2(fmaf(sacc[0][2 * r], scale_log2, -base));
-        const float p01 = ex2(fmaf(sacc[0][2 * r + 1], scale_log2, -base));
-        const float p10 = ex2(fmaf(sacc[1][2 * r], scale_log2, -base));
-        const float p11 = ex2(fmaf(sacc[1][2 * r + 1], scale_log2, -base));
-        l_run[r] = fmaf(l_run[r], alpha, (p00 + p01) + (p10 + p11));  // lane-local part of the row sum
+        float sum = 0.f;   // lane-local part of the row sum
+#pragma unroll
+        for (int kb = 0; kb < kBlocks; ++kb) {
+          const float p00 = ex2(fmaf(sacc[2 * kb][2 * r], scale_log2, -base));
+          const float p01 = ex2(fmaf(sacc[2 * kb][2 * r + 1], scale_log2, -base));
+          const float p10 = ex2(fmaf(sacc[2 * kb + 1][2 * r], scale_log2, -base));
+          const float p11 = ex2(fmaf(sacc[2 * kb + 1][2 * r + 1], scale_log2, -base));
+          sum += (p00 + p01) + (p10 + p11);
+          pa[kb][r] = pack2<kBf16>(p00, p01);       // a0a1 (row g) / a2a3 (row g+8): keys 2t, 2t+1
+          pa[kb][2 + r] = pack2<kBf16>(p10, p11);   // a4a5 / a6a7: keys 2t+8, 2t+9
+        }
+        l_run[r] = fmaf(l_run[r], alpha, sum);
         m_run[r] = m_new;
-        pa[r] = pack2<kBf16>(p00, p01);       // a0a1 (row g) / a2a3 (row g+8): keys 2t, 2t+1
-        pa[2 + r] = pack2<kBf16>(p10, p11);   // a4a5 / a6a7: keys 2t+8, 2t+9
 #pragma unroll
         for (int i = 0; i < D / 8; ++i) {
           oacc[i][2 * r] *= alpha;
@@ -243,30 +278,32 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         }
       }
       // Rows of V past key_end get p = 0, but 0 * NaN = NaN: with a device-side length those rows are
-      // whatever the cache buffer holds, so this warp zeroes them in its 16-key slice of the tile first.
-      {
-        const int first_bad = key_end - (key_begin + t * kTileKeys);  // tile-relative; >= 64 when all rows are valid
-        if (first_bad < kw + 16) {
-          const int r0 = max(first_bad, kw);
-          for (int i = lane; i < (kw + 16 - r0) * 8 * (D / 64); i += 32) {
-            const int row = r0 + i / (8 * (D / 64)), rem = i % (8 * (D / 64));
-            *reinterpret_cast<uint4*>(smem + s * L::kStage + L::kTile + (rem >> 3) * L::kHalf + row * 128 + (rem & 7) * 16) =
-                make_uint4(0u, 0u, 0u, 0u);
-          }
-          __syncwarp();
+      // whatever the cache buffer holds, so this warp zeroes them in its tile first.
+      if (left < kTileKeys) {
+        for (int i = lane; i < (kTileKeys - left) * 8 * (D / 64); i += 32) {
+          const int row = left + i / (8 * (D / 64)), rem = i % (8 * (D / 64));
+          *reinterpret_cast<uint4*>(smem + s * L::kStage + L::kTile + (rem >> 3) * L::kHalf + row * 128 + (rem & 7) * 16) =
+              make_uint4(0u, 0u, 0u, 0u);
         }
+        __syncwarp();
       }
-      // O[16 x D] += P[16 x 16 keys] V[16 keys x D]
+      // O[16 x D] += P[16 x 64 keys] V[64 keys x D]
 #pragma unroll
-      for (int dn = 0; dn < D / 16; ++dn) {
-        // matrices: (keys 0-7, d c0) (keys 8-15, d c0) (keys 0-7, d c1) (keys 8-15, d c1), transposed on load
-        const int key = kw + (mat & 1) * 8 + mrow;
-        const int dchunk = dn * 2 + (mat >> 1);
-        uint32_t r0, r1, r2, r3;
-        ldmatrix_x4_trans(v_base + (dchunk >> 3) * L::kHalf + swz(key, dchunk & 7), r0, r1, r2, r3);
-        mma16816<kBf16>(oacc[2 * dn], pa, r0, r1);
-        mma16816<kBf16>(oacc[2 * dn + 1], pa, r2, r3);
-      }
+      for (int kb = 0; kb < kBlocks; ++kb)
+#pragma unroll
+        for (int dn = 0; dn < D / 16; ++dn) {
+          // matrices: (keys 0-7, d c0) (keys 8-15, d c0) (keys 0-7, d c1) (keys 8-15, d c1), transposed on load
+          const int key = kb * 16 + (mat & 1) * 8 + mrow;
+          const int dchunk = dn * 2 + (mat >> 1);
+          uint32_t r0, r1, r2, r3;
+          ldmatrix_x4_trans(v_base + (dchunk >> 3) * L::kHalf + swz(key, dchunk & 7), r0, r1, r2, r3);
+          mma16816<kBf16>(oacc[2 * dn], pa[kb], r0, r1);
+          mma16816<kBf16>(oacc[2 * dn + 1], pa[kb], r2, r3);
+        }
+      // The stage is refilled through the async proxy: this warp's reads of it have to be over before it is given back.
+      // (Without the fence the next tile overwrote rows still being read: with K and V in L2 and several CTAs per SM,
+      // 19 of 20 calls at B = 8, Hk = 4, 1000..4096 keys had wrong heads, errors up to 0.1.)
+      fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty[s]);
     }
@@ -278,7 +315,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     }
   }
 
-  // ------------------------------------------------------------------ merge the four warps
+  // ------------------------------------------------------------------ merge the warps
   __syncthreads();  // every tile has been consumed (or the CTA is aborting): the ring is free
   float* scratch = reinterpret_cast<float*>(smem);
   constexpr int kPerWarp = kRows * (D + 2);
@@ -301,7 +338,8 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     }
   }
   __syncthreads();
-  const bool direct = splits == 1 && !force_partial;   // otherwise (O, m, l) goes to `partial` for a later merge
+  const bool direct = splits == 1 && !force_partial;   // otherwise (O, m, l) goes to `partial`, or to `own` for the cluster
+  float* own = scratch + kConsumerWarps * kPerWarp;
   float* out_partial = partial + (((size_t)b * gridDim.y + blockIdx.y) * splits + split) * kPerWarp;
   for (int idx = threadIdx.x; idx < rows * D; idx += kThreads) {
     const int r = idx / D, d = idx - r * D;
@@ -316,7 +354,13 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       acc = fmaf(f, scratch[w * kPerWarp + r * D + d], acc);
       l_all = fmaf(f, scratch[w * kPerWarp + kRows * D + kRows + r], l_all);
     }
-    if (direct) {
+    if (clustered) {
+      own[r * D + d] = acc;
+      if (d == 0) {
+        own[kRows * D + r] = m_all;
+        own[kRows * D + kRows + r] = l_all;
+      }
+    } else if (direct) {
       o[((size_t)b * H + h0 + r) * D + d] = pack1<kBf16>(l_all > 0.f ? acc / l_all : 0.f);  // no valid key: zeros
     } else {
       out_partial[r * D + d] = acc;
@@ -326,6 +370,35 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       }
     }
   }
+  if (!clustered) return;
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  // splits <= 8: this CTA merges elements split, split + splits, ... of the group's output
+  const uint32_t own_addr = smem_u32(own);
+  for (int idx = threadIdx.x * splits + split; idx < rows * D; idx += kThreads * splits) {
+    const int r = idx / D, d = idx - r * D;
+    float m[8], l[8], a[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const bool there = c < splits;
+      m[c] = there ? ld_cluster(own_addr + (kRows * D + r) * 4, c) : -INFINITY;
+      l[c] = there ? ld_cluster(own_addr + (kRows * D + kRows + r) * 4, c) : 0.f;
+      a[c] = there ? ld_cluster(own_addr + (r * D + d) * 4, c) : 0.f;
+    }
+    float m_all = m[0];
+#pragma unroll
+    for (int c = 1; c < 8; ++c) m_all = fmaxf(m_all, m[c]);
+    const float base = (m_all == -INFINITY) ? 0.f : m_all;
+    float acc = 0.f, l_all = 0.f;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const float f = ex2(m[c] - base);
+      acc = fmaf(f, a[c], acc);
+      l_all = fmaf(f, l[c], l_all);
+    }
+    if (!aborted) o[((size_t)b * H + h0 + r) * D + d] = pack1<kBf16>(l_all > 0.f ? acc / l_all : 0.f);
+  }
+  // no CTA leaves while another one still reads its sums
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // Combines the per-split partials of one (batch, query head).  `sets` > 1: several partial buffers of the same layout,
@@ -384,46 +457,43 @@ attn_decode_merge_kernel(const float* __restrict__ partial, uint16_t* __restrict
 }
 
 struct SplitPlan {
-  int chunks, splits, keys_per_split;
+  int chunks, splits;
+  bool clustered;
 };
 
+// How many CTAs share the keys of one (batch, kv head, chunk) group.  Measured at 24 shapes of 4..512 groups and 225..16384
+// keys, best of unsplit / clusters of 2..8 / 2..48 splits with a merge kernel:
+//   * more than 64 groups: one CTA each.  A second wave of CTAs or half-empty rings cost more than an uneven tail
+//     (64 x 4 groups of 4096 keys: 43.0 us, best split 48.7; 40 x 4 of 300..1200: 11.7, split 12.0).
+//   * otherwise as many as fit the GPU at once, one per SM, as a cluster of at most eight (8 x 4 groups of 1000..4096:
+//     8.6 us; three splits and a merge kernel 11.1).  Every CTA keeps two tiles (545 keys: 4.1 us, unsplit 4.8), and a
+//     group of fewer than eight tiles is quicker alone (225 keys: 4.3 against 5.3).
+//   * a handful of groups with long caches: eight CTAs each leave most of the chip idle, and from 16 tiles of D = 64 per
+//     CTA on that costs more than the merge kernel, whose own cost grows with the splits (4 groups of 16384 keys: eight in
+//     a cluster 11.4 us, 16 to 32 and a merge 9.7; 4096 keys: 6.7 and 6.8; one group of 131072: 48 splits 16.3, 148 19.6).
 SplitPlan plan_splits(int B, int H, int Hk, int Nk, int D) {
-  // Choose the number of key splits so that the grid fills whole waves of resident CTAs
-  // (3 per SM at D = 64, 1 at D = 128: shared memory) while every split keeps at least 2 tiles.
+  constexpr int kMinTiles = 8;
+  // Clusters of 1..8 such CTAs that fit at once: cudaOccupancyMaxActiveClusters gives 148, 74, 45, 33, 26, 22, 15, 15; a
+  // little less here, since which SMs a chip has differs.  (With one cluster too many, 16 of eight, 3072 keys took 13 us
+  // instead of 9.6.)
+  constexpr int kFit[9] = {0, 148, 64, 44, 32, 24, 20, 14, 14};
   SplitPlan p;
-  const int G = H / Hk;
-  p.chunks = ceil_div(G, kRows);
+  p.chunks = ceil_div(H / Hk, kRows);
+  p.splits = 1;
+  p.clustered = false;
   const long long groups = (long long)B * Hk * p.chunks;
   const int tiles = ceil_div(Nk, kTileKeys);
-  const long long slots = (long long)sm_count() * (D == 64 ? 3 : 1);
-  int best = 1;
-  double best_score = -1.0;
-  const int max_splits = tiles >= 4 ? (tiles / 2 < 128 ? tiles / 2 : 128) : 1;
-  for (int s = 1; s <= max_splits; ++s) {
-    const int per = ceil_div(tiles, s);
-    const int real = ceil_div(tiles, per);           // splits actually launched
-    if (real != s) continue;
-    const double waves = (double)(groups * real) / (double)slots;
-    const double full = waves <= 1.0 ? 1.0 : (double)(long long)(waves + 0.999999);
-    // time ~ full waves x tiles per split (+1 tile of fixed cost per CTA); lower is better
-    const double cost = full * (per + 1.0) + (waves <= 1.0 ? (1.0 - waves) * 0.01 : 0.0);
-    const double score = 1.0 / cost;
-    if (score > best_score * 1.0001) { best_score = score; best = real; }
+  if (tiles < kMinTiles || groups > kFit[2]) return p;
+  int cluster = 8;
+  while (cluster > 1 && (cluster * 2 > tiles || groups > kFit[cluster])) --cluster;
+  p.splits = cluster;
+  p.clustered = cluster > 1;
+  const int at_once = sm_count() / (int)groups;
+  if (at_once >= 2 * cluster && ceil_div(tiles, cluster) * (D / 64) > 16) {
+    const int wanted = ceil_div(tiles, 10) < 48 ? ceil_div(tiles, 10) : 48;
+    p.splits = wanted < at_once ? wanted : at_once;
+    p.clustered = false;
   }
-  // A split plan needs the merge kernel, a second launch worth about 12 key tiles of a CTA; when the unsplit plan is
-  // within that, it wins (end-to-end decode of the 22-layer model at a cache of 784: 0.849 -> 0.843 ms per step at batch
-  // 1, 1.125 -> 1.099 at batch 8, 1.630 -> 1.548 at batch 32; with 24 tiles a lone 1024-key call gets slower).
-  constexpr double kMergeCostTiles = 12.0;
-  if (best > 1) {
-    const int per = ceil_div(tiles, best);
-    const double waves = (double)(groups * best) / (double)slots;
-    const double full = waves <= 1.0 ? 1.0 : (double)(long long)(waves + 0.999999);
-    const double unsplit = (double)(long long)((double)groups / (double)slots + 0.999999) * (tiles + 1.0);
-    if (full * (per + 1.0) + kMergeCostTiles >= unsplit) best = 1;
-  }
-  const int tiles_per_split = ceil_div(tiles, best);
-  p.keys_per_split = tiles_per_split * kTileKeys;
-  p.splits = ceil_div(Nk, p.keys_per_split);
   return p;
 }
 
@@ -445,9 +515,9 @@ int launch(const Problem& p, const SplitPlan& plan, const CUtensorMap& tk, const
            unsigned int* status, cudaStream_t stream, bool partial_only = false) {
   const dim3 grid_probe(plan.splits, p.Hk * plan.chunks, p.B);
   const long long ctas = (long long)grid_probe.x * grid_probe.y * grid_probe.z;
-  if (ctas <= sm_count() && ceil_div(plan.keys_per_split, kTileKeys) > kStagesShallow)
+  if (ctas <= sm_count() && ceil_div(ceil_div(p.Nk, kTileKeys), plan.splits) > shallow_stages<D>())
     return launch_stages<D, kBf16, deep_stages<D>()>(p, plan, tk, tv, partial, status, stream, partial_only);
-  return launch_stages<D, kBf16, kStagesShallow>(p, plan, tk, tv, partial, status, stream, partial_only);
+  return launch_stages<D, kBf16, shallow_stages<D>()>(p, plan, tk, tv, partial, status, stream, partial_only);
 }
 
 template <int D, bool kBf16, int kStages>
@@ -462,11 +532,25 @@ int launch_stages(const Problem& p, const SplitPlan& plan, const CUtensorMap& tk
     KFB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kAlloc));
     configured[dev] = true;
   }
-  const dim3 grid(plan.splits, p.Hk * plan.chunks, p.B);
-  if (int rc = launch_kernel("attn_decode_kernel", kernel, grid, dim3(kThreads), L::kAlloc, stream, tk, tv,
-                             (const uint16_t*)p.q, (uint16_t*)p.o, partial, p.H, p.Hk, p.Nk, plan.keys_per_split,
-                             p.scale * 1.4426950408889634f, status, p.kv_len_dev, partial_only ? 1 : 0))
-    return rc;
+  const bool clustered = plan.clustered && !partial_only;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(plan.splits, p.Hk * plan.chunks, p.B);
+  cfg.blockDim = dim3(L::kThreads);
+  cfg.dynamicSmemBytes = L::kAlloc;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = plan.splits;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = clustered ? 2 : 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, tk, tv, (const uint16_t*)p.q, (uint16_t*)p.o, partial, p.H, p.Hk, p.Nk,
+                                     p.scale * 1.4426950408889634f, status, p.kv_len_dev, partial_only ? 1 : 0, clustered ? 1 : 0);
+  if (e != cudaSuccess) return fail(KFB_ERR_CUDA, "launch of attn_decode_kernel failed: %s", cudaGetErrorString(e));
+  if (clustered) return KFB_OK;
   if (plan.splits > 1 && !partial_only)
     return launch_merge_lanes<D, kBf16>((const float*)partial, (uint16_t*)p.o, p.B, p.H, p.Hk, plan.splits, 1, 0LL, stream);
   return KFB_OK;
@@ -474,6 +558,7 @@ int launch_stages(const Problem& p, const SplitPlan& plan, const CUtensorMap& tk
 
 }  // namespace
 
+// (a cluster's splits do not touch it: what is reported covers either form of the plan)
 size_t decode_ws_bytes(int B, int H, int Hk, int Nk, int D) {
   const SplitPlan plan = plan_splits(B, H, Hk, Nk, D);
   if (plan.splits <= 1) return 0;
@@ -501,7 +586,8 @@ int launch_decode(const Problem& p, void* ws, size_t ws_bytes, cudaStream_t stre
   if (p.Hk * ceil_div(p.H / p.Hk, kRows) > 65535 || p.B > 65535 || p.H > 65535)
     return fail(KFB_ERR_INVALID, "B, H and Hk * ceil(H/Hk/16) must each be <= 65535");
   const SplitPlan plan = plan_splits(p.B, p.H, p.Hk, p.Nk, p.D);
-  const size_t need = partial_only ? decode_partial_bytes(p.B, p.H, p.Hk, p.Nk, p.D, nullptr) : decode_ws_bytes(p.B, p.H, p.Hk, p.Nk, p.D);
+  const size_t need = partial_only ? decode_partial_bytes(p.B, p.H, p.Hk, p.Nk, p.D, nullptr)
+                      : plan.clustered ? 0 : decode_ws_bytes(p.B, p.H, p.Hk, p.Nk, p.D);
   if (need > 0 && (!ws || ws_bytes < need))
     return fail(KFB_ERR_WORKSPACE, "decode attention needs a %zu-byte workspace, got %zu", need, ws_bytes);
   if (need > 0 && !aligned16(ws)) return fail(KFB_ERR_ALIGNMENT, "workspace must be 16-byte aligned");
