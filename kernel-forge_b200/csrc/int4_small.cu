@@ -155,6 +155,8 @@ int4_small_kernel(const uint16_t* __restrict__ x, const uint32_t* __restrict__ p
   for (int d = 0; d < kDepth; ++d) fetch(d, g0 + d);
   if (fu.early) pdl_wait(x);
   pdl_launch_dependents();
+  if (!kBf16 && fu.residual != nullptr && threadIdx.x < M)   // what the epilogue adds: on its way while the product is computed
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(fu.residual + (size_t)threadIdx.x * N + r0));
 
   float acc[RB][MB][4];
 #pragma unroll

@@ -101,12 +101,6 @@ class LlamaInt4Decoder:
         # predecessor before touching activations); with tensor parallelism only when the gathers are this library's
         # peer-memory kernels too (NCCL kernels in between know nothing of the protocol)
         self.pdl = programmatic_launch and (tp_group is None or peer_gather)
-        # The 5-kernels-per-layer step (_step_fused, batch <= 2: RMSNorm in the prologue of the consuming GEMV, residual adds
-        # and pair epilogues in the producing ones) is available but not the default: a fused prologue (norm over the whole
-        # row, two block barriers) sits on every GEMV's critical path and costs what the two launches it removes would have.
-        # Measured, ms per step on the TinyLlama-1.1B shape with programmatic dependent launch: batch 1 0.624 fused against
-        # 0.620 separate, batch 2 0.80 against 0.64 (the separate step runs on the prepacked GEMV there).
-        self.fused = False
         s = shape
         self.tp_group = tp_group
         self.world = 1
@@ -127,18 +121,25 @@ class LlamaInt4Decoder:
         # epilogues of the GEMV want (ops.interleave_qkv_for_rope / interleave_gate_up), so RoPE + cache write and
         # SiLU * up happen in the epilogue of the projection (8 kernels per layer instead of 10).  Rows are quantised
         # independently, so this is exact; prefill reads the same matrices and undoes the order with a view.
-        # Batch 2..8 on one GPU: the decode-step GEMVs run on private fragment-order copies of the weights
-        # (ops.prepack_int4; as much memory again as the packed weights), with the same pair epilogues.  Measured,
-        # ms per step on the TinyLlama-1.1B shape, dispatcher kernels -> prepacked: batch 1 0.675 -> 0.681 (a tie: the
-        # CUDA-core GEMV stays, and the memory is saved), batch 2 0.80 -> 0.70, batch 8 1.01 -> 0.75.
+        # Batch 3 and more (2 where the fused step below does not apply): the decode-step GEMVs run on private
+        # fragment-order copies of the weights (ops.prepack_int4; as much memory again as the packed weights), with the
+        # same pair epilogues.  Measured, ms per step on the TinyLlama-1.1B shape, dispatcher kernels -> prepacked:
+        # batch 2 0.80 -> 0.70, batch 8 1.01 -> 0.75.
         # With tensor parallelism the same holds for the rank's own rows (local heads, local share of the hidden and
         # intermediate features); only the four gathers per layer are added.
+        # Batch <= 2 on one GPU: five kernels per layer (_step_fused), both RMSNorms in the prologue of the projection behind
+        # them and the residual adds in the epilogues, where the hidden size is within what the projection kernel with a norm
+        # takes (16 warps of 128 inputs).  Measured, ms per step on the TinyLlama-1.1B shape: batch 1 0.593 -> 0.510,
+        # batch 2 0.615 (prepacked weights) -> 0.556; the prepacked copies are not made then.
+        hidden_groups = s.hidden // group
+        self.fused = (self.plan is None and batch <= ops.FUSED_GEMV_MAX_M and s.hidden % group == 0 and s.hidden <= 2048
+                      and (hidden_groups <= 16 or hidden_groups % 2 == 0))
         hidden_loc = s.hidden if self.plan is None else self.plan["hidden_rows"][1] - self.plan["hidden_rows"][0]
         kdims = (s.hidden, s.heads * s.head_dim, s.intermediate)
         ndims = ((self.h_loc + 2 * self.hk_loc) * s.head_dim, hidden_loc, 2 * self.inter_loc)
         groups = s.hidden // group     # (the pair epilogues above 8 batch rows exist for K split 8 ways, <= 12 blocks of 64 per warp)
         wide_ok = batch <= 8 or (groups >= 8 and -(-groups // 8) * (group // 64) <= 12)
-        self.prepacked = (prepack and 2 <= batch <= ops.PREPACKED_GEMV_MAX_M and wide_ok
+        self.prepacked = (prepack and not self.fused and 2 <= batch <= ops.PREPACKED_GEMV_MAX_M and wide_ok
                           and all(k % 64 == 0 and k % group == 0 and k <= 12288 for k in kdims) and all(n % 16 == 0 for n in ndims))
         self.pair_rows = batch <= ops.FUSED_GEMV_MAX_M or self.prepacked
         f16 = lambda t: t.to(self.dev, torch.float16).contiguous()
@@ -332,8 +333,8 @@ class LlamaInt4Decoder:
         keys are split), o, add + norm, gate_up, silu * up, down; the last residual add is fused into the next layer's
         norm; the embedding gather is fused into the first norm) -- 7 or 8 at batch <= 2 on one GPU, where rope +
         cache write and silu * up run in the epilogues of the qkv and gate_up GEMVs -- then final norm, lm_head with fused argmax, and
-        one kernel that publishes the token and advances position and KV length.  Every kernel of the step is one
-        of this library's: no torch or cuBLAS kernel is left in the graph."""
+        one kernel that publishes the token and advances position and KV length (batch <= 2: _step_fused instead, where it
+        applies).  Every kernel of the step is one of this library's: no torch or cuBLAS kernel is left in the graph."""
         if self.persistent:
             return self._step_persistent()
         if self.plan is None and self.b <= ops.FUSED_GEMV_MAX_M and self.fused:

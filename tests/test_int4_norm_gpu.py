@@ -1,0 +1,51 @@
+"""RMSNorm fused with the INT4 linear behind it, against the two separate kernels: row counts around the 16-row blocks, around
+two blocks per SM and where a CTA owns three, four and five blocks; the smallest and largest share of K per warp; both group
+sizes; the residual epilogue of the linears without a norm."""
+
+import pytest
+import torch
+
+from kernelforge import ops, quantize
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m", [1, 2])
+@pytest.mark.parametrize("n,k,group", [
+    (2, 128, 128), (16, 64, 64), (18, 256, 64), (2560, 2048, 128), (4736, 2048, 128), (4738, 2048, 128), (7106, 1024, 64),
+    (9474, 2048, 64), (11264, 2048, 128), (14000, 1024, 128), (1000, 4096, 128), (640, 3072, 64), (48, 4096, 64), (5000, 4096, 128),
+])
+def test_norm_linear(m, n, k, group):
+    g = torch.Generator(device="cuda").manual_seed(n + k + m)
+    rn = lambda *s: torch.randn(*s, generator=g, device="cuda").half()
+    qw = quantize.quantize_weight(rn(n, k) * 0.05, group)
+    x, w, res = rn(m, k) * 3, 1 + 0.1 * rn(k), rn(m, n)
+    wd = quantize.dequantize(qw, torch.float32)
+    want = ops.add_rmsnorm(x, w, 1e-5)[0].float() @ wd.T
+    tol = 2e-3 * want.abs().max().item()
+    got = ops.int4_gemv_fused(x, qw.packed, qw.scales, group, ops.XFORM_RMSNORM, w, 1e-5)
+    assert (got.float() - want).abs().max().item() <= tol
+    got = ops.int4_gemv_silu_pair(x, qw.packed, qw.scales, group, w, 1e-5)
+    act = torch.nn.functional.silu(want[:, 0::2]) * want[:, 1::2]
+    assert (got.float() - act).abs().max().item() <= 4e-3 * max(act.abs().max().item(), want.abs().max().item())
+    got = ops.int4_gemv_fused(x, qw.packed, qw.scales, group, residual=res)
+    want = x.float() @ wd.T + res.float()
+    assert (got.float() - want).abs().max().item() <= 2e-3 * want.abs().max().item()
+
+
+@pytest.mark.parametrize("b", [1, 2])
+def test_norm_rope_kv(b):
+    h, hk, d, k, lmax, pos = 32, 4, 64, 2048, 24, 9
+    g = torch.Generator(device="cuda").manual_seed(b)
+    rn = lambda *s: torch.randn(*s, generator=g, device="cuda").half()
+    qw = quantize.quantize_weight(rn((h + 2 * hk) * d, k) * 0.05, 128)
+    x, w = rn(b, k), 1 + 0.1 * rn(k)
+    ang = torch.outer(torch.arange(lmax, device="cuda").float(), 1e4 ** (-torch.arange(0, d, 2, device="cuda").float() / d))
+    cos, sin = (f(torch.cat([ang, ang], -1)).contiguous() for f in (torch.cos, torch.sin))
+    at = torch.tensor([pos], device="cuda")
+    caches = [torch.zeros(b, hk, lmax, d, dtype=torch.float16, device="cuda") for _ in range(4)]
+    got = ops.int4_gemv_rope_kv(x, qw.packed, qw.scales, 128, cos, sin, at, caches[0], caches[1], h, w, 1e-5)
+    want = ops.int4_gemv_rope_kv(ops.add_rmsnorm(x, w, 1e-5)[0], qw.packed, qw.scales, 128, cos, sin, at, caches[2], caches[3], h)
+    for a, c in ((got, want), (caches[0], caches[2]), (caches[1], caches[3])):
+        assert (a.float() - c.float()).abs().max().item() <= 2e-3 * c.float().abs().max().item()
+    assert not caches[0][:, :, :pos].any() and not caches[1][:, :, pos + 1:].any()
