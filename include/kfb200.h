@@ -65,14 +65,14 @@ int kfb_device_status_reset(void* stream);
  * reference (csrc/common/check.cuh:11-24 turns CUDA errors into exceptions; it has no in-kernel waits). */
 int kfb_selftest_wait_expiry(unsigned long long timeout_ns, unsigned int* outcome_dev, void* stream);
 
-/* Programmatic dependent launch for every kernel of a decode step (the INT4 GEMVs, decode attention, the fused
- * element-wise kernels, lm_head, finalize).  When on, launches carry the CUDA attribute that lets a kernel become
- * resident while the one in front of it in the stream is still running; each kernel waits for that one
- * (griddepcontrol.wait) before it touches any activation and only then releases its own successor, so results are
- * those of the plain stream order while launch latency -- and, for the GEMVs and the lm_head, the first round trip
- * of the weight stream -- is hidden behind the previous kernel.  Works in CUDA-graph capture.  Process-wide switch,
- * off by default; returns the previous setting.  The reference has no counterpart (its decode step is launch-bound:
- * docs/phase5-notes.md). */
+/* Every launch of this library carries the attribute that lets a kernel become resident while the one in front of it in
+ * the stream is still running (programmatic dependent launch); each kernel waits for that one (griddepcontrol.wait)
+ * before it touches anything that one may have written, and only then releases its own successor, so results are those of
+ * the plain stream order.  This switch adds one promise by the caller: weights, scales and norm weights are OLDER than the
+ * kernel in front of the one that reads them, so the linears, the lm_head and the norms may request them before their
+ * wait -- true of a decode step, not of a weight quantised by the launch before.  Works in CUDA-graph capture.
+ * Process-wide, off by default; returns the previous setting.  The reference has no counterpart (its decode step is
+ * launch-bound: docs/phase5-notes.md). */
 int kfb_set_programmatic_launch(int enable);
 
 /* ---------------------------------------------------------------------------------------
@@ -121,9 +121,8 @@ int kfb_int4_linear_silu_pairs(const void* x, const void* packed, const void* sc
  * memory and multiplied on mma.sync fragments in their masked unsigned form (exact), with
  * a per-group correction from sums of x; a CUDA-core kernel (one FMA per weight, like the
  * reference's) remains for comparison and for very long K.
- * flags: bit 0 = launch with programmatic dependent launch (the weight prefetch of this
- * call may overlap the tail of the previous kernel on the stream; x is read and y written
- * only after the previous kernel has completed).
+ * flags: bit 0 = the weights are older than the kernel in front on the stream: they may be
+ * requested before that one has completed (x is read and y written only after it has).
  *        bit 1 = use the CUDA-core kernel;  bit 2 = use the mma.sync kernel (bits 1 and 2 exclude each other;
  *        with neither, the faster one for the shape is chosen). */
 int kfb_int4_gemv(const void* x, const void* packed, const void* scales, void* y,
@@ -300,7 +299,8 @@ int kfb_peer_allgather(const void* src, void* const* dst_all, void* const* peer_
  *   cache[:, :, :Nk] needs no copy.
  *   Prefill (Nq > 1): TMA-staged swizzled tiles, tcgen05 MMA, accumulators in TMEM.  The workspace is optional there: with
  *   kfb_flash_attn_ws_bytes bytes (16-byte aligned) a problem with few query tiles is split along the keys.
- *   Decode (Nq == 1): split-KV kernel; partial (o, m, l) per split go through `ws`.
+ *   Decode (Nq == 1): split-KV kernel; up to eight splits are merged inside a thread-block cluster, with more the partial
+ *   (o, m, l) per split go through `ws` (kfb_flash_attn_ws_bytes covers either form).
  * ------------------------------------------------------------------------------------- */
 size_t kfb_flash_attn_ws_bytes(int B, int H, int Hk, int Nq, int Nk, int D);
 int kfb_flash_attn_fwd(const void* q, const void* k, const void* v, void* o, int dtype,
@@ -400,8 +400,8 @@ int kfb_flash_attn_fwd_tokens(const void* q, const void* k, const void* v, void*
  * performs no cudaMalloc / cudaFree and uses no allocating library routine.
  *   - A problem whose split plan needs more than 4 MiB (kfb_flash_attn_ws_bytes tells) is refused
  *     with KFB_ERR_WORKSPACE: the array holds 992 (batch x kv-head x split) partials at D = 64
- *     and 504 at D = 128.  Small batches fit (B = 1..8 with 4 KV heads: at most 416 partials);
- *     e.g. B = 32, Hk = 4, Nk = 16384 (1280 partials) does not.
+ *     and 504 at D = 128.  (Today's plans use it only where a few groups with long caches are split
+ *     more than eight ways, at most one partial per SM.)
  *   - The first call on each device resolves the array's device address (cudaGetSymbolAddress);
  *     make that first call outside any stream capture.
  *   - All calls on a device share the one array.  Nothing in it has to be cleared between calls

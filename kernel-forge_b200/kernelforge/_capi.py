@@ -184,8 +184,9 @@ def raise_on_device_status(device: torch.device) -> None:
 
 
 class programmatic_launch:
-    """Context manager: the kernels launched inside carry the programmatic-dependent-launch attribute
-    (kfb_set_programmatic_launch).  Process-wide; restores the previous setting on exit."""
+    """Context manager: the caller promises that weights are older than the kernel in front of the one that reads them, so
+    kernels launched inside may request them early (kfb_set_programmatic_launch).  Process-wide; restores the previous
+    setting on exit."""
 
     def __init__(self, enable: bool = True):
         self.enable, self.prev = enable, 0
