@@ -274,6 +274,7 @@ __device__ __forceinline__ bool wait_full(Ctx& c) {
   return mbar_wait_warp(&c.sh->full[slot], parity, c.abort, kStatusWeightRing);
 }
 __device__ __forceinline__ void release_slot(Ctx& c) {   // every consumer warp, after its last read of the slot
+  fence_proxy_async_smem();   // the reads are over before the next bulk copy may land
   __syncwarp();
   if (c.lane == 0) mbar_arrive(&c.sh->empty[c.it % kSlots]);
   if (c.tid == 0) c.sh->consumed = c.it + 1;

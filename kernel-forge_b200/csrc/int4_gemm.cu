@@ -373,6 +373,7 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
           for (int e = 0; e < 2; ++e)
             *reinterpret_cast<uint4*>(&pw[4 * e]) = *reinterpret_cast<const uint4*>(words + (((4 * (turn & 1) + 2 * h + e) ^ (r & 7)) << 4));
           if (h == 1) {
+            fence_proxy_async_smem();   // these reads are over before the next copy of words may land
             __syncwarp();
             if (lane == 0) mbar_arrive(&w_free[ws]);
           }
