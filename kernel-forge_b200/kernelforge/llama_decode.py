@@ -121,10 +121,11 @@ class LlamaInt4Decoder:
         # epilogues of the GEMV want (ops.interleave_qkv_for_rope / interleave_gate_up), so RoPE + cache write and
         # SiLU * up happen in the epilogue of the projection (8 kernels per layer instead of 10).  Rows are quantised
         # independently, so this is exact; prefill reads the same matrices and undoes the order with a view.
-        # Batch 3 and more (2 where the fused step below does not apply): the decode-step GEMVs run on private
-        # fragment-order copies of the weights (ops.prepack_int4; as much memory again as the packed weights), with the
-        # same pair epilogues.  Measured, ms per step on the TinyLlama-1.1B shape, dispatcher kernels -> prepacked:
-        # batch 2 0.80 -> 0.70, batch 8 1.01 -> 0.75.
+        # Batch 3 and more (2 where the fused step below does not apply): the qkv and gate_up projections run on private
+        # fragment-order copies of their weights (ops.prepack_int4; as much memory again), with the same pair epilogues;
+        # o and down on the public format (int4_linear).  Measured, us per step on the TinyLlama-1.1B shape at batch 3 / 8 /
+        # 16 / 32: everything on fragment-order copies 597 / 620 / 764 / 1065, this 534 / 554 / 687 / 991, gate_up by
+        # int4_linear too 577 / 610 / 739 / 994.
         # With tensor parallelism the same holds for the rank's own rows (local heads, local share of the hidden and
         # intermediate features); only the four gathers per layer are added.
         # Batch <= 2 on one GPU: five kernels per layer (_step_fused), both RMSNorms in the prologue of the projection behind
@@ -164,9 +165,9 @@ class LlamaInt4Decoder:
             self.layers.append({
                 "in_norm": f16(lw["in_norm"]), "post_norm": f16(lw["post_norm"]),
                 "qkv": _Int4(qkv_rows, group, self.prepacked),
-                "o": _Int4(f16(o), group, self.prepacked),
+                "o": _Int4(f16(o), group),
                 "gate_up": _Int4(gate_up_rows, group, self.prepacked),
-                "down": _Int4(f16(down), group, self.prepacked),
+                "down": _Int4(f16(down), group),
             })
         self.k_cache = torch.zeros(s.layers, batch, self.hk_loc, max_len, s.head_dim, dtype=torch.float16, device=self.dev)
         self.v_cache = torch.zeros_like(self.k_cache)
@@ -357,8 +358,7 @@ class LlamaInt4Decoder:
                 q = ops.rope_kv_write(qkv, self.cos, self.sin, self.pos, self.k_cache[li], self.v_cache[li], self.h_loc)
             a = ops.flash_attn_decode(q, self.k_cache[li], self.v_cache[li], self.kv_len)
             a = self._gather(a.view(b, self.h_loc * s.head_dim), "attn_bounds")
-            o = ops.int4_gemv_prepacked(a, L["o"].pre, L["o"].scales, L["o"].group) if self.prepacked else L["o"](a)
-            o = self._gather(o, "hidden_bounds")
+            o = self._gather(L["o"](a), "hidden_bounds")
             h, x = ops.add_rmsnorm(x, L["post_norm"], s.rms_eps, o)
             if self.prepacked:
                 act = ops.int4_gemv_prepacked_silu_pair(h, L["gate_up"].pre, L["gate_up"].scales, L["gate_up"].group)
@@ -367,8 +367,7 @@ class LlamaInt4Decoder:
             else:
                 act = ops.silu_mul(L["gate_up"](h))
             act = self._gather(act, "inter_bounds")
-            res = ops.int4_gemv_prepacked(act, L["down"].pre, L["down"].scales, L["down"].group) if self.prepacked else L["down"](act)
-            res = self._gather(res, "hidden_bounds")
+            res = self._gather(L["down"](act), "hidden_bounds")
         h, x = ops.add_rmsnorm(x, self.final_norm, s.rms_eps, res)
         ops.lm_head_argmax(h, self.lm_head, self.step_logits, self.best)
         ops.decode_finalize(self.best, self.tok, self.pos, self.kv_len)
