@@ -43,10 +43,10 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
-// three-input maximum (one instruction on sm_100)
+// three-input maximum (one instruction on sm_100); NaN if any of the three is
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float y;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
   return y;
 }
 
@@ -169,7 +169,7 @@ __device__ __forceinline__ void max32(const uint32_t (&v)[32], float (&mx)[4]) {
 #pragma unroll
   for (int i = 0; i < 32; i += 2) mx[(i >> 1) & 3] = max3(mx[(i >> 1) & 3], __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
 }
-__device__ __forceinline__ float max_of(const float (&mx)[4]) { return fmaxf(max3(mx[0], mx[1], mx[2]), mx[3]); }
+__device__ __forceinline__ float max_of(const float (&mx)[4]) { return max3(max3(mx[0], mx[1], mx[2]), mx[3], mx[3]); }
 
 // Two scores, p = 2^(x * scale - base), rounded to the I/O type into one register; the unrounded p are added to `sum`.
 // Scale-and-subtract and the sums use the two-wide FP32 instructions of sm_100 (results per element are those of the scalar
@@ -187,7 +187,8 @@ constexpr float kExp2C1 = 0.693146944f, kExp2C2 = 0.240221202f, kExp2C3 = 0.0555
 
 // The same on the FMA pipe instead of the exponential unit: 2^x = 2^r 2^f with r = rint(x), f in [-1/2, 1/2] (Cody and
 // Waite's reduction), 2^f by a degree-5 polynomial fitted for least relative error there (2^-22, like ex2.approx), r added
-// to the exponent.  x below -125 counts as -125: far below the last bit of any sum it enters.
+// to the exponent.  x below -125 counts as -125: far below the last bit of any sum it enters.  So does NaN: rows with a
+// score that is NaN or +infinity are told by their maximum instead (see l_run).
 template <bool kBf16>
 __device__ __forceinline__ uint32_t exp_pair_fma(uint32_t v0, uint32_t v1, float2 sc2, float2 nb2, float2& sum) {
   float2 x = __ffma2_rn(make_float2(__uint_as_float(v0), __uint_as_float(v1)), sc2, nb2);
@@ -531,7 +532,8 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       }
       chunk(3);
       const float2 t = __fadd2_rn(sum[0], sum[1]);
-      l_run = fmaf(l_run, alpha, t.x + t.y);
+      // A score that is NaN or +infinity makes its row NaN, whichever way its exponential was taken.
+      l_run = m_step < INFINITY ? fmaf(l_run, alpha, t.x + t.y) : __int_as_float(0x7FFFFFFF);
       if (!pv_waited) {   // PV(j-1) must have finished reading the P columns before they are overwritten: by now it has
         if (!wait_all(&pv_done[X], ph ^ 1u, kWaitPvDone)) break;
         tc_fence_after_sync();
@@ -614,7 +616,7 @@ __global__ void __launch_bounds__(256) attn_prefill_merge_kernel(const float* __
 #pragma unroll 4
   for (int s = 0; s < splits; ++s) {
     const float2 w = ml[s * rows + row];
-    if (w.x == -INFINITY) continue;   // no step of this split reached the row (its O was not written)
+    if (w.x == -INFINITY && !isnan(w.y)) continue;   // no step of this split reached the row (its O was not written)
     const float f = ex2(w.x - m);
     const float4 v = *reinterpret_cast<const float4*>(partial + (s * rows + row) * D + c);
     acc.x = fmaf(f, v.x, acc.x); acc.y = fmaf(f, v.y, acc.y); acc.z = fmaf(f, v.z, acc.z); acc.w = fmaf(f, v.w, acc.w);
