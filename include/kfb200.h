@@ -298,11 +298,14 @@ int kfb_peer_allgather(const void* src, void* const* dst_all, void* const* peer_
  *   k and v (each a multiple of 8; the D axis must be dense), so a KV-cache view
  *   cache[:, :, :Nk] needs no copy.
  *   Prefill (Nq > 1): TMA-staged swizzled tiles, tcgen05 MMA, accumulators in TMEM.  The workspace is optional there: with
- *   kfb_flash_attn_ws_bytes bytes (16-byte aligned) a problem with few query tiles is split along the keys.
+ *   kfb_flash_attn_ws_bytes bytes (16-byte aligned) a problem with few query tiles is split along the keys, without it is
+ *   cut as well as can be without splits.
  *   Decode (Nq == 1): split-KV kernel; up to eight splits are merged inside a thread-block cluster, with more the partial
  *   (o, m, l) per split go through `ws` (kfb_flash_attn_ws_bytes covers either form).
  * ------------------------------------------------------------------------------------- */
 size_t kfb_flash_attn_ws_bytes(int B, int H, int Hk, int Nq, int Nk, int D);
+/* How a prefill (Nq > 1) is cut when its workspace has ws_bytes bytes: query tiles per CTA (1 or 2) and key splits (1: none). */
+int kfb_flash_attn_plan(int B, int H, int Hk, int Nq, int Nk, int D, int causal, size_t ws_bytes, int* tiles_per_cta, int* splits);
 int kfb_flash_attn_fwd(const void* q, const void* k, const void* v, void* o, int dtype,
                        int B, int H, int Hk, int Nq, int Nk, int D, int causal, float scale,
                        const int64_t* kv_strides, void* ws, size_t ws_bytes, void* stream);

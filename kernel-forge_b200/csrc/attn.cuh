@@ -24,8 +24,10 @@ struct Problem {
 };
 
 // Prefill / general path: tiles of 128 query rows, TMA + tcgen05 + TMEM (attn_prefill.cu).  The workspace is optional: a
-// problem with few tiles is split along the keys when it has prefill_ws_bytes bytes.
+// problem with few tiles is split along the keys when it has prefill_ws_bytes bytes (enough with and without the causal mask).
 size_t prefill_ws_bytes(int B, int H, int Hk, int Nq, int Nk, int D);
+// The plan that launch_prefill takes with a workspace of ws_bytes.
+void prefill_plan(const Problem& p, size_t ws_bytes, int* tiles_per_cta, int* splits);
 int launch_prefill(const Problem& p, void* ws, size_t ws_bytes, cudaStream_t stream);
 
 // Decode path (Nq == 1): split-KV, one CTA per (batch, kv head, split) (attn_decode.cu).

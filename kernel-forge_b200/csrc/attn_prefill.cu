@@ -630,12 +630,12 @@ __global__ void __launch_bounds__(256) attn_prefill_merge_kernel(const float* __
 
 }  // namespace tiles
 
-// How a problem is cut (see the header of the kernel).
+// How a problem is cut (see the header of the kernel); max_splits = 1 where there is no workspace for the pieces.
 struct PrefillPlan {
   int heads_per_tile, tiles, units, per_cta, splits;
 };
 
-PrefillPlan plan_prefill(const Problem& p) {
+PrefillPlan plan_prefill(const Problem& p, int max_splits = 32) {
   PrefillPlan c;
   const int G = p.H / p.Hk, q_tiles = ceil_div(p.Nq, kBlockM), sms = sm_count();
   c.heads_per_tile = 0;
@@ -660,7 +660,7 @@ PrefillPlan plan_prefill(const Problem& p) {
   c.per_cta = 1;
   c.splits = 1;
   for (int per_cta = 1; per_cta <= 2; ++per_cta)
-    for (int s = 1; s <= steps && s <= 32; ++s) {
+    for (int s = 1; s <= steps && s <= max_splits; ++s) {
       const int per = ceil_div(steps, s);
       if (ceil_div(steps, per) != s) continue;   // an empty split
       const long long ctas = (long long)c.units * ceil_div(c.tiles, per_cta) * s;
@@ -724,7 +724,17 @@ size_t partial_bytes(const Problem& p, const PrefillPlan& plan) {
 size_t prefill_ws_bytes(int B, int H, int Hk, int Nq, int Nk, int D) {
   Problem p = {};
   p.B = B; p.H = H; p.Hk = Hk; p.Nq = Nq; p.Nk = Nk; p.D = D;
-  return partial_bytes(p, plan_prefill(p));
+  const size_t full = partial_bytes(p, plan_prefill(p));
+  p.causal = 1;   // (its plan may have more splits)
+  const size_t causal = partial_bytes(p, plan_prefill(p));
+  return full > causal ? full : causal;
+}
+
+void prefill_plan(const Problem& p, size_t ws_bytes, int* tiles_per_cta, int* splits) {
+  PrefillPlan plan = plan_prefill(p);
+  if (ws_bytes < partial_bytes(p, plan)) plan = plan_prefill(p, 1);   // the workspace is optional
+  *tiles_per_cta = plan.per_cta;
+  *splits = plan.splits;
 }
 
 int launch_prefill(const Problem& given, void* ws, size_t ws_bytes, cudaStream_t stream) {
@@ -734,7 +744,7 @@ int launch_prefill(const Problem& given, void* ws, size_t ws_bytes, cudaStream_t
   unsigned int* status = device_status_word();
   if (!status) return fail(KFB_ERR_CUDA, "cannot resolve the device status word");
   PrefillPlan plan = plan_prefill(p);
-  if (!ws || !aligned16(ws) || ws_bytes < partial_bytes(p, plan)) plan.splits = 1;   // the workspace is optional
+  if (!ws || !aligned16(ws) || ws_bytes < partial_bytes(p, plan)) plan = plan_prefill(p, 1);   // the workspace is optional
   CUtensorMap tq, tk, tv;
   const uint64_t D = p.D;
   const uint64_t qd[4] = {D, (uint64_t)p.Nq, (uint64_t)p.H, (uint64_t)p.B};

@@ -36,6 +36,17 @@ extern "C" size_t kfb_flash_attn_ws_bytes(int B, int H, int Hk, int Nq, int Nk, 
   return attn::decode_ws_bytes(B, H, Hk, Nk, D);
 }
 
+extern "C" int kfb_flash_attn_plan(int B, int H, int Hk, int Nq, int Nk, int D, int causal, size_t ws_bytes, int* tiles_per_cta, int* splits) {
+  if (int rc = check_shape(KFB_F16, B, H, Hk, Nq, Nk, D, causal)) return rc;
+  if (Nq < 2) return fail(KFB_ERR_INVALID, "flash_attn_plan describes prefill, Nq >= 2");
+  if (!tiles_per_cta || !splits) return fail(KFB_ERR_INVALID, "null pointer");
+  attn::Problem p = {};
+  p.B = B; p.H = H; p.Hk = Hk; p.Nq = Nq; p.Nk = Nk; p.D = D;
+  p.causal = causal ? 1 : 0;
+  attn::prefill_plan(p, ws_bytes, tiles_per_cta, splits);
+  return KFB_OK;
+}
+
 extern "C" int kfb_flash_attn_fwd(const void* q, const void* k, const void* v, void* o, int dtype, int B, int H,
                                   int Hk, int Nq, int Nk, int D, int causal, float scale, const int64_t* kv_strides,
                                   void* ws, size_t ws_bytes, void* stream) {

@@ -105,6 +105,37 @@ def test_custom_ops_registered_with_fakes():
         assert torch.ops.kernelforge.int4_matmul(x, p, s, 128).shape == (3, 40)
 
 
+def test_prefill_workspace_covers_the_plan_with_and_without_the_causal_mask():
+    """The bytes that kfb_flash_attn_ws_bytes reports are enough for the plan a call takes, causal or not (it is not told
+    which); without a workspace the call is planned for no splits, not a split plan run unsplit.  Host logic."""
+    import ctypes
+    import random
+    from kernelforge import _capi
+    lib = _capi.lib()
+
+    def plan(shape, causal, ws):
+        tiles, splits = ctypes.c_int(), ctypes.c_int()
+        assert lib.kfb_flash_attn_plan(*shape, causal, ws, ctypes.byref(tiles), ctypes.byref(splits)) == 0
+        return tiles.value, splits.value
+
+    rng = random.Random(1)
+    shapes = [(2, 1, 1, 3907, 3907, 64), (1, 8, 8, 1557, 1557, 128), (1, 12, 2, 509, 4093, 128)]
+    for _ in range(3000):
+        hk, n = rng.choice((1, 2, 4, 8)), int(2 ** rng.uniform(1, 13))
+        shapes.append((rng.choice((1, 2, 3, 8)), hk * rng.choice((1, 2, 6, 8)), hk, n, n + rng.choice((0, 0, 300, 4000)), rng.choice((64, 128))))
+    split = 0
+    for shape in shapes:
+        ws = lib.kfb_flash_attn_ws_bytes(*shape)
+        for causal in (0, 1):
+            best = plan(shape, causal, 1 << 60)
+            assert plan(shape, causal, ws) == best, (shape, causal)
+            assert plan(shape, causal, 0)[1] == 1
+            split += best[1] > 1
+    assert split > 100
+    # 1557 queries of 8 heads: with splits two tiles per CTA are best, without them one
+    assert plan(shapes[1], 1, 1 << 60)[0] == 2 and plan(shapes[1], 1, 0) == (1, 1)
+
+
 def test_int4_matmul_routing_table():
     """Which kernel int4_matmul picks by shape (pure host logic): GEMV up to M = 8, the same kernel with more batch columns
     for 8 < M <= 16 where it measured faster, the tcgen05 GEMM otherwise."""
