@@ -300,8 +300,8 @@ int kfb_peer_allgather(const void* src, void* const* dst_all, void* const* peer_
  *   Prefill (Nq > 1): TMA-staged swizzled tiles, tcgen05 MMA, accumulators in TMEM.  The workspace is optional there: with
  *   kfb_flash_attn_ws_bytes bytes (16-byte aligned) a problem with few query tiles is split along the keys, without it is
  *   cut as well as can be without splits.
- *   Decode (Nq == 1): split-KV kernel; up to eight splits are merged inside a thread-block cluster, with more the partial
- *   (o, m, l) per split go through `ws` (kfb_flash_attn_ws_bytes covers either form).
+ *   Decode (Nq == 1): split-KV kernel; up to eight splits are merged inside a thread-block cluster and need no workspace, with
+ *   more the partial (o, m, l) per split go through `ws`.
  * ------------------------------------------------------------------------------------- */
 size_t kfb_flash_attn_ws_bytes(int B, int H, int Hk, int Nq, int Nk, int D);
 /* How a prefill (Nq > 1) is cut when its workspace has ws_bytes bytes: query tiles per CTA (1 or 2) and key splits (1: none). */
@@ -398,13 +398,11 @@ int kfb_flash_attn_fwd_tokens(const void* q, const void* k, const void* v, void*
  * between cudaStreamBeginCapture and EndCapture (cudaMalloc is not allowed there), a host runtime
  * without a device allocator.  This entry point has no counterpart in the reference.
  * It computes exactly what kfb_flash_attn_fwd computes for Nq == 1, but the split-KV partial
- * results go through a 4 MiB array that is part of the library image (each GPU that loads the
- * library holds those 4 MiB until the process exits) instead of a caller workspace; the call
+ * results go through a 2 MiB array that is part of the library image (each GPU that loads the
+ * library holds those 2 MiB until the process exits) instead of a caller workspace; the call
  * performs no cudaMalloc / cudaFree and uses no allocating library routine.
- *   - A problem whose split plan needs more than 4 MiB (kfb_flash_attn_ws_bytes tells) is refused
- *     with KFB_ERR_WORKSPACE: the array holds 992 (batch x kv-head x split) partials at D = 64
- *     and 504 at D = 128.  (Today's plans use it only where a few groups with long caches are split
- *     more than eight ways, at most one partial per SM.)
+ *   - Partials are written only where a few groups with long caches are split more than eight ways,
+ *     at most one per SM, so every problem fits on a GPU of up to 252 SMs; KFB_ERR_WORKSPACE otherwise.
  *   - The first call on each device resolves the array's device address (cudaGetSymbolAddress);
  *     make that first call outside any stream capture.
  *   - All calls on a device share the one array.  Nothing in it has to be cleared between calls

@@ -468,7 +468,7 @@ struct SplitPlan {
 //   * otherwise as many as fit the GPU at once, one per SM, as a cluster of at most eight (8 x 4 groups of 1000..4096:
 //     8.6 us; three splits and a merge kernel 11.1).  Every CTA keeps two tiles (545 keys: 4.1 us, unsplit 4.8), and a
 //     group of fewer than eight tiles is quicker alone (225 keys: 4.3 against 5.3).
-//   * a handful of groups with long caches: eight CTAs each leave most of the chip idle, and from 16 tiles of D = 64 per
+//   * a handful of groups with long caches (the only plans that write partials, at most one per SM): eight CTAs each leave most of the chip idle, and from 16 tiles of D = 64 per
 //     CTA on that costs more than the merge kernel, whose own cost grows with the splits (4 groups of 16384 keys: eight in
 //     a cluster 11.4 us, 16 to 32 and a merge 9.7; 4096 keys: 6.7 and 6.8; one group of 131072: 48 splits 16.3, 148 19.6).
 SplitPlan plan_splits(int B, int H, int Hk, int Nk, int D) {
@@ -558,10 +558,10 @@ int launch_stages(const Problem& p, const SplitPlan& plan, const CUtensorMap& tk
 
 }  // namespace
 
-// (a cluster's splits do not touch it: what is reported covers either form of the plan)
+// (the splits of a cluster are merged through shared memory)
 size_t decode_ws_bytes(int B, int H, int Hk, int Nk, int D) {
   const SplitPlan plan = plan_splits(B, H, Hk, Nk, D);
-  if (plan.splits <= 1) return 0;
+  if (plan.splits <= 1 || plan.clustered) return 0;
   return (size_t)B * Hk * plan.chunks * plan.splits * kRows * (D + 2) * sizeof(float);
 }
 
@@ -586,8 +586,7 @@ int launch_decode(const Problem& p, void* ws, size_t ws_bytes, cudaStream_t stre
   if (p.Hk * ceil_div(p.H / p.Hk, kRows) > 65535 || p.B > 65535 || p.H > 65535)
     return fail(KFB_ERR_INVALID, "B, H and Hk * ceil(H/Hk/16) must each be <= 65535");
   const SplitPlan plan = plan_splits(p.B, p.H, p.Hk, p.Nk, p.D);
-  const size_t need = partial_only ? decode_partial_bytes(p.B, p.H, p.Hk, p.Nk, p.D, nullptr)
-                      : plan.clustered ? 0 : decode_ws_bytes(p.B, p.H, p.Hk, p.Nk, p.D);
+  const size_t need = partial_only ? decode_partial_bytes(p.B, p.H, p.Hk, p.Nk, p.D, nullptr) : decode_ws_bytes(p.B, p.H, p.Hk, p.Nk, p.D);
   if (need > 0 && (!ws || ws_bytes < need))
     return fail(KFB_ERR_WORKSPACE, "decode attention needs a %zu-byte workspace, got %zu", need, ws_bytes);
   if (need > 0 && !aligned16(ws)) return fail(KFB_ERR_ALIGNMENT, "workspace must be 16-byte aligned");
@@ -633,7 +632,8 @@ namespace kfb {
 namespace attn {
 namespace {
 
-constexpr size_t kMaxScratchBytes = 4u << 20;  // 4 MiB: up to 992 (group, split) partials at D = 64, 504 at D = 128
+// A plan that is not a cluster's has at most one partial per SM (plan_splits): 1.2 MB on 148 SMs at D = 128.  2 MiB hold 252.
+constexpr size_t kMaxScratchBytes = 2u << 20;
 static __device__ __align__(256) unsigned char g_decode_scratch[kMaxScratchBytes];
 
 std::mutex g_scratch_mutex;

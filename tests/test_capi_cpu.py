@@ -136,6 +136,24 @@ def test_prefill_workspace_covers_the_plan_with_and_without_the_causal_mask():
     assert plan(shapes[1], 1, 1 << 60)[0] == 2 and plan(shapes[1], 1, 0) == (1, 1)
 
 
+def test_every_decode_plan_fits_the_array_of_the_allocation_free_entry():
+    """kfb_flash_attn_decode_noalloc has 2 MiB for partials: no plan needs more, over groups, keys and head dims.  A workspace is
+    asked for only where partials are written, so most plans need none.  Host logic."""
+    from kernelforge import _capi
+    lib = _capi.lib()
+    most, none, some = 0, 0, 0
+    for d in (64, 128):
+        for b in list(range(1, 80)) + [100, 148, 149, 300]:
+            for h, hk in ((1, 1), (16, 1), (17, 1), (40, 1), (8, 2), (32, 4), (34, 2), (64, 8)):
+                for nk in (1, 64, 449, 512, 1000, 1025, 2048, 4096, 5000, 16384, 65536, 131072, 1 << 20):
+                    need = lib.kfb_flash_attn_ws_bytes(b, h, hk, 1, nk, d)
+                    most, none, some = max(most, need), none + (need == 0), some + (need > 0)
+    assert 0 < most <= 2 << 20
+    assert some > 50 and none > some
+    assert lib.kfb_flash_attn_ws_bytes(8, 32, 4, 1, 4608, 64) == 0      # a cluster of four
+    assert lib.kfb_flash_attn_ws_bytes(1, 32, 4, 1, 16384, 64) > 0      # more than eight splits
+
+
 def test_int4_matmul_routing_table():
     """Which kernel int4_matmul picks by shape (pure host logic): GEMV up to M = 8, the same kernel with more batch columns
     for 8 < M <= 16 where it measured faster, the tcgen05 GEMM otherwise."""
