@@ -301,8 +301,10 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
           mma16816<kBf16>(oacc[2 * dn + 1], pa[kb], r2, r3);
         }
       // The stage is refilled through the async proxy: this warp's reads of it have to be over before it is given back.
-      // (Without the fence the next tile overwrote rows still being read: with K and V in L2 and several CTAs per SM,
-      // 19 of 20 calls at B = 8, Hk = 4, 1000..4096 keys had wrong heads, errors up to 0.1.)
+      // (An earlier form of this kernel, four warps on every tile, released it without the fence: 8 of 100 calls at B = 8, Hk = 4,
+      // 1152..4608 keys and 5 of 100 at B = 64, 1024..4096 were off by up to 0.03 from one another.  The fence alone, nothing else
+      // changed, made all of them equal and right, although there too an mma.sync had taken every loaded word before the arrive:
+      // that the words have been used does not order the reads before the copy.)
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty[s]);

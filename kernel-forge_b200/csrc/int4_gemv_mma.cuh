@@ -397,6 +397,7 @@ int4_gemv_mma_split_kernel(const __half* __restrict__ x, const __grid_constant__
     load_scales<G, 1>(srow, r0, nr, vec_scales, sc);
     if (!__all_sync(0xffffffffu, wait_stage(&my_bars[i % S], (uint32_t)(i / S) & 1u, ctx))) break;
     chunk_compute<G, 1, (NB <= 2 ? 2 : 1), NB>(lm, my_ring + (uint32_t)(i % S) * kStage, sx, r0, nr, sc, unpack, acc, [&] {
+      fence_proxy_async_smem();   // this warp's reads of the stage are over before its next copy may land
       __syncwarp();
       if (i + S < n_c) issue(i + S);
     });
@@ -568,6 +569,7 @@ int4_gemv_mma_stream_kernel(const __half* __restrict__ x, const __grid_constant_
       load_scales<G, T>(srow, r0, nr, vec_scales, sc);   // before the wait: overlaps it
       if (!__all_sync(0xffffffffu, wait_stage(&my_bars[q % S], (uint32_t)(q / S) & 1u, ctx))) { ok = false; return; }
       chunk_compute<G, T, RG, NB, XS>(lm, my_ring + (uint32_t)(q % S) * kStage, sx, r0, nr, sc, unpack, acc, [&] {
+        fence_proxy_async_smem();   // (as above; 152 us with it, 145 without, at 720896 x 2048, M = 1)
         __syncwarp();
         issue_next();
       });
