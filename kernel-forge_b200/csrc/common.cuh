@@ -56,7 +56,8 @@ int require_sm100();
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // `fresh`: pointers to what the kernel in front may have written.  Their values pass through the asm, so no load through
 // them can be moved above the wait (the compiler may move loads through `const T* __restrict__`, which it takes to be
-// invariant, across any memory clobber), nor become a non-coherent one.
+// invariant, across any memory clobber), nor become a non-coherent one.  For the same reason no kernel of this library asks
+// for a non-coherent load itself (__ldg, ld.global.nc).
 template <class... P>
 __device__ __forceinline__ void pdl_wait(P&... fresh) {
   asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -73,7 +73,8 @@ int4_norm_kernel(const __half* __restrict__ x, const uint32_t* __restrict__ pack
   __half* hx = reinterpret_cast<__half*>(part + M * kMaxWarps);
 
   // ---- before the wait: whatever does not depend on the kernel in front
-  if (!fu.early) pdl_wait(x, packed, scales);   // (early: the weights are older than it)
+  const __half* norm_w = fu.norm_w;
+  if (!fu.early) pdl_wait(x, packed, scales, norm_w);   // (early: the weights are older than it)
   uint2 wv[RB][2][NG][H];
   __half sv[RB][2][NG];
 #pragma unroll
@@ -87,7 +88,7 @@ int4_norm_kernel(const __half* __restrict__ x, const uint32_t* __restrict__ pack
       for (int i = 0; i < NG; ++i) {
 #pragma unroll
         for (int b = 0; b < H; ++b) wv[rb][h][i][b] = load_words(w + i * (G / 8) + b * 8);
-        sv[rb][h][i] = __ldg(s + i);
+        sv[rb][h][i] = s[i];
       }
     }
   uint32_t early[kEarlyUnpack ? H : 1][4][4];       // [64 k][word][pair]
@@ -102,9 +103,9 @@ int4_norm_kernel(const __half* __restrict__ x, const uint32_t* __restrict__ pack
   }
   const int pieces = K / 8;                         // 16-byte pieces of a row of activations: at most two per thread
   const int c0 = threadIdx.x, c1 = threadIdx.x + blockDim.x;
-  const uint4* nw = reinterpret_cast<const uint4*>(fu.norm_w);
+  const uint4* nw = reinterpret_cast<const uint4*>(norm_w);
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-  const uint4 w0 = c0 < pieces ? __ldg(nw + c0) : zero, w1 = c1 < pieces ? __ldg(nw + c1) : zero;
+  const uint4 w0 = c0 < pieces ? nw[c0] : zero, w1 = c1 < pieces ? nw[c1] : zero;
   const float inv_k = 1.0f / (float)K;
   for (int i = threadIdx.x; i < M * kMaxWarps; i += blockDim.x) part[i] = 0.f;
   __syncthreads();

@@ -146,7 +146,7 @@ int4_small_kernel(const uint16_t* __restrict__ x, const uint32_t* __restrict__ p
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           load_words(wbuf[slot][rb][h], wrow[rb][h] + (size_t)gi * (G / 8));
-          sbuf[slot][rb][h] = __half2float(__ldg(srow[rb][h] + gi));
+          sbuf[slot][rb][h] = __half2float(srow[rb][h][gi]);
         }
     }
   };

@@ -108,9 +108,7 @@ def test_custom_ops_registered_with_fakes():
 def test_prefill_workspace_covers_the_plan_with_and_without_the_causal_mask():
     """The bytes that kfb_flash_attn_ws_bytes reports are enough for the plan a call takes, causal or not (it is not told
     which); without a workspace the call is planned for no splits, not a split plan run unsplit.  Host logic."""
-    import ctypes
     import random
-    from kernelforge import _capi
     lib = _capi.lib()
 
     def plan(shape, causal, ws):
@@ -139,7 +137,6 @@ def test_prefill_workspace_covers_the_plan_with_and_without_the_causal_mask():
 def test_every_decode_plan_fits_the_array_of_the_allocation_free_entry():
     """kfb_flash_attn_decode_noalloc has 2 MiB for partials: no plan needs more, over groups, keys and head dims.  A workspace is
     asked for only where partials are written, so most plans need none.  Host logic."""
-    from kernelforge import _capi
     lib = _capi.lib()
     most, none, some = 0, 0, 0
     for d in (64, 128):
@@ -152,6 +149,16 @@ def test_every_decode_plan_fits_the_array_of_the_allocation_free_entry():
     assert some > 50 and none > some
     assert lib.kfb_flash_attn_ws_bytes(8, 32, 4, 1, 4608, 64) == 0      # a cluster of four
     assert lib.kfb_flash_attn_ws_bytes(1, 32, 4, 1, 16384, 64) > 0      # more than eight splits
+
+
+def test_no_kernel_asks_for_non_coherent_loads():
+    """Kernels are resident while the one in front still writes (programmatic dependent launch): what they read has to go through
+    coherent loads behind pdl_wait.  __ldg and ld.global.nc are taken to be invariant and may be moved above it."""
+    found = []
+    for src in sorted((ROOT / "kernel-forge_b200" / "csrc").iterdir()):
+        code = re.sub(r"//[^\n]*", "", src.read_text())
+        found += [f"{src.name}: {hit}" for hit in re.findall(r"__ldg\s*\(|ld\.global\.nc", code)]
+    assert not found, found
 
 
 def test_int4_matmul_routing_table():
