@@ -334,6 +334,8 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         }
       }
     }
+    } else {
+      cluster_wait();   // the two warps that only fill the warpgroup: every arrive has its wait before the next one
     }
   } else if (warp < kDequantWarps) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsDequant));

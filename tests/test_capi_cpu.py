@@ -253,3 +253,19 @@ def test_private_row_orders_are_permutations_prefill_can_undo():
     gate, up = (torch.randn(inter, k, generator=g, dtype=torch.float64) for _ in range(2))
     gu = (x @ ops.interleave_gate_up(gate, up).T).view(b, t, inter, 2)
     assert torch.equal(gu[..., 0], x @ gate.T) and torch.equal(gu[..., 1], x @ up.T)
+
+
+def test_every_role_of_the_gemm_waits_for_the_cluster_once():
+    """int4_gemm_kernel arrives on the cluster barrier before its roles part: each role has to wait for that phase before the
+    arrive of the teardown (two arrives in a row are not defined).  Read from the source: no run shows it."""
+    code = re.sub(r"//[^\n]*", "", (ROOT / "kernel-forge_b200" / "csrc" / "int4_gemm.cu").read_text())
+    code = code[code.index("int4_gemm_kernel("):]
+    first = code.index("cluster_arrive();")
+    roles, teardown = code[first:code.index("cluster_arrive_relaxed();")], code[code.index("cluster_arrive_relaxed();"):]
+    assert roles.count("cluster_arrive") == 1 and teardown.index("cluster_wait();") > 0
+    inner = roles[roles.index("if (warp >= kProducerWarp) {"):]
+    producer, rest = inner.split("} else if (warp == kMmaWarp) {", 1)
+    mma, rest = rest.split("} else {\n      cluster_wait();", 1)       # the filling warps
+    dequant, epilogue = rest.split("} else if (warp < kDequantWarps) {", 1)[1].split("} else {\n", 1)
+    assert producer.count("cluster_wait();") == 1 and mma.count("cluster_wait();") == 1
+    assert dequant.count("cluster_wait();") + epilogue.count("cluster_wait();") == 3   # (dequantise: at its first block, or at the end)
