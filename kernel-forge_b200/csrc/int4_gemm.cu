@@ -419,8 +419,10 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     const int wg = (warp - kDequantWarps) >> 2, r = (warp & 3) * 32 + lane;
     const uint32_t lane_bits = (uint32_t)((warp & 3) * 32) << 16;
     const int chunks = sh.mt / 32;
-    // A wait expired earlier on this device: nothing is written (the read's latency passes during the products).
-    bool ok = __all_sync(0xffffffffu, *reinterpret_cast<volatile unsigned int*>(status) == 0);
+    // A wait expired earlier on this device: nothing is written (the read's latency passes during the products), but the
+    // accumulators are still given back: without that the MMA warp's wait for one would run out too, 2 s in every call.
+    const bool muted = __any_sync(0xffffffffu, *reinterpret_cast<volatile unsigned int*>(status) != 0);
+    bool ok = true;
     cluster_wait();
     uint32_t ic = 0;
     for (int it = pair; ok && it < items; it += pairs, ++ic) {
@@ -432,6 +434,10 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[buf], use & 1u, ctx, kWaitAcc));
       if (!ok) break;
       tc_fence_after_sync();
+      if (muted) {
+        if (lane == 0 && it + (two_acc ? 2 : 1) * pairs < items) mbar_arrive_at(&acc_free[buf], 0);
+        continue;
+      }
       const uint32_t acc = tmem_base + buf * 128u + lane_bits;
       if (sh.splits > 1) {   // FP32 partials: a warp's 32 rows are 128 contiguous bytes of every batch row
         float* dst = partial + ((size_t)w.split * sh.M + w.m0) * sh.N + row;

@@ -10,6 +10,7 @@ import torch
 
 from helpers import ATTN_ATOL, attn_oracle, qkv_case
 from kernelforge import _capi, ops
+from kernelforge import quantize as kq
 
 pytestmark = pytest.mark.gpu
 
@@ -43,6 +44,37 @@ def test_expired_wait_is_reported_and_cleared():
     out = ops.flash_attn(qc, kc, vc, causal=True)
     assert np.abs(out.float().cpu().numpy() - attn_oracle(q, k, v, True)).max() <= ATTN_ATOL[torch.float16]
     assert _capi.device_status(dev) == 0
+
+
+@pytest.mark.parametrize("m", [1024, 3000])   # several tiles per CTA pair, no splits along K
+def test_gemm_returns_at_once_while_the_status_word_is_set(m):
+    """The persistent GEMM writes nothing then, and none of its own waits runs out (2 s each) for want of the accumulators."""
+    dev = torch.device("cuda", 0)
+    lib = _capi.lib()
+    g = torch.Generator(device=dev).manual_seed(1)
+    x = torch.randn(m, 1536, generator=g, device=dev, dtype=torch.float16)
+    qw = kq.quantize_weight(torch.randn(8960, 1536, generator=g, device=dev, dtype=torch.float16) * 0.02, 128)
+    want = ops.int4_linear(x, qw.packed, qw.scales, 128)
+    assert lib.kfb_int4_linear_ws_bytes(m, 8960, 1536, 128, 0) == 0
+    y = torch.full_like(want, 7.0)
+    outcome = torch.zeros(1, dtype=torch.int32, device=dev)
+    start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    try:
+        with _capi.on_device(dev):
+            _capi.check(lib.kfb_selftest_wait_expiry(2_000_000, outcome.data_ptr(), _capi.stream_ptr(dev)))
+        torch.cuda.synchronize()
+        assert _capi.device_status(dev) == 0x601
+        start.record()
+        _capi.check(lib.kfb_int4_linear(x.data_ptr(), qw.packed.data_ptr(), qw.scales.data_ptr(), None, y.data_ptr(), m, 8960, 1536, 128, 0,
+                                        None, 0, _capi.stream_ptr(dev)))
+        end.record()
+        torch.cuda.synchronize()
+        assert bool((y == 7.0).all()) and start.elapsed_time(end) < 500.0
+        assert _capi.device_status(dev) == 0x601
+    finally:
+        _capi.device_status_reset(dev)
+        torch.cuda.synchronize()
+    assert torch.equal(ops.int4_linear(x, qw.packed, qw.scales, 128), want)
 
 
 def test_selftest_rejects_limits_out_of_range():
