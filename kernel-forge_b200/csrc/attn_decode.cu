@@ -463,31 +463,46 @@ struct SplitPlan {
   bool clustered;
 };
 
-// How many CTAs share the keys of one (batch, kv head, chunk) group.  Measured at 24 shapes of 4..512 groups and 225..16384
-// keys, best of unsplit / clusters of 2..8 / 2..48 splits with a merge kernel:
-//   * more than 64 groups: one CTA each.  A second wave of CTAs or half-empty rings cost more than an uneven tail
-//     (64 x 4 groups of 4096 keys: 43.0 us, best split 48.7; 40 x 4 of 300..1200: 11.7, split 12.0).
-//   * otherwise as many as fit the GPU at once, one per SM, as a cluster of at most eight (8 x 4 groups of 1000..4096:
-//     8.6 us; three splits and a merge kernel 11.1).  Every CTA keeps two tiles (545 keys: 4.1 us, unsplit 4.8), and a
-//     group of fewer than eight tiles is quicker alone (225 keys: 4.3 against 5.3).
-//   * a handful of groups with long caches (the only plans that write partials, at most one per SM): eight CTAs each leave most of the chip idle, and from 16 tiles of D = 64 per
-//     CTA on that costs more than the merge kernel, whose own cost grows with the splits (4 groups of 16384 keys: eight in
-//     a cluster 11.4 us, 16 to 32 and a merge 9.7; 4096 keys: 6.7 and 6.8; one group of 131072: 48 splits 16.3, 148 19.6).
+// How many CTAs share the keys of one (batch, kv head, chunk) group.  Only the capacity of the cache is known here, not the
+// valid lengths.  Measured in a graph over 24..256 groups of 300..16384 keys, all lengths equal to the capacity / to half of it /
+// spread from a quarter to the whole (us), best of unsplit / clusters of 2..8 / 3..48 splits with a merge kernel:
+//   * as many as fit the GPU at once, one per SM, as a cluster of at most eight (8 x 4 groups of 1000..4096: 8.6; three splits
+//     and a merge kernel 11.1).  Every CTA keeps two tiles (545 keys: 4.1, unsplit 4.8), a group of fewer than eight tiles is
+//     quicker alone (225 keys: 4.3 against 5.3).  Two or three CTAs need longer caches to pay for the merge: 64 groups of 1000
+//     keys 7.1 / 5.6 / 7.1 unsplit against 7.4 / 6.2 / 6.9 in pairs, of 2000 11.1 / 7.4 / 10.7 against 10.6 / 7.5 / 8.9.
+//   * more groups than clusters of two (74: the SMs come in pairs; 68 groups of 8192: pairs 26.1 / 12.5 / 18.7, unsplit 30.4 /
+//     17.0 / 29.9): one CTA each; a second wave of CTAs or half-empty rings cost more than an uneven tail, except (D = 64,
+//     three shallow CTAs per SM) where caches are so long that the longest sequence's CTA is on its own for most of the time:
+//     80 groups of 16384: clusters of four 53.6 / 30.2 / 40.6, unsplit 59.3 / 31.0 / 55.5; 160 of 8192: pairs 53.8 / 30.8 /
+//     40.9, unsplit 62.6 / 34.0 / 55.7.
+//   * 45 to 51 groups of very long caches: pairs would leave a third of the SMs idle, six shallow CTAs each do not
+//     (48 groups of 16384: 36.1 / 18.8 / 27.4, pairs 35.2 / 19.1 / 32.2).
+//   * a handful of groups with long caches (the only plans that write partials, at most one per SM): eight CTAs each leave most
+//     of the chip idle, and from 16 tiles of D = 64 per CTA on that costs more than the merge kernel, whose own cost grows with
+//     the splits (4 groups of 16384 keys: eight in a cluster 11.4, 16 to 32 and a merge 9.7; 4096 keys: 6.7 and 6.8; one group
+//     of 131072: 48 splits 16.3, 148 19.6).
 SplitPlan plan_splits(int B, int H, int Hk, int Nk, int D) {
-  constexpr int kMinTiles = 8;
-  // Clusters of 1..8 such CTAs that fit at once: cudaOccupancyMaxActiveClusters gives 148, 74, 45, 33, 26, 22, 15, 15; a
-  // little less here, since which SMs a chip has differs.  (With one cluster too many, 16 of eight, 3072 keys took 13 us
-  // instead of 9.6.)
-  constexpr int kFit[9] = {0, 148, 64, 44, 32, 24, 20, 14, 14};
+  // Clusters of 1..8 CTAs, one per SM, that fit at once: cudaOccupancyMaxActiveClusters gives 148, 74, 45, 33, 26, 22, 15, 15;
+  // from three on a little less here, since which SMs a chip has differs.  (With one cluster too many, 16 of eight, 3072 keys
+  // took 13 us instead of 9.6.)
+  constexpr int kFit[9] = {0, 148, 74, 44, 32, 24, 20, 14, 14};
+  constexpr int kLeastTiles[9] = {0, 8, 24, 12, 8, 10, 12, 14, 16};   // of the capacity, for a cluster of that size
   SplitPlan p;
   p.chunks = ceil_div(H / Hk, kRows);
   p.splits = 1;
   p.clustered = false;
   const long long groups = (long long)B * Hk * p.chunks;
   const int tiles = ceil_div(Nk, kTileKeys);
-  if (tiles < kMinTiles || groups > kFit[2]) return p;
-  int cluster = 8;
-  while (cluster > 1 && (cluster * 2 > tiles || groups > kFit[cluster])) --cluster;
+  if (tiles < kLeastTiles[1]) return p;
+  int cluster = 1;
+  if (D == 64 && groups > kFit[3] && groups <= 51 && tiles >= 256) cluster = 6;
+  else if (D == 64 && groups > kFit[2] && groups <= 88 && tiles >= 128) cluster = 4;
+  else if (D == 64 && groups > kFit[1] && groups <= 192 && tiles >= 64) cluster = 2;
+  else if (groups <= kFit[2]) {
+    cluster = 8;
+    while (cluster > 1 && (cluster * 2 > tiles || groups > kFit[cluster])) --cluster;
+    if (tiles < kLeastTiles[cluster]) return p;
+  }
   p.splits = cluster;
   p.clustered = cluster > 1;
   const int at_once = sm_count() / (int)groups;

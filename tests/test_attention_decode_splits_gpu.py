@@ -21,8 +21,14 @@ pytestmark = pytest.mark.gpu
     (8, 32, 4, 64, 4608, (1000, 4096, 4608, 63, 2047, 2048, 2049, 3333)),
     (5, 8, 4, 64, 2048, (2048, 2000, 1, 129, 640)),      # 20 groups: clusters of six
     (3, 8, 8, 128, 1500, (1500, 64, 1437)),              # 24 groups: clusters of five
-    (11, 4, 4, 64, 700, tuple(range(640, 651))),         # 44 groups: clusters of three
-    (16, 8, 4, 128, 1000, tuple(range(0, 1000, 63))),    # 64 groups: pairs
+    (11, 4, 4, 64, 700, tuple(range(640, 651))),         # 44 groups, 11 tiles: too short for clusters of three
+    (11, 4, 4, 64, 705, tuple(range(640, 706, 6))),      # 12 tiles: clusters of three
+    (16, 8, 4, 128, 1000, tuple(range(0, 1000, 63))),    # 64 groups, 16 tiles: too short for pairs
+    (16, 8, 4, 128, 1473, tuple(range(1, 1473, 95))),   # 24 tiles: pairs
+    (37, 2, 2, 64, 1600, tuple(range(0, 1600, 44))),     # 74 groups: as many pairs as there are
+    (12, 4, 4, 64, 16321, tuple(range(1, 16321, 1483))), # 48 groups of very long caches: clusters of six on the shallow ring
+    (20, 4, 4, 64, 8129, tuple(range(0, 8129, 427))),    # 80 groups of long caches: clusters of four on the shallow ring
+    (40, 4, 4, 64, 4033, tuple(range(64, 4033, 100))),   # 160 groups of long caches: pairs on the shallow ring
     (1, 34, 2, 64, 16384, (16321,)),                     # 34 / 2 = 17 heads: two chunks; splits and a merge kernel
     (40, 8, 4, 64, 2000, tuple(range(1, 2000, 50))),     # more groups than SMs: the shallow ring, three CTAs per SM
     (40, 8, 8, 128, 900, tuple(range(20, 900, 22))),     # the same at D = 128, two per SM
