@@ -15,6 +15,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cmath>
@@ -66,14 +67,12 @@ struct OnDevice {
 };
 inline void* stream_of(const at::Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
 
+// C++ exceptions become the Python ones that torch's own functions raise (torch.OutOfMemoryError and so on).
 template <class F>
 PyObject* guarded(F&& body) {
-  try {
-    return body();
-  } catch (const std::exception& e) {   // out of memory and the like: torch's message
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
-  }
+  HANDLE_TH_ERRORS
+  return body();
+  END_HANDLE_TH_ERRORS
 }
 
 PyObject* pair_of(at::Tensor first, PyObject* second /* new reference or null */) {
