@@ -792,6 +792,37 @@ def single_kernel_main(args):
 
 
 # ----------------------------------------------------------------------------------------------
+# the printed line
+# ----------------------------------------------------------------------------------------------
+
+def digits(x, n: int = 4):
+    """x with its floating-point numbers rounded to n significant digits."""
+    if isinstance(x, dict):
+        return {k: digits(v, n) for k, v in x.items()}
+    if isinstance(x, (list, tuple)):
+        return [digits(v, n) for v in x]
+    return float(f"{x:.{n}g}") if isinstance(x, float) else x
+
+
+def brief(also: dict) -> dict:
+    """One number per workload and its share of the measured peak: [value, share].  Values are tok/s, TFLOP/s where the bound is
+    the tensor pipe, GB/s otherwise.  The records themselves go to stderr: with them the line was 20 KB long, and whoever keeps
+    only the last 3000 characters of a program's output could not parse it."""
+    out = {}
+    for name, rec in also.items():
+        short = name.replace("_tinyllama_arch", "").replace("_flash_attn", "").replace("_int4_linear", "").replace("decode_", "dec_")
+        if "error" in rec:
+            out[short] = rec["error"][:60]
+        elif name.startswith("c2_sweep"):
+            out[short] = {k: round(r["tflops"]) for k, r in rec.items() if k.startswith(("n2048", "n8192"))}
+        elif not name.startswith("c4") or rec["K"] * rec["N"] > 4 << 20:
+            kind = rec.get("roofline", {}).get("bound")
+            value = rec.get("tok_per_s") or (rec["tflops"] if kind == "tensor" else rec.get("gbs"))
+            out[short] = digits([value, rec.get("roofline", {}).get("frac")], 3)
+    return out
+
+
+# ----------------------------------------------------------------------------------------------
 # main
 # ----------------------------------------------------------------------------------------------
 
@@ -815,9 +846,9 @@ def main():
         return single_kernel_main(args)
 
     config = {"workload": "flash_attn fwd MHA fp16 B=2 H=16 N=2048 D=64 non-causal, scale 1/sqrt(64)",
-              "l2": "inputs rotate over distinct sets totalling > 2x the 126 MB L2",
-              "per_gpu": "same batch shape on every GPU (batch x heads shard, no communication)",
-              "timing": "blocks of K steps, each one CUDA-graph replay between barrier + synchronize, CUDA events; median block, max over ranks"}
+              "l2": "inputs rotate over sets of > 2x L2",
+              "per_gpu": "same shape on every GPU (batch x heads shard)",
+              "timing": "blocks of K steps, one CUDA-graph replay each, CUDA events; median block, max over ranks"}
     base = {"metric": "flash_attn TFLOPS (% peak) [headline]; int4_linear M=1 HBM GB/s [headline_alt]; decode tok/s and the rest under `also`",
             "unit": "TFLOP/s", "n_gpus": args.gpus, "steps": args.steps,
             "warmup": args.warmup, "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f16",
@@ -867,16 +898,19 @@ def main():
         "roofline": roofline("tensor", fa["tflops"] / world, peaks, kind,
                              # dram__bytes_read.sum + dram__bytes_write.sum of one launch of this workload from an ncu capture
                              # (q, k, v read once = 25.2 MB; o stays in L2 until after the launch)
-                             traffic=25205760, kernel="attn_prefill_pair_kernel<64,fp16>"),
+                             traffic=25205760, kernel="attn_prefill_kernel<64,fp16,2>"),
     })
     c1 = also.get("c1_int4_linear_m1_5632x2048")
     if c1:
         line["headline_alt"] = {"metric": "int4_linear M=1 K=2048 N=5632 g128 HBM GB/s", "value": c1["gbs"], "unit": "GB/s",
                                 "us_per_call": c1["us_per_call"], "roofline": c1["roofline"]}
-    line["also"] = also
     if rank == 0:
-        line["cpu_baseline"] = cpu_attention(HEADLINE, False, args.cpu_seconds) if full else None
-        print(json.dumps(line))
+        cpu = cpu_attention(HEADLINE, False, args.cpu_seconds) if full else None
+        print(json.dumps({"records": dict(also, headline=line["roofline"], cpu_baseline=cpu)}), file=sys.stderr)
+        line["also"] = brief(also)
+        line["cpu_baseline"] = cpu and {k: cpu[k] for k in ("value", "unit", "cores", "kind")}
+        line["roofline"] = {k: line["roofline"][k] for k in ("bound", "achieved", "peak", "unit", "frac", "kernel")}
+        print(json.dumps(digits(line, 6), separators=(",", ":")))
     if world > 1:
         import torch.distributed as dist
         dist.destroy_process_group()
