@@ -27,9 +27,16 @@ INT4_GROUP_SIZES = (64, 128)
 def _resolve_scale(scale: float | None, head_dim: int) -> float:
     if scale is None:
         return 1.0 / math.sqrt(head_dim)
-    if scale <= 0:
+    if not scale > 0:   # (NaN too)
         raise ValueError(f"scale must be positive, got {scale}")
     return float(scale)
+
+
+def _native(out, what: str, args: str = "arguments"):
+    """The result of a native call that has nothing behind it: declined arguments are an error there, never a None."""
+    if out is None:
+        raise ValueError(f"{what}: {args} must be non-empty contiguous fp16 CUDA tensors of matching shapes")
+    return out
 
 
 # ---------------------------------------------------------------------------
@@ -360,7 +367,8 @@ def int4_matmul(x: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, gro
     if x.shape[0] == 0 or packed.shape[0] == 0:
         return torch.empty(x.shape[0], packed.shape[0], dtype=x.dtype, device=x.device)
     # tensor subclasses and the like: plain views of the same memory
-    return _linear_launch(x.as_subclass(torch.Tensor), packed.as_subclass(torch.Tensor), scales.as_subclass(torch.Tensor), group_size, None)
+    plain = lambda t: t.as_subclass(torch.Tensor)
+    return _native(_linear_launch(plain(x), plain(packed), plain(scales), int(group_size), None), "int4_matmul", "x, packed and scales")
 
 
 def _linear_launch(x, packed, scales, group_size, bias):
@@ -395,6 +403,8 @@ def _check_attn(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool,
             raise ValueError(f"{name} must be contiguous (call .contiguous() first)")
     if not (q.dtype == k.dtype == v.dtype):
         raise TypeError(f"q, k, v must share a dtype, got {q.dtype}, {k.dtype}, {v.dtype}")
+    if not (q.device == k.device == v.device):
+        raise ValueError(f"q, k and v must be on the same CUDA device, got {q.device}, {k.device}, {v.device}")
     if k.shape != v.shape:
         raise ValueError(f"k and v must have the same shape, got {tuple(k.shape)} and {tuple(v.shape)}")
     (b, h, nq, d), (bk, hk, nk, dk) = q.shape, k.shape
@@ -419,7 +429,7 @@ def _attn_launch(q, k, v, causal: bool, scale: float) -> torch.Tensor:
         raise ValueError("attention needs at least one key (Nk >= 1)")
     # tensor subclasses, or K / V views that cannot be read in place
     plain = lambda t: t.contiguous().as_subclass(torch.Tensor)
-    return _capi.host().flash_attn(plain(q), plain(k), plain(v), causal, scale, False)
+    return _native(_capi.host().flash_attn(plain(q), plain(k), plain(v), causal, scale, False), "flash_attn", "q, k and v")
 
 
 @torch.library.custom_op("kernelforge::flash_attn", mutates_args=())
@@ -584,12 +594,6 @@ def int4_linear_silu_pairs(x: torch.Tensor, packed: torch.Tensor, scales: torch.
 # Fused element-wise steps of a decode step (not part of the reference's operator surface, which leaves
 # them to torch; used by kernelforge.llama_decode)
 # ---------------------------------------------------------------------------
-
-def _native(out, what: str):
-    if out is None:
-        raise ValueError(f"{what}: arguments must be non-empty contiguous fp16 CUDA tensors of matching shapes")
-    return out
-
 
 def add_rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float, residual: torch.Tensor | None = None):
     """(y, s): s = x + residual (x itself when residual is None), y = RMSNorm(s) * weight.  fp16 [rows, hidden]."""

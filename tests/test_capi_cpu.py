@@ -269,3 +269,13 @@ def test_every_role_of_the_gemm_waits_for_the_cluster_once():
     dequant, epilogue = rest.split("} else if (warp < kDequantWarps) {", 1)[1].split("} else {\n", 1)
     assert producer.count("cluster_wait();") == 1 and mma.count("cluster_wait();") == 1
     assert dequant.count("cluster_wait();") + epilogue.count("cluster_wait();") == 3   # (dequantise: at its first block, or at the end)
+
+
+@pytest.mark.parametrize("call", ["flash_attn", "flash_attn_kv_view"])
+def test_attention_refuses_tensors_of_different_devices(call):
+    """The native path declines them; what stands behind it has to raise, not to return None."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    with FakeTensorMode(allow_non_fake_inputs=True):
+        q, k = (torch.empty(1, 2, 16, 64, dtype=torch.float16, device=f"cuda:{i}") for i in (0, 1))
+        with pytest.raises(ValueError, match="same CUDA device"):
+            getattr(ops, call)(q, k, k)

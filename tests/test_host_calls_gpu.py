@@ -23,3 +23,19 @@ def test_a_result_that_does_not_fit_raises_torchs_out_of_memory_error():
         ops.int4_linear(x, packed, scales, 64)
     torch.cuda.empty_cache()
     assert not ops.int4_linear(x[:3], packed, scales, 64).any()    # and the next call works
+
+
+@pytest.mark.parametrize("call", ["flash_attn", "flash_attn_kv_view", "flash_attn_decode"])
+def test_a_scale_that_is_not_a_number_is_refused(call):
+    q, kv = torch.zeros(1, 2, 1, 64, dtype=torch.float16, device="cuda"), torch.zeros(1, 2, 70, 64, dtype=torch.float16, device="cuda")
+    lengths = (torch.ones(1, dtype=torch.int32, device="cuda"),) if call == "flash_attn_decode" else ()
+    with pytest.raises(ValueError, match="scale must be positive"):
+        getattr(ops, call)(q, kv, kv, *lengths, scale=float("nan"))
+
+
+@pytest.mark.parametrize("m", [1, 5, 40])
+def test_group_size_may_be_any_number_equal_to_it(m):
+    qw = weight(256, 512)
+    x = torch.randn(m, 512, device="cuda", dtype=torch.float16)
+    got = ops.int4_matmul(x, qw.packed, qw.scales, 128.0)
+    assert got is not None and torch.equal(got, ops.int4_matmul(x, qw.packed, qw.scales, 128))
