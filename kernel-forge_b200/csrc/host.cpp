@@ -24,11 +24,13 @@
 
 namespace {
 
-// A plain torch.Tensor (or nn.Parameter) on a CUDA device: what the kernels take without further questions.
+// A plain torch.Tensor (or nn.Parameter) on a CUDA device: what the kernels take without further questions.  The wrappers of
+// torch.func (vmap, grad, jvp) have the type of a plain tensor, but no memory of their own.
 inline const at::Tensor* plain(PyObject* o) {
   if (!THPVariable_CheckTypeExact(Py_TYPE(o))) return nullptr;
   const at::Tensor& t = THPVariable_Unpack(o);
-  return t.is_cuda() && t.layout() == at::kStrided ? &t : nullptr;
+  constexpr c10::DispatchKeySet wrappers({c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper});
+  return t.is_cuda() && t.layout() == at::kStrided && !t.key_set().has_any(wrappers) ? &t : nullptr;
 }
 
 inline bool int_arg(PyObject* o, long long* out) {
@@ -74,6 +76,12 @@ PyObject* guarded(F&& body) {
   return body();
   END_HANDLE_TH_ERRORS
 }
+
+// The interpreter lock is free while this lives.  An exception that passes through takes it back first (data_ptr() throws).
+struct NoGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~NoGil() { PyEval_RestoreThread(state); }
+};
 
 PyObject* pair_of(at::Tensor first, PyObject* second /* new reference or null */) {
   PyObject* f = second ? THPVariable_Wrap(std::move(first)) : nullptr;
@@ -124,12 +132,13 @@ PyObject* int4_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (ws_bytes) ws = new_tensor({(int64_t)ws_bytes}, at::kByte, *x);
     void *stream = stream_of(*x), *wsp = ws_bytes ? ws.data_ptr() : nullptr;
     int rc;
-    Py_BEGIN_ALLOW_THREADS
-    if (silu) rc = kfb_int4_linear_silu_pairs(x->data_ptr(), packed->data_ptr(), scales->data_ptr(), y.data_ptr(), (int)m, (int)rows, (int)k,
-                                              (int)group, wsp, ws_bytes, stream);
-    else rc = kfb_int4_linear(x->data_ptr(), packed->data_ptr(), scales->data_ptr(), bias ? bias->data_ptr() : nullptr, y.data_ptr(), (int)m,
-                              (int)rows, (int)k, (int)group, code, wsp, ws_bytes, stream);
-    Py_END_ALLOW_THREADS
+    {
+      NoGil free;
+      if (silu) rc = kfb_int4_linear_silu_pairs(x->data_ptr(), packed->data_ptr(), scales->data_ptr(), y.data_ptr(), (int)m, (int)rows, (int)k,
+                                                (int)group, wsp, ws_bytes, stream);
+      else rc = kfb_int4_linear(x->data_ptr(), packed->data_ptr(), scales->data_ptr(), bias ? bias->data_ptr() : nullptr, y.data_ptr(), (int)m,
+                                (int)rows, (int)k, (int)group, code, wsp, ws_bytes, stream);
+    }
     return rc ? raise_status(rc) : THPVariable_Wrap(std::move(y));
   });
 }
@@ -194,11 +203,12 @@ PyObject* flash_attn(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (ws_bytes) ws = new_tensor({(int64_t)ws_bytes}, at::kByte, *p.q);
     void* stream = stream_of(*p.q);
     int rc;
-    Py_BEGIN_ALLOW_THREADS
-    rc = kfb_flash_attn_fwd(p.q->data_ptr(), p.k->data_ptr(), p.v->data_ptr(), o.data_ptr(), dtype_code(p.q->scalar_type()), (int)p.b, (int)p.h,
-                            (int)p.hk, (int)p.nq, (int)p.nk, (int)p.d, causal, scale, p.strided ? p.strides : nullptr,
-                            ws_bytes ? ws.data_ptr() : nullptr, ws_bytes, stream);
-    Py_END_ALLOW_THREADS
+    {
+      NoGil free;
+      rc = kfb_flash_attn_fwd(p.q->data_ptr(), p.k->data_ptr(), p.v->data_ptr(), o.data_ptr(), dtype_code(p.q->scalar_type()), (int)p.b, (int)p.h,
+                              (int)p.hk, (int)p.nq, (int)p.nk, (int)p.d, causal, scale, p.strided ? p.strides : nullptr,
+                              ws_bytes ? ws.data_ptr() : nullptr, ws_bytes, stream);
+    }
     return rc ? raise_status(rc) : THPVariable_Wrap(std::move(o));
   });
 }
@@ -219,11 +229,12 @@ PyObject* flash_attn_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (ws_bytes) ws = new_tensor({(int64_t)ws_bytes}, at::kByte, *p.q);
     void* stream = stream_of(*p.q);
     int rc;
-    Py_BEGIN_ALLOW_THREADS
-    rc = kfb_flash_attn_decode_kvlen(p.q->data_ptr(), p.k->data_ptr(), p.v->data_ptr(), o.data_ptr(), dtype_code(p.q->scalar_type()), (int)p.b,
-                                     (int)p.h, (int)p.hk, (int)p.nk, (int)p.d, scale, p.strided ? p.strides : nullptr,
-                                     static_cast<const int32_t*>(len->data_ptr()), ws_bytes ? ws.data_ptr() : nullptr, ws_bytes, stream);
-    Py_END_ALLOW_THREADS
+    {
+      NoGil free;
+      rc = kfb_flash_attn_decode_kvlen(p.q->data_ptr(), p.k->data_ptr(), p.v->data_ptr(), o.data_ptr(), dtype_code(p.q->scalar_type()), (int)p.b,
+                                       (int)p.h, (int)p.hk, (int)p.nk, (int)p.d, scale, p.strided ? p.strides : nullptr,
+                                       static_cast<const int32_t*>(len->data_ptr()), ws_bytes ? ws.data_ptr() : nullptr, ws_bytes, stream);
+    }
     return rc ? raise_status(rc) : THPVariable_Wrap(std::move(o));
   });
 }
@@ -241,9 +252,10 @@ PyObject* quantize_pack(PyObject*, PyObject* const* a, Py_ssize_t n) {
     at::Tensor packed = new_tensor({rows, k / 8}, at::kInt, *w), scales = new_tensor({rows, k / group}, at::kHalf, *w);
     void* stream = stream_of(*w);
     int rc;
-    Py_BEGIN_ALLOW_THREADS
-    rc = kfb_quantize_pack(w->data_ptr(), dtype_code(w->scalar_type()), (int)rows, (int)k, (int)group, packed.data_ptr(), scales.data_ptr(), stream);
-    Py_END_ALLOW_THREADS
+    {
+      NoGil free;
+      rc = kfb_quantize_pack(w->data_ptr(), dtype_code(w->scalar_type()), (int)rows, (int)k, (int)group, packed.data_ptr(), scales.data_ptr(), stream);
+    }
     if (rc) return raise_status(rc);
     return pair_of(std::move(packed), THPVariable_Wrap(std::move(scales)));
   });
@@ -271,10 +283,11 @@ PyObject* add_rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (res) s = new_tensor(x->sizes(), at::kHalf, *x);
     void* stream = stream_of(*x);
     int rc;
-    Py_BEGIN_ALLOW_THREADS
-    rc = kfb_add_rmsnorm(x->data_ptr(), res ? res->data_ptr() : nullptr, w->data_ptr(), y.data_ptr(), res ? s.data_ptr() : nullptr,
-                         (int)x->size(0), (int)x->size(1), (float)eps, stream);
-    Py_END_ALLOW_THREADS
+    {
+      NoGil free;
+      rc = kfb_add_rmsnorm(x->data_ptr(), res ? res->data_ptr() : nullptr, w->data_ptr(), y.data_ptr(), res ? s.data_ptr() : nullptr,
+                           (int)x->size(0), (int)x->size(1), (float)eps, stream);
+    }
     if (rc) return raise_status(rc);
     if (res) return pair_of(std::move(y), THPVariable_Wrap(std::move(s)));
     Py_INCREF(a[0]);
@@ -302,10 +315,11 @@ PyObject* rope_tokens(PyObject*, PyObject* const* a, Py_ssize_t n) {
     at::Tensor q = new_tensor({b, t, h, d}, at::kHalf, *qkv);
     void* stream = stream_of(*qkv);
     int rc;
-    Py_BEGIN_ALLOW_THREADS
-    rc = kfb_rope_tokens(qkv->data_ptr(), cos->data_ptr(), sin->data_ptr(), q.data_ptr(), kc->data_ptr(), vc->data_ptr(), (int)b, (int)t, (int)h,
-                         (int)hk, (int)d, (int)lmax, pairs, stream);
-    Py_END_ALLOW_THREADS
+    {
+      NoGil free;
+      rc = kfb_rope_tokens(qkv->data_ptr(), cos->data_ptr(), sin->data_ptr(), q.data_ptr(), kc->data_ptr(), vc->data_ptr(), (int)b, (int)t, (int)h,
+                           (int)hk, (int)d, (int)lmax, pairs, stream);
+    }
     return rc ? raise_status(rc) : THPVariable_Wrap(std::move(q));
   });
 }
@@ -329,10 +343,11 @@ PyObject* attention_tokens(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (ws_bytes) ws = new_tensor({(int64_t)ws_bytes}, at::kByte, *q);
     void* stream = stream_of(*q);
     int rc;
-    Py_BEGIN_ALLOW_THREADS
-    rc = kfb_flash_attn_fwd_tokens(q->data_ptr(), kc->data_ptr(), vc->data_ptr(), o.data_ptr(), KFB_F16, (int)b, (int)h, (int)hk, (int)t, (int)nk,
-                                   (int)d, causal, (float)(1.0 / std::sqrt((double)d)), strides, ws_bytes ? ws.data_ptr() : nullptr, ws_bytes, stream);
-    Py_END_ALLOW_THREADS
+    {
+      NoGil free;
+      rc = kfb_flash_attn_fwd_tokens(q->data_ptr(), kc->data_ptr(), vc->data_ptr(), o.data_ptr(), KFB_F16, (int)b, (int)h, (int)hk, (int)t, (int)nk,
+                                     (int)d, causal, (float)(1.0 / std::sqrt((double)d)), strides, ws_bytes ? ws.data_ptr() : nullptr, ws_bytes, stream);
+    }
     return rc ? raise_status(rc) : THPVariable_Wrap(std::move(o));
   });
 }
@@ -349,10 +364,11 @@ PyObject* silu_mul(PyObject*, PyObject* const* a, Py_ssize_t n) {
     at::Tensor act = new_tensor({rows, inter}, at::kHalf, *gu);
     void* stream = stream_of(*gu);
     int rc;
-    Py_BEGIN_ALLOW_THREADS
-    rc = pairs ? kfb_silu_mul_pairs(gu->data_ptr(), act.data_ptr(), (int)rows, (int)inter, stream)
-               : kfb_silu_mul(gu->data_ptr(), act.data_ptr(), (int)rows, (int)inter, stream);
-    Py_END_ALLOW_THREADS
+    {
+      NoGil free;
+      rc = pairs ? kfb_silu_mul_pairs(gu->data_ptr(), act.data_ptr(), (int)rows, (int)inter, stream)
+                 : kfb_silu_mul(gu->data_ptr(), act.data_ptr(), (int)rows, (int)inter, stream);
+    }
     return rc ? raise_status(rc) : THPVariable_Wrap(std::move(act));
   });
 }

@@ -39,3 +39,29 @@ def test_group_size_may_be_any_number_equal_to_it(m):
     x = torch.randn(m, 512, device="cuda", dtype=torch.float16)
     got = ops.int4_matmul(x, qw.packed, qw.scales, 128.0)
     assert got is not None and torch.equal(got, ops.int4_matmul(x, qw.packed, qw.scales, 128))
+
+
+def test_wrappers_of_torch_func_are_never_read_as_memory():
+    """The operands of vmap, grad and jvp look like plain tensors and have no memory: a call raises, or (where torch can take it
+    apart) gives what the calls one by one give.  It does not crash."""
+    qw = weight(256, 512)
+    x = torch.randn(2, 4, 512, device="cuda", dtype=torch.float16)
+    q, kv = torch.randn(2, 1, 2, 3, 64, device="cuda", dtype=torch.float16), torch.randn(2, 1, 2, 70, 64, device="cuda", dtype=torch.float16)
+    linear = lambda t: ops.int4_linear(t, qw.packed, qw.scales)
+    attend = lambda t: ops.flash_attn(t, kv[0], kv[0])
+    one_by_one = torch.stack([ops.flash_attn(q[i], kv[i], kv[i]) for i in range(2)])
+    calls = [(lambda: torch.func.vmap(linear)(x), linear(x)), (lambda: torch.func.jvp(linear, (x[0],), (x[1],))[0], linear(x[0])),
+             (lambda: torch.func.grad(lambda t: linear(t).float().sum())(x[0]), torch.zeros_like(x[0])),
+             (lambda: torch.func.vmap(ops.flash_attn)(q, kv, kv), one_by_one), (lambda: torch.func.vmap(ops.flash_attn_kv_view)(q, kv, kv), one_by_one),
+             (lambda: torch.func.jvp(attend, (q[0],), (q[1],))[0], attend(q[0])),
+             (lambda: torch.func.vmap(lambda w: kq.quantize_weight(w).packed)(x), torch.stack([kq.quantize_weight(w).packed for w in x]))]
+    raised = 0
+    for call, want in calls:
+        try:
+            got = call()
+        except (RuntimeError, ValueError):
+            raised += 1
+        else:
+            assert torch.equal(got, want)
+    assert raised >= 3
+    assert torch.isfinite(linear(x)).all()
