@@ -13,6 +13,7 @@
 
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/GradMode.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -32,6 +33,9 @@ inline const at::Tensor* plain(PyObject* o) {
   constexpr c10::DispatchKeySet wrappers({c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper});
   return t.is_cuda() && t.layout() == at::kStrided && !t.key_set().has_any(wrappers) ? &t : nullptr;
 }
+
+// Whether a tensor is being differentiated, in either mode.
+inline bool differentiated(const at::Tensor& t) { return (t.requires_grad() && c10::GradMode::is_enabled()) || t._fw_grad(0).defined(); }
 
 inline bool int_arg(PyObject* o, long long* out) {
   *out = PyLong_AsLongLong(o);
@@ -113,7 +117,8 @@ PyObject* int4_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const bool silu = PyUnicode_Check(a[4]);
     if (a[4] != Py_None && !silu) {
       bias = plain(a[4]);
-      if (!bias || bias->scalar_type() != type || bias->dim() != 1 || !bias->is_contiguous() || bias->device() != x->device()) NOT_PLAIN;
+      if (!bias || differentiated(*bias)) NOT_PLAIN;   // (`y + bias` in Python then)
+      if (bias->scalar_type() != type || bias->dim() != 1 || !bias->is_contiguous() || bias->device() != x->device()) NOT_PLAIN;
     }
     if (x->dim() < 1 || packed->dim() != 2 || scales->dim() != 2 || !x->is_contiguous() || !packed->is_contiguous() || !scales->is_contiguous()) NOT_PLAIN;
     if (packed->device() != x->device() || scales->device() != x->device()) NOT_PLAIN;
@@ -140,6 +145,15 @@ PyObject* int4_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
                                 (int)rows, (int)k, (int)group, code, wsp, ws_bytes, stream);
     }
     return rc ? raise_status(rc) : THPVariable_Wrap(std::move(y));
+  });
+}
+
+// plain_constant(t) -> whether t may go into a kernel as a bias: a plain CUDA tensor outside autograd and torch.func
+PyObject* plain_constant(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  ARGS(1)
+  return guarded([&]() -> PyObject* {
+    const at::Tensor* t = plain(a[0]);
+    return PyBool_FromLong(t && !differentiated(*t));
   });
 }
 
@@ -376,6 +390,7 @@ PyObject* silu_mul(PyObject*, PyObject* const* a, Py_ssize_t n) {
 #define METHOD(name, doc) {#name, (PyCFunction)(void*)name, METH_FASTCALL, doc}
 PyMethodDef methods[] = {
     METHOD(int4_linear, "int4_linear(x, packed, scales, group_size, bias) -> y, or None when the call is not a plain one"),
+    METHOD(plain_constant, "plain_constant(t) -> whether t may go into a kernel as a bias"),
     METHOD(flash_attn, "flash_attn(q, k, v, causal, scale, views) -> o, or None when the call is not a plain one"),
     METHOD(flash_attn_decode, "flash_attn_decode(q, k_cache, v_cache, kv_len, scale) -> o, or None when the call is not a plain one"),
     METHOD(quantize_pack, "quantize_pack(weight, group_size) -> (packed, scales), or None when the call is not a plain one"),

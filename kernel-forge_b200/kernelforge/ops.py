@@ -375,12 +375,13 @@ def _linear_launch(x, packed, scales, group_size, bias):
     """The native dispatcher, or the private prepacked copy of the weight where there is one; None for a call that is not
     a plain one (the caller validates then)."""
     if _PREPACKED and isinstance(x, torch.Tensor) and x.dtype == torch.float16 and x.is_contiguous() and x.dim() >= 1 and x.shape[-1] and (
-            bias is None or (bias.dtype == torch.float16 and bias.is_contiguous() and bias.shape == packed.shape[:1])):
+            bias is None or (_capi.host().plain_constant(bias) and bias.dtype == torch.float16 and bias.is_contiguous()
+                             and bias.shape == packed.shape[:1])):
         m = x.numel() // x.shape[-1]
         if 1 <= m <= PREPACKED_GEMV_MAX_M:
             private = _prepacked_for(packed)          # set by prepack_weight_(packed)
             if private is not None and _prepacked_wins(m, packed.shape[0], x.shape[-1]):
-                x2 = x.reshape(-1, x.shape[-1])
+                x2 = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
                 _check_int4(x2, packed, scales, group_size)
                 _check_int4_storage(x2, packed, scales, group_size)
                 return int4_gemv_prepacked(x2, private, scales, group_size, bias).reshape(*x.shape[:-1], packed.shape[0])
@@ -571,7 +572,7 @@ def int4_linear(x: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, gro
         if y is not None:
             return y
     lead = x.shape[:-1]
-    x2 = x.reshape(-1, x.shape[-1])
+    x2 = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])   # (under torch.func a reshape would wrap it)
     if not x2.is_contiguous():
         x2 = x2.contiguous()
     _check_int4(x2, packed, scales, group_size, allow_bf16=True)

@@ -65,3 +65,30 @@ def test_wrappers_of_torch_func_are_never_read_as_memory():
             assert torch.equal(got, want)
     assert raised >= 3
     assert torch.isfinite(linear(x)).all()
+
+
+@pytest.mark.parametrize("prepacked", [False, True])
+@pytest.mark.parametrize("m", [1, 4, 40])
+def test_a_bias_that_is_trained_batched_or_dual_is_added_by_torch(m, prepacked):
+    """The product has no backward, its bias is an ordinary addend: gradients, vmap and forward mode over it work."""
+    n, k = 256, 512
+    qw = weight(n, k)
+    if prepacked:
+        ops.prepack_weight_(qw.packed)
+    x = torch.randn(m, k, device="cuda", dtype=torch.float16)
+    y = ops.int4_linear(x, qw.packed, qw.scales)
+    bias = torch.randn(n, device="cuda", dtype=torch.float16)
+    linear = lambda b: ops.int4_linear(x, qw.packed, qw.scales, 128, b)
+    assert torch.equal(linear(bias), y + bias)
+    trained = torch.nn.Parameter(bias.clone())
+    out = linear(trained)
+    out.backward(torch.ones_like(out))
+    assert torch.equal(out, y + bias) and torch.equal(trained.grad, torch.full_like(bias, m))
+    with torch.no_grad():
+        assert not linear(trained).requires_grad
+    several = torch.randn(3, n, device="cuda", dtype=torch.float16)
+    assert torch.equal(torch.func.vmap(linear)(several), y + several[:, None])
+    if prepacked:
+        return   # (its entry allocates in Python: a transform of torch.func that wraps every new tensor is refused)
+    value, tangent = torch.func.jvp(linear, (bias,), (several[0],))
+    assert torch.equal(value, y + bias) and torch.equal(tangent, several[0].expand(m, n))
