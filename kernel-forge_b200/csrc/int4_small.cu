@@ -95,7 +95,7 @@ __device__ __forceinline__ void store_rows(float a0, float a1, const gemv::Fusio
       case gemv::kEpiSiluPair: gemv::store_pair<gemv::kEpiSiluPair>(a0, a1, fu, out, m, n, N); break;
       case gemv::kEpiRopeKv: gemv::store_pair<gemv::kEpiRopeKv>(a0, a1, fu, out, m, n, N); break;
       default:
-        if ((N & 1) == 0) {   // one 4-byte store (n + 1 < N then)
+        if ((N & 1) == 0 && (reinterpret_cast<uintptr_t>(y) & 3u) == 0) {   // one 4-byte store (n + 1 < N then)
           *reinterpret_cast<__half2*>(out + (size_t)m * N + n) =
               __halves2half2(gemv::finish(a0, fu, m, n, N), gemv::finish(a1, fu, m, n + 1, N));
         } else {

@@ -69,3 +69,17 @@ def test_silu_pairs_epilogue(m, n, k):
     want = torch.nn.functional.silu(gate) * up
     assert got.shape == want.shape
     assert (got.float() - want.float()).abs().max() <= 3e-3 * want.float().abs().max()
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 512, 1024), (2, 512, 1024), (8, 512, 1024), (32, 1536, 1024)])
+def test_result_buffer_of_two_byte_alignment(m, n, k):
+    """A caller of the C ABI may hand over any element of an fp16 buffer: the 4-byte stores look at the address first."""
+    from kernelforge import _capi
+    _, x, packed, scales, ref = int4_case(m, n, k, 128, seed=m)
+    x, packed, scales = (torch.from_numpy(t).cuda() for t in (x, packed, scales))
+    buf = torch.full((m * n + 2,), 7.0, dtype=torch.float16, device="cuda")
+    _capi.check(_capi.lib().kfb_int4_linear(x.data_ptr(), packed.data_ptr(), scales.data_ptr(), None, buf.data_ptr() + 2, m, n, k, 128, 0, None, 0,
+                                            _capi.stream_ptr(x.device)))
+    assert_int4_close(buf[1:-1].view(m, n), ref)
+    assert buf[0] == 7.0 and buf[-1] == 7.0
+    assert torch.equal(buf[1:-1].view(m, n), ops.int4_linear(x, packed, scales, 128))
