@@ -374,18 +374,27 @@ int4_gemv_kernel(const __half* __restrict__ x, const uint4* __restrict__ packed,
   }
 }
 
+// Shared memory that a CTA asks for so that no SM takes more than its share of the grid.  A grid of a few CTAs per SM, all of
+// which would fit on a part of the chip, is not spread evenly by the hardware: 5632 x 2048, M = 1, 352 CTAs 4.3 us, kept to three
+// per SM 3.6; 2048 x 5632, 512 CTAs 6.1 and 5.3; 7000 x 3072, 438 CTAs 6.1 and 5.2; one more per SM than its share: no gain.
+size_t spread(int grid) {
+  const int share = ceil_div(grid, sm_count());
+  return share < 2048 / kThreads ? (size_t)(228 * 1024 / (share + 1)) : 0;   // share + 1 of them do not fit
+}
+
 template <int M, int R, int G, int XF = kXformNone, int EPI = kEpiNone>
 int launch(const void* x, const void* packed, const void* scales, void* y, int N, int K, int ksplit_log2, int flags,
            cudaStream_t stream, const Fusion& fu = Fusion{}) {
   const int tiles = ceil_div(N, R);
   const int grid = ceil_div(tiles, kWarps >> ksplit_log2);
-  const size_t smem = XF != kXformNone ? (size_t)M * K * sizeof(__half) : 0;
+  const size_t smem = XF != kXformNone ? (size_t)M * K * sizeof(__half) : spread(grid);
   if (smem > 48 * 1024) {
     static bool configured[64] = {false};
     int dev = 0;
     KFB_CUDA_TRY(cudaGetDevice(&dev));
     if (dev >= 0 && dev < 64 && !configured[dev]) {
-      KFB_CUDA_TRY(cudaFuncSetAttribute(int4_gemv_kernel<M, R, G, XF, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
+      KFB_CUDA_TRY(cudaFuncSetAttribute(int4_gemv_kernel<M, R, G, XF, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (XF != kXformNone ? 64 : 114) * 1024));
       configured[dev] = true;
     }
   }
