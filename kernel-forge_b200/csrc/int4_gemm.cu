@@ -37,6 +37,7 @@ constexpr int kBlockK = 128;     // k per pipeline stage: two 64-wide (128-byte)
 constexpr int kMaxTile = 256;    // most batch rows of a tile (MMA N)
 constexpr int kStages = 4;       // K blocks of dequantised weights in TMEM
 constexpr int kMaxXStages = 16;  // K blocks of activations in shared memory: as many as fit (4 at 256 batch rows per tile)
+constexpr int kMaxSplits = 16;   // of K
 constexpr int kWordStages = 4;   // copies of packed words in flight, two K blocks each
 constexpr int kDequantGroups = 2;  // warpgroups; they take the K blocks in turn
 constexpr int kDequantWarps = 4 * kDequantGroups, kEpilogueWarps = 8;
@@ -539,8 +540,12 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
 }
 
 // y[m, col0 + n] = 16-bit(sum over splits, in split order, of partial[s][m][n]) (+ bias), in every output buffer.  V: columns
-// per thread (4 where rows allow 16-byte loads).
-template <int V>
+// per thread (4 where rows allow 16-byte loads).  S: all pieces of an element are requested before the first one is added (in
+// split order): a kernel of few elements is bound by the round trips to L2.  With 5 to 16 pieces, four at a time and the rest one
+// by one before: 512 x 12288, M = 48 11.3 us the whole call, now 9.7; 1536 x 8960, M = 33 12.1 and 10.5.  S = 0, up to four
+// pieces or one column per thread: a plain loop; with registers for 16 pieces 2048 x 5632, M = 512 takes 23.5 instead of 20.9,
+// 1001 x 2048, M = 33 8.3 instead of 7.8.
+template <int V, int S>
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restrict__ partial, const __grid_constant__ OutSpec out,
                                                             int M, int N, int splits) {
   pdl_wait(partial);
@@ -551,31 +556,47 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restr
 #pragma unroll
     for (int e = 0; e < V; ++e) acc[e] = 0.f;
     const float* p = partial + i * V;
+    if constexpr (S > 0) {
+      alignas(16) float v[S][V];
+#pragma unroll
+      for (int s = 0; s < S; ++s)
+        if (s < splits) {
+          if constexpr (V == 4) *reinterpret_cast<float4*>(v[s]) = *reinterpret_cast<const float4*>(p + (size_t)s * elems);
+          else v[s][0] = p[(size_t)s * elems];
+        }
+#pragma unroll
+      for (int s = 0; s < S; ++s)
+        if (s < splits) {
+#pragma unroll
+          for (int e = 0; e < V; ++e) acc[e] += v[s][e];
+        }
+    } else {
 #pragma unroll 4
-    for (int s = 0; s < splits; ++s) {
-      if constexpr (V == 4) {
-        const float4 v = *reinterpret_cast<const float4*>(p + (size_t)s * elems);
-        acc[0] += v.x; acc[1] += v.y; acc[2] += v.z; acc[3] += v.w;
-      } else {
-        acc[0] += p[(size_t)s * elems];
+      for (int s = 0; s < splits; ++s) {
+        if constexpr (V == 4) {
+          const float4 v = *reinterpret_cast<const float4*>(p + (size_t)s * elems);
+          acc[0] += v.x; acc[1] += v.y; acc[2] += v.z; acc[3] += v.w;
+        } else {
+          acc[0] += p[(size_t)s * elems];
+        }
       }
     }
     const long long m = i * V / N;
     const int n = (int)(i * V - m * N);
-    uint16_t v[V];
+    uint16_t r[V];
 #pragma unroll
-    for (int e = 0; e < V; ++e) v[e] = out.bias ? round16_bias(acc[e], out.bias[n + e], out.bf16 != 0) : round16(acc[e], out.bf16 != 0);
+    for (int e = 0; e < V; ++e) r[e] = out.bias ? round16_bias(acc[e], out.bias[n + e], out.bf16 != 0) : round16(acc[e], out.bf16 != 0);
     if constexpr (V == 4) {
       if (out.silu) {
         *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(out.y[0]) + m * out.ld + n / 2) =
-            silu_pair(v[0] | ((uint32_t)v[1] << 16)) | ((uint32_t)silu_pair(v[2] | ((uint32_t)v[3] << 16)) << 16);
+            silu_pair(r[0] | ((uint32_t)r[1] << 16)) | ((uint32_t)silu_pair(r[2] | ((uint32_t)r[3] << 16)) << 16);
         continue;
       }
     }
     for (int o = 0; o < out.count; ++o) {
       uint16_t* dst = reinterpret_cast<uint16_t*>(out.y[o]) + m * out.ld + out.col0 + n;
-      if constexpr (V == 4) *reinterpret_cast<uint2*>(dst) = make_uint2(v[0] | ((uint32_t)v[1] << 16), v[2] | ((uint32_t)v[3] << 16));
-      else dst[0] = v[0];
+      if constexpr (V == 4) *reinterpret_cast<uint2*>(dst) = make_uint2(r[0] | ((uint32_t)r[1] << 16), r[2] | ((uint32_t)r[3] << 16));
+      else dst[0] = r[0];
     }
   }
 }
@@ -591,7 +612,7 @@ Shape make_plan(int M, int N, int K, int group, bool bf16) {
   for (int mt = 32; mt <= kMaxTile; mt += 32) {
     const int m_tiles = ceil_div(M, mt);
     if (mt > 32 && m_tiles == ceil_div(M, mt - 32)) continue;   // the same tiles, more padding
-    for (int sp = 1; sp <= 16; ++sp) {
+    for (int sp = 1; sp <= kMaxSplits; ++sp) {
       const int per = ceil_div(ceil_div(kblocks, sp), 2) * 2;
       const int splits = ceil_div(kblocks, per);
       if (splits != sp) continue;
@@ -632,8 +653,8 @@ int launch(const Shape& p, const CUtensorMap& tw, const CUtensorMap& tx, const v
     long long blocks = (work + 255) / 256;
     const long long cap = (long long)sm_count() * 8;
     if (blocks > cap) blocks = cap;
-    return launch_kernel("splitk_reduce_kernel", vec ? splitk_reduce_kernel<4> : splitk_reduce_kernel<1>, dim3((unsigned)blocks), dim3(256), 0, stream,
-                         (const float*)partial, out, p.M, p.N, p.splits);
+    auto reduce = !vec ? splitk_reduce_kernel<1, 0> : p.splits <= 4 ? splitk_reduce_kernel<4, 0> : splitk_reduce_kernel<4, kMaxSplits>;
+    return launch_kernel("splitk_reduce_kernel", reduce, dim3((unsigned)blocks), dim3(256), 0, stream, (const float*)partial, out, p.M, p.N, p.splits);
   }
   return KFB_OK;
 }
