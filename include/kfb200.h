@@ -106,6 +106,8 @@ int kfb_dequantize(const void* packed, const void* scales, int N, int K, int gro
  * shape.  x, bias and y are of `dtype` (KFB_F16 or KFB_BF16); bias [N] or NULL is added to the rounded product and the
  * sum rounded again, like `y + bias`.  Workspace: kfb_int4_linear_ws_bytes bytes, 16-byte aligned (0: none needed). */
 size_t kfb_int4_linear_ws_bytes(int M, int N, int K, int group, int dtype);
+/* Which kernel that is: 0 CUDA-core GEMV, 1 persistent streaming kernel, 2 small-batch kernel, 3 tcgen05 GEMM. */
+int kfb_int4_linear_route(int M, int N, int K, int dtype, int with_bias);
 int kfb_int4_linear(const void* x, const void* packed, const void* scales, const void* bias, void* y,
                     int M, int N, int K, int group, int dtype, void* ws, size_t ws_bytes, void* stream);
 

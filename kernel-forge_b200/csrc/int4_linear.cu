@@ -3,7 +3,7 @@
 // The reference's dispatcher (kernelforge/ops.py:193-214) knows a GEMV up to M = 7 and a GEMM above; here:
 //   M = 1                 CUDA-core GEMV (int4_gemv.cu): one row of activations, nothing for an MMA to share
 //   fp16, N >= 75776      persistent streaming kernel (int4_gemv_mma.cuh) up to M = 16, where it has no bias to add
-//   M <= 32               small-batch kernel (int4_small.cu)
+//   M <= 32               small-batch kernel (int4_small.cu), but for few rows of a long K above M = 16
 //   otherwise             tcgen05 GEMM (int4_gemm.cu)
 #include "int4_gemm.cuh"
 #include "int4_small.cuh"
@@ -17,17 +17,26 @@ enum class Route { kGemv, kStream, kSmall, kGemm };
 // Where the lines lie (graph of L2-cold calls, us):
 //   M = 1: GEMV / small-batch kernel 5632x2048 4.1/4.7, 1536x8960 5.2/6.2, 2560x2048 3.7/3.7, but 8960x1536 5.0/4.8,
 //     11264x2048 8.0/7.3: the GEMV's four or eight rows per warp leave it too few warps there.
-//   M = 32: small-batch kernel / GEMM 2048x5632 8.7/12.3, 1536x8960 11.5/13.5, 8960x1536 10.7/11.6, 5632x2048 11.7/11.4,
-//     11264x2048 17.4/13.2; the kernel's activation reads grow with M * N, the GEMM's time hardly with M.
+//   16 < M <= 32: small-batch kernel / GEMM, M = 32, 2048x5632 8.1/9.5, 2048x8192 10.4/11.3, 1024x4096 6.0/7.9, 5632x2048
+//     11.7/11.4, 11264x2048 17.4/13.2; its activation reads grow with M * N, the GEMM's time hardly with M.  Few rows and a long
+//     K leave a warp too many groups one after the other, while the GEMM splits K over the chip: M = 17 / 24 / 32, 512x8192 8.2/8.4,
+//     8.7/8.6, 9.7/8.7, 1536x8960 9.8/9.5, 10.0/9.8, 11.0/10.3, 512x12288 10.8/9.2, 11.5/9.4, 12.8/9.5; bf16, whose unpacking
+//     costs more: 512x6144 7.6/8.4, 7.8/8.6, 8.5/8.7, 512x8192 9.4/8.9, 9.9/9.0, 10.6/9.1, 2048x8192 9.9/11.7, 10.1/11.8, 11.0/12.3.
 Route route(int M, int N, int K, int dtype, bool bias) {
   const bool fp16 = dtype == KFB_F16;
   if (fp16 && N >= 75776 && !bias && M <= 16) return M <= 8 ? Route::kGemv : Route::kStream;
   if (fp16 && M == 1 && N < 8192) return Route::kGemv;
-  if (M <= 16 || (M <= 32 && (long long)N * K <= 16LL << 20)) return Route::kSmall;
-  return Route::kGemm;
+  if (M > 32 || (M > 16 && (long long)N * K > 16LL << 20)) return Route::kGemm;
+  if (M > 16 && N <= 1536 && K >= 8192 && (!fp16 || (long long)K * (M + 8) > 8192 * 32)) return Route::kGemm;
+  return Route::kSmall;
 }
 
 }  // namespace
+
+extern "C" int kfb_int4_linear_route(int M, int N, int K, int dtype, int with_bias) {
+  if (M < 1 || N < 1 || K < 1 || (dtype != KFB_F16 && dtype != KFB_BF16)) return fail(KFB_ERR_INVALID, "no such linear: M=%d N=%d K=%d", M, N, K);
+  return (int)route(M, N, K, dtype, with_bias != 0);
+}
 
 extern "C" size_t kfb_int4_linear_ws_bytes(int M, int N, int K, int group, int dtype) {
   return M <= 16 ? 0 : route(M, N, K, dtype, false) == Route::kGemm ? gemm::ws_bytes(M, N, K, group, dtype == KFB_BF16) : 0;

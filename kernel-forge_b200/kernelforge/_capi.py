@@ -45,6 +45,7 @@ _SIGNATURES = {
     "kfb_pack_int4": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p]),
     "kfb_dequantize": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_void_p]),
     "kfb_int4_linear_ws_bytes": (c_size_t, [c_int, c_int, c_int, c_int, c_int]),
+    "kfb_int4_linear_route": (c_int, [c_int, c_int, c_int, c_int, c_int]),
     "kfb_int4_linear": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p,
                                 c_size_t, c_void_p]),
     "kfb_int4_linear_silu_pairs": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]),

@@ -322,17 +322,6 @@ SMALL_BATCH_MAX_M = 32
 GEMV_MAX_M = 8
 
 
-def _small_batch_wins(m: int, n: int, k: int) -> bool:
-    """For callers that choose between the entry points int4_small_batch and int4_gemm themselves (int4_matmul has a
-    kernel of its own there): where int4_small_batch measured faster for 8 < M <= 16 (same method as above, us):
-    M = 12: 5632x2048 10.1/12.3, 2048x2048 5.9/8.3, 8960x1536 9.1/13.1, 11264x2048 16.6/18.0, 128256x4096 128/153, but
-    1536x8960 16.1/12.3, 2048x5632 12.1/11.4 and 32000x2048 26.8/24.4;  M = 16: 5632x2048 11.3/12.6, 2048x2048 6.5/8.3,
-    8960x1536 9.6/13.3, 11264x2048 18.3/18.0, 128256x4096 133/153.  From M = 24 on the GEMM wins everywhere."""
-    if n >= 75776:                       # the persistent streaming kernel
-        return m <= 16
-    return m <= 16 and k <= 2048 and n <= 16384
-
-
 def int4_gemm(x: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, group_size: int = 128) -> torch.Tensor:
     """Fused INT4 dequant GEMM on the tcgen05 tensor cores, any M, N a multiple of 64."""
     _check_int4(x, packed, scales, group_size)
@@ -353,8 +342,10 @@ def int4_gemm_ragged(x: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor
 def int4_matmul(x: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, group_size: int = 128) -> torch.Tensor:
     """y = x @ W_hat^T for INT4 weights from kernelforge.quantize, choosing the kernel by M (kfb_int4_linear).
 
-    M = 1: the CUDA-core GEMV; M <= 32: the small-batch kernel (FP32 accumulation in both).  Larger M: the tcgen05 GEMM.
-    bf16 activations (not in the reference, README.md:103) take the same route.  A weight with a private prepacked copy
+    The lines are in csrc/int4_linear.cu: the CUDA-core GEMV for one fp16 row and fewer than 8192 features, the small-batch
+    kernel up to M = 16 and, where features x K and K allow, 32, streaming kernels for very many features, the tcgen05 GEMM
+    otherwise.  FP32 accumulation in all of them.  bf16 activations (not in the reference, README.md:103) never take the
+    GEMV.  A weight with a private prepacked copy
     (prepack_weight_) runs batches of up to PREPACKED_GEMV_MAX_M rows on it.
     """
     y = _linear_launch(x, packed, scales, group_size, None) if isinstance(x, torch.Tensor) and x.dim() == 2 else None

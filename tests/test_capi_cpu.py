@@ -130,8 +130,8 @@ def test_prefill_workspace_covers_the_plan_with_and_without_the_causal_mask():
             assert plan(shape, causal, 0)[1] == 1
             split += best[1] > 1
     assert split > 100
-    # 1557 queries of 8 heads: with splits two tiles per CTA are best, without them one
-    assert plan(shapes[1], 1, 1 << 60)[0] == 2 and plan(shapes[1], 1, 0) == (1, 1)
+    # 3907 queries of one head: with splits two tiles per CTA are best, without them one
+    assert plan(shapes[0], 1, 1 << 60)[0] == 2 and plan(shapes[0], 1, 0) == (1, 1)
 
 
 def test_every_decode_plan_fits_the_array_of_the_allocation_free_entry():
@@ -162,15 +162,21 @@ def test_no_kernel_asks_for_non_coherent_loads():
 
 
 def test_int4_matmul_routing_table():
-    """Which kernel int4_matmul picks by shape (pure host logic): GEMV up to M = 8, the same kernel with more batch columns
-    for 8 < M <= 16 where it measured faster, the tcgen05 GEMM otherwise."""
-    from kernelforge import ops
-    assert ops.GEMV_MAX_M == 8 and ops.SMALL_BATCH_MAX_M == 32
-    wins = ops._small_batch_wins
-    assert wins(12, 5632, 2048) and wins(16, 2048, 2048) and wins(16, 8960, 1536)
-    assert wins(16, 128256, 4096)                      # large N: the persistent streaming kernel
-    assert not wins(12, 1536, 8960)                    # long K, few rows: the GEMM was faster
-    assert not wins(12, 32000, 2048)                   # between the two regimes
+    """Which kernel int4_linear / int4_matmul takes by shape (pure host logic, kfb_int4_linear_route), on both sides of each line."""
+    gemv, stream, small, gemm = range(4)
+    route = _capi.lib().kfb_int4_linear_route
+    fp16, bf16 = (_capi.dtype_code(t) for t in (torch.float16, torch.bfloat16))
+    for m, n, k, want in ((1, 8191, 2048, gemv), (1, 8192, 2048, small), (1, 75776, 2048, gemv), (8, 75776, 2048, gemv), (9, 75776, 2048, stream),
+                          (16, 75776, 2048, stream), (17, 75776, 2048, gemm), (2, 5632, 2048, small), (16, 11264, 2048, small), (17, 11264, 2048, gemm),
+                          (32, 2048, 8192, small), (32, 2049, 8192, gemm), (33, 256, 1024, gemm), (24, 1536, 8192, small), (25, 1536, 8192, gemm),
+                          (25, 1537, 8192, small), (16, 1536, 12288, small), (17, 1024, 12288, gemm), (32, 1536, 8128, small)):
+        assert route(m, n, k, fp16, 0) == want, (m, n, k)
+    for m, n, k, want in ((1, 100, 2048, small), (1, 80000, 2048, small), (16, 80000, 1024, small), (17, 1536, 8192, gemm), (17, 1536, 8128, small),
+                          (17, 1537, 8192, small), (33, 64, 64, gemm)):
+        assert route(m, n, k, bf16, 0) == want, (m, n, k)
+    assert route(8, 75776, 2048, fp16, 1) == small      # the streaming kernels have no bias to add
+    assert route(0, 64, 64, fp16, 0) < 0
+    assert ops.GEMV_MAX_M == 8 and ops.SMALL_BATCH_MAX_M == 32 and ops.PREPACKED_GEMV_MAX_M == 32
 
 
 def test_decoder_refuses_steps_that_do_not_fit_the_cache():
