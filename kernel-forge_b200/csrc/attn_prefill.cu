@@ -139,6 +139,7 @@ struct TileLayout {
   static constexpr int kMisc = kBars + kNumBars * 8;
   static constexpr int kBytes = kMisc + 16;
   static constexpr int kAlloc = kBytes + 1024;        // room to align the tiles to 1024 bytes
+  static constexpr int kAllocAlone = 116 * 1024;      // more than half of what an SM has
   static_assert((NT == 1 ? 2 : 1) * kAlloc <= 227 * 1024, "two one-tile CTAs, or a two-tile CTA, must fit on an SM");
   static_assert(NT == 1 || 2 * kAlloc > 228 * 1024, "one two-tile CTA per SM: it allocates all 512 TMEM columns");
   static constexpr uint32_t kColS = 0;                              // + 128 X
@@ -633,6 +634,7 @@ __global__ void __launch_bounds__(256) attn_prefill_merge_kernel(const float* __
 // How a problem is cut (see the header of the kernel); max_splits = 1 where there is no workspace for the pieces.
 struct PrefillPlan {
   int heads_per_tile, tiles, units, per_cta, splits;
+  bool alone;   // a one-tile CTA that has its SM to itself
 };
 
 PrefillPlan plan_prefill(const Problem& p, int max_splits = 32) {
@@ -648,33 +650,54 @@ PrefillPlan plan_prefill(const Problem& p, int max_splits = 32) {
     c.tiles = G / c.heads_per_tile;
     c.units = p.B * p.Hk;
   }
-  // Tiles per CTA and key splits, by a cost model in us fitted to measurements on B200: a key step takes a two-tile CTA
-  // 2.05 (head dim 64: 1.44), a one-tile CTA 1.7 (1.1) alone on its SM and 2.085 (1.65) beside another one; set-up and drain
-  // 5.3 and 4.6; the merge kernel 2.5 and its traffic at ~4 TB/s.  So a grid smaller than the GPU takes one tile per CTA
-  // (1 x 16 x 1093 queries D = 128: 20.1 us against 23.6) and splits the keys; long ones share K / V between two tiles
-  // (2 x 16 x 8192 D = 128 causal: 514 against 542).
-  const int steps = ceil_div(p.Nk, kBlockN);
+  // Tiles per CTA, CTAs per SM and key splits, by a cost model in us fitted to 1194 shapes, 3650 measured plans in graphs on
+  // B200 (mean deviation 5 %): a CTA takes `step` per 128 keys and `fixed` for set-up and drain; the merge kernel 2.7, 0.2 per
+  // split and its traffic at 5.1 TB/s.  So a grid smaller than the GPU takes one tile per CTA and splits the keys (1 x 8 x 1024
+  // queries, D = 128: 17.4 us, two tiles 18.7), long ones share K / V between two tiles (2 x 16 x 8192 D = 128 causal: 514
+  // against 542).
+  // One-tile CTAs fit in pairs on an SM, and the hardware does pair them while other SMs stay idle.  Where the grid has at
+  // most one for each SM, and under a causal mask also for longer grids, where short CTAs even out what is left over, they are
+  // kept apart (by the shared memory they ask for): 1 x 8 x 1024, two splits 21.2 -> 17.0; 1 x 16 x 2048 causal 39.2 -> 35.2.
+  // CTAs of one or two steps gain nothing from it (1 x 2 queries, 4002 keys, 32 splits: 13.8 us apart, 11.6 in pairs).
+  struct Kind {
+    int per_cta;
+    bool alone;
+    double step, fixed, wave, tail;   // wave: `fixed` where CTAs follow one another on an SM; tail: share of the longest CTA that
+  };                                  // a causal grid of more CTAs than slots ends with
   const bool wide = p.D == 128;
-  const double merge_mb = (double)p.B * p.H * p.Nq * p.D * 8.0 / 4.0e6;
+  const Kind kinds[3] = {{1, false, wide ? 2.15 : 1.72, wide ? 5.7 : 5.25, wide ? 5.25 : 3.75, 0.30},
+                         {1, true, wide ? 1.71 : 1.30, wide ? 4.1 : 3.6, wide ? 5.6 : 3.4, wide ? 0.09 : 0.18},
+                         {2, false, wide ? 2.00 : 1.51, wide ? 5.6 : 4.8, wide ? 5.75 : 4.6, 0.27}};
+  const int steps = ceil_div(p.Nk, kBlockN), hidden = ceil_div(p.Nk - p.Nq, kBlockN);   // hidden: steps that every causal tile has
+  const bool uneven = p.causal && !c.heads_per_tile && p.Nq > p.Nk / 2;   // CTAs of all lengths, longest first
+  const double merge_us = (double)p.B * p.H * p.Nq * p.D * 8.0 / 5.1e6 + 0.2;
   double best = 1e30;
   c.per_cta = 1;
   c.splits = 1;
-  for (int per_cta = 1; per_cta <= 2; ++per_cta)
+  c.alone = false;
+  for (const Kind& k : kinds)
     for (int s = 1; s <= steps && s <= max_splits; ++s) {
-      const int per = ceil_div(steps, s);
-      if (ceil_div(steps, per) != s) continue;   // an empty split
-      const long long ctas = (long long)c.units * ceil_div(c.tiles, per_cta) * s;
+      const int longest = ceil_div(steps, s);
+      if (ceil_div(steps, longest) != s) continue;   // an empty split
+      const int per_unit = ceil_div(c.tiles, k.per_cta);
+      const long long ctas = (long long)c.units * per_unit * s;
       if (s > 1 && ctas > 2 * sms) break;
-      // Waves of CTAs; a causal grid has CTAs of all lengths, longest first, and fills its last wave.
-      const long long slots = per_cta == 2 ? sms : 2 * sms;
-      const double waves = p.causal && p.Nq > p.Nk / 2 ? (double)ctas / slots : (double)((ctas + slots - 1) / slots);
-      const double len = p.causal && ctas > slots ? per * (1.0 - 0.5 * p.Nq / p.Nk) + 0.5 : per;
-      double cost = 0.0;
-      if (per_cta == 2) cost = (ctas <= sms ? 1.0 : waves) * (len * (wide ? 2.05 : 1.44) + 5.3);
-      else if (ctas <= sms) cost = per * (wide ? 1.7 : 1.1) + 4.6;
-      else cost = (ctas <= slots ? 1.0 : waves) * (len * (wide ? 2.085 : 1.65) + 4.6);
-      if (s > 1) cost += 2.5 + s * merge_mb;
-      if (cost < best) { best = cost; c.per_cta = per_cta; c.splits = s; }
+      if (k.per_cta == 1 && !k.alone && ctas <= sms) continue;
+      if (k.alone && ctas > sms && (s > 1 || longest < 8)) continue;
+      const long long slots = k.per_cta == 2 || k.alone ? sms : 2 * sms;
+      const double one = longest * k.step + k.fixed;
+      double cost = one;
+      if (ctas > slots && uneven && per_unit > 1) {
+        const double total = (double)c.units * (k.per_cta * (per_unit - 1.0) * per_unit / 2 + (per_unit - 1.0) * hidden + steps);
+        const double shared = (total * k.step + ctas * k.wave) / slots + k.tail * longest * k.step;
+        cost = one > shared ? one : shared;
+      } else if (ctas > slots) {   // (the last wave of pairs: CTAs on their own where there is an SM for each)
+        const long long last = ctas % slots;
+        const Kind& left = slots > sms && last <= sms ? kinds[1] : k;
+        cost = (double)(ctas / slots) * (longest * k.step + k.wave) + (last ? longest * left.step + left.wave : 0.0);
+      }
+      if (s > 1) cost += 2.7 + s * merge_us;
+      if (cost < best) { best = cost; c.per_cta = k.per_cta; c.splits = s; c.alone = k.alone && longest >= 3; }
     }
   return c;
 }
@@ -688,7 +711,7 @@ int launch_tiles(const Problem& p, const PrefillPlan& plan, const CUtensorMap& t
   int dev = 0;
   KFB_CUDA_TRY(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    KFB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kAlloc));
+    KFB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, NT == 1 ? L::kAllocAlone : L::kAlloc));
     configured[dev] = true;
   }
   const Strides o_st{p.o_stride_b, p.o_stride_h, p.o_stride_n};
@@ -699,7 +722,7 @@ int launch_tiles(const Problem& p, const PrefillPlan& plan, const CUtensorMap& t
   if (ctas > 0x7fffffffLL) return fail(KFB_ERR_INVALID, "too many query tiles for one launch");
   tiles::Params pr = {p.B, p.H, p.Hk, p.Nq, p.Nk, p.causal, p.scale * 1.4426950408889634f, plan.heads_per_tile, plan.tiles, units_per_group,
                      plan.splits, partial};
-  if (int rc = launch_kernel("attn_prefill_kernel", kernel, dim3((unsigned)ctas, plan.splits), dim3(L::kThreads), L::kAlloc, stream, tq, tk, tv,
+  if (int rc = launch_kernel("attn_prefill_kernel", kernel, dim3((unsigned)ctas, plan.splits), dim3(L::kThreads), plan.alone ? L::kAllocAlone : L::kAlloc, stream, tq, tk, tv,
                              p.o, o_st, pr, status))
     return rc;
   if (plan.splits == 1) return KFB_OK;
