@@ -147,6 +147,9 @@ int kfb_int4_small_batch(const void* x, const void* packed, const void* scales, 
  *   xform 2: x [M, 2 K] is gate | up; the product uses fp16(fp16(silu(gate)) * up)   (K <= 8192 for xform 1, 2);
  *   then y = fp16(sum), + bias[N] when not NULL, + residual[M, N] when not NULL (fp16 additions, in that order).
  * Larger M: KFB_ERR_UNSUPPORTED (run the separate kernels).  flags: bit 0 as kfb_int4_gemv. */
+/* 1 where xform 1 runs on the kernel that holds its weights in registers while it normalises (csrc/int4_norm.cu), 0 where the
+ * CUDA-core GEMV does it in a prologue: a caller with a norm kernel of its own may prefer that one then. */
+int kfb_int4_norm_fits(int M, int N, int K, int group);
 int kfb_int4_gemv_fused(const void* x, const void* packed, const void* scales, void* y,
                         int M, int N, int K, int group, int xform, const void* norm_weight, float eps,
                         const void* bias, const void* residual, int flags, void* stream);

@@ -537,6 +537,10 @@ int fused_common(const char* what, const void* x, const void* packed, const void
 
 }  // namespace
 
+extern "C" int kfb_int4_norm_fits(int M, int N, int K, int group) {
+  return (group == 64 || group == 128) && K >= group && K % group == 0 && normed::fits(M, N, K, group);
+}
+
 extern "C" int kfb_int4_gemv_fused(const void* x, const void* packed, const void* scales, void* y, int M, int N, int K, int group,
                                    int xform, const void* norm_weight, float eps, const void* bias, const void* residual,
                                    int flags, void* stream) {

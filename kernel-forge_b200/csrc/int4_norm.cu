@@ -257,12 +257,16 @@ int row_blocks(int N) {
 
 }  // namespace
 
-// Up to 128 k per warp (K <= 2048) every N; up to 256 k only where one block of rows per CTA is enough: with more the
-// weights do not fit in the registers.
+// Up to 128 k per warp (K <= 2048) every N that keeps the SMs busy; up to 256 k only where one block of rows per CTA is enough:
+// with more the weights do not fit in the registers.  A CTA per SM and five blocks per CTA are one wave; a second one that is
+// half empty costs more than the norm kernels and launches saved (step of 8 layers at batch 1, us, this kernel / separate norms:
+// gate_up of 11264 rows 201 / 224, 13824 238 / 229, 16384 245 / 224, 17920 237 / 226, 22016 276 / 291).
 bool fits(int M, int N, int K, int group) {
   const int ng = groups_per_warp(K / group);
   if (M < 1 || M > 2 || N < 1 || ng == 0 || ng * group > 256) return false;
   const int warps = K / (group * ng), rb = row_blocks(N);
+  const long long wave = (long long)kMaxRB * sm_count(), blocks = ceil_div(N, 16), waves = (blocks + wave - 1) / wave;
+  if (waves > 1 && blocks * 100 < waves * wave * 85) return false;
   return (rb == 1 || ng * group <= 128) && K / 8 <= 2 * warps * 32 && smem_bytes(warps, rb, M, K) <= 48 * 1024;
 }
 

@@ -50,6 +50,7 @@ _SIGNATURES = {
                                 c_size_t, c_void_p]),
     "kfb_int4_linear_silu_pairs": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]),
     "kfb_int4_gemv": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p]),
+    "kfb_int4_norm_fits": (c_int, [c_int, c_int, c_int, c_int]),
     "kfb_int4_gemv_fused": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_float,
                                     c_void_p, c_void_p, c_int, c_void_p]),
     "kfb_int4_gemv_silu_pair": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_float,

@@ -32,7 +32,7 @@ from dataclasses import dataclass
 
 import torch
 
-from . import ops
+from . import _capi, ops
 from . import quantize as kq
 
 
@@ -121,27 +121,32 @@ class LlamaInt4Decoder:
         # epilogues of the GEMV want (ops.interleave_qkv_for_rope / interleave_gate_up), so RoPE + cache write and
         # SiLU * up happen in the epilogue of the projection (8 kernels per layer instead of 10).  Rows are quantised
         # independently, so this is exact; prefill reads the same matrices and undoes the order with a view.
-        # Batch 3 and more (2 where the fused step below does not apply): the qkv and gate_up projections run on private
-        # fragment-order copies of their weights (ops.prepack_int4; as much memory again), with the same pair epilogues;
-        # o and down on the public format (int4_linear).  Measured, us per step on the TinyLlama-1.1B shape at batch 3 / 8 /
-        # 16 / 32: everything on fragment-order copies 597 / 620 / 764 / 1065, this 534 / 554 / 687 / 991, gate_up by
-        # int4_linear too 577 / 610 / 739 / 994.
+        # Batch 2 and more: the qkv and gate_up projections run on private fragment-order copies of their weights
+        # (ops.prepack_int4; as much memory again), with the same pair epilogues; o and down on the public format
+        # (int4_linear).  Measured, us per step on the TinyLlama-1.1B shape at batch 3 / 8 / 16 / 32: everything on
+        # fragment-order copies 597 / 620 / 764 / 1065, this 534 / 554 / 687 / 991, gate_up by int4_linear too 577 / 610 / 739 /
+        # 994 (so at batch 32 the copy of gate_up saves no time worth its memory).
         # With tensor parallelism the same holds for the rank's own rows (local heads, local share of the hidden and
         # intermediate features); only the four gathers per layer are added.
-        # Batch <= 2 on one GPU: five kernels per layer (_step_fused), both RMSNorms in the prologue of the projection behind
-        # them and the residual adds in the epilogues, where the hidden size is within what the projection kernel with a norm
-        # takes (16 warps of 128 inputs).  Measured, ms per step on the TinyLlama-1.1B shape: batch 1 0.593 -> 0.510,
-        # batch 2 0.615 (prepacked weights) -> 0.556; the prepacked copies are not made then.
-        hidden_groups = s.hidden // group
-        self.fused = (self.plan is None and batch <= ops.FUSED_GEMV_MAX_M and s.hidden % group == 0 and s.hidden <= 2048
-                      and (hidden_groups <= 16 or hidden_groups % 2 == 0))
+        # Batch 1 on one GPU: five kernels per layer (_step_fused), both RMSNorms in the prologue of the projection behind them
+        # and the residual adds in the epilogues, where both projections suit the kernel that does this (kfb_int4_norm_fits) and
+        # the hidden size makes it worth while.  Measured, us per step of 8 layers, fused / separate norm kernels: hidden 512
+        # 123 / 119, 768 134 / 128, 1024 148 / 144, 1280 177 / 177, 1536 (8192 gate / up rows) 168 / 183, 2048 (11264) 201 / 224.
+        # Above 2048 the weights of a projection with a norm do not fit in the registers: separate kernels.
+        # Batch 2: the private copies are faster at each of these sizes (132 / 142, 151 / 153, 154 / 167, 185 / 195, 176 / 187,
+        # 208 / 219 us), so the fused step is for decoders without them.
+        qkv_rows, gate_up_rows = (self.h_loc + 2 * self.hk_loc) * s.head_dim, 2 * self.inter_loc
+        fits = _capi.lib().kfb_int4_norm_fits
+        self.fused = (self.plan is None and batch <= ops.FUSED_GEMV_MAX_M and s.hidden >= 1536
+                      and all(fits(batch, n, s.hidden, group) for n in (qkv_rows, gate_up_rows)))
         hidden_loc = s.hidden if self.plan is None else self.plan["hidden_rows"][1] - self.plan["hidden_rows"][0]
         kdims = (s.hidden, s.heads * s.head_dim, s.intermediate)
         ndims = ((self.h_loc + 2 * self.hk_loc) * s.head_dim, hidden_loc, 2 * self.inter_loc)
         groups = s.hidden // group     # (the pair epilogues above 8 batch rows exist for K split 8 ways, <= 12 blocks of 64 per warp)
         wide_ok = batch <= 8 or (groups >= 8 and -(-groups // 8) * (group // 64) <= 12)
-        self.prepacked = (prepack and not self.fused and 2 <= batch <= ops.PREPACKED_GEMV_MAX_M and wide_ok
+        self.prepacked = (prepack and 2 <= batch <= ops.PREPACKED_GEMV_MAX_M and wide_ok
                           and all(k % 64 == 0 and k % group == 0 and k <= 12288 for k in kdims) and all(n % 16 == 0 for n in ndims))
+        self.fused = self.fused and not self.prepacked
         self.pair_rows = batch <= ops.FUSED_GEMV_MAX_M or self.prepacked
         f16 = lambda t: t.to(self.dev, torch.float16).contiguous()
         self.embed = f16(weights["embed"])
@@ -197,7 +202,6 @@ class LlamaInt4Decoder:
     # ------------------------------------------------------------------ construction helpers
     def _persistent_descriptor(self):
         """The argument block of kfb_decode_step_persistent: a device table of 12 pointers per layer, the workspace."""
-        from . import _capi
         s = self.s
         rows = [[L["qkv"].packed.data_ptr(), L["qkv"].scales.data_ptr(), L["o"].packed.data_ptr(), L["o"].scales.data_ptr(),
                  L["gate_up"].packed.data_ptr(), L["gate_up"].scales.data_ptr(), L["down"].packed.data_ptr(),
@@ -221,7 +225,6 @@ class LlamaInt4Decoder:
     def _step_persistent(self):
         """The whole step as one persistent cooperative kernel, then the kernel that publishes token / position / length."""
         import ctypes
-        from . import _capi
         with _capi.on_device(self.dev):
             _capi.check(_capi.lib().kfb_decode_step_persistent(ctypes.byref(self._step_desc), _capi.stream_ptr(self.dev)))
         ops.decode_finalize(self.best, self.tok, self.pos, self.kv_len)
@@ -377,7 +380,6 @@ class LlamaInt4Decoder:
         step writes cache row `pos`, which the first real step rewrites with the same values)."""
         if self._host_pos >= self.max_len:
             raise ValueError(f"the KV cache ({self.max_len} rows) is full: no room for the warm-up step")
-        from . import _capi
         saved = (self.tok.clone(), self.pos.clone(), self.kv_len.clone())
         side = torch.cuda.Stream(self.dev)
         with torch.cuda.stream(side), _capi.programmatic_launch(self.pdl):
@@ -418,6 +420,5 @@ class LlamaInt4Decoder:
                 logs.append(self.step_logits.clone())
         self._host_pos += steps
         if check_status:
-            from . import _capi
             _capi.raise_on_device_status(self.dev)
         return torch.stack(toks, 1), (torch.stack(logs, 1) if keep_logits else None)

@@ -285,3 +285,20 @@ def test_attention_refuses_tensors_of_different_devices(call):
         q, k = (torch.empty(1, 2, 16, 64, dtype=torch.float16, device=f"cuda:{i}") for i in (0, 1))
         with pytest.raises(ValueError, match="same CUDA device"):
             getattr(ops, call)(q, k, k)
+
+
+def test_where_a_decode_step_has_its_norms_in_the_projections():
+    """kfb_int4_norm_fits (148 SMs without a GPU) and the decoder's use of it: hidden sizes and widths on both sides of the lines."""
+    from kernelforge.llama_decode import LlamaInt4Decoder, LlamaShape
+    fits = _capi.lib().kfb_int4_norm_fits
+    for m, n, k, group, want in ((1, 11264, 2048, 128, 1), (2, 11840, 2048, 128, 1), (1, 11841, 2048, 128, 0), (1, 16384, 2048, 128, 0),
+                                 (1, 22016, 2048, 128, 1), (1, 4736, 4096, 128, 1), (1, 4752, 4096, 128, 0), (3, 256, 2048, 128, 0),
+                                 (1, 256, 2048, 96, 0), (1, 256, 100, 64, 0), (0, 256, 2048, 128, 0)):
+        assert fits(m, n, k, group) == want, (m, n, k, group)
+
+    def fused(hidden, intermediate):
+        shape = LlamaShape(hidden=hidden, layers=1, heads=hidden // 64, kv_heads=1, head_dim=64, intermediate=intermediate, vocab=16)
+        return LlamaInt4Decoder.random_init(shape, "cpu", batch=1, max_len=4).fused
+
+    assert fused(1536, 256) and not fused(1408, 256) and not fused(2176, 256)
+    assert not fused(1536, 5952)     # 11904 gate and up rows: a second wave of CTAs, nearly empty

@@ -1,5 +1,5 @@
 """RMSNorm fused with the INT4 linear behind it, against the two separate kernels: row counts around the 16-row blocks, around
-two blocks per SM and where a CTA owns three, four and five blocks; the smallest and largest share of K per warp; both group
+two blocks per SM and where a CTA owns three, four and five blocks, in a full second wave and in one that is left to the other kernel; the smallest and largest share of K per warp; both group
 sizes; the residual epilogue of the linears without a norm."""
 
 import pytest
@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("m", [1, 2])
 @pytest.mark.parametrize("n,k,group", [
     (2, 128, 128), (16, 64, 64), (18, 256, 64), (2560, 2048, 128), (4736, 2048, 128), (4738, 2048, 128), (7106, 1024, 64),
-    (9474, 2048, 64), (11264, 2048, 128), (14000, 1024, 128), (1000, 4096, 128), (640, 3072, 64), (48, 4096, 64), (5000, 4096, 128),
+    (9474, 2048, 64), (11264, 2048, 128), (14000, 1024, 128), (22016, 512, 128), (1000, 4096, 128), (640, 3072, 64), (48, 4096, 64), (5000, 4096, 128),
 ])
 def test_norm_linear(m, n, k, group):
     g = torch.Generator(device="cuda").manual_seed(n + k + m)
