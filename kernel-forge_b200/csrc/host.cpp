@@ -235,7 +235,7 @@ PyObject* flash_attn_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
     float scale;
     const at::Tensor* len = plain(a[3]);
     if (!attention_args(a, true, &p) || p.nq != 1 || !scale_arg(a[4], p.d, &scale)) NOT_PLAIN;
-    if (!len || len->scalar_type() != at::kInt || len->numel() != p.b || len->device() != p.q->device()) NOT_PLAIN;
+    if (!len || len->scalar_type() != at::kInt || len->numel() != p.b || !len->is_contiguous() || len->device() != p.q->device()) NOT_PLAIN;
     OnDevice dev(*p.q);
     at::Tensor o = new_tensor(p.q->sizes(), p.q->scalar_type(), *p.q);
     const size_t ws_bytes = kfb_flash_attn_ws_bytes((int)p.b, (int)p.h, (int)p.hk, 1, (int)p.nk, (int)p.d);

@@ -497,7 +497,7 @@ def flash_attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
     if q.numel() == 0:
         return torch.empty_like(q)
     plain = lambda t: t.as_subclass(torch.Tensor)
-    o = _capi.host().flash_attn_decode(plain(q), plain(k_cache), plain(v_cache), plain(kv_len), scale)
+    o = _capi.host().flash_attn_decode(plain(q), plain(k_cache), plain(v_cache), plain(kv_len).contiguous(), scale)
     if o is None:
         raise ValueError("q, k_cache, v_cache and kv_len must be non-empty and on one CUDA device")
     return o
@@ -511,6 +511,8 @@ def flash_attn_decode_partial(q: torch.Tensor, k_shard: torch.Tensor, v_shard: t
     _check_attn(q, k_shard, v_shard, False, strided_kv=True)
     b, h, _, d = q.shape
     hk, nk = k_shard.shape[1], k_shard.shape[2]
+    if kv_len is not None:
+        kv_len = kv_len.contiguous()
     lib = _capi.lib()
     nbytes = lib.kfb_flash_attn_decode_partial_bytes(b, h, hk, nk, d, None)
     partial = torch.empty(nbytes // 4, dtype=torch.float32, device=q.device)

@@ -92,3 +92,13 @@ def test_a_bias_that_is_trained_batched_or_dual_is_added_by_torch(m, prepacked):
         return   # (its entry allocates in Python: a transform of torch.func that wraps every new tensor is refused)
     value, tangent = torch.func.jvp(linear, (bias,), (several[0],))
     assert torch.equal(value, y + bias) and torch.equal(tangent, several[0].expand(m, n))
+
+
+def test_lengths_may_be_a_strided_view():
+    q, kv = (torch.randn(3, 4, n, 64, device="cuda", dtype=torch.float16) for n in (1, 900))
+    table = torch.tensor([[900, 1], [7, 2], [450, 3]], dtype=torch.int32, device="cuda")
+    lengths = table[:, 0]
+    want = ops.flash_attn_decode(q, kv, kv, lengths.contiguous())
+    assert torch.equal(ops.flash_attn_decode(q, kv, kv, lengths), want)
+    part = lambda n: ops.flash_attn_merge_partials(ops.flash_attn_decode_partial(q, kv, kv, n), q, 4, 900)
+    assert torch.equal(part(lengths), part(lengths.contiguous()))
