@@ -382,6 +382,7 @@ class LlamaInt4Decoder:
             raise ValueError(f"the KV cache ({self.max_len} rows) is full: no room for the warm-up step")
         saved = (self.tok.clone(), self.pos.clone(), self.kv_len.clone())
         side = torch.cuda.Stream(self.dev)
+        side.wait_stream(torch.cuda.current_stream(self.dev))   # weights, cache and state may still be on their way there
         with torch.cuda.stream(side), _capi.programmatic_launch(self.pdl):
             self._step()
             side.synchronize()

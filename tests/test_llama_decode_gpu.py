@@ -13,7 +13,7 @@ from transformers import LlamaConfig, LlamaForCausalLM  # noqa: E402
 
 from kernelforge import modules as km  # noqa: E402
 from kernelforge import quantize as kq  # noqa: E402
-from kernelforge.llama_decode import LlamaInt4Decoder  # noqa: E402
+from kernelforge.llama_decode import LlamaInt4Decoder, LlamaShape  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 
@@ -179,3 +179,21 @@ def test_persistent_step_at_tinyllama_size():
     (ta, la), (tb, lb) = outs
     err, scale = assert_same_decode(ta, la, tb, lb, 4e-3)
     print(f"PARITY persistent step vs separate kernels, tinyllama-arch: max_abs_diff {err:.3e} logit scale {scale:.3f}")
+
+
+def test_capture_waits_for_pending_work_of_the_current_stream():
+    """decode() right after prefill(), without a capture before: the warm-up step has to see the position that the current
+    stream is about to set, or it writes the key and value of one token into another's row of the cache."""
+    shape = LlamaShape(hidden=256, layers=2, heads=4, kv_heads=2, head_dim=64, intermediate=512, vocab=300)
+    model = LlamaInt4Decoder.random_init(shape, "cuda", batch=1, max_len=40, seed=3)
+    ids = torch.randint(0, 300, (1, 20), generator=torch.Generator().manual_seed(1))
+    model.prefill(ids)
+    rows = model.k_cache[:, :, :, :20].clone()
+    model.pos.fill_(0)
+    torch.cuda.synchronize()
+    torch.cuda._sleep(100_000_000)          # some 50 ms on the current stream, then the state that prefill sets
+    model.pos.fill_(20)
+    tokens, _ = model.decode(4)
+    assert torch.equal(model.k_cache[:, :, :, :20], rows)
+    model.prefill(ids)
+    assert torch.equal(model.decode(4)[0], tokens)
