@@ -318,6 +318,10 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   }
 
   // ------------------------------------------------------------------ merge the warps
+  if (!aborted && *abort_word != 0) {   // a wait expired: let copies in flight land before the ring is reused or freed
+    const unsigned long long t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+  }
   __syncthreads();  // every tile has been consumed (or the CTA is aborting): the ring is free
   float* scratch = reinterpret_cast<float*>(smem);
   constexpr int kPerWarp = kRows * (D + 2);

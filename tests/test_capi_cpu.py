@@ -302,3 +302,12 @@ def test_where_a_decode_step_has_its_norms_in_the_projections():
 
     assert fused(1536, 256) and not fused(1408, 256) and not fused(2176, 256)
     assert not fused(1536, 6016)     # 12032 gate and up rows: a second wave of CTAs, nearly empty
+
+
+def test_decode_attention_waits_for_its_copies_before_it_reuses_their_ring():
+    """After an expired wait copies may still be in flight: they get time to land before the ring becomes the scratch of the merge
+    and the CTA leaves.  Read from the source: a run would need a wait that expires in mid-copy."""
+    code = re.sub(r"//[^\n]*", "", (ROOT / "kernel-forge_b200" / "csrc" / "attn_decode.cu").read_text())
+    kernel = code[code.index("attn_decode_kernel("):code.index("attn_decode_merge_kernel(")]
+    consumed, merge = kernel.split("float* scratch", 1)
+    assert "*abort_word != 0" in consumed[consumed.index("mbar_arrive(&empty[s])"):]
