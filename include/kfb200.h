@@ -391,6 +391,10 @@ int kfb_decode_finalize(void* best, void* tok, void* pos, void* kv_len, int M, v
  * weight with the rounding of kfb_add_rmsnorm.  embed: fp16 [vocab, hidden]. */
 int kfb_embed_rmsnorm(const void* tok, const void* embed, const void* weight, void* y, void* x_out, int rows,
                       int hidden, int vocab, float eps, void* stream);
+/* The same for ids that come from a caller (a prompt): negative ids count from the end of the table, and an id outside it leaves
+ * 0x702 in the device status word (a valid row is read; nothing faults). */
+int kfb_embed_prompt(const void* tok, const void* embed, const void* weight, void* y, void* x_out, int rows,
+                     int hidden, int vocab, float eps, void* stream);
 
 /* kfb_flash_attn_fwd for token-major q and o, [B, Nq, H, D]: what a projection writes and the next one reads, without
  * the two transposes.  K, V, strides and workspace as there. */

@@ -148,17 +148,23 @@ __global__ void decode_finalize_kernel(unsigned long long* __restrict__ best, lo
   if (m == 0) pos[0] += 1;
 }
 
+constexpr unsigned int kStatusTokenId = 0x702;   // a prompt holds an id outside the embedding table
+
 // One CTA (256 threads) per token: x_out[row] = embed[tok[row]], y[row] = fp16(fp16(x * rsqrt(mean(x^2) + eps)) * w).
 constexpr int kWidestVec = 16;  // hidden <= 256 * 8 * 16
 // kMaxVec: 16-byte vectors of the row a thread holds
 template <int kMaxVec>
 __global__ void __launch_bounds__(kThreads)
 embed_rmsnorm_kernel(const long long* __restrict__ tok, const __half* __restrict__ embed, const __half* __restrict__ w,
-                     __half* __restrict__ y, __half* __restrict__ x_out, int hidden, int vocab, float eps) {
+                     __half* __restrict__ y, __half* __restrict__ x_out, int hidden, int vocab, float eps, unsigned int* status) {
   __shared__ float warp_part[kWarps];
   pdl_wait(tok, embed, w);
   pdl_launch_dependents();
   long long id = tok[blockIdx.x];
+  if (status) {   // ids of a caller: negative ones count from the end, as in `embed[ids]`
+    if (id < 0) id += vocab;
+    if ((id < 0 || id >= vocab) && threadIdx.x == 0) atomicCAS(status, 0u, kStatusTokenId);
+  }
   id = id < 0 ? 0 : (id >= vocab ? vocab - 1 : id);   // an id outside the table reads a valid row instead of faulting
   const size_t src = (size_t)id * hidden, dst = (size_t)blockIdx.x * hidden;
   const int nvec = hidden / 8;
@@ -243,8 +249,10 @@ extern "C" int kfb_decode_finalize(void* best, void* tok, void* pos, void* kv_le
                        static_cast<long long*>(pos), static_cast<int*>(kv_len), M);
 }
 
-extern "C" int kfb_embed_rmsnorm(const void* tok, const void* embed, const void* weight, void* y, void* x_out, int rows,
-                                 int hidden, int vocab, float eps, void* stream) {
+namespace {
+
+int embed_rmsnorm(const void* tok, const void* embed, const void* weight, void* y, void* x_out, int rows, int hidden, int vocab, float eps,
+                  unsigned int* status, void* stream) {
   if (int rc = require_sm100()) return rc;
   if (rows < 1 || vocab < 1 || hidden < 8 || hidden % 8 || hidden > lmhead::kThreads * 8 * lmhead::kWidestVec)
     return fail(KFB_ERR_INVALID, "embed_rmsnorm needs rows, vocab >= 1 and hidden a multiple of 8 up to %d, got %d x %d",
@@ -257,5 +265,19 @@ extern "C" int kfb_embed_rmsnorm(const void* tok, const void* embed, const void*
                                                                                      : lmhead::embed_rmsnorm_kernel<lmhead::kWidestVec>;
   return launch_kernel("embed_rmsnorm_kernel", kernel, dim3(rows), dim3(lmhead::kThreads), 0,
                        (cudaStream_t)stream, static_cast<const long long*>(tok), static_cast<const __half*>(embed),
-                       static_cast<const __half*>(weight), static_cast<__half*>(y), static_cast<__half*>(x_out), hidden, vocab, eps);
+                       static_cast<const __half*>(weight), static_cast<__half*>(y), static_cast<__half*>(x_out), hidden, vocab, eps, status);
+}
+
+}  // namespace
+
+extern "C" int kfb_embed_rmsnorm(const void* tok, const void* embed, const void* weight, void* y, void* x_out, int rows,
+                                 int hidden, int vocab, float eps, void* stream) {
+  return embed_rmsnorm(tok, embed, weight, y, x_out, rows, hidden, vocab, eps, nullptr, stream);
+}
+
+extern "C" int kfb_embed_prompt(const void* tok, const void* embed, const void* weight, void* y, void* x_out, int rows, int hidden, int vocab,
+                                float eps, void* stream) {
+  unsigned int* status = device_status_word();
+  if (!status) return fail(KFB_ERR_CUDA, "cannot resolve the device status word");
+  return embed_rmsnorm(tok, embed, weight, y, x_out, rows, hidden, vocab, eps, status, stream);
 }

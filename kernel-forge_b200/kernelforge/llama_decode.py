@@ -280,14 +280,20 @@ class LlamaInt4Decoder:
     @torch.no_grad()
     def prefill(self, ids: torch.Tensor) -> torch.Tensor:
         """ids [B, T] -> logits [B, T, vocab] (fp16); fills the cache and arms the decode state with the
-        greedy next token."""
+        greedy next token.  Ids as in `embed[ids]`: negative ones count from the end.  One outside the vocabulary raises
+        IndexError when the ids are on the host; on the GPU it leaves 0x702 in the device status word, which decode() raises."""
         s, (b, t) = self.s, ids.shape
+        if ids.dtype not in (torch.int64, torch.int32):
+            raise IndexError(f"token ids must be int64 or int32, got {ids.dtype}")
+        if not ids.is_cuda and ids.numel() and not (-s.vocab <= int(ids.min()) and int(ids.max()) < s.vocab):
+            raise IndexError(f"token ids must lie in [-{s.vocab}, {s.vocab}), got {int(ids.min())} .. {int(ids.max())}")
         if t >= self.max_len:
             raise ValueError(f"prompt of {t} tokens leaves no room in a cache of {self.max_len} rows for a decode step")
         nq, rows = self.h_loc * s.head_dim, b * t
         # eight or nine kernels per layer (SiLU * up sits in the epilogue of the gate / up projection when its rows are paired) and no copy in between: activations stay token-major [B * T, features], RoPE writes the
         # cache and undoes the pair order of the rows, attention reads the cache in place
-        h, x = ops.embed_rmsnorm(ids.to(self.dev, torch.long).reshape(rows).contiguous(), self.embed, self.layers[0]["in_norm"], s.rms_eps)
+        h, x = ops.embed_rmsnorm(ids.to(self.dev, torch.long).reshape(rows).contiguous(), self.embed, self.layers[0]["in_norm"], s.rms_eps,
+                                prompt=True)
         res = None
         for li, L in enumerate(self.layers):
             k_cache, v_cache = self.k_cache[li], self.v_cache[li]

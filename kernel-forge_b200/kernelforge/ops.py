@@ -650,12 +650,14 @@ def decode_finalize(best: torch.Tensor, tok: torch.Tensor, pos: torch.Tensor, kv
                                                     tok.numel(), _capi.stream_ptr(tok.device)))
 
 
-def embed_rmsnorm(tok: torch.Tensor, embed: torch.Tensor, weight: torch.Tensor, eps: float):
-    """(y, x): x = embed[tok] (tok int64 [rows]), y = RMSNorm(x) * weight, in one pass."""
+def embed_rmsnorm(tok: torch.Tensor, embed: torch.Tensor, weight: torch.Tensor, eps: float, prompt: bool = False):
+    """(y, x): x = embed[tok] (tok int64 [rows]), y = RMSNorm(x) * weight, in one pass.  Ids are clamped to the table; `prompt`:
+    negative ids count from its end and an id outside it leaves 0x702 in the device status word."""
     rows, (vocab, hidden) = tok.numel(), embed.shape
     y = torch.empty(rows, hidden, dtype=torch.float16, device=embed.device)
     x = torch.empty_like(y)
+    entry = _capi.lib().kfb_embed_prompt if prompt else _capi.lib().kfb_embed_rmsnorm
     with _capi.on_device(embed.device):
-        _capi.check(_capi.lib().kfb_embed_rmsnorm(tok.data_ptr(), embed.data_ptr(), weight.data_ptr(), y.data_ptr(), x.data_ptr(),
-                                                  rows, hidden, vocab, eps, _capi.stream_ptr(embed.device)))
+        _capi.check(entry(tok.data_ptr(), embed.data_ptr(), weight.data_ptr(), y.data_ptr(), x.data_ptr(),
+                          rows, hidden, vocab, eps, _capi.stream_ptr(embed.device)))
     return y, x

@@ -311,3 +311,12 @@ def test_decode_attention_waits_for_its_copies_before_it_reuses_their_ring():
     kernel = code[code.index("attn_decode_kernel("):code.index("attn_decode_merge_kernel(")]
     consumed, merge = kernel.split("float* scratch", 1)
     assert "*abort_word != 0" in consumed[consumed.index("mbar_arrive(&empty[s])"):]
+
+
+def test_prefill_refuses_ids_that_are_no_indices():
+    from kernelforge.llama_decode import LlamaInt4Decoder, LlamaShape
+    shape = LlamaShape(hidden=128, layers=1, heads=2, kv_heads=1, head_dim=64, intermediate=128, vocab=64)
+    dec = LlamaInt4Decoder.random_init(shape, "cpu", batch=1, max_len=8)
+    for ids in (torch.ones(1, 4), torch.ones(1, 4, dtype=torch.int16), torch.tensor([[1, 64]]), torch.tensor([[0, -65]])):
+        with pytest.raises(IndexError):
+            dec.prefill(ids)

@@ -4,7 +4,7 @@ bit where no transcendental is involved)."""
 import pytest
 import torch
 
-from kernelforge import ops
+from kernelforge import _capi, ops
 
 pytestmark = pytest.mark.gpu
 
@@ -53,3 +53,23 @@ def test_rmsnorm_widths(hidden):
     want = (f * torch.rsqrt(f.pow(2).mean(-1, keepdim=True) + 1e-5)).half() * w
     assert torch.equal(s, x + r)
     assert (y.float() - want.float()).abs().max() <= 2e-3 * want.float().abs().max()
+
+
+def test_prompt_ids_are_table_indices():
+    """Negative ids count from the end, as torch indexing has them; an id outside the table is reported, nothing faults."""
+    g = torch.Generator(device="cuda").manual_seed(4)
+    embed = torch.randn(300, 256, generator=g, device="cuda", dtype=torch.float16)
+    w = torch.ones(256, device="cuda", dtype=torch.float16)
+    ids = torch.tensor([0, 299, -1, -300, 17], device="cuda")
+    assert torch.equal(ops.embed_rmsnorm(ids, embed, w, 1e-5, prompt=True)[1], embed[ids])
+    dev = torch.device("cuda", 0)
+    assert _capi.device_status(dev) == 0
+    try:
+        for bad in (300, -301, 1 << 40):
+            ops.embed_rmsnorm(torch.tensor([5, bad], device="cuda"), embed, w, 1e-5, prompt=True)
+            torch.cuda.synchronize()
+            assert _capi.device_status(dev) == 0x702
+            _capi.device_status_reset(dev)
+    finally:
+        _capi.device_status_reset(dev)
+        torch.cuda.synchronize()
