@@ -514,8 +514,10 @@ extern "C" int kfb_int4_gemv(const void* x, const void* packed, const void* scal
 namespace {
 
 int fused_common(const char* what, const void* x, const void* packed, const void* scales, void* y, int M, int N, int K, int group,
-                 int xform, int flags, void* stream, const gemv::Fusion& fu) {
+                 int xform, int flags, void* stream, const gemv::Fusion& given) {
   if (int rc = require_sm100()) return rc;
+  gemv::Fusion fu = given;
+  fu.early = flags & 1;
   if (M < 1 || M > 2) return fail(KFB_ERR_UNSUPPORTED, "%s handles M in [1, 2], got M=%d", what, M);
   if (group != 64 && group != 128) return fail(KFB_ERR_INVALID, "group_size must be one of (64, 128), got %d", group);
   if (N < 1 || K < group || K % group) return fail(KFB_ERR_INVALID, "K=%d is not a multiple of group_size=%d", K, group);

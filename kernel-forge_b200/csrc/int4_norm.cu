@@ -273,7 +273,7 @@ bool fits(int M, int N, int K, int group) {
 int run(const void* x, const void* packed, const void* scales, void* y, int M, int N, int K, int group, cudaStream_t stream,
         const gemv::Fusion& given) {
   gemv::Fusion fu = given;
-  fu.early = constants_are_old();
+  fu.early = given.early || constants_are_old();
   const int ng = groups_per_warp(K / group), rb = row_blocks(N);
 #define KFB_NORM(G, NG, RB) \
   if (group == G && ng == NG && rb == RB) return launch<G, NG, RB>(x, packed, scales, y, M, N, K, stream, fu)

@@ -257,7 +257,7 @@ int launch(const void* x, const void* packed, const void* scales, void* y, int M
 int run(const void* x, const void* packed, const void* scales, void* y, int M, int N, int K, int group, bool bf16, cudaStream_t stream,
         const gemv::Fusion& given) {
   gemv::Fusion fu = given;
-  fu.early = constants_are_old();
+  fu.early = given.early || constants_are_old();
   // Few row blocks (at most one CTA per SM) and a long K: 16 shares of K instead of 8, so that a warp has half as many
   // groups one after the other (2048 x 5632, M = 8: 5.3 us against 6.1; at K = 2048 there is nothing to gain).
   // 9 <= M <= 16 and more row blocks than the three CTAs per SM hold: two row blocks per warp share the activations

@@ -4,6 +4,7 @@ import pytest
 import torch
 
 from kernelforge import ops
+from kernelforge import quantize as kq
 
 pytestmark = pytest.mark.gpu
 
@@ -292,3 +293,24 @@ def test_prepacked_gemv_epilogues_match_the_separate_kernels(m):
     close(q_got, q_want, "rope q"); close(kc1, kc0, "k cache"); close(vc1, vc0, "v cache")
     untouched = [i for i in range(lmax) if i != pos]
     assert torch.equal(kc1[:, :, untouched], base[:, :, untouched]) and torch.equal(vc1[:, :, untouched], (base * 2)[:, :, untouched])
+
+
+@pytest.mark.parametrize("hidden", [512, 2048, 2560])   # the kernel with a norm prologue; too wide for it: the CUDA-core one
+def test_flag_for_old_weights_gives_the_same_bits(hidden):
+    """Bit 0 (weights are older than the kernel in front) on every route of kfb_int4_gemv_fused: norm, residual, neither."""
+    from kernelforge import _capi
+    lib, n = _capi.lib(), 768
+    g = torch.Generator(device="cuda").manual_seed(hidden)
+    rn = lambda *s: torch.randn(*s, generator=g, device="cuda", dtype=torch.float16)
+    qw = kq.quantize_weight(rn(n, hidden) * 0.02, 128)
+    x, norm, res = rn(2, hidden), rn(hidden), rn(2, n)
+    torch.cuda.synchronize()
+    for xform, norm_w, residual in ((1, norm, None), (0, None, res), (0, None, None)):
+        out = []
+        for flags in (0, 1):
+            y = torch.empty(2, n, dtype=torch.float16, device="cuda")
+            _capi.check(lib.kfb_int4_gemv_fused(x.data_ptr(), qw.packed.data_ptr(), qw.scales.data_ptr(), y.data_ptr(), 2, n, hidden, 128, xform,
+                                                norm_w.data_ptr() if xform else None, 1e-5, None,
+                                                residual.data_ptr() if residual is not None else None, flags, _capi.stream_ptr(x.device)))
+            out.append(y)
+        assert torch.equal(*out)
