@@ -310,7 +310,13 @@ def test_decode_attention_waits_for_its_copies_before_it_reuses_their_ring():
     code = re.sub(r"//[^\n]*", "", (ROOT / "kernel-forge_b200" / "csrc" / "attn_decode.cu").read_text())
     kernel = code[code.index("attn_decode_kernel("):code.index("attn_decode_merge_kernel(")]
     consumed, merge = kernel.split("float* scratch", 1)
-    assert "*abort_word != 0" in consumed[consumed.index("mbar_arrive(&empty[s])"):]
+    for wait in ("if (!mbar_wait(&empty[s]", "if (!ok)"):     # the producer's wait and the consumers'
+        assert consumed.count(wait) == 1
+        expired = consumed[consumed.index(wait):]
+        assert "let_copies_land();" in expired[:expired.index("break;")]
+    assert consumed.count("break;") == 2      # no other way out of the loops
+    helper = code[code.index("void let_copies_land()"):]
+    assert "200000ull" in helper[:helper.index("\n}")]
 
 
 def test_prefill_refuses_ids_that_are_no_indices():
