@@ -65,14 +65,15 @@ int kfb_device_status_reset(void* stream);
  * reference (csrc/common/check.cuh:11-24 turns CUDA errors into exceptions; it has no in-kernel waits). */
 int kfb_selftest_wait_expiry(unsigned long long timeout_ns, unsigned int* outcome_dev, void* stream);
 
-/* Every launch of this library carries the attribute that lets a kernel become resident while the one in front of it in
- * the stream is still running (programmatic dependent launch); each kernel waits for that one (griddepcontrol.wait)
- * before it touches anything that one may have written, and only then releases its own successor, so results are those of
- * the plain stream order.  This switch adds one promise by the caller: weights, scales and norm weights are OLDER than the
- * kernel in front of the one that reads them, so the linears, the lm_head and the norms may request them before their
- * wait -- true of a decode step, not of a weight quantised by the launch before.  Works in CUDA-graph capture.
- * Process-wide, off by default; returns the previous setting.  The reference has no counterpart (its decode step is
- * launch-bound: docs/phase5-notes.md). */
+/* The launches of the attention, linear, norm and decode-step kernels carry the attribute that lets a kernel become
+ * resident while the one in front of it in the stream is still running (programmatic dependent launch; not those of
+ * pack, unpack, dequantise, the persistent step and the self-tests, and the streaming linear kernels only with this
+ * switch); each kernel waits for that one (griddepcontrol.wait) before it touches anything that one may have written,
+ * and only then releases its own successor, so results are those of the plain stream order.  This switch adds one
+ * promise by the caller: weights, scales and norm weights are OLDER than the kernel in front of the one that reads
+ * them, so the linears, the lm_head and the norms may request them before their wait -- true of a decode step, not of
+ * a weight quantised by the launch before.  Works in CUDA-graph capture. Process-wide, off by default; returns the
+ * previous setting.  The reference has no counterpart (its decode step is launch-bound: docs/phase5-notes.md). */
 int kfb_set_programmatic_launch(int enable);
 
 /* ---------------------------------------------------------------------------------------

@@ -109,11 +109,12 @@ __device__ __forceinline__ TileOrder decode_tile_order(unsigned int block, int n
 //   * the two tiles take turns on the exponential units (a "baton"): one tile's exponentials run under the other's score
 //     load, maxima, P store and products.  Left alone the tiles fall into step and compete for the same unit;
 //   * head dim 64 computes some exponentials on the FMA pipe (exp_pair_fma), which is idle otherwise.
-// Measured (TFLOP/s, graph of calls; the kernels before: event-loop issuers at head dim 64, one tile per CTA and two passes
-// over S at head dim 128): B=2 H=16 N=2048 D=64 582 -> 610, causal 479 -> 521; N=8192 D=128 causal 1009 -> 1083;
-// 509 queries on 4093 keys, 12 heads, D=128: 59 us -> 30 (key splits).
-// Also measured at D=64, N=2048 (us; this kernel 56.4): scores of step j+1 loaded chunk by chunk under the exponentials of
-// step j 64; no baton 64; baton passed after all exponentials 66; polynomial for 4 of 16 pairs 58.6, for 5 59.2.
+// Measured (us per call through the public operator; the kernels before had event-loop issuers at head dim 64, one tile per CTA
+// and two passes over S at head dim 128): B=2 H=16 N=2048 D=64 62.6 -> 58.4 (588 TFLOP/s); N=8192 D=128 causal 632 -> 572
+// (961 TFLOP/s; 1083 in a burst too short for the power limit); 509 queries on 4093 keys, 12 heads over 2, D=128 60 -> 27.4.
+// Also measured at D=64, N=2048 (us in a graph; this kernel 56.4): scores of step j+1 loaded chunk by chunk under the
+// exponentials of step j 64; no baton 64; baton passed after all exponentials 66; polynomial for 4 of 16 pairs 58.6, for 5
+// 59.2.
 //
 // Split over keys: a problem with few tiles (short chunks against a long cache) is cut along the keys too; a CTA then
 // writes its unnormalised O and (m, l) per row and attn_prefill_merge_kernel puts the pieces together in order.
@@ -654,7 +655,7 @@ PrefillPlan plan_prefill(const Problem& p, int max_splits = 32) {
   // B200 (mean deviation 5 %): a CTA takes `step` per 128 keys and `fixed` for set-up and drain; the merge kernel 2.7, 0.2 per
   // split and its traffic at 5.1 TB/s.  So a grid smaller than the GPU takes one tile per CTA and splits the keys (1 x 8 x 1024
   // queries, D = 128: 17.4 us, two tiles 18.7), long ones share K / V between two tiles (2 x 16 x 8192 D = 128 causal: 514
-  // against 542).
+  // against 542; bursts too short for the power limit).
   // One-tile CTAs fit in pairs on an SM, and the hardware does pair them while other SMs stay idle.  Where the grid has at
   // most one for each SM, and under a causal mask also for longer grids, where short CTAs even out what is left over, they are
   // kept apart (by the shared memory they ask for): 1 x 8 x 1024, two splits 21.2 -> 17.0; 1 x 16 x 2048 causal 39.2 -> 35.2.

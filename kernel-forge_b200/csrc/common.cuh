@@ -43,13 +43,14 @@ int require_sm100();
                          __FILE__, __LINE__);                                               \
   } while (0)
 
-// Programmatic dependent launch: every launch of this library carries the attribute.  Such a kernel may become resident
-// while the kernel in front of it in the stream is still running; it calls pdl_wait() before it touches anything that
-// kernel may have written (or still reads), and releases its own successor with pdl_launch_dependents() after that wait,
-// so at most two grids overlap and the order of all memory operations is that of the plain stream.  It hides launch and
-// set-up behind the predecessor's tail; and between plain launches the hardware was measured to start a kernel only at
-// multiples of 2.05 us after the one in front (a 3.0 us kernel costs 4.1 us, a 4.2 us one 6.1), with the attribute 0.5 us
-// after it.  Both instructions are no-ops without a predecessor.
+// Programmatic dependent launch: the launches of the attention, linear, norm and decode-step kernels carry the attribute
+// (not pack, unpack, dequantise, the persistent decode step and the self-tests; the streaming INT4 kernels only when
+// constants are old, below). Such a kernel may become resident while the kernel in front of it in the stream is still
+// running; it calls pdl_wait() before it touches anything that kernel may have written (or still reads), and releases its
+// own successor with pdl_launch_dependents() after that wait, so at most two grids overlap and the order of all memory
+// operations is that of the plain stream.  It hides launch and set-up behind the predecessor's tail; and between plain
+// launches the hardware was measured to start a kernel only at multiples of 2.05 us after the one in front (a 3.0 us kernel
+// costs 4.1 us, a 4.2 us one 6.1), with the attribute 0.5 us after it.  Both instructions are no-ops without a predecessor.
 // A kernel may read CONSTANTS (weights, scales, norm weights) before its wait only where the caller knows that they are
 // older than the kernel in front: kfb_set_programmatic_launch (constants_are_old() below), used for decode steps.
 #ifdef __CUDACC__

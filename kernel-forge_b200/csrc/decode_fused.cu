@@ -3,8 +3,10 @@
 // The reference leaves these operations to Hugging Face / torch (RMSNorm, rotary embedding, KV-cache
 // write, SiLU * up, residual add: kernelforge/modules.py swaps only the linears and the attention
 // function), which costs ~45 tiny kernels per layer.  At batch 1 a decode step is launch-bound (631 MB
-// per token are 0.1 ms of HBM time), so the step is cut to 11 kernels per layer with three fused
-// element-wise kernels.  All three are HBM / latency trivial; they exist to remove launches.
+// per token are 0.1 ms of HBM time), so these kernels exist to remove launches; all are HBM / latency
+// trivial.  In a step the norms run twice per layer unless the projections take them into their
+// prologues (int4_norm.cu); RoPE + cache write and SiLU * up are the projections' epilogues where their
+// rows are paired (int4_epilogue.cuh), and kernels of this file otherwise and for the tokens of a prompt.
 //
 // Rounding follows what the torch formulation does in fp16 models, so results track the unfused path:
 //   add_rmsnorm : s = fp16(x + r);  y = fp16( fp16(s * rsqrt(mean(s^2) + eps)) * w )

@@ -1,5 +1,5 @@
-// Epilogues shared by the M <= 8 INT4 GEMV kernels (the CUDA-core kernel of int4_gemv.cu, the fragment-order kernel of
-// int4_gemv_frag.cu): what happens to a pair of adjacent result rows before it is stored.
+// Epilogues shared by the small-batch INT4 kernels (int4_gemv.cu on CUDA cores, int4_small.cu, int4_norm.cu, and
+// int4_gemv_frag.cu on private copies): what happens to a pair of adjacent result rows before it is stored.
 #pragma once
 
 #include "common.cuh"

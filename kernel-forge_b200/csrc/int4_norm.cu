@@ -15,8 +15,8 @@
 //     561, 141 of five 513).
 // Weights staged in shared memory with asynchronous copies instead of registers were slower (+2 us per layer), and so was
 // this structure without the norm (o and down projection: int4_small.cu, which has fewer and smaller CTAs there).
-// Step of the 22-layer model: 593 us with separate norm kernels and the CUDA-core GEMV -> 510 at batch 1, 615 (fragment-order
-// weights) -> 556 at batch 2; from batch 4 on the fragment-order kernels are faster (635 against 647).
+// Step of the 22-layer model at batch 1: 593 us with separate norm kernels and the CUDA-core GEMV -> 503.  At batch 2 the step
+// with the norms apart on fragment-order copies of qkv and gate_up is the faster one (LlamaInt4Decoder decides).
 // The fragment layout and the unpacking are those of int4_small.cu.
 #include "common.cuh"
 #include "int4_epilogue.cuh"

@@ -7,13 +7,13 @@ Here the step runs `ops.flash_attn_decode`, which reads the valid cache length f
 `ops.int4_linear` for the seven decoder linears of every layer; token ids, position and KV length all live
 on the device, so a step is a pure graph replay with no host synchronisation.
 
-Prefill runs nine kernels per layer (ops.add_rmsnorm, rope_tokens, attention_tokens, silu_mul and the four linears);
+Prefill runs eight or nine kernels per layer (ops.add_rmsnorm twice, rope_tokens, attention_tokens, the four linears, and
+silu_mul where the gate / up rows are not paired), plus a merge or reduction kernel where an attention or a linear is split;
 written with torch for everything but the two hot paths, as the reference does, it was ~45 and bound by their launches.
-Only the lm_head over all prompt positions is torch's matmul.  The decode step is launch-bound at batch 1 too, so there the
-element-wise steps run as three fused kernels (ops.add_rmsnorm, ops.rope_kv_write, ops.silu_mul) and q/k/v and
-gate/up are stored as one quantised matrix each: 11 kernels per layer instead of ~48 (2.39 -> 0.85 ms per step
-on the TinyLlama-1.1B architecture).  The embedding lookup is fused into the first norm (ops.embed_rmsnorm), the fp16
-lm_head is this library's streaming GEMV with the greedy argmax fused (ops.lm_head_argmax: the lm_head is the largest
+Only the lm_head over all prompt positions is torch's matmul.  In the decode step q/k/v and gate/up are stored as one
+quantised matrix each, and what surrounds the projections runs in their epilogues where the rows allow it: five kernels
+per layer with the norms in the projections too, seven with the norms apart, nine without epilogues (written with torch it
+was ~48).  The embedding lookup is fused into the first norm (ops.embed_rmsnorm), the fp16 lm_head is this library's streaming GEMV with the greedy argmax fused (ops.lm_head_argmax: the lm_head is the largest
 single read of a step), and one kernel publishes the token and advances the device-side counters
 (ops.decode_finalize).
 
@@ -188,7 +188,7 @@ class LlamaInt4Decoder:
         self.best = torch.zeros(batch, dtype=torch.int64, device=self.dev)   # argmax keys of the step, see ops.lm_head_argmax
         # Batch <= 2, head dim 64, one GPU: the whole step can run as ONE persistent cooperative kernel
         # (kfb_decode_step_persistent) plus the finalize kernel: set `persistent = True` before capture().  Not the default:
-        # measured on the TinyLlama-1.1B shape it takes 0.98 ms per step at batch 1 against 0.68 ms for the step of
+        # measured on the TinyLlama-1.1B shape it takes 0.92 ms per step at batch 1 against 0.50 ms for the step of
         # separate kernels chained by programmatic dependent launch -- five grid-wide barriers per layer at ~2 us each
         # plus the L2 round trip that re-reads the activations after each of them cost more than the launches they replace.
         self.persistent_ok = self.pair_rows and self.plan is None and batch <= 2 and s.head_dim == 64
@@ -290,8 +290,8 @@ class LlamaInt4Decoder:
         if t >= self.max_len:
             raise ValueError(f"prompt of {t} tokens leaves no room in a cache of {self.max_len} rows for a decode step")
         nq, rows = self.h_loc * s.head_dim, b * t
-        # eight or nine kernels per layer (SiLU * up sits in the epilogue of the gate / up projection when its rows are paired) and no copy in between: activations stay token-major [B * T, features], RoPE writes the
-        # cache and undoes the pair order of the rows, attention reads the cache in place
+        # Eight or nine kernels per layer (SiLU * up sits in the epilogue of the gate / up projection when its rows are
+        # paired) and no copy in between: activations stay token-major [B * T, features], RoPE writes the cache and undoes the pair order of the rows, attention reads the cache in place
         h, x = ops.embed_rmsnorm(ids.to(self.dev, torch.long).reshape(rows).contiguous(), self.embed, self.layers[0]["in_norm"], s.rms_eps,
                                 prompt=True)
         res = None
@@ -320,7 +320,7 @@ class LlamaInt4Decoder:
     # ------------------------------------------------------------------ one decode step (graph body)
     @torch.no_grad()
     def _step_fused(self):
-        """The step for batch <= 2 on one GPU with everything fused: 5 kernels per layer.  Both RMSNorms run in the
+        """The step with everything fused (one GPU, where __init__ finds it the faster one): five kernels per layer.  Both RMSNorms run in the
         prologue of the GEMV that consumes them, RoPE + cache write and SiLU * up in the epilogue of the GEMV that
         produces their input, both residual adds in the epilogues of o_proj and down_proj; only the attention itself
         stays a kernel of its own."""
@@ -339,12 +339,12 @@ class LlamaInt4Decoder:
 
     @torch.no_grad()
     def _step(self):
-        """One decode step: 9 or 10 kernels per layer (add + norm, qkv, rope + cache write, attention (+ merge when the
-        keys are split), o, add + norm, gate_up, silu * up, down; the last residual add is fused into the next layer's
-        norm; the embedding gather is fused into the first norm) -- 7 or 8 at batch <= 2 on one GPU, where rope +
-        cache write and silu * up run in the epilogues of the qkv and gate_up GEMVs -- then final norm, lm_head with fused argmax, and
-        one kernel that publishes the token and advances position and KV length (batch <= 2: _step_fused instead, where it
-        applies).  Every kernel of the step is one of this library's: no torch or cuBLAS kernel is left in the graph."""
+        """One decode step: nine kernels per layer (add + norm, qkv, rope + cache write, attention, o, add + norm, gate_up,
+        silu * up, down), seven where the rows of qkv and gate_up are paired, since rope + cache write and silu * up then run in
+        the epilogues of those projections; one more each where the attention (more than eight splits) or a projection (split
+        K) needs a kernel that puts pieces together.  The last residual add is fused into the next layer's norm, the embedding
+        gather into the first one.  Then final norm, lm_head with fused argmax, and one kernel that publishes the token and
+        advances position and KV length.  _step_fused takes its place where self.fused says so.  Every kernel of the step is one of this library's: no torch or cuBLAS kernel is left in the graph."""
         if self.persistent:
             return self._step_persistent()
         if self.plan is None and self.b <= ops.FUSED_GEMV_MAX_M and self.fused:

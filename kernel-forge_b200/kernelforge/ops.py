@@ -143,7 +143,7 @@ def int4_gemv_fused(x: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor,
 # private prepacked weight cache (the reference's stated next step, docs/phase4-notes.md:59): a copy of the packed words
 # in MMA-fragment order, keyed on the public tensor, which stays the format callers exchange
 # ----------------------------------------------------------------------------------------------------------------
-PREPACKED_GEMV_MAX_M = 32   # measured against the dispatcher's kernels on the public format: faster at every M <= 32
+PREPACKED_GEMV_MAX_M = 32   # what the kernel takes; where it is the faster one: _prepacked_wins
 _PREPACKED: dict[int, tuple[int, torch.Tensor]] = {}
 
 
@@ -166,9 +166,9 @@ def prepack_int4(packed: torch.Tensor) -> torch.Tensor:
 
 def prepack_weight_(packed: torch.Tensor) -> torch.Tensor:
     """Builds (once) and caches the private fragment-order copy of `packed`; afterwards int4_linear / int4_matmul run
-    batches of up to PREPACKED_GEMV_MAX_M rows on it (M = 1: only where it measured faster, see _prepacked_wins).  The cache entry is keyed on the public tensor (identity and
-    version counter: an in-place change of the weight rebuilds the copy) and dies with it.  Costs as much memory again
-    as the packed weight."""
+    batches of up to PREPACKED_GEMV_MAX_M rows on it (see _prepacked_wins for what that gives).  The cache entry is keyed on
+    the public tensor (identity and version counter: an in-place change of the weight rebuilds the copy) and dies with it.
+    Costs as much memory again as the packed weight."""
     import weakref
     key = id(packed)
     hit = _PREPACKED.get(key)
@@ -182,9 +182,16 @@ def prepack_weight_(packed: torch.Tensor) -> torch.Tensor:
 
 
 def _prepacked_wins(m: int, n: int, k: int) -> bool:
-    """Measured (B200, graph of L2-cold calls): the fragment-order GEMV is flat in M and wins from M = 2 on at every
-    shape tried; at M = 1 it loses where N is small and K long (1536 x 8960: 8.2 against 5.3 us -- 96 CTAs of 18 K
-    blocks per warp) and is within 0.3 us elsewhere."""
+    """Where a weight with a private copy runs on it: from M = 2 on, and at M = 1 unless N is small and K long.  Measured
+    (B200, graph of L2-cold calls, us on the public format / on the copy at M = 1, 2, 8, 16, 32):
+        5632 x 2048   4.0 / 3.8   5.1 / 3.9   5.5 / 4.1    6.0 / 6.0   11.4 / 10.6
+        2560 x 2048   3.5 / 2.9   3.5 / 3.0   3.7 / 3.1    4.4 / 3.9    6.3 / 6.5
+       11264 x 2048   7.4 / 5.7   7.4 / 6.0   8.2 / 6.0   10.6 / 9.2   12.3 / 16.0
+        2048 x 5632   5.8 / 5.7   4.6 / 5.8   4.8 / 6.0    5.7 / 6.8    8.3 / 8.5
+        1536 x 8960   5.0 / 8.0   6.1 / 8.0   6.3 / 8.6    7.3 / 9.6   11.2 / 11.9
+    So the copy pays at K = 2048 up to 16 rows; at a longer K with few rows (96 to 128 CTAs, 11 to 18 blocks of K per warp)
+    and for many rows at M = 32 the public kernels have become the faster ones, and a weight of that kind is better left
+    without a copy."""
     return m >= 2 or n * 8 >= k * 5
 
 
@@ -345,8 +352,7 @@ def int4_matmul(x: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, gro
     The lines are in csrc/int4_linear.cu: the CUDA-core GEMV for one fp16 row and fewer than 8192 features, the small-batch
     kernel up to M = 16 and, where features x K and K allow, 32, streaming kernels for very many features, the tcgen05 GEMM
     otherwise.  FP32 accumulation in all of them.  bf16 activations (not in the reference, README.md:103) never take the
-    GEMV.  A weight with a private prepacked copy
-    (prepack_weight_) runs batches of up to PREPACKED_GEMV_MAX_M rows on it.
+    GEMV.  A weight with a private prepacked copy (prepack_weight_) runs batches of up to PREPACKED_GEMV_MAX_M rows on it.
     """
     y = _linear_launch(x, packed, scales, group_size, None) if isinstance(x, torch.Tensor) and x.dim() == 2 else None
     if y is not None:
