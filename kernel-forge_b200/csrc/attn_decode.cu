@@ -378,7 +378,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         own[kRows * D + kRows + r] = l_all;
       }
     } else if (direct) {
-      o[((size_t)b * H + h0 + r) * D + d] = pack1<kBf16>(l_all > 0.f ? acc / l_all : 0.f);  // no valid key: zeros
+      o[((size_t)b * H + h0 + r) * D + d] = pack1<kBf16>(l_all == 0.f ? 0.f : acc / l_all);  // no valid key: zeros; a score that is NaN or +infinity: NaN
     } else {
       out_partial[r * D + d] = acc;
       if (d == 0) {
@@ -412,7 +412,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       acc = fmaf(f, a[c], acc);
       l_all = fmaf(f, l[c], l_all);
     }
-    if (!aborted) o[((size_t)b * H + h0 + r) * D + d] = pack1<kBf16>(l_all > 0.f ? acc / l_all : 0.f);
+    if (!aborted) o[((size_t)b * H + h0 + r) * D + d] = pack1<kBf16>(l_all == 0.f ? 0.f : acc / l_all);
   }
   // no CTA leaves while another one still reads its sums
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -446,13 +446,11 @@ attn_decode_merge_kernel(const float* __restrict__ partial, uint16_t* __restrict
     const int t = i / splits, sp = i - t * splits;
     const float* ps = base_ptr + (size_t)t * set_stride + (size_t)sp * kPer;
     const float m_s = ps[kRows * D + r], l_s = ps[kRows * D + kRows + r], o_s = ps[r * D + d];
-    const float m_new = fmaxf(m_run, m_s);
-    if (m_new > -INFINITY) {
-      const float keep = ex2(m_run - m_new), f = ex2(m_s - m_new);   // ex2(-inf) = 0
-      acc = fmaf(f, o_s, acc * keep);
-      l_run = fmaf(f, l_s, l_run * keep);
-      m_run = m_new;
-    }
+    const float m_new = fmaxf(m_run, m_s), base = m_new == -INFINITY ? 0.f : m_new;
+    const float keep = ex2(m_run - base), f = ex2(m_s - base);   // ex2(-inf) = 0; a sum that is NaN stays in any case
+    acc = fmaf(f, o_s, acc * keep);
+    l_run = fmaf(f, l_s, l_run * keep);
+    m_run = m_new;
   }
   sm_m[j][d] = m_run; sm_a[j][d] = acc; sm_l[j][d] = l_run;
   __syncthreads();
@@ -460,16 +458,15 @@ attn_decode_merge_kernel(const float* __restrict__ partial, uint16_t* __restrict
     float m_all = -INFINITY;
 #pragma unroll
     for (int k = 0; k < kMergeLanes; ++k) m_all = fmaxf(m_all, sm_m[k][d]);
+    const float base = m_all == -INFINITY ? 0.f : m_all;
     float a = 0.f, l = 0.f;
-    if (m_all > -INFINITY) {
 #pragma unroll
-      for (int k = 0; k < kMergeLanes; ++k) {
-        const float f = ex2(sm_m[k][d] - m_all);
-        a = fmaf(f, sm_a[k][d], a);
-        l = fmaf(f, sm_l[k][d], l);
-      }
+    for (int k = 0; k < kMergeLanes; ++k) {
+      const float f = ex2(sm_m[k][d] - base);
+      a = fmaf(f, sm_a[k][d], a);
+      l = fmaf(f, sm_l[k][d], l);
     }
-    o[((size_t)b * H + h) * D + d] = pack1<kBf16>(l > 0.f ? a / l : 0.f);  // no valid key: zeros
+    o[((size_t)b * H + h) * D + d] = pack1<kBf16>(l == 0.f ? 0.f : a / l);  // no valid key: zeros; a score that is NaN or +infinity: NaN
   }
 }
 

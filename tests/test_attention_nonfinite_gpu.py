@@ -52,3 +52,38 @@ def test_score_of_plus_infinity_makes_its_row_nan(d, place):
     ref, bad = expected(q, k, v, True)
     assert bad.sum() == 1
     check(ops.flash_attn(q.cuda(), k.cuda(), v.cuda(), causal=True).float().cpu(), ref, bad, ATTN_ATOL[torch.bfloat16])
+
+
+# (sequences, heads, KV heads, keys): one CTA per group; clusters of splits; more than eight splits and the merge kernel
+DECODE = [(40, 8, 4, 300), (8, 32, 4, 2000), (1, 34, 2, 16384)]
+
+
+@pytest.mark.parametrize("score", ["nan", "inf", "all nan"])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("b,h,hk,nk", DECODE)
+def test_decode_makes_the_rows_that_see_it_nan(b, h, hk, nk, d, score):
+    q, k, v = qkv_case(b, h, hk, 1, nk, d, torch.bfloat16, seed=d)
+    lens = torch.full((b,), nk, dtype=torch.int32)
+    lens[-1] = nk - 70
+    k[-1, :, nk - 70:] = float("nan")          # not valid keys: nothing sees them
+    v[-1, :, nk - 70:] = float("nan")
+    valid = torch.arange(nk)[None, :] < lens[:, None]
+    clean = lambda t: torch.where(valid[:, None, :, None], t, torch.zeros((), dtype=t.dtype))
+    ref = torch.cat([torch.from_numpy(attn_oracle(q[i:i + 1], clean(k)[i:i + 1, :, :lens[i]], clean(v)[i:i + 1, :, :lens[i]], False)) for i in range(b)])
+    group = h // hk
+    bad = torch.zeros(b, h, 1, dtype=torch.bool)
+    if score == "inf":      # the product overflows FP32 for one head; the others of its group have no such feature
+        q[..., 0] = 0.0
+        k[:, :, :, 0] = 0.0
+        ref = torch.cat([torch.from_numpy(attn_oracle(q[i:i + 1], clean(k)[i:i + 1, :, :lens[i]], clean(v)[i:i + 1, :, :lens[i]], False)) for i in range(b)])
+        q[0, 1, 0, 0] = k[0, 1 // group, 77, 0] = 3e38
+        bad[0, 1] = True
+    else:                   # one key, or the first 64 keys: the first piece of the row then has no number at all
+        k[0, 0, 0 if score == "nan" else slice(0, nk // 16)] = float("nan")
+        bad[0, :group] = True
+    got = ops.flash_attn_decode(q.cuda(), k.cuda(), v.cuda(), lens.cuda()).float().cpu()
+    check(got, ref, bad, ATTN_ATOL[torch.bfloat16])
+    if b == 1:
+        return
+    none = ops.flash_attn_decode(q.cuda(), k.cuda(), v.cuda(), torch.zeros_like(lens).cuda())
+    assert not none.any()      # no valid key: zeros, whatever the cache holds
