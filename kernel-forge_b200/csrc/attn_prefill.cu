@@ -110,8 +110,8 @@ __device__ __forceinline__ TileOrder decode_tile_order(unsigned int block, int n
 //     load, maxima, P store and products.  Left alone the tiles fall into step and compete for the same unit;
 //   * head dim 64 computes some exponentials on the FMA pipe (exp_pair_fma), which is idle otherwise.
 // Measured (us per call through the public operator; the kernels before had event-loop issuers at head dim 64, one tile per CTA
-// and two passes over S at head dim 128): B=2 H=16 N=2048 D=64 62.6 -> 58.4 (588 TFLOP/s); N=8192 D=128 causal 632 -> 572
-// (961 TFLOP/s; 1083 in a burst too short for the power limit); 509 queries on 4093 keys, 12 heads over 2, D=128 60 -> 27.4.
+// and two passes over S at head dim 128): B=2 H=16 N=2048 D=64 62.6 -> 58.4 (588 TFLOP/s); N=8192 D=128 causal 632 -> 572..580
+// (950 TFLOP/s; 1083 in a burst too short for the power limit); 509 queries on 4093 keys, 12 heads over 2, D=128 60 -> 27.4.
 // Also measured at D=64, N=2048 (us in a graph; this kernel 56.4): scores of step j+1 loaded chunk by chunk under the
 // exponentials of step j 64; no baton 64; baton passed after all exponentials 66; polynomial for 4 of 16 pairs 58.6, for 5
 // 59.2.
