@@ -90,9 +90,9 @@ __device__ __forceinline__ TileOrder decode_tile_order(unsigned int block, int n
 //              descriptors are then uniform registers (inside `if (lane == 0)` every MMA costs ~95 clocks of moves into
 //              them); it sleeps in blocking waits, because polling takes issue slots from two of the softmax warps.
 // NT = 1: one tile, 192 threads (warps 0-3, 4, 5), half of the TMEM columns, two CTAs per SM: smaller pieces, for grids
-// that would leave SMs idle (plan_prefill).
-// TMEM (NT = 2: all 512 columns), head dim 64:  S_X [128 X, +128)   O_X [256 + 64 X, +64)   P_X [384 + 64 X, +64)
-//                          head dim 128: S_X [128 X, +128)   O_X [256 + 128 X, +128), P_X aliased on S_X [.., +64)
+// that would leave SMs idle (plan_prefill).  kDouble (head dim 128): one tile with the SM to itself and two buffers of scores.
+// TMEM: S_X [128 X, +128), then head dim 64: O_X [128 NT + 64 X, +64), P_X [192 NT + 64 X, +64);  head dim 128: P_X on the first
+// 64 columns of S_X, O_X [128 NT + 128 X, +128);  kDouble: S(j) [128 (j % 2), +128), P(j) on its first 64 columns, O [256, +128)
 // Both tiles read the same K/V tiles, so each is brought into shared memory once for 256 query rows.
 //
 // What a tile's rows are.  Two or more query tiles per head: 128 consecutive queries of one head, tiles A and B neighbours.
@@ -102,19 +102,27 @@ __device__ __forceinline__ TileOrder decode_tile_order(unsigned int block, int n
 // What bounds it: the exponentials (a 128 x 128 tile costs 1024 clocks of the SM's exponential units) and, at head dim
 // 128, equally the tensor pipe (1024 clocks per tile and step).  Either is reached only if a softmax warp never waits, so
 // its own chain -- scores, maximum, exponentials, P, PV, next QK -- is what counts:
-//   * a softmax thread loads the 128 scores of its row into registers in one go.  Head dim 64 then releases the S buffer,
-//     and QK(j+1) runs under step j; P has columns of its own;
+//   * exponentials do not wait for the maximum of their step: they are taken with the base of the steps before, while the
+//     maxima of the row run under them, and in the rare step whose maximum outgrows the base the first two of four chunks are
+//     taken again (the results are those of looking first).  Only the first step of a CTA looks first;
+//   * the scores are loaded in chunks of 32, one ahead.  Head dim 64 releases the S buffer after the last, and QK(j+1) runs
+//     under step j; P has columns of its own;
 //   * head dim 128: P(j) overwrites half of S(j), so QK(j+1) can only follow PV(j).  P is handed over in two halves, and
-//     PV starts on the first 64 keys while the exponentials of the others run;
-//   * the two tiles take turns on the exponential units (a "baton"): one tile's exponentials run under the other's score
-//     load, maxima, P store and products.  Left alone the tiles fall into step and compete for the same unit;
+//     PV starts on the first 64 keys while the exponentials of the others run.  With two buffers (kDouble) QK(j+1) is
+//     complete before step j ends and the softmax warps never wait for a product;
+//   * two tiles of a CTA take turns on the exponential units (a "baton"): one tile's exponentials run under the other's score
+//     load, P store and products.  Left alone the tiles fall into step and compete for the same unit;
 //   * head dim 64 computes some exponentials on the FMA pipe (exp_pair_fma), which is idle otherwise.
-// Measured (us per call through the public operator; the kernels before had event-loop issuers at head dim 64, one tile per CTA
-// and two passes over S at head dim 128): B=2 H=16 N=2048 D=64 62.6 -> 58.4 (588 TFLOP/s); N=8192 D=128 causal 632 -> 572..580
-// (950 TFLOP/s; 1083 in a burst too short for the power limit); 509 queries on 4093 keys, 12 heads over 2, D=128 60 -> 27.4.
-// Also measured at D=64, N=2048 (us in a graph; this kernel 56.4): scores of step j+1 loaded chunk by chunk under the
-// exponentials of step j 64; no baton 64; baton passed after all exponentials 66; polynomial for 4 of 16 pairs 58.6, for 5
-// 59.2.
+// What is left (clocks of one step of 128 keys, stamps of the clock in a copy of the kernel, two tiles at head dim 128): 3200 for
+// the pair of tiles, each 1200 from its last P to its next scores and 1640 of exponentials (1024 at the unit's rate; a single
+// warp per scheduler reaches 86 % of it), which overlap with the other tile's.
+// Measured (us in a graph, before -> after the exponentials stopped waiting, one-tile CTAs with an SM to themselves got two
+// buffers and head dim 64 one-tile CTAs wherever keys are not split): B=2 H=16 N=2048 D=64 58.0 -> 53.9, N=8192 701 -> 651; 32 x 32 heads
+// x 200 tokens D=64 causal 50.6 -> 45.3; N=2048 D=128 75.4 -> 69.8; N=8192 D=128 causal 495 -> 471 (577 -> 549 back to back at the
+// power limit's clock); 1 x 16 x 2048 D=128 causal 34.0 -> 29.5; 509 queries on 4093 keys, 12 heads over 2, D=128 26.5 -> 23.5.
+// Also measured: D=64, N=2048, two tiles per CTA 56.8, without baton 58.1; two pairs of 16 by polynomial 56.7, four 57.2; the last
+// chunk of scores read twice, to save registers, 55.3; the first step on the path that takes exponentials again (registers spill) 73.  D=128, N=2048 (70.0): no baton 86.7, baton after two chunks 83.7, after
+// four 75.1; one polynomial pair in 16 73.7; P handed over in three pieces 70.6.
 //
 // Split over keys: a problem with few tiles (short chunks against a long cache) is cut along the keys too; a CTA then
 // writes its unnormalised O and (m, l) per row and attn_prefill_merge_kernel puts the pieces together in order.
@@ -123,14 +131,15 @@ namespace tiles {
 
 constexpr int kPolyPairs = 3;       // head dim 64: of 16 pairs of scores, this many take exp_pair_fma
 
-template <int D, int NT>
+template <int D, int NT, bool kDouble>
 struct TileLayout {
   static constexpr int kProducerWarp = 4 * NT, kMmaWarp = 4 * NT + 1;   // (then one issuer warp per tile)
   static constexpr int kThreads = NT == 2 ? 384 : 192;
-  static constexpr uint32_t kTmemCols = 256u * NT;
+  static constexpr uint32_t kTmemCols = kDouble ? 512u : 256u * NT;
   static constexpr bool kAliasP = D == 128;
   static constexpr int kHalves = kAliasP ? 2 : 1;     // pieces in which P is handed to the tensor cores
-  static constexpr int kStages = (D == 64 ? 2 : 1) * NT;
+  static constexpr int kScores = kDouble ? 2 : 1;     // buffers of scores
+  static constexpr int kStages = kDouble ? 2 : D == 64 ? 2 * NT : NT;
   static constexpr int kTile = kBlockN * D * 2;       // bytes of one 128-row tile (Q, K or V)
   static constexpr int kQ = 0;                        // Q_A, Q_B
   static constexpr int kK = NT * kTile;
@@ -140,11 +149,12 @@ struct TileLayout {
   static constexpr int kMisc = kBars + kNumBars * 8;
   static constexpr int kBytes = kMisc + 16;
   static constexpr int kAlloc = kBytes + 1024;        // room to align the tiles to 1024 bytes
-  static constexpr int kAllocAlone = 116 * 1024;      // more than half of what an SM has
-  static_assert((NT == 1 ? 2 : 1) * kAlloc <= 227 * 1024, "two one-tile CTAs, or a two-tile CTA, must fit on an SM");
-  static_assert(NT == 1 || 2 * kAlloc > 228 * 1024, "one two-tile CTA per SM: it allocates all 512 TMEM columns");
-  static constexpr uint32_t kColS = 0;                              // + 128 X
-  static constexpr uint32_t kColO = 128 * NT;                       // + D X
+  static constexpr int kAllocAlone = kDouble ? kAlloc : 116 * 1024;   // more than half of what an SM has
+  static_assert(!kDouble || (NT == 1 && kAliasP), "for a tile whose P lies on its scores; two tiles leave no room in TMEM");
+  static_assert((NT == 1 && !kDouble ? 2 : 1) * kAlloc <= 227 * 1024, "two one-tile CTAs, or a two-tile CTA, must fit on an SM");
+  static_assert((NT == 1 && !kDouble) || 2 * kAlloc > 228 * 1024, "one CTA per SM where it allocates all 512 TMEM columns");
+  static constexpr uint32_t kColS = 0;                              // + 128 X (+ 128 for the second buffer)
+  static constexpr uint32_t kColO = 128 * NT * kScores;             // + D X
   static constexpr uint32_t kColP = kAliasP ? 0u : 192u * NT;       // + (kAliasP ? 128 : 64) X
   static constexpr uint32_t kStrideP = kAliasP ? 128u : 64u;
 };
@@ -210,14 +220,16 @@ __device__ __forceinline__ uint32_t exp_pair_fma(uint32_t v0, uint32_t v1, float
   return pack2<kBf16>(y.x, y.y);
 }
 
-template <int D, bool kBf16, int NT>
-__global__ void __launch_bounds__(TileLayout<D, NT>::kThreads, NT == 2 ? 1 : 2)
+template <int D, bool kBf16, int NT, bool kDouble>
+__global__ void __launch_bounds__(TileLayout<D, NT, kDouble>::kThreads, NT == 2 || kDouble ? 1 : 2)
 attn_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                          const __grid_constant__ CUtensorMap tm_v, void* __restrict__ o_ptr, const Strides o_st,
                          const __grid_constant__ Params pr, unsigned int* status) {
-  using L = TileLayout<D, NT>;
+  using L = TileLayout<D, NT, kDouble>;
   constexpr int S = L::kStages, kHalves = L::kHalves;
   constexpr bool kAliasP = L::kAliasP;
+  constexpr bool kBaton = NT == 2;               // the two tiles take turns
+  constexpr int kBatonAfter = kAliasP ? 2 : 1;   // the chunk after which the other tile may start
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBars);
@@ -345,46 +357,50 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       const uint32_t s_col = tmem_base + L::kColS + 128u * X, o_col = tmem_base + L::kColO + (uint32_t)D * X;
       const uint32_t p_col = tmem_base + L::kColP + L::kStrideP * X;
       const int n = n_of(X);
+      constexpr int kAhead = kDouble ? 2 : 1;   // steps by which the scores of an aliased P are ahead of its products
       bool ok = true;
       auto wait_for = [&](uint64_t* bar, uint32_t parity, uint32_t code) {
         ok = ok && __all_sync(0xffffffffu, mbar_wait(bar, parity, ctx, code));
         return ok;
       };
       // S(j) = Q K(j)^T
-      auto qk = [&](int j) {
-        const int s = j % S;
-        if (!wait_for(&k_full[s], (uint32_t)(j / S) & 1u, kWaitKFull)) return;
+      auto await_k = [&](int j) { return wait_for(&k_full[j % S], (uint32_t)(j / S) & 1u, kWaitKFull); };
+      auto qk = [&](int j) {   // K(j) has been awaited
+        const int s = j % S, buf = kDouble ? j & 1 : 0;
         tc_fence_after_sync();
         const uint64_t kd = k_desc + (uint64_t)(s * (L::kTile >> 4));
-        if (elect_one()) {
+        if (ok && elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
             const uint64_t off = (uint64_t)(((kk / 4) * kHalfBytes + (kk % 4) * 32) >> 4);
-            mma_ss(s_col, q_desc + off, kd + off, idesc_qk, kk > 0 ? 1u : 0u);
+            mma_ss(s_col + 128u * buf, q_desc + off, kd + off, idesc_qk, kk > 0 ? 1u : 0u);
           }
-          tc_commit(&s_full[X]);
+          tc_commit(&s_full[kDouble ? buf : X]);
         }
         __syncwarp();
       };
       // O += P(j) V(j), in kHalves pieces of the 128 keys
       auto pv = [&](int j) {
         const int s = j % S;
+        const uint32_t p_at = p_col + (kDouble ? 128u * (j & 1) : 0u);
         constexpr int kPer = kBlockN / 16 / kHalves;
         if (!wait_for(&v_full[s], (uint32_t)(j / S) & 1u, kWaitVFull)) return;
         const uint64_t vd = v_desc + (uint64_t)(s * (L::kTile >> 4));
 #pragma unroll
         for (int half = 0; half < kHalves; ++half) {
-          if (!wait_for(&p_ready[2 * X + half], (uint32_t)j & 1u, kWaitPReady)) return;
+          // (the next product follows at once: its keys are awaited before the last piece of P)
+          if (half + 1 == kHalves && kAliasP && j + kAhead < n && !await_k(j + kAhead)) return;
+          if (!wait_for(&p_ready[2 * (kDouble ? j & 1 : X) + half], (uint32_t)(kDouble ? j >> 1 : j) & 1u, kWaitPReady)) return;
           tc_fence_after_sync();
           if (elect_one()) {
 #pragma unroll
             for (int kk = 0; kk < kPer; ++kk) {
               // 16 keys per MMA: 16 rows of 128 bytes; the second 64-column block of V is kHalfBytes away
               const int k = half * kPer + kk;
-              mma_ts(o_col, p_col + (uint32_t)k * 8u, vd + (uint64_t)(k * (2048 >> 4)), idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
+              mma_ts(o_col, p_at + (uint32_t)k * 8u, vd + (uint64_t)(k * (2048 >> 4)), idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
             }
-            // (aliased P: S(j + 1) complete implies PV(j) complete, so only the last step needs a commit of its own)
-            if (half + 1 == kHalves && (!kAliasP || j + 1 == n)) tc_commit(&pv_done[X]);
+            // (aliased P, one buffer: S(j + 1) complete implies PV(j) complete, so only the last step needs a commit of its own)
+            if (half + 1 == kHalves && (!kAliasP || kDouble || j + 1 == n)) tc_commit(&pv_done[X]);
           }
           __syncwarp();
         }
@@ -396,11 +412,14 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       // A commit keeps the issuing thread for some 50-130 clocks, so the ones that only return a stage come last.
       if (n > 0) {
         wait_for(q_full, 0, kWaitQ);
-        qk(0);
-        release(&k_empty[0]);
+        for (int j = 0; j < kAhead && j < n; ++j) {
+          if (await_k(j)) qk(j);
+          release(&k_empty[j % S]);
+        }
         for (int j = 0; ok && j < n; ++j) {
-          const int next = j + 1;
+          const int next = j + kAhead;
           if (!kAliasP && next < n) {   // S(j + 1) as soon as the scores of step j are in registers
+            await_k(next);
             wait_for(&s_free[X], (uint32_t)j & 1u, kWaitSFull);
             qk(next);
           }
@@ -443,66 +462,57 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       return ok;
     };
     auto wait_turn = [&](int i) { return wait_all(&turn[X], (X == 1 ? (uint32_t)i : (uint32_t)i + 1u) & 1u, kWaitTurn); };
+    // With two buffers of scores those of the next step are there before this one ends: their first chunk of 32 is requested
+    // then.  (Head dim 64, whose next product has only been started in the middle of the step, two tiles: 62.0 us with that, 57.0
+    // without.)
+    constexpr bool kPrefetch = kDouble;
+    uint32_t v[4][32];         // the 128 scores of this row
+    auto await_scores = [&](int i) {
+      if (!wait_all(&s_full[kDouble ? i & 1 : X], (uint32_t)(kDouble ? i >> 1 : i) & 1u, kWaitSFull)) return false;
+      tc_fence_after_sync();
+      return true;
+    };
+    auto fetch = [&](int i, int c) { tmem_ld_x32(s_tmem + (kDouble ? 128u * (i & 1) : 0u) + c * 32, v[c]); };
+    if (kPrefetch && n > 0 && await_scores(0)) fetch(0, 0);
     for (int i = 0; ok && i < n; ++i) {
       const uint32_t ph = (uint32_t)i & 1u;
-      if (!wait_all(&s_full[X], ph, kWaitSFull)) break;
-      tc_fence_after_sync();
-      uint32_t v[4][32];         // the 128 scores of this row
+      const uint32_t p_at = p_tmem + (kDouble ? 128u * (i & 1) : 0u);
       float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
       const int k0 = (j0 + i) * kBlockN;
       const bool masked = k0 + kBlockN - 1 > tile_limit;
-      auto fetch = [&](int c) { tmem_ld_x32(s_tmem + c * 32, v[c]); };
-      auto scan = [&](int c) {
+      auto mask = [&](int c) {
         if (masked) mask32(v[c], c * 32, row_limit - k0);
-        max32(v[c], mx);
       };
-      fetch(0);
-      fetch(1);
+      if (!kPrefetch) {
+        if (!await_scores(i)) break;
+        fetch(i, 0);
+      }
       tmem_wait_ld_regs(v[0]);
-      tmem_wait_ld_regs(v[1]);
-      fetch(2);
-      fetch(3);
-      scan(0);
-      scan(1);
-      tmem_wait_ld_regs(v[2]);
-      tmem_wait_ld_regs(v[3]);
-      if constexpr (!kAliasP && NT == 2) {   // the S buffer can take the next product already
-        tc_fence_before_sync();
-        mbar_arrive(&s_free[X]);
-      }
-      scan(2);
-      scan(3);
-      const float m_step = max_of(mx) * pr.scale_log2;
-      // lazy rescale: move the base only when the maximum outgrew it by more than the threshold
-      const bool grow = m_step > m_base + kRescaleThreshold;   // (-inf + 8 = -inf: the first finite maximum counts)
-      const float alpha = grow ? ex2(m_base - m_step) : 1.0f;  // 0 when m_base is still -inf
-      m_base = grow ? m_step : m_base;
-      const float base = (m_base == -INFINITY) ? 0.f : m_base;
-      bool pv_waited = kAliasP || i == 0;   // (with aliased P, S(j) complete implies PV(j-1) complete)
-      if (i > 0 && __any_sync(0xffffffffu, grow)) {
-        // O is rescaled between PV(j-1), which must have finished accumulating, and PV(j), which cannot have
-        // started (it waits for this step's P).  Rare after the first steps.
-        if (!pv_waited && !wait_all(&pv_done[X], ph ^ 1u, kWaitPvDone)) break;
-        pv_waited = true;
-        tc_fence_after_sync();
+      fetch(i, 1);
+      fetch(i, 2);
+      fetch(i, 3);
+      mask(0);
+      if (i == 0) {   // the first step has no base to guess with
+        tmem_wait_ld_regs(v[1]);
+        tmem_wait_ld_regs(v[2]);
+        tmem_wait_ld_regs(v[3]);
 #pragma unroll
-        for (int c = 0; c < D / 32; ++c) {
-          uint32_t o[32];
-          tmem_ld_x32(o_tmem + c * 32, o);
-          tmem_wait_ld();
-#pragma unroll
-          for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
-          tmem_st_x32(o_tmem + c * 32, o);
+        for (int c = 0; c < 4; ++c) {
+          if (c > 0) mask(c);
+          max32(v[c], mx);
         }
+        m_base = max_of(mx) * pr.scale_log2;
       }
-      if (NT == 2 && (X == 1 || i > 0) && !wait_turn(i)) break;
-      const float2 nb2 = make_float2(-base, -base);
+      float base = (m_base == -INFINITY) ? 0.f : m_base;
+      if (kBaton && (X == 1 || i > 0) && !wait_turn(i)) break;
+      float2 nb2 = make_float2(-base, -base);
       float2 sum[2] = {{0.f, 0.f}, {0.f, 0.f}};
       uint32_t p[4][16];
       auto expo = [&](int c, int e) {
         if (!kAliasP && e < kPolyPairs) p[c][e] = exp_pair_fma<kBf16>(v[c][2 * e], v[c][2 * e + 1], sc2, nb2, sum[e & 1]);
         else p[c][e] = exp_pair<kBf16>(v[c][2 * e], v[c][2 * e + 1], sc2, nb2, sum[e & 1]);
       };
+      auto seen = [&](int c, int e) { mx[e & 3] = max3(mx[e & 3], __uint_as_float(v[c][2 * e]), __uint_as_float(v[c][2 * e + 1])); };
       auto chunk = [&](int c) {   // (the order spreads the polynomials among the others)
 #pragma unroll
         for (int e = 0; e < 16; ++e) expo(c, (e * 5) & 15);
@@ -510,48 +520,113 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       auto pass_baton = [&]() {   // (the operands keep the exponentials summed so far in front of it)
         asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0]; // %1 %2" ::"r"(smem_u32(&turn[X ^ 1])), "f"(sum[0].x), "f"(sum[1].x) : "memory");
       };
-      chunk(0);
-      // One-tile CTAs have 168 registers a thread: the last chunk is read once more instead of being kept.
-      if constexpr (NT == 1) fetch(3);
-      chunk(1);
-      if (NT == 2 && !kAliasP) pass_baton();
-      if constexpr (kHalves == 2) {
-        tmem_st_x16(p_tmem, p[0]);
-        tmem_st_x16(p_tmem + 16, p[1]);
+      // The maxima run under the exponentials of the first two chunks, which are taken with the base of the steps before: it
+      // only moves when a maximum outgrows it by more than the threshold, and then they are taken again.
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        expo(0, (e * 5) & 15);
+        seen(0, e);
+      }
+      tmem_wait_ld_regs(v[1]);
+      tmem_wait_ld_regs(v[2]);
+      tmem_wait_ld_regs(v[3]);
+      if (i > 0) {
+        mask(1);
+        mask(2);
+        mask(3);
+      }
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        expo(1, (e * 5) & 15);
+        seen(1, e);
+        seen(2, e);
+        seen(3, e);
+      }
+      const float m_step = max_of(mx) * pr.scale_log2;
+      // lazy rescale: move the base only when the maximum outgrew it by more than the threshold
+      const bool grow = m_step > m_base + kRescaleThreshold;   // (-inf + 8 = -inf: the first finite maximum counts)
+      float alpha = 1.0f;
+      // PV(j-1) must have finished accumulating before O is rescaled, and reading before P is overwritten.  (One buffer with
+      // aliased P: S(j) complete implies PV(j-1) complete.)
+      bool pv_waited = (kAliasP && !kDouble) || i == 0;
+      auto wait_pv = [&]() {
+        if (!pv_waited) {
+          if (!wait_all(&pv_done[X], ph ^ 1u, kWaitPvDone)) return false;
+          pv_waited = true;
+        }
+        tc_fence_after_sync();
+        return true;
+      };
+      if (__any_sync(0xffffffffu, grow)) {   // (not in the first step)
+        // O is rescaled between PV(j-1) and PV(j), which cannot have started (it waits for this step's P).  Rare after the
+        // first steps.
+        if (grow) {
+          alpha = ex2(m_base - m_step);  // 0 when m_base is still -inf
+          m_base = m_step;
+        }
+        if (!wait_pv()) break;
+#pragma unroll 1
+        for (int c = 0; c < D / 32; ++c) {
+          uint32_t o[32];
+          tmem_ld_x32(o_tmem + c * 32, o);
+          tmem_wait_ld_regs(o);
+#pragma unroll
+          for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
+          tmem_st_x32(o_tmem + c * 32, o);
+        }
+        base = (m_base == -INFINITY) ? 0.f : m_base;
+        nb2 = make_float2(-base, -base);
+        sum[0] = sum[1] = make_float2(0.f, 0.f);
+        fetch(i, 0);
+        fetch(i, 1);
+        tmem_wait_ld_regs(v[0]);
+        tmem_wait_ld_regs(v[1]);
+        mask(0);
+        mask(1);
+        chunk(0);
+        chunk(1);
+      }
+      if constexpr (!kAliasP) {   // the S buffer can take the next product already
+        tc_fence_before_sync();
+        mbar_arrive(&s_free[X]);
+      }
+      // (two buffers of scores: only so that the wait after the last step is for one phase)
+      if (kDouble && i + 1 == n && !wait_pv()) break;
+      if constexpr (kAliasP) {
+        tmem_st_x16(p_at, p[0]);
+        tmem_st_x16(p_at + 16, p[1]);
         tmem_wait_st();
         tc_fence_before_sync();
-        mbar_arrive(&p_ready[2 * X]);
+        mbar_arrive(&p_ready[2 * (kDouble ? i & 1 : X)]);
       }
+      if (kBaton && kBatonAfter == 1) pass_baton();
       chunk(2);
-      if (NT == 2 && kAliasP) pass_baton();
-      if constexpr (NT == 1) {
-        tmem_wait_ld_regs(v[3]);
-        if (masked) mask32(v[3], 96, row_limit - k0);
-        if constexpr (!kAliasP) {
-          tc_fence_before_sync();
-          mbar_arrive(&s_free[X]);
-        }
-      }
+      if constexpr (kAliasP) tmem_st_x16(p_at + 32, p[2]);
+      if (kBaton && kBatonAfter == 2) pass_baton();
       chunk(3);
+      if constexpr (kAliasP) tmem_st_x16(p_at + 48, p[3]);
       const float2 t = __fadd2_rn(sum[0], sum[1]);
       // A score that is NaN or +infinity makes its row NaN, whichever way its exponential was taken.
       l_run = m_step < INFINITY ? fmaf(l_run, alpha, t.x + t.y) : __int_as_float(0x7FFFFFFF);
-      if (!pv_waited) {   // PV(j-1) must have finished reading the P columns before they are overwritten: by now it has
-        if (!wait_all(&pv_done[X], ph ^ 1u, kWaitPvDone)) break;
-        tc_fence_after_sync();
-      }
+      if constexpr (!kAliasP) {   // (each chunk stored on its own, as above, is slower here: 61.5 us at 2 x 16 x 2048)
+        if (!wait_pv()) break;
 #pragma unroll
-      for (int c = kHalves == 2 ? 2 : 0; c < 4; ++c) tmem_st_x16(p_tmem + 16 * c, p[c]);
+        for (int c = 0; c < 4; ++c) tmem_st_x16(p_at + 16 * c, p[c]);
+      }
       tmem_wait_st();
       tc_fence_before_sync();
-      mbar_arrive(&p_ready[2 * X + kHalves - 1]);
+      mbar_arrive(&p_ready[2 * (kDouble ? i & 1 : X) + kHalves - 1]);
+      if (kPrefetch && i + 1 < n) {
+        if (!await_scores(i + 1)) break;
+        fetch(i + 1, 0);
+      }
     }
-    for (int i = n; NT == 2 && ok && i < n_max; ++i) {   // steps that only the other tile has: pass the baton on
+    for (int i = n; kBaton && ok && i < n_max; ++i) {   // steps that only the other tile has: pass the baton on
       if ((X == 1 || i > 0) && !wait_turn(i)) break;
       mbar_arrive(&turn[X ^ 1]);
     }
     // PVs complete in issue order: the last one done means all are
-    if (ok && n > 0) wait_all(&pv_done[X], kAliasP ? 0u : (uint32_t)(n - 1) & 1u, kWaitPvDone);
+    if (ok && n > 0) wait_all(&pv_done[X], kAliasP && !kDouble ? 0u : (uint32_t)(n - 1) & 1u, kWaitPvDone);
     if (ok) {
       tc_fence_after_sync();
       const long long grow_row = ((long long)b * H + head) * Nq + query;   // row of the dense [B H Nq] order of the partials
@@ -651,27 +726,28 @@ PrefillPlan plan_prefill(const Problem& p, int max_splits = 32) {
     c.tiles = G / c.heads_per_tile;
     c.units = p.B * p.Hk;
   }
-  // Tiles per CTA, CTAs per SM and key splits, by a cost model in us fitted to 1194 shapes, 3650 measured plans in graphs on
-  // B200 (mean deviation 5 %): a CTA takes `step` per 128 keys and `fixed` for set-up and drain; the merge kernel 2.7, 0.2 per
-  // split and its traffic at 5.1 TB/s.  So a grid smaller than the GPU takes one tile per CTA and splits the keys (1 x 8 x 1024
-  // queries, D = 128: 17.4 us, two tiles 18.7), long ones share K / V between two tiles (2 x 16 x 8192 D = 128 causal: 514
-  // against 542; bursts too short for the power limit).
+  // Tiles per CTA, CTAs per SM and key splits, by a cost model in us fitted to 700 shapes, 4713 measured plans in graphs on
+  // B200 (mean deviation 4 % at head dim 64, 9 % at 128; the plan it picks is on average 0.5 % slower than the best one measured,
+  // before the fit to these kernels 4 %): a CTA takes `step` per 128 keys and `fixed` for set-up and drain; the merge kernel
+  // 2.4 or 3.2, 0.2 or 0.3 per split and its traffic at 5.1 TB/s.  So a grid smaller than the GPU takes one tile per CTA and may
+  // split the keys (1 x 12 heads x 509 queries, 4093 keys, D = 128: three splits 23.5 us, two tiles per CTA in six 26.2), long
+  // ones share K / V between two tiles (2 x 16 x 2048 D = 128: 70.6 against 75.6 for one in pairs, 101 for one apart).
   // One-tile CTAs fit in pairs on an SM, and the hardware does pair them while other SMs stay idle.  Where the grid has at
   // most one for each SM, and under a causal mask also for longer grids, where short CTAs even out what is left over, they are
-  // kept apart (by the shared memory they ask for): 1 x 8 x 1024, two splits 21.2 -> 17.0; 1 x 16 x 2048 causal 39.2 -> 35.2.
-  // CTAs of one or two steps gain nothing from it (1 x 2 queries, 4002 keys, 32 splits: 13.8 us apart, 11.6 in pairs).
+  // kept apart: at D = 128 with the TMEM of the whole SM (1 x 16 x 2048 causal: in pairs 35.9, apart 29.5), at D = 64, where
+  // that gains nothing, by the shared memory they ask for (1 x 4 heads x 7: in pairs 4.5, apart 4.1).
   struct Kind {
     int per_cta;
     bool alone;
     double step, fixed, wave, tail;   // wave: `fixed` where CTAs follow one another on an SM; tail: share of the longest CTA that
   };                                  // a causal grid of more CTAs than slots ends with
   const bool wide = p.D == 128;
-  const Kind kinds[3] = {{1, false, wide ? 2.15 : 1.72, wide ? 5.7 : 5.25, wide ? 5.25 : 3.75, 0.30},
-                         {1, true, wide ? 1.71 : 1.30, wide ? 4.1 : 3.6, wide ? 5.6 : 3.4, wide ? 0.09 : 0.18},
-                         {2, false, wide ? 2.00 : 1.51, wide ? 5.6 : 4.8, wide ? 5.75 : 4.6, 0.27}};
+  const Kind kinds[3] = {{1, false, wide ? 2.06 : 1.44, wide ? 4.5 : 3.8, wide ? 6.5 : 4.6, wide ? 0.24 : 0.17},
+                         {1, true, wide ? 1.33 : 0.97, wide ? 3.7 : 3.6, wide ? 4.0 : 3.9, wide ? 0.24 : 0.33},
+                         {2, false, wide ? 1.80 : 1.46, wide ? 3.9 : 3.3, wide ? 4.7 : 4.4, wide ? 0.39 : 0.20}};
   const int steps = ceil_div(p.Nk, kBlockN), hidden = ceil_div(p.Nk - p.Nq, kBlockN);   // hidden: steps that every causal tile has
   const bool uneven = p.causal && !c.heads_per_tile && p.Nq > p.Nk / 2;   // CTAs of all lengths, longest first
-  const double merge_us = (double)p.B * p.H * p.Nq * p.D * 8.0 / 5.1e6 + 0.2;
+  const double merge_us = (double)p.B * p.H * p.Nq * p.D * 8.0 / 5.1e6 + (wide ? 0.30 : 0.22);
   double best = 1e30;
   c.per_cta = 1;
   c.splits = 1;
@@ -684,7 +760,10 @@ PrefillPlan plan_prefill(const Problem& p, int max_splits = 32) {
       const long long ctas = (long long)c.units * per_unit * s;
       if (s > 1 && ctas > 2 * sms) break;
       if (k.per_cta == 1 && !k.alone && ctas <= sms) continue;
-      if (k.alone && ctas > sms && (s > 1 || longest < 8)) continue;
+      if (k.alone && ctas > sms && (wide ? longest < 6 : s > 1 || longest < 8)) continue;
+      // Two tiles per CTA: not for short CTAs (D = 128, 320 of at most four steps: 37.2 us, in pairs of one tile 34.1), and at D = 64
+      // only where the keys are split (2 x 16 x 8192: 694 us, one tile 664; 4 heads x 5806 causal: two splits 45.0, one tile 50.6)
+      if (k.per_cta == 2 && (longest < 5 || (!wide && s == 1))) continue;
       const long long slots = k.per_cta == 2 || k.alone ? sms : 2 * sms;
       const double one = longest * k.step + k.fixed;
       double cost = one;
@@ -697,17 +776,17 @@ PrefillPlan plan_prefill(const Problem& p, int max_splits = 32) {
         const Kind& left = slots > sms && last <= sms ? kinds[1] : k;
         cost = (double)(ctas / slots) * (longest * k.step + k.wave) + (last ? longest * left.step + left.wave : 0.0);
       }
-      if (s > 1) cost += 2.7 + s * merge_us;
-      if (cost < best) { best = cost; c.per_cta = k.per_cta; c.splits = s; c.alone = k.alone && longest >= 3; }
+      if (s > 1) cost += (wide ? 3.2 : 2.4) + s * merge_us;
+      if (cost < best) { best = cost; c.per_cta = k.per_cta; c.splits = s; c.alone = k.alone; }
     }
   return c;
 }
 
-template <int D, bool kBf16, int NT>
+template <int D, bool kBf16, int NT, bool kDouble>
 int launch_tiles(const Problem& p, const PrefillPlan& plan, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, float* partial,
                  unsigned int* status, cudaStream_t stream) {
-  using L = tiles::TileLayout<D, NT>;
-  auto kernel = tiles::attn_prefill_kernel<D, kBf16, NT>;
+  using L = tiles::TileLayout<D, NT, kDouble>;
+  auto kernel = tiles::attn_prefill_kernel<D, kBf16, NT, kDouble>;
   static bool configured[64] = {false};
   int dev = 0;
   KFB_CUDA_TRY(cudaGetDevice(&dev));
@@ -735,8 +814,11 @@ int launch_tiles(const Problem& p, const PrefillPlan& plan, const CUtensorMap& t
 template <int D, bool kBf16>
 int launch(const Problem& p, const PrefillPlan& plan, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, float* partial,
            unsigned int* status, cudaStream_t stream) {
-  return plan.per_cta == 2 ? launch_tiles<D, kBf16, 2>(p, plan, tq, tk, tv, partial, status, stream)
-                           : launch_tiles<D, kBf16, 1>(p, plan, tq, tk, tv, partial, status, stream);
+  if (plan.per_cta == 2) return launch_tiles<D, kBf16, 2, false>(p, plan, tq, tk, tv, partial, status, stream);
+  if constexpr (D == 128) {
+    if (plan.alone) return launch_tiles<D, kBf16, 1, true>(p, plan, tq, tk, tv, partial, status, stream);
+  }
+  return launch_tiles<D, kBf16, 1, false>(p, plan, tq, tk, tv, partial, status, stream);
 }
 
 size_t partial_bytes(const Problem& p, const PrefillPlan& plan) {
