@@ -327,6 +327,14 @@ int kfb_flash_attn_decode_kvlen(const void* q, const void* k, const void* v, voi
                                 const int64_t* kv_strides, const int32_t* kv_len_dev,
                                 void* ws, size_t ws_bytes, void* stream);
 
+/* The same inside a decode step, with one more promise by the caller: the kernel in front of this launch in the stream wrote q and at
+ * most ONE row of each sequence's cache, the last valid one; kv_len_dev and all other valid rows are older.  The launch may then read
+ * those before that kernel has finished (it carries the attribute described at kfb_set_programmatic_launch). */
+int kfb_flash_attn_decode_step(const void* q, const void* k, const void* v, void* o, int dtype,
+                               int B, int H, int Hk, int Nk, int D, float scale,
+                               const int64_t* kv_strides, const int32_t* kv_len_dev,
+                               void* ws, size_t ws_bytes, void* stream);
+
 /* Decode attention over a KV cache that is SHARDED ALONG THE SEQUENCE (one shard per GPU for a single long sequence,
  * or any other split the caller makes).  The reference is single-GPU; these entries have no counterpart there.
  *   kfb_flash_attn_decode_partial: runs the split-KV kernel on one shard (k, v: [B, Hk, Nk, D] of this shard, kv_len_dev

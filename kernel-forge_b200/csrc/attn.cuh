@@ -21,6 +21,8 @@ struct Problem {
   long long o_stride_b = 0, o_stride_h = 0, o_stride_n = 0;
   // decode only: device array of B valid lengths (<= Nk, the capacity of the cache); nullptr = all Nk keys
   const int* kv_len_dev = nullptr;
+  // decode only: kv_len_dev and all valid rows but the last are older than the kernel in front (kfb_flash_attn_decode_step)
+  bool old_rows = false;
 };
 
 // Prefill / general path: tiles of 128 query rows, TMA + tcgen05 + TMEM (attn_prefill.cu).  The workspace is optional: a

@@ -18,6 +18,9 @@
 //   * per-warp online softmax (base 2, FP32), warps merged in shared memory in fixed order.  Up to
 //     eight splits form a thread-block cluster and are merged through distributed shared memory, in
 //     split order, every CTA a share of the output: one launch, nothing goes through global memory.
+//     Each CTA sends its sums to the CTA that needs them, so one cluster barrier is enough and no load
+//     crosses the cluster (reading them from one another took two barriers and a round trip: 4 sequences
+//     of 800..1100 keys 5.7 us, now 4.8; 8 of 1000..4096 8.4 and 7.9).
 //     More splits write one partial (O, m, l) each to the caller's workspace, combined in split order
 //     by a second small kernel.  Both are deterministic; with one split the result is written directly.
 #include "attn.cuh"
@@ -38,6 +41,7 @@ template <int D> constexpr int shallow_stages() { return D == 64 ? 4 : 3; }
 template <int D> constexpr int deep_stages() { return D == 64 ? 12 : 6; }
 template <int D, int kStages> constexpr int consumer_warps() { return kStages == shallow_stages<D>() ? kStages : 6; }
 constexpr int kRows = 16;  // query heads per CTA (MMA M)
+constexpr int kMaxCluster = 8;
 
 enum WaitCode : uint32_t { kWaitFull = 0x201, kWaitEmpty };
 
@@ -53,10 +57,14 @@ struct Layout {
   static constexpr int kStage = 2 * kTile;            // K then V
   static constexpr int kBars = kStages * kStage;
   static constexpr int kMisc = kBars + 2 * kStages * 8;
-  static constexpr int kBytes = kMisc + 16;
-  static constexpr int kAlloc = kBytes + 1024;
+  // what the CTAs of a cluster send this one, outside the ring, which may still be in use then: its share of the output from each
+  // (shares are multiples of four elements), then m[16] and l[16] of each
+  static constexpr int kSent = kMisc + 16;
+  static constexpr int kSentStats = kRows * D + 4 * kMaxCluster;   // floats before the first m
+  static constexpr int kBytes = kSent + (kSentStats + kMaxCluster * 2 * kRows) * 4;
+  static constexpr int kAlloc = kBytes + 1024, kAllocSingle = kSent + 1024;   // in a cluster, and not
   // the cross-warp merge reuses the tile ring: per warp O[16][D] + m[16] + l[16] floats
-  static constexpr int kMergeBytes = (kWarps + 1) * kRows * (D + 2) * 4;
+  static constexpr int kMergeBytes = kWarps * kRows * (D + 2) * 4;
   static_assert(kMergeBytes <= kBars, "merge scratch must fit in the tile ring");
 };
 
@@ -109,11 +117,10 @@ __device__ __forceinline__ uint16_t pack1(float x) {
   }
 }
 
-__device__ __forceinline__ float ld_cluster(uint32_t local_addr, uint32_t rank) {
-  float v;
-  asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %1, %2;\n\tld.shared::cluster.f32 %0, [ra];\n\t}"
-               : "=f"(v) : "r"(local_addr), "r"(rank) : "memory");
-  return v;
+// To the same place in the shared memory of CTA `rank` of the cluster.
+__device__ __forceinline__ void st_cluster(const float* at, uint32_t rank, float v) {
+  asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, %1;\n\tst.shared::cluster.f32 [ra], %2;\n\t}" ::"r"(smem_u32(at)),
+               "r"(rank), "f"(v) : "memory");
 }
 
 // byte offset of (key row r, 16-byte chunk c of the 128-byte row) inside a 128B-swizzled 64-key half tile
@@ -132,12 +139,16 @@ __device__ __noinline__ void let_copies_land() {
 template <int D>
 __host__ __device__ constexpr int partial_floats() { return kRows * (D + 2); }
 
-template <int D, bool kBf16, int kStages>
+// kOldRows: kv_len and all valid rows but the last are older than the kernel in front (kfb_flash_attn_decode_step): the tiles are on
+// their way while that kernel ends (step of the 22-layer model at batch 1, 512 keys, with the merge above: 513 us -> 481; batch 32
+// 996 -> 964).  kClustered and kOldRows are variants and not arguments: with them as arguments calls without either got slower (22
+// sequences of 6000..7000 keys 27.6 us -> 29.5; 42 of 700..2600 12.0 -> 12.7 even where only kClustered was one).
+template <int D, bool kBf16, int kStages, bool kClustered, bool kOldRows>
 __global__ void __launch_bounds__((consumer_warps<D, kStages>() + 1) * 32)
 attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                    const uint16_t* __restrict__ q, uint16_t* __restrict__ o, float* __restrict__ partial, int H, int Hk,
                    int Nk, float scale_log2, unsigned int* status, const int* __restrict__ kv_len,
-                   int force_partial, int clustered) {
+                   int force_partial) {
   using L = Layout<D, kStages>;
   constexpr int kConsumerWarps = L::kWarps, kThreads = L::kThreads;
   extern __shared__ uint8_t smem_raw[];
@@ -163,9 +174,14 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     *abort_word = *reinterpret_cast<volatile unsigned int*>(status);  // non-zero: an earlier wait expired
     fence_mbar_init();
   }
+  if constexpr (kClustered) cluster_arrive_relaxed();   // (its counterpart: before this CTA writes to the others)
   __syncthreads();
-  pdl_wait(q, kv_len);      // q, the cache rows and kv_len may be the output of the kernel in front
-  pdl_launch_dependents();
+  // q, the cache rows and kv_len may be the output of the kernel in front.  kOldRows: only q and the last valid row, so that every
+  // tile in front of that row's is requested before the wait.
+  if constexpr (!kOldRows) {
+    pdl_wait(q, kv_len);
+    pdl_launch_dependents();
+  }
   // a static KV cache holds Nk rows of which only kv_len[b] are valid (read on the device, so the
   // same launch can be replayed from a CUDA graph while the cache fills up)
   const int valid = kv_len ? min(Nk, max(kv_len[b], 0)) : Nk;
@@ -174,7 +190,8 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   const int key_end = min(valid, key_begin + per_split * kTileKeys);
   const int n_tiles = key_end > key_begin ? (key_end - key_begin + kTileKeys - 1) / kTileKeys : 0;
   const bool aborted = *abort_word != 0;   // uniform: written before the barrier, nothing has been issued yet
-  if (aborted && !clustered) return;
+  if (kOldRows && aborted) pdl_wait();     // (whoever waits for this kernel relies on its having waited)
+  if (aborted && !kClustered) return;
 
   float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
   float oacc[D / 8][4];
@@ -190,8 +207,10 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     if (lane == 0) {
       tma_prefetch_desc(&tm_k);
       tma_prefetch_desc(&tm_v);
+      const int first_new = min(kStages, (valid - 1 - key_begin) / kTileKeys);
       for (int t = 0; t < n_tiles; ++t) {
         const int s = t % kStages;
+        if (kOldRows && t == first_new) pdl_wait();
         if (!mbar_wait(&empty[s], ((uint32_t)(t / kStages) & 1u) ^ 1u, ctx, kWaitEmpty)) {
           let_copies_land();
           break;
@@ -206,9 +225,17 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         }
       }
     }
+    if constexpr (kOldRows) {
+      pdl_wait();
+      pdl_launch_dependents();
+    }
   } else {
     // ------------------------------------------------------------------ consumers
     const int g = lane >> 2, t4 = lane & 3;
+    if constexpr (kOldRows) {
+      pdl_wait(q);
+      pdl_launch_dependents();
+    }
     // Q fragments (A operand, 16 heads x D), rows >= `rows` are zero
     uint32_t qa[D / 16][4];
     {
@@ -355,67 +382,78 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     }
   }
   __syncthreads();
-  const bool direct = splits == 1 && !force_partial;   // otherwise (O, m, l) goes to `partial`, or to `own` for the cluster
-  float* own = scratch + kConsumerWarps * kPerWarp;
-  float* out_partial = partial + (((size_t)b * gridDim.y + blockIdx.y) * splits + split) * kPerWarp;
-  for (int idx = threadIdx.x; idx < rows * D; idx += kThreads) {
-    const int r = idx / D, d = idx - r * D;
-    float m_all = -INFINITY;
+  float m_all = -INFINITY, acc = 0.f, l_all = 0.f;
+  auto merge_warps = [&](int r, int d) {
+    m_all = -INFINITY;
 #pragma unroll
     for (int w = 0; w < kConsumerWarps; ++w) m_all = fmaxf(m_all, scratch[w * kPerWarp + kRows * D + r]);
     const float base = (m_all == -INFINITY) ? 0.f : m_all;
-    float acc = 0.f, l_all = 0.f;
+    acc = l_all = 0.f;
 #pragma unroll
     for (int w = 0; w < kConsumerWarps; ++w) {  // fixed order
       const float f = ex2(scratch[w * kPerWarp + kRows * D + r] - base);
       acc = fmaf(f, scratch[w * kPerWarp + r * D + d], acc);
       l_all = fmaf(f, scratch[w * kPerWarp + kRows * D + kRows + r], l_all);
     }
-    if (clustered) {
-      own[r * D + d] = acc;
-      if (d == 0) {
-        own[kRows * D + r] = m_all;
-        own[kRows * D + kRows + r] = l_all;
+  };
+  if constexpr (!kClustered) {
+    const bool direct = splits == 1 && !force_partial;   // otherwise (O, m, l) goes to `partial`
+    float* out_partial = partial + (((size_t)b * gridDim.y + blockIdx.y) * splits + split) * kPerWarp;
+    for (int idx = threadIdx.x; idx < rows * D; idx += kThreads) {
+      const int r = idx / D, d = idx - r * D;
+      merge_warps(r, d);
+      if (direct) {
+        o[((size_t)b * H + h0 + r) * D + d] = pack1<kBf16>(l_all == 0.f ? 0.f : acc / l_all);  // no valid key: zeros; a score that is NaN or +infinity: NaN
+      } else {
+        out_partial[r * D + d] = acc;
+        if (d == 0) {
+          out_partial[kRows * D + r] = m_all;
+          out_partial[kRows * D + kRows + r] = l_all;
+        }
       }
-    } else if (direct) {
-      o[((size_t)b * H + h0 + r) * D + d] = pack1<kBf16>(l_all == 0.f ? 0.f : acc / l_all);  // no valid key: zeros; a score that is NaN or +infinity: NaN
-    } else {
-      out_partial[r * D + d] = acc;
-      if (d == 0) {
-        out_partial[kRows * D + r] = m_all;
-        out_partial[kRows * D + kRows + r] = l_all;
+    }
+  } else {
+    float* sent = reinterpret_cast<float*>(smem + L::kSent);
+    float* sent_stats = sent + L::kSentStats;
+    const int share = ((rows * D + splits - 1) / splits + 3) & ~3;   // elements of the output that a CTA of the cluster puts together
+    cluster_wait();   // every CTA has started: its shared memory may be written
+#pragma unroll 1
+    for (int idx = threadIdx.x; idx < rows * D; idx += kThreads) {
+      const int r = idx / D, d = idx - r * D, owner = idx / share;
+      merge_warps(r, d);
+      st_cluster(sent + split * share + idx - owner * share, owner, acc);
+      if (d < splits) {   // m and l to CTA d
+        st_cluster(sent_stats + split * 2 * kRows + r, d, m_all);
+        st_cluster(sent_stats + split * 2 * kRows + kRows + r, d, l_all);
       }
+    }
+    // After this barrier nobody touches another CTA's memory: no second one before the end.
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+#pragma unroll 1
+    for (int i = threadIdx.x; i < share && split * share + i < rows * D; i += kThreads) {
+      const int idx = split * share + i, r = idx / D, d = idx - r * D;
+      float m[kMaxCluster], l[kMaxCluster], a[kMaxCluster];
+#pragma unroll
+      for (int c = 0; c < kMaxCluster; ++c) {
+        const bool there = c < splits;
+        m[c] = there ? sent_stats[c * 2 * kRows + r] : -INFINITY;
+        l[c] = there ? sent_stats[c * 2 * kRows + kRows + r] : 0.f;
+        a[c] = there ? sent[c * share + i] : 0.f;
+      }
+      m_all = m[0];
+#pragma unroll
+      for (int c = 1; c < kMaxCluster; ++c) m_all = fmaxf(m_all, m[c]);
+      const float base = (m_all == -INFINITY) ? 0.f : m_all;
+      acc = l_all = 0.f;
+#pragma unroll
+      for (int c = 0; c < kMaxCluster; ++c) {
+        const float f = ex2(m[c] - base);
+        acc = fmaf(f, a[c], acc);
+        l_all = fmaf(f, l[c], l_all);
+      }
+      if (!aborted) o[((size_t)b * H + h0 + r) * D + d] = pack1<kBf16>(l_all == 0.f ? 0.f : acc / l_all);
     }
   }
-  if (!clustered) return;
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-  // splits <= 8: this CTA merges elements split, split + splits, ... of the group's output
-  const uint32_t own_addr = smem_u32(own);
-  for (int idx = threadIdx.x * splits + split; idx < rows * D; idx += kThreads * splits) {
-    const int r = idx / D, d = idx - r * D;
-    float m[8], l[8], a[8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const bool there = c < splits;
-      m[c] = there ? ld_cluster(own_addr + (kRows * D + r) * 4, c) : -INFINITY;
-      l[c] = there ? ld_cluster(own_addr + (kRows * D + kRows + r) * 4, c) : 0.f;
-      a[c] = there ? ld_cluster(own_addr + (r * D + d) * 4, c) : 0.f;
-    }
-    float m_all = m[0];
-#pragma unroll
-    for (int c = 1; c < 8; ++c) m_all = fmaxf(m_all, m[c]);
-    const float base = (m_all == -INFINITY) ? 0.f : m_all;
-    float acc = 0.f, l_all = 0.f;
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const float f = ex2(m[c] - base);
-      acc = fmaf(f, a[c], acc);
-      l_all = fmaf(f, l[c], l_all);
-    }
-    if (!aborted) o[((size_t)b * H + h0 + r) * D + d] = pack1<kBf16>(l_all == 0.f ? 0.f : acc / l_all);
-  }
-  // no CTA leaves while another one still reads its sums
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // Combines the per-split partials of one (batch, query head).  `sets` > 1: several partial buffers of the same layout,
@@ -526,7 +564,7 @@ SplitPlan plan_splits(int B, int H, int Hk, int Nk, int D) {
   return p;
 }
 
-template <int D, bool kBf16, int kStages>
+template <int D, bool kBf16, int kStages, bool kClustered, bool kOldRows>
 int launch_stages(const Problem& p, const SplitPlan& plan, const CUtensorMap& tk, const CUtensorMap& tv, float* partial,
                   unsigned int* status, cudaStream_t stream, bool partial_only);
 
@@ -544,28 +582,35 @@ int launch(const Problem& p, const SplitPlan& plan, const CUtensorMap& tk, const
            unsigned int* status, cudaStream_t stream, bool partial_only = false) {
   const dim3 grid_probe(plan.splits, p.Hk * plan.chunks, p.B);
   const long long ctas = (long long)grid_probe.x * grid_probe.y * grid_probe.z;
-  if (ctas <= sm_count() && ceil_div(ceil_div(p.Nk, kTileKeys), plan.splits) > shallow_stages<D>())
-    return launch_stages<D, kBf16, deep_stages<D>()>(p, plan, tk, tv, partial, status, stream, partial_only);
-  return launch_stages<D, kBf16, shallow_stages<D>()>(p, plan, tk, tv, partial, status, stream, partial_only);
+  const bool deep = ctas <= sm_count() && ceil_div(ceil_div(p.Nk, kTileKeys), plan.splits) > shallow_stages<D>();
+  constexpr int kDeep = deep_stages<D>(), kShallow = shallow_stages<D>();
+  int (*run)(const Problem&, const SplitPlan&, const CUtensorMap&, const CUtensorMap&, float*, unsigned int*, cudaStream_t, bool);
+  if (plan.clustered && !partial_only)
+    run = p.old_rows ? (deep ? launch_stages<D, kBf16, kDeep, true, true> : launch_stages<D, kBf16, kShallow, true, true>)
+                     : (deep ? launch_stages<D, kBf16, kDeep, true, false> : launch_stages<D, kBf16, kShallow, true, false>);
+  else
+    run = p.old_rows ? (deep ? launch_stages<D, kBf16, kDeep, false, true> : launch_stages<D, kBf16, kShallow, false, true>)
+                     : (deep ? launch_stages<D, kBf16, kDeep, false, false> : launch_stages<D, kBf16, kShallow, false, false>);
+  return run(p, plan, tk, tv, partial, status, stream, partial_only);
 }
 
-template <int D, bool kBf16, int kStages>
+template <int D, bool kBf16, int kStages, bool kClustered, bool kOldRows>
 int launch_stages(const Problem& p, const SplitPlan& plan, const CUtensorMap& tk, const CUtensorMap& tv, float* partial,
                   unsigned int* status, cudaStream_t stream, bool partial_only) {
   using L = Layout<D, kStages>;
-  auto kernel = attn_decode_kernel<D, kBf16, kStages>;
+  auto kernel = attn_decode_kernel<D, kBf16, kStages, kClustered, kOldRows>;
+  constexpr int kSmem = kClustered ? L::kAlloc : L::kAllocSingle;
   static bool configured[64] = {false};
   int dev = 0;
   KFB_CUDA_TRY(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    KFB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kAlloc));
+    KFB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
     configured[dev] = true;
   }
-  const bool clustered = plan.clustered && !partial_only;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(plan.splits, p.Hk * plan.chunks, p.B);
   cfg.blockDim = dim3(L::kThreads);
-  cfg.dynamicSmemBytes = L::kAlloc;
+  cfg.dynamicSmemBytes = kSmem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -575,11 +620,11 @@ int launch_stages(const Problem& p, const SplitPlan& plan, const CUtensorMap& tk
   attr[1].val.clusterDim.y = 1;
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = clustered ? 2 : 1;
+  cfg.numAttrs = kClustered ? 2 : 1;
   cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, tk, tv, (const uint16_t*)p.q, (uint16_t*)p.o, partial, p.H, p.Hk, p.Nk,
-                                     p.scale * 1.4426950408889634f, status, p.kv_len_dev, partial_only ? 1 : 0, clustered ? 1 : 0);
+                                     p.scale * 1.4426950408889634f, status, p.kv_len_dev, partial_only ? 1 : 0);
   if (e != cudaSuccess) return fail(KFB_ERR_CUDA, "launch of attn_decode_kernel failed: %s", cudaGetErrorString(e));
-  if (clustered) return KFB_OK;
+  if (kClustered) return KFB_OK;
   if (plan.splits > 1 && !partial_only)
     return launch_merge_lanes<D, kBf16>((const float*)partial, (uint16_t*)p.o, p.B, p.H, p.Hk, plan.splits, 1, 0LL, stream);
   return KFB_OK;

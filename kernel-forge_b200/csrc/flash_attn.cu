@@ -92,9 +92,8 @@ extern "C" int kfb_flash_attn_fwd_tokens(const void* q, const void* k, const voi
 }
 
 // Decode attention against a static KV cache whose valid length lives on the device.
-extern "C" int kfb_flash_attn_decode_kvlen(const void* q, const void* k, const void* v, void* o, int dtype, int B, int H,
-                                           int Hk, int Nk, int D, float scale, const int64_t* kv_strides,
-                                           const int32_t* kv_len_dev, void* ws, size_t ws_bytes, void* stream) {
+static int decode_kvlen(const void* q, const void* k, const void* v, void* o, int dtype, int B, int H, int Hk, int Nk, int D, float scale,
+                        const int64_t* kv_strides, const int32_t* kv_len_dev, void* ws, size_t ws_bytes, void* stream, bool old_rows) {
   if (int rc = require_sm100()) return rc;
   if (int rc = check_shape(dtype, B, H, Hk, 1, Nk, D, 0)) return rc;
   if (!(scale > 0.0f)) return fail(KFB_ERR_INVALID, "scale must be positive, got %g", (double)scale);
@@ -107,8 +106,21 @@ extern "C" int kfb_flash_attn_decode_kvlen(const void* q, const void* k, const v
   p.causal = 0;
   p.scale = scale;
   p.kv_len_dev = kv_len_dev;
+  p.old_rows = old_rows;
   if (int rc = set_kv_strides(&p, kv_strides)) return rc;
   return attn::launch_decode(p, ws, ws_bytes, (cudaStream_t)stream);
+}
+
+extern "C" int kfb_flash_attn_decode_kvlen(const void* q, const void* k, const void* v, void* o, int dtype, int B, int H,
+                                           int Hk, int Nk, int D, float scale, const int64_t* kv_strides,
+                                           const int32_t* kv_len_dev, void* ws, size_t ws_bytes, void* stream) {
+  return decode_kvlen(q, k, v, o, dtype, B, H, Hk, Nk, D, scale, kv_strides, kv_len_dev, ws, ws_bytes, stream, false);
+}
+
+extern "C" int kfb_flash_attn_decode_step(const void* q, const void* k, const void* v, void* o, int dtype, int B, int H, int Hk, int Nk,
+                                          int D, float scale, const int64_t* kv_strides, const int32_t* kv_len_dev, void* ws,
+                                          size_t ws_bytes, void* stream) {
+  return decode_kvlen(q, k, v, o, dtype, B, H, Hk, Nk, D, scale, kv_strides, kv_len_dev, ws, ws_bytes, stream, true);
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -100,6 +100,8 @@ _SIGNATURES = {
     "kfb_decode_step_persistent": (c_int, [ctypes.POINTER(DecodeStep), c_void_p]),
     "kfb_flash_attn_decode_kvlen": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                                             c_float, ctypes.POINTER(c_int64), c_void_p, c_void_p, c_size_t, c_void_p]),
+    "kfb_flash_attn_decode_step": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
+                                           c_float, ctypes.POINTER(c_int64), c_void_p, c_void_p, c_size_t, c_void_p]),
     "kfb_flash_attn_decode_partial_bytes": (c_size_t, [c_int, c_int, c_int, c_int, c_int, ctypes.POINTER(c_int)]),
     "kfb_flash_attn_decode_partial": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float,
                                               ctypes.POINTER(c_int64), c_void_p, c_void_p, c_size_t, c_void_p]),

@@ -3,7 +3,7 @@
 What the reference measures with `bench/e2e_model.py::graph_decode` (97-141): prefill on a static KV cache,
 then one captured decode step replayed per token.  There the captured step has to use SDPA because the
 reference's attention kernel takes the KV length from the tensor shape (docstring 91-92, README.md:101).
-Here the step runs `ops.flash_attn_decode`, which reads the valid cache length from a device tensor, and
+Here the step runs `ops.flash_attn_decode_step`, which reads the valid cache length from a device tensor, and
 `ops.int4_linear` for the seven decoder linears of every layer; token ids, position and KV length all live
 on the device, so a step is a pure graph replay with no host synchronisation.
 
@@ -329,7 +329,7 @@ class LlamaInt4Decoder:
         for li, L in enumerate(self.layers):
             q = ops.int4_gemv_rope_kv(x, L["qkv"].packed, L["qkv"].scales, L["qkv"].group, self.cos, self.sin, self.pos,
                                       self.k_cache[li], self.v_cache[li], self.h_loc, L["in_norm"], s.rms_eps)
-            a = ops.flash_attn_decode(q, self.k_cache[li], self.v_cache[li], self.kv_len).view(b, self.h_loc * s.head_dim)
+            a = ops.flash_attn_decode_step(q, self.k_cache[li], self.v_cache[li], self.kv_len).view(b, self.h_loc * s.head_dim)
             x = ops.int4_gemv_fused(a, L["o"].packed, L["o"].scales, L["o"].group, residual=x)
             act = ops.int4_gemv_silu_pair(x, L["gate_up"].packed, L["gate_up"].scales, L["gate_up"].group, L["post_norm"], s.rms_eps)
             x = ops.int4_gemv_fused(act, L["down"].packed, L["down"].scales, L["down"].group, residual=x)
@@ -365,7 +365,7 @@ class LlamaInt4Decoder:
             else:
                 qkv = L["qkv"](h)
                 q = ops.rope_kv_write(qkv, self.cos, self.sin, self.pos, self.k_cache[li], self.v_cache[li], self.h_loc)
-            a = ops.flash_attn_decode(q, self.k_cache[li], self.v_cache[li], self.kv_len)
+            a = ops.flash_attn_decode_step(q, self.k_cache[li], self.v_cache[li], self.kv_len)
             a = self._gather(a.view(b, self.h_loc * s.head_dim), "attn_bounds")
             o = self._gather(L["o"](a), "hidden_bounds")
             h, x = ops.add_rmsnorm(x, L["post_norm"], s.rms_eps, o)

@@ -509,6 +509,27 @@ def flash_attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
     return o
 
 
+def flash_attn_decode_step(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, kv_len: torch.Tensor) -> torch.Tensor:
+    """flash_attn_decode for a loop whose kernel in front of this one wrote q and at most the last valid row of each sequence's cache:
+    kv_len and all other rows are older, and are read before that kernel has finished (kfb_flash_attn_decode_step)."""
+    _check_attn(q, k_cache, v_cache, False, strided_kv=True)
+    b, h, nq, d = q.shape
+    hk, nk = k_cache.shape[1], k_cache.shape[2]
+    if nq != 1 or kv_len.dtype != torch.int32 or not kv_len.is_cuda or not kv_len.is_contiguous() or kv_len.numel() != b:
+        raise ValueError("flash_attn_decode_step takes one query position per sequence and a contiguous int32 CUDA kv_len")
+    if k_cache.stride() != v_cache.stride() or k_cache.stride(3) != 1:
+        raise ValueError("k_cache and v_cache must share strides, with a dense D axis")
+    lib, o = _capi.lib(), torch.empty_like(q)
+    nbytes = lib.kfb_flash_attn_ws_bytes(b, h, hk, 1, nk, d)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=q.device) if nbytes else None
+    strides = (ctypes.c_int64 * 3)(*k_cache.stride()[:3])
+    with _capi.on_device(q.device):
+        _capi.check(lib.kfb_flash_attn_decode_step(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), o.data_ptr(), _capi.dtype_code(q.dtype),
+                                                   b, h, hk, nk, d, _resolve_scale(None, d), strides, kv_len.data_ptr(),
+                                                   ws.data_ptr() if nbytes else None, nbytes, _capi.stream_ptr(q.device)))
+    return o
+
+
 def flash_attn_decode_partial(q: torch.Tensor, k_shard: torch.Tensor, v_shard: torch.Tensor,
                               kv_len: torch.Tensor | None = None, scale: float | None = None) -> torch.Tensor:
     """Softmax partials of one decode step over ONE SHARD of the keys (see kfb_flash_attn_decode_partial): a flat fp32
