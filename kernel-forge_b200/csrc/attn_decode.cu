@@ -516,10 +516,12 @@ struct SplitPlan {
 // How many CTAs share the keys of one (batch, kv head, chunk) group.  Only the capacity of the cache is known here, not the
 // valid lengths.  Measured in a graph over 24..256 groups of 300..16384 keys, all lengths equal to the capacity / to half of it /
 // spread from a quarter to the whole (us), best of unsplit / clusters of 2..8 / 3..48 splits with a merge kernel:
-//   * as many as fit the GPU at once, one per SM, as a cluster of at most eight (8 x 4 groups of 1000..4096: 8.6; three splits
-//     and a merge kernel 11.1).  Every CTA keeps two tiles (545 keys: 4.1, unsplit 4.8), a group of fewer than eight tiles is
-//     quicker alone (225 keys: 4.3 against 5.3).  Two or three CTAs need longer caches to pay for the merge: 64 groups of 1000
-//     keys 7.1 / 5.6 / 7.1 unsplit against 7.4 / 6.2 / 6.9 in pairs, of 2000 11.1 / 7.4 / 10.7 against 10.6 / 7.5 / 8.9.
+//   * as many as fit the GPU at once, one per SM, as a cluster of at most eight (8 x 4 groups of 1000..4096: 7.9; three splits
+//     and a merge kernel 11.1).  A CTA may have as little as one tile, at D = 64 two from nine tiles on (sum of the three length
+//     patterns; 8 groups of 6 tiles: unsplit 12.3, six CTAs 11.6, D = 128 16.4 and 15.2; of 9 tiles: four CTAs 12.4, five 11.7,
+//     eight 11.8; D = 128 four 16.4, five 15.6, eight 15.1); of four tiles a group is as quick alone.  Two or three CTAs need
+//     longer caches to pay for the merge: 44 groups of 6 tiles 12.9 alone, 13.3 in threes, of 8 tiles 14.0 and 13.5; 64 groups of
+//     12 tiles 16.0 alone, 16.2 in pairs, of 16 tiles 17.8 and 17.4.
 //   * more groups than clusters of two (74: the SMs come in pairs; 68 groups of 8192: pairs 26.1 / 12.5 / 18.7, unsplit 30.4 /
 //     17.0 / 29.9): one CTA each; a second wave of CTAs or half-empty rings cost more than an uneven tail, except (D = 64,
 //     three shallow CTAs per SM) where caches are so long that the longest sequence's CTA is on its own for most of the time:
@@ -536,7 +538,7 @@ SplitPlan plan_splits(int B, int H, int Hk, int Nk, int D) {
   // from three on a little less here, since which SMs a chip has differs.  (With one cluster too many, 16 of eight, 3072 keys
   // took 13 us instead of 9.6.)
   constexpr int kFit[9] = {0, 148, 74, 44, 32, 24, 20, 14, 14};
-  constexpr int kLeastTiles[9] = {0, 8, 24, 12, 8, 10, 12, 14, 16};   // of the capacity, for a cluster of that size
+  constexpr int kLeastTiles[9] = {0, 6, 16, 8, 6, 6, 6, 6, 6};   // of the capacity, for a cluster of that size
   SplitPlan p;
   p.chunks = ceil_div(H / Hk, kRows);
   p.splits = 1;
@@ -549,8 +551,9 @@ SplitPlan plan_splits(int B, int H, int Hk, int Nk, int D) {
   else if (D == 64 && groups > kFit[2] && groups <= 88 && tiles >= 128) cluster = 4;
   else if (D == 64 && groups > kFit[1] && groups <= 192 && tiles >= 64) cluster = 2;
   else if (groups <= kFit[2]) {
-    cluster = 8;
-    while (cluster > 1 && (cluster * 2 > tiles || groups > kFit[cluster])) --cluster;
+    const int wanted = D == 64 && tiles > 8 ? ceil_div(tiles, 2) : tiles;
+    cluster = wanted < kMaxCluster ? wanted : kMaxCluster;
+    while (cluster > 1 && groups > kFit[cluster]) --cluster;
     if (tiles < kLeastTiles[cluster]) return p;
   }
   p.splits = cluster;
