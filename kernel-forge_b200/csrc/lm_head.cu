@@ -8,7 +8,7 @@
 //     into mma.sync.m16n8k16 A fragments (16 vocabulary rows per warp; a lane's 16 bytes of a row are 8 consecutive k,
 //     and the same 8 k of x are its B fragment -- any consistent assignment of k to fragment slots gives the same dot
 //     product, so no shared-memory staging or transposition is needed); FP32 accumulation, one rounding to fp16;
-//     the greedy argmax is fused: every warp reduces its 16 rows per batch column and merges into a 64-bit key per
+//     the greedy argmax is fused: every CTA reduces its rows per batch column and merges into a 64-bit key per
 //     batch row with atomicMax (value in the high word, inverted row index in the low word: the maximum is unique, so
 //     the result does not depend on the order of the atomics; ties go to the lowest index like torch.argmax);
 //   * decode_finalize_kernel: turns the keys into next-token ids (int64, what the embedding reads), clears the keys
@@ -23,7 +23,6 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kRowsPerWarp = 16;
-constexpr int kUnroll = 8;   // k chunks of 32 in flight per lane: 2 rows x 16 B x 8 = 256 B per lane, 8 KB per warp (4 gave 51 % of the HBM rate: too few bytes in flight at 13 warps per SM)
 
 __device__ __forceinline__ uint4 ldg_stream(const uint4* p) {
   uint4 v;
@@ -47,23 +46,24 @@ __device__ __forceinline__ uint32_t ordered_bits(float f) {
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
-// NB: blocks of 8 batch columns.  Lane = 4 g + t: vocabulary rows row0 + g and row0 + g + 8, k chunk t of every 32.
-template <int NB>
-__global__ void __launch_bounds__(kThreads)
+// NB: blocks of 8 batch columns; KU: k chunks of 32 requested at once, one batch of them ahead of the one being multiplied.
+// Lane = 4 g + t: vocabulary rows row0 + g and row0 + g + 8, k chunk t of every 32.
+// What bounds it: HBM up to 8 columns (32000 x 2048, M = 1 23.2 us, 5.6 TB/s; one batch of 8 chunks at a time, loads and products in
+// turn, 24.8), then the reads of the activations, each of which serves 16 rows.  The keys of a CTA's warps are brought together in
+// shared memory: an atomic per warp and column, 2000 of them on each of 32 addresses at the same time, took 15 us of 51.  Both, M = 8 /
+// 16 / 24 / 32: 31.2 / 41.3 / 47.6 / 56.5 -> 23.8 / 29.0 / 30.7 / 37.4.  Also measured at M = 32: two row blocks per warp 41.5
+// (without keys; this kernel 36), one or three chunks at once 38.4 and 39.8; at M = 16 two chunks 34.1, at M = 1 three 26.3.
+template <int NB, int KU>
+__global__ void __launch_bounds__(kThreads, 2)
 lm_head_gemv_kernel(const __half* __restrict__ x, const __half* __restrict__ w, __half* __restrict__ y,
                     unsigned long long* __restrict__ best, int M, int N, int K, int early) {
+  __shared__ unsigned long long keys[kWarps][8 * NB];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int row0 = (blockIdx.x * kWarps + warp) * kRowsPerWarp;
-  if (row0 >= N) {
-    pdl_wait();
-    pdl_launch_dependents();
-    return;
-  }
+  const int row0 = (blockIdx.x * kWarps + warp) * kRowsPerWarp;   // (a warp past N works on the last row and stores nothing)
   if (!early) pdl_wait(x, w);   // the weights may be the work of the kernel in front
-  const int ra = min(row0 + g, N - 1), rb = min(row0 + g + 8, N - 1);   // rows past N: a valid row, never stored
-  const uint4* wa = reinterpret_cast<const uint4*>(w + (size_t)ra * K) + t;
-  const uint4* wb = reinterpret_cast<const uint4*>(w + (size_t)rb * K) + t;
+  const uint4* wa = reinterpret_cast<const uint4*>(w + (size_t)min(row0 + g, N - 1) * K) + t;
+  const uint4* wb = reinterpret_cast<const uint4*>(w + (size_t)min(row0 + g + 8, N - 1) * K) + t;
   const uint4* xr[NB];
 #pragma unroll
   for (int nb = 0; nb < NB; ++nb) xr[nb] = reinterpret_cast<const uint4*>(x + (size_t)min(8 * nb + g, M - 1) * K) + t;
@@ -75,29 +75,39 @@ lm_head_gemv_kernel(const __half* __restrict__ x, const __half* __restrict__ w, 
     for (int e = 0; e < 4; ++e) acc[nb][e] = 0.f;
 
   const int chunks = K / 32;   // a chunk = 32 k: four lanes x 16 bytes
-  for (int c0 = 0; c0 < chunks; c0 += kUnroll) {
-    uint4 va[kUnroll], vb[kUnroll];
+  uint4 va[2][KU], vb[2][KU];
+  auto fetch = [&](int buf, int c0) {
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
+    for (int u = 0; u < KU; ++u) {
       const int c = min(c0 + u, chunks - 1);
-      va[u] = ldg_stream(wa + c * 4);
-      vb[u] = ldg_stream(wb + c * 4);
+      va[buf][u] = ldg_stream(wa + c * 4);
+      vb[buf][u] = ldg_stream(wb + c * 4);
     }
-    if (c0 == 0) {   // (early) the first loads are in flight before the wait for the kernel in front
-      pdl_wait();
-      pdl_launch_dependents();
-    }
+  };
+  auto multiply = [&](int buf, int c0) {
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
+    for (int u = 0; u < KU; ++u) {
       if (c0 + u < chunks) {
+        const uint4 a = va[buf][u], b = vb[buf][u];
 #pragma unroll
         for (int nb = 0; nb < NB; ++nb) {
           const uint4 xv = ldg_cached(xr[nb] + (c0 + u) * 4);
           // fragment slots (2t, 2t+1 | 2t+8, 2t+9) <- this lane's k (0,1 | 2,3), then (4,5 | 6,7)
-          mma16816(acc[nb], va[u].x, vb[u].x, va[u].y, vb[u].y, xv.x, xv.y);
-          mma16816(acc[nb], va[u].z, vb[u].z, va[u].w, vb[u].w, xv.z, xv.w);
+          mma16816(acc[nb], a.x, b.x, a.y, b.y, xv.x, xv.y);
+          mma16816(acc[nb], a.z, b.z, a.w, b.w, xv.z, xv.w);
         }
       }
+    }
+  };
+  fetch(0, 0);
+  pdl_wait();   // (early) the first loads are in flight before the wait for the kernel in front
+  pdl_launch_dependents();
+  for (int c0 = 0; c0 < chunks; c0 += 2 * KU) {
+    if (c0 + KU < chunks) fetch(1, c0 + KU);
+    multiply(0, c0);
+    if (c0 + KU < chunks) {
+      if (c0 + 2 * KU < chunks) fetch(0, c0 + 2 * KU);
+      multiply(1, c0 + KU);
     }
   }
 
@@ -128,9 +138,17 @@ lm_head_gemv_kernel(const __half* __restrict__ x, const __half* __restrict__ w, 
           const unsigned long long other = __shfl_xor_sync(0xffffffffu, key, off);
           key = other > key ? other : key;
         }
-        if (g == 0 && m < M) atomicMax(best + m, key);
+        if (g == 0) keys[warp][m] = key;
       }
     }
+  }
+  if (best == nullptr) return;
+  __syncthreads();
+  if (threadIdx.x < M) {
+    unsigned long long key = keys[0][threadIdx.x];
+#pragma unroll
+    for (int i = 1; i < kWarps; ++i) key = keys[i][threadIdx.x] > key ? keys[i][threadIdx.x] : key;
+    atomicMax(best + threadIdx.x, key);
   }
 }
 
@@ -224,20 +242,22 @@ extern "C" int kfb_fp16_gemv_argmax(const void* x, const void* w, void* y, void*
   if (!x || !w || !y) return fail(KFB_ERR_INVALID, "null pointer");
   if (!aligned16(x) || !aligned16(w) || (best && (reinterpret_cast<uintptr_t>(best) & 7u)))
     return fail(KFB_ERR_ALIGNMENT, "x and w must be 16-byte aligned, the argmax keys 8-byte aligned");
-  const int grid = ceil_div(N, lmhead::kWarps * lmhead::kRowsPerWarp);
   auto s = (cudaStream_t)stream;
   auto* b = static_cast<unsigned long long*>(best);
   const auto* xp = static_cast<const __half*>(x);
   const auto* wp = static_cast<const __half*>(w);
   auto* yp = static_cast<__half*>(y);
-  const dim3 gd(grid), bd(lmhead::kThreads);
   const int early = constants_are_old();
+#define KFB_LM(NB, KU)                                                                                                \
+  return launch_kernel("lm_head_gemv_kernel", lmhead::lm_head_gemv_kernel<NB, KU>, dim3(ceil_div(N, lmhead::kWarps * lmhead::kRowsPerWarp)), \
+                       dim3(lmhead::kThreads), 0, s, xp, wp, yp, b, M, N, K, early)
   switch (ceil_div(M, 8)) {
-    case 1: return launch_kernel("lm_head_gemv_kernel", lmhead::lm_head_gemv_kernel<1>, gd, bd, 0, s, xp, wp, yp, b, M, N, K, early);
-    case 2: return launch_kernel("lm_head_gemv_kernel", lmhead::lm_head_gemv_kernel<2>, gd, bd, 0, s, xp, wp, yp, b, M, N, K, early);
-    case 3: return launch_kernel("lm_head_gemv_kernel", lmhead::lm_head_gemv_kernel<3>, gd, bd, 0, s, xp, wp, yp, b, M, N, K, early);
-    default: return launch_kernel("lm_head_gemv_kernel", lmhead::lm_head_gemv_kernel<4>, gd, bd, 0, s, xp, wp, yp, b, M, N, K, early);
+    case 1: KFB_LM(1, 4);
+    case 2: KFB_LM(2, 4);
+    case 3: KFB_LM(3, 3);
+    default: KFB_LM(4, 2);
   }
+#undef KFB_LM
 }
 
 extern "C" int kfb_decode_finalize(void* best, void* tok, void* pos, void* kv_len, int M, void* stream) {
