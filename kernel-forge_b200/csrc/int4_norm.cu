@@ -13,6 +13,9 @@
 //   * one CTA per SM where there are more than two blocks of 16 rows for each: a second wave would fetch its weights and
 //     normalise after the first one has finished (11264 rows, step of 22 layers: 704 CTAs of one block 583 us, 235 of three
 //     561, 141 of five 513).
+//   * with RB > 1 the packed nibbles are multiplied as they are, subnormal fp16 numbers, which takes 10 clocks of unpacking per word
+//     instead of 18 (unpack_tiny; step of 22 layers 484 us -> 477; the error against 64 bits is the same, 4.41e-4 of a SiLU output).
+//     With one row block the product that makes up for the offset costs as much as it saves.
 // Weights staged in shared memory with asynchronous copies instead of registers were slower (+2 us per layer), and so was
 // this structure without the norm (o and down projection: int4_small.cu, which has fewer and smaller CTAs there).
 // Step of the 22-layer model at batch 1: 593 us with separate norm kernels and the CUDA-core GEMV -> 503.  At batch 2 the step
@@ -43,6 +46,15 @@ __device__ __forceinline__ void unpack(uint32_t w, uint32_t (&q)[4]) {
   asm("sub.f16x2 %0, %1, %2;" : "=r"(q[1]) : "r"(v1), "r"(0x54805480u));   // - 72
   asm("sub.f16x2 %0, %1, %2;" : "=r"(q[2]) : "r"(v2), "r"(0x64086408u));
   asm("sub.f16x2 %0, %1, %2;" : "=r"(q[3]) : "r"(v3), "r"(0x54805480u));
+}
+
+// The same pairs as subnormal fp16 numbers, u = q + 8 times 2^-24 (s even) or 2^-20 (s odd), exact: no additions.
+__device__ __forceinline__ void unpack_tiny(uint32_t w, uint32_t (&q)[4]) {
+  const uint32_t h = w >> 8;
+  q[0] = w & 0x000F000Fu;
+  q[1] = w & 0x00F000F0u;
+  q[2] = h & 0x000F000Fu;
+  q[3] = h & 0x00F000F0u;
 }
 
 __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -177,27 +189,48 @@ int4_norm_kernel(const __half* __restrict__ x, const uint32_t* __restrict__ pack
     for (int b = 0; b < H; ++b)
 #pragma unroll
       for (int e = 0; e < 2; ++e) xv[b][e] = *reinterpret_cast<const uint4*>(xs + i * G + b * 64 + e * 8);
+    // With several row blocks the unpacking is what a scheduler spends its time on; there the nibbles go into the product as they
+    // are (unpack_tiny), and what that is too large by, 8 times the sum of the group's activations, is what the sums start with:
+    // a product with a constant, once for all row blocks.  Even and odd pairs have a sum each, which differ by 2^4.
+    float start[4] = {0.f, 0.f, 0.f, 0.f};
+    if constexpr (RB > 1) {
+      constexpr uint32_t kMinusEight = 0x80088008u;   // -8 * 2^-24, twice
+#pragma unroll
+      for (int b = 0; b < H; ++b)
+#pragma unroll
+        for (int s = 0; s < 4; ++s)
+          mma16816(start, kMinusEight, kMinusEight, kMinusEight, kMinusEight, reinterpret_cast<const uint32_t*>(&xv[b][0])[s],
+                   reinterpret_cast<const uint32_t*>(&xv[b][1])[s]);
+    }
 #pragma unroll
     for (int rb = 0; rb < RB; ++rb) {
-      float c[4] = {0.f, 0.f, 0.f, 0.f};
+      float c[2][4] = {{start[0], start[1], start[2], start[3]}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
       for (int b = 0; b < H; ++b) {
         uint32_t q[4][4];
         if constexpr (!kEarlyUnpack) {
-          unpack(wv[rb][0][i][b].x, q[0]);
-          unpack(wv[rb][1][i][b].x, q[1]);
-          unpack(wv[rb][0][i][b].y, q[2]);
-          unpack(wv[rb][1][i][b].y, q[3]);
+          auto take = [](uint32_t w, uint32_t (&to)[4]) {
+            if constexpr (RB > 1) unpack_tiny(w, to);
+            else unpack(w, to);
+          };
+          take(wv[rb][0][i][b].x, q[0]);
+          take(wv[rb][1][i][b].x, q[1]);
+          take(wv[rb][0][i][b].y, q[2]);
+          take(wv[rb][1][i][b].y, q[3]);
         }
         const uint32_t (&u)[4][4] = kEarlyUnpack ? early[kEarlyUnpack ? b : 0] : q;
 #pragma unroll
         for (int s = 0; s < 4; ++s)
-          mma16816(c, u[0][s], u[1][s], u[2][s], u[3][s], reinterpret_cast<const uint32_t*>(&xv[b][0])[s],
+          mma16816(c[RB > 1 ? s & 1 : 0], u[0][s], u[1][s], u[2][s], u[3][s], reinterpret_cast<const uint32_t*>(&xv[b][0])[s],
                    reinterpret_cast<const uint32_t*>(&xv[b][1])[s]);
       }
-      const float s0 = __half2float(sv[rb][0][i]), s1 = __half2float(sv[rb][1][i]);
+      constexpr float kUnit = RB > 1 ? 16777216.0f : 1.0f;
+      const float s0 = __half2float(sv[rb][0][i]) * kUnit, s1 = __half2float(sv[rb][1][i]) * kUnit;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) acc[rb][e] = i == 0 ? (e < 2 ? s0 : s1) * c[e] : fmaf(e < 2 ? s0 : s1, c[e], acc[rb][e]);
+      for (int e = 0; e < 4; ++e) {
+        const float v = RB > 1 ? fmaf(c[1][e], 0.0625f, c[0][e]) : c[0][e];
+        acc[rb][e] = i == 0 ? (e < 2 ? s0 : s1) * v : fmaf(e < 2 ? s0 : s1, v, acc[rb][e]);
+      }
     }
   }
 

@@ -49,3 +49,23 @@ def test_norm_rope_kv(b):
     for a, c in ((got, want), (caches[0], caches[2]), (caches[1], caches[3])):
         assert (a.float() - c.float()).abs().max().item() <= 2e-3 * c.float().abs().max().item()
     assert not caches[0][:, :, :pos].any() and not caches[1][:, :, pos + 1:].any()
+
+
+@pytest.mark.parametrize("mean", [0.0, 4.0, -4.0])
+@pytest.mark.parametrize("m,n,k,group", [(1, 7106, 1024, 64), (2, 9474, 2048, 64), (1, 11264, 2048, 128), (2, 11000, 2048, 128)])
+def test_nibbles_multiplied_as_they_are(m, n, k, group, mean):
+    """Several row blocks per CTA take nibbles without their offset of 8, which is made up for by the sum of the activations: also
+    where that sum is large because they have one sign."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    qw = quantize.quantize_weight((torch.randn(n, k, generator=g, device="cuda") * 0.05).half(), group)
+    x, w = (torch.randn(m, k, generator=g, device="cuda") + mean).half(), torch.ones(k, device="cuda").half()
+    got = ops.int4_gemv_fused(x, qw.packed, qw.scales, group, ops.XFORM_RMSNORM, w, 1e-5).double()
+    h, wd = ops.add_rmsnorm(x, w, 1e-5)[0].double(), quantize.dequantize(qw, torch.float32).double()
+    ref = h @ wd.T
+    # FP32 sums of nibble * activation, nibbles up to 15 with an offset of 8: at most 2 * 2^-24 of the sum of their magnitudes for each
+    # of the additions that a sum goes through (k / 16 in the tensor core, 32 around it); the norm's own rounding may differ by one
+    # step of fp16 in an activation here and there; one rounding to fp16
+    terms = h.abs() @ (wd.abs() + 8 * qw.scales.double().repeat_interleave(group, 1)).T
+    bound = 2 * (k / 16 + 32) * 2.0 ** -24 * terms + 2.0 ** -10 * (h.abs() @ wd.abs().T) / 16 + ref.abs() * 2.0 ** -11
+    assert ((got - ref).abs() <= bound).all()
+    assert (got - ref).mean().abs().item() <= 0.1 * 2.0 ** -11 * ref.abs().max().item()     # unbiased
