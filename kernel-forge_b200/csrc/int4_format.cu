@@ -48,11 +48,19 @@ __device__ __forceinline__ float rcp_approx(float x) {
   return y;
 }
 
+// Largest magnitude of three (one instruction on sm_100); NaN only if all are.
+__device__ __forceinline__ float max_abs3(float a, float b, float c) {
+  float y;
+  asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+  return y;
+}
+
 // One lane per packed word (8 consecutive k); G / 8 neighbouring lanes share a group.  Words and groups are contiguous
 // over the whole tensor, so a CTA takes a run of kUnroll * 256 flat word indices and knows no rows.
 //
 // HBM-bound by design (2.5 bytes per fp16 weight), bound by issue slots in fact.  One IEEE division per weight (a dozen
-// instructions) and 8-byte loads took 42.8 us for 11264 x 2048 fp16; this kernel takes 15 us (3.9 TB/s).  A weight is
+// instructions) and 8-byte loads took 42.8 us for 11264 x 2048 fp16; this kernel takes 14.9 us (3.9 TB/s; with one weight per
+// floating-point instruction 15.1, bf16 16.8 and now 16.3).  A weight is
 // multiplied with the group's reciprocal and rounded by the magic-number addition of one FMA.  The product is off by at
 // most 2^-22 of itself, so the result can only differ from the definition's next to a half integer; a lane that sees such
 // a weight (or a quotient above 7.4, infinity, NaN) packs its word by the definition.
@@ -79,9 +87,7 @@ __global__ void __launch_bounds__(kQuantThreads, 8) quantize_pack_kernel(const T
 #pragma unroll
   for (int u = 0; u < kQuantUnroll; ++u) {
     const int i = u * kQuantThreads + threadIdx.x;
-    float amax = fabsf(v[u][0]);
-#pragma unroll
-    for (int j = 1; j < 8; ++j) amax = fmaxf(amax, fabsf(v[u][j]));
+    float amax = max_abs3(max_abs3(v[u][0], v[u][1], v[u][2]), max_abs3(v[u][3], v[u][4], v[u][5]), max_abs3(v[u][6], v[u][7], v[u][7]));
 #pragma unroll
     for (int off = kLanes / 2; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
     // scale = fp16(max(absmax / 7, smallest normal fp16)); exactly 1 for an all-zero group
@@ -94,17 +100,21 @@ __global__ void __launch_bounds__(kQuantThreads, 8) quantize_pack_kernel(const T
     constexpr float kMagic = 12582912.0f;
     constexpr uint32_t kBits = 0x4B400000u, kSum = 0u - (kBits - 8u) * 0x11111111u;
     const float lo = inv * (1.0f - 1.0f / 1048576.0f), hi = inv * (1.0f + 1.0f / 1048576.0f);
+    const float2 lo2 = make_float2(lo, lo), hi2 = make_float2(hi, hi), magic2 = make_float2(kMagic, kMagic);
     uint32_t word = kSum, differ = 0;
-    float sum = 0.0f;   // not finite if any weight is (amax does not see NaN)
+    float2 sum = make_float2(0.0f, 0.0f);   // not finite if any weight is (amax does not see NaN)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float t = fmaf(v[u][j], lo, kMagic);
-      const uint32_t a = __float_as_uint(t), b = __float_as_uint(fmaf(v[u][j], hi, kMagic));
-      sum += t;
-      differ |= a ^ b;
-      word += a << (4 * nibble_pos(j));
+    for (int j = 0; j < 8; j += 2) {   // two weights per floating-point instruction
+      const float2 w2 = make_float2(v[u][j], v[u][j + 1]);
+      const float2 t = __ffma2_rn(w2, lo2, magic2), q = __ffma2_rn(w2, hi2, magic2);
+      const uint32_t a0 = __float_as_uint(t.x), a1 = __float_as_uint(t.y);
+      sum = __fadd2_rn(sum, t);
+      differ |= a0 ^ __float_as_uint(q.x);
+      differ |= a1 ^ __float_as_uint(q.y);
+      word += a0 << (4 * nibble_pos(j));
+      word += a1 << (4 * nibble_pos(j + 1));
     }
-    if (!(differ == 0 && amax * inv < 7.4f && sum < 1e9f)) {
+    if (!(differ == 0 && amax * inv < 7.4f && sum.x + sum.y < 1e9f)) {
       Eight w8;
 #pragma unroll
       for (int j = 0; j < 8; ++j) w8.v[j] = v[u][j];
