@@ -109,13 +109,14 @@ __device__ __forceinline__ void store_rows(float a0, float a1, const gemv::Fusio
 template <int KS, int RB, int MB>
 constexpr int min_blocks() { return KS == 16 ? 1 : RB * MB == 1 ? 4 : RB == 1 && MB == 2 ? 3 : 2; }
 
-// G: group size; KS: warps of a CTA = shares of K; RB: 16-row blocks per warp; MB: blocks of 8 batch columns.
-template <int G, int KS, int RB, int MB, bool kBf16>
+// G: group size; KS: warps of a CTA = shares of K; RB: 16-row blocks per warp; MB: blocks of 8 batch columns; kHalves: see run.
+template <int G, int KS, int RB, int MB, bool kBf16, bool kHalves>
 __global__ void __launch_bounds__(KS * 32, min_blocks<KS, RB, MB>())
 int4_small_kernel(const uint16_t* __restrict__ x, const uint32_t* __restrict__ packed, const __half* __restrict__ scales,
                   uint16_t* __restrict__ y, int M, int N, int K, const gemv::Fusion fu) {
-  constexpr int W = G / 32;                         // packed words per lane, row and group; and 16-byte pieces of x
-  constexpr int kDepth = (KS == 16 && MB == 1 ? 4 : 2) * (128 / G);   // groups a warp keeps in flight
+  constexpr int U = kHalves ? 64 : G;               // K is walked in scale groups, or in blocks of 64
+  constexpr int W = U / 32;                         // packed words per lane, row and unit; and 16-byte pieces of x
+  constexpr int kDepth = (KS == 16 && MB == 1 ? 4 : 2) * (128 / U);   // units a warp keeps in flight
   constexpr int kRows = 16 * RB, kPad = kRows + 4;
   extern __shared__ float red[];                    // [warp][8 MB][kPad]
 
@@ -124,7 +125,7 @@ int4_small_kernel(const uint16_t* __restrict__ x, const uint32_t* __restrict__ p
   const int g = lane >> 2, t = lane & 3;
   const int r0 = blockIdx.x * kRows;
   const int SG = K / G, KW = K / 8;
-  const int g0 = (int)((long long)SG * warp / warps), g1 = (int)((long long)SG * (warp + 1) / warps);
+  const int units = K / U, g0 = (int)((long long)units * warp / warps), g1 = (int)((long long)units * (warp + 1) / warps);   // of this warp
 
   if (!fu.early) pdl_wait(x, packed, scales);   // (early: the weights are older than the kernel in front)
   const uint32_t* wrow[RB][2];
@@ -145,8 +146,8 @@ int4_small_kernel(const uint16_t* __restrict__ x, const uint32_t* __restrict__ p
       for (int rb = 0; rb < RB; ++rb)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          load_words(wbuf[slot][rb][h], wrow[rb][h] + (size_t)gi * (G / 8));
-          sbuf[slot][rb][h] = __half2float(srow[rb][h][gi]);
+          load_words(wbuf[slot][rb][h], wrow[rb][h] + (size_t)gi * (U / 8));
+          sbuf[slot][rb][h] = __half2float(srow[rb][h][gi / (G / U)]);
         }
     }
   };
@@ -170,7 +171,7 @@ int4_small_kernel(const uint16_t* __restrict__ x, const uint32_t* __restrict__ p
 #pragma unroll
     for (int j = 0; j < MB; ++j) {
       const bool real = 8 * j + g < M;
-      const uint4* p = reinterpret_cast<const uint4*>(xrow + (size_t)(8 * j) * K + (size_t)gi * G);
+      const uint4* p = reinterpret_cast<const uint4*>(xrow + (size_t)(8 * j) * K + (size_t)gi * U);
 #pragma unroll
       for (int i = 0; i < W; ++i) xv[j][i] = real ? p[(i >> 1) * 8 + (i & 1)] : make_uint4(0u, 0u, 0u, 0u);
     }
@@ -242,10 +243,10 @@ int4_small_kernel(const uint16_t* __restrict__ x, const uint32_t* __restrict__ p
   }
 }
 
-template <int G, int KS, int RB, int MB, bool kBf16>
+template <int G, int KS, int RB, int MB, bool kBf16, bool kHalves = false>
 int launch(const void* x, const void* packed, const void* scales, void* y, int M, int N, int K,
            cudaStream_t stream, const gemv::Fusion& fu) {
-  auto kernel = int4_small_kernel<G, KS, RB, MB, kBf16>;
+  auto kernel = int4_small_kernel<G, KS, RB, MB, kBf16, kHalves>;
   constexpr size_t smem = (size_t)KS * (8 * MB) * (16 * RB + 4) * sizeof(float);
   static_assert(smem <= 48 * 1024, "no opt-in for more shared memory is made");
   return launch_kernel("int4_small_kernel", kernel, dim3(ceil_div(N, 16 * RB)), dim3(KS * 32), smem, stream,
@@ -265,12 +266,19 @@ int run(const void* x, const void* packed, const void* scales, void* y, int M, i
   const int row_blocks = ceil_div(N, 16), sms = sm_count();
   const bool long_k = row_blocks <= sms && K >= 4096;
   const bool two_rows = M > 8 && M <= 16 && row_blocks > 3 * sms;
+  // Above M = 16 the activations of a group of 128 take 64 registers, which costs a resident CTA and loads in flight: with more than 48
+  // row blocks K is walked in blocks of 64 (us, M = 19, 5824 x 1920 9.1 -> 7.5; M = 22, 6464 x 1536 bf16 9.1 -> 7.0; M = 23, 1600 x
+  // 1792 4.7 -> 4.1; step of the 22-layer model at batch 32 952 -> 921).  Fewer row blocks (M = 22, 371 x 1792 3.8 and 3.9; M = 29, 512
+  // x 2560 4.8 and 4.9) and smaller M (M = 16, 1536 x 8960 6.8 and 7.5; M = 4, 1216 x 2688 3.5 and 4.0) gain nothing from it.
+  const bool halves = group == 128 && row_blocks > 48;
 #define KFB_SMALL(G, KS, RB, MB, BF) return launch<G, KS, RB, MB, BF>(x, packed, scales, y, M, N, K, stream, fu)
 #define KFB_SMALL_KS(G, BF)                                                            \
   {                                                                                    \
     if (two_rows) KFB_SMALL(G, 8, 2, 2, BF);                                           \
     if (M <= 8) { if (long_k) KFB_SMALL(G, 16, 1, 1, BF); KFB_SMALL(G, 8, 1, 1, BF); } \
     if (M <= 16) { if (long_k) KFB_SMALL(G, 16, 1, 2, BF); KFB_SMALL(G, 8, 1, 2, BF); } \
+    if (long_k && halves) return launch<G, 16, 1, 4, BF, true>(x, packed, scales, y, M, N, K, stream, fu); \
+    if (halves) return launch<G, 8, 1, 4, BF, true>(x, packed, scales, y, M, N, K, stream, fu);            \
     if (long_k) KFB_SMALL(G, 16, 1, 4, BF);                                            \
     KFB_SMALL(G, 8, 1, 4, BF);                                                         \
   }

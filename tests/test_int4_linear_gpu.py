@@ -83,3 +83,10 @@ def test_result_buffer_of_two_byte_alignment(m, n, k):
     assert_int4_close(buf[1:-1].view(m, n), ref)
     assert buf[0] == 7.0 and buf[-1] == 7.0
     assert torch.equal(buf[1:-1].view(m, n), ops.int4_linear(x, packed, scales, 128))
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m,n,k", [(17, 768, 640), (17, 769, 640), (24, 800, 128), (25, 1000, 4224), (32, 769, 8064), (32, 2400, 1152)])
+def test_blocks_of_64_above_16_rows(m, n, k, dtype):
+    """Groups of 128 walked in blocks of 64, from 49 row blocks on: both sides of the line, fewer blocks than warps, a long K."""
+    check(m, n, k, 128, dtype, True)
