@@ -126,6 +126,7 @@ class LlamaInt4Decoder:
         # (int4_linear).  Measured, us per step on the TinyLlama-1.1B shape at batch 3 / 8 / 16 / 32: everything on
         # fragment-order copies 597 / 620 / 764 / 1065, this 534 / 554 / 687 / 991, gate_up by int4_linear too 577 / 610 / 739 /
         # 994 (so at batch 32 the copy of gate_up saves no time worth its memory).
+        # (Later attention, lm_head and linear kernels, at batch 8 / 16 / 32 on 200 cached tokens: 554 / 689 / 991 -> 528 / 651 / 921.)
         # With tensor parallelism the same holds for the rank's own rows (local heads, local share of the hidden and
         # intermediate features); only the four gathers per layer are added.
         # Batch 1 on one GPU: five kernels per layer (_step_fused), both RMSNorms in the prologue of the projection behind them
@@ -188,7 +189,7 @@ class LlamaInt4Decoder:
         self.best = torch.zeros(batch, dtype=torch.int64, device=self.dev)   # argmax keys of the step, see ops.lm_head_argmax
         # Batch <= 2, head dim 64, one GPU: the whole step can run as ONE persistent cooperative kernel
         # (kfb_decode_step_persistent) plus the finalize kernel: set `persistent = True` before capture().  Not the default:
-        # measured on the TinyLlama-1.1B shape it takes 0.92 ms per step at batch 1 against 0.50 ms for the step of
+        # measured on the TinyLlama-1.1B shape it takes 0.92 ms per step at batch 1 against 0.48 ms for the step of
         # separate kernels chained by programmatic dependent launch -- five grid-wide barriers per layer at ~2 us each
         # plus the L2 round trip that re-reads the activations after each of them cost more than the launches they replace.
         self.persistent_ok = self.pair_rows and self.plan is None and batch <= 2 and s.head_dim == 64
