@@ -69,3 +69,24 @@ def test_nibbles_multiplied_as_they_are(m, n, k, group, mean):
     bound = 2 * (k / 16 + 32) * 2.0 ** -24 * terms + 2.0 ** -10 * (h.abs() @ wd.abs().T) / 16 + ref.abs() * 2.0 ** -11
     assert ((got - ref).abs() <= bound).all()
     assert (got - ref).mean().abs().item() <= 0.1 * 2.0 ** -11 * ref.abs().max().item()     # unbiased
+
+
+@pytest.mark.parametrize("at", [[0], [3], [517], [1022], [64, 700], [1, 2, 3]])
+@pytest.mark.parametrize("m,n,k,group", [(1, 2048, 1024, 128), (1, 7106, 1024, 64), (2, 7107, 2048, 64), (2, 9474, 2048, 128), (1, 11264, 2048, 128), (2, 11264, 1024, 64)])
+def test_activations_that_overflow(m, n, k, group, at):
+    """A normalised activation past the largest fp16 number: results are what the definition gives, infinite with the sign of the product and
+    NaN where the nibble is zero or two infinities differ in sign.  The other batch row stays as it is."""
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    qw = quantize.quantize_weight((torch.randn(n, k, generator=g, device="cuda") * 0.05).half(), group)
+    x, w = torch.randn(m, k, generator=g, device="cuda").half(), torch.ones(k, device="cuda").half()
+    for i, j in enumerate(at):
+        x[0, j], w[j] = (-1.0) ** i * 20.0, 60000.0
+    x[1:, at] = 0.0
+    h, wd = ops.add_rmsnorm(x, w, 1e-5)[0].double(), quantize.dequantize(qw, torch.float32).double()
+    assert h[0, at].isinf().all() and h.isinf().sum() == len(at)
+    want = torch.stack([(row * wd).sum(1) for row in h])
+    got = ops.int4_gemv_fused(x, qw.packed, qw.scales, group, ops.XFORM_RMSNORM, w, 1e-5).double()
+    assert not want[0].isfinite().any() and want[1:].isfinite().all()
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got[got.isinf()], want[want.isinf()])
+    if m > 1:
+        assert (got[1] - want[1]).abs().max().item() <= 2e-3 * want[1].abs().max().item()
