@@ -492,13 +492,7 @@ def flash_attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
     o = _capi.host().flash_attn_decode(q, k_cache, v_cache, kv_len, scale)
     if o is not None:
         return o
-    _check_attn(q, k_cache, v_cache, False, strided_kv=True)
-    if q.shape[2] != 1:
-        raise ValueError(f"flash_attn_decode takes one query position per sequence, got Nq={q.shape[2]}")
-    if kv_len.dtype != torch.int32 or not kv_len.is_cuda or kv_len.numel() != q.shape[0]:
-        raise TypeError("kv_len must be an int32 CUDA tensor with one entry per batch item")
-    if k_cache.stride() != v_cache.stride() or k_cache.stride(3) != 1 or any(s % 8 for s in k_cache.stride()[:3]):
-        raise ValueError("k_cache and v_cache must share strides, with a dense D axis and strides that are multiples of 8")
+    _check_decode(q, k_cache, v_cache, kv_len)
     scale = _resolve_scale(scale, q.shape[-1])
     if q.numel() == 0:
         return torch.empty_like(q)
@@ -511,14 +505,15 @@ def flash_attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
 
 def flash_attn_decode_step(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, kv_len: torch.Tensor) -> torch.Tensor:
     """flash_attn_decode for a loop whose kernel in front of this one wrote q and at most the last valid row of each sequence's cache:
-    kv_len and all other rows are older, and are read before that kernel has finished (kfb_flash_attn_decode_step)."""
-    _check_attn(q, k_cache, v_cache, False, strided_kv=True)
-    b, h, nq, d = q.shape
+    kv_len and all other rows are older, and are read before that kernel has finished (kfb_flash_attn_decode_step).  kv_len has to be
+    contiguous: a copy of it would be younger."""
+    _check_decode(q, k_cache, v_cache, kv_len)
+    if not kv_len.is_contiguous():
+        raise ValueError("flash_attn_decode_step takes a contiguous kv_len")
+    if q.numel() == 0:
+        return torch.empty_like(q)
+    b, h, _, d = q.shape
     hk, nk = k_cache.shape[1], k_cache.shape[2]
-    if nq != 1 or kv_len.dtype != torch.int32 or not kv_len.is_cuda or not kv_len.is_contiguous() or kv_len.numel() != b:
-        raise ValueError("flash_attn_decode_step takes one query position per sequence and a contiguous int32 CUDA kv_len")
-    if k_cache.stride() != v_cache.stride() or k_cache.stride(3) != 1:
-        raise ValueError("k_cache and v_cache must share strides, with a dense D axis")
     lib, o = _capi.lib(), torch.empty_like(q)
     nbytes = lib.kfb_flash_attn_ws_bytes(b, h, hk, 1, nk, d)
     ws = torch.empty(nbytes, dtype=torch.uint8, device=q.device) if nbytes else None
@@ -528,6 +523,22 @@ def flash_attn_decode_step(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torc
                                                    b, h, hk, nk, d, _resolve_scale(None, d), strides, kv_len.data_ptr(),
                                                    ws.data_ptr() if nbytes else None, nbytes, _capi.stream_ptr(q.device)))
     return o
+
+
+def _check_decode(q, k_cache, v_cache, kv_len):
+    _check_attn(q, k_cache, v_cache, False, strided_kv=True)
+    if q.shape[2] != 1:
+        raise ValueError(f"flash_attn_decode takes one query position per sequence, got Nq={q.shape[2]}")
+    _check_kv_len(q, kv_len)
+    if k_cache.stride() != v_cache.stride() or k_cache.stride(3) != 1 or any(s % 8 for s in k_cache.stride()[:3]):
+        raise ValueError("k_cache and v_cache must share strides, with a dense D axis and strides that are multiples of 8")
+
+
+def _check_kv_len(q, kv_len):
+    if kv_len.dtype != torch.int32 or not kv_len.is_cuda or kv_len.numel() != q.shape[0]:
+        raise TypeError("kv_len must be an int32 CUDA tensor with one entry per batch item")
+    if kv_len.device != q.device:
+        raise ValueError(f"q and kv_len must be on one CUDA device, got {q.device} and {kv_len.device}")
 
 
 def flash_attn_decode_partial(q: torch.Tensor, k_shard: torch.Tensor, v_shard: torch.Tensor,
