@@ -227,7 +227,8 @@ PyObject* flash_attn(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
-// flash_attn_decode(q, k_cache, v_cache, kv_len, scale or None) -> o
+// flash_attn_decode(q, k_cache, v_cache, kv_len, scale or None) -> o, and flash_attn_decode_step with the same arguments
+template <decltype(&kfb_flash_attn_decode_kvlen) Entry>
 PyObject* flash_attn_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   ARGS(5)
   return guarded([&]() -> PyObject* {
@@ -245,9 +246,9 @@ PyObject* flash_attn_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
     int rc;
     {
       NoGil free;
-      rc = kfb_flash_attn_decode_kvlen(p.q->data_ptr(), p.k->data_ptr(), p.v->data_ptr(), o.data_ptr(), dtype_code(p.q->scalar_type()), (int)p.b,
-                                       (int)p.h, (int)p.hk, (int)p.nk, (int)p.d, scale, p.strided ? p.strides : nullptr,
-                                       static_cast<const int32_t*>(len->data_ptr()), ws_bytes ? ws.data_ptr() : nullptr, ws_bytes, stream);
+      rc = Entry(p.q->data_ptr(), p.k->data_ptr(), p.v->data_ptr(), o.data_ptr(), dtype_code(p.q->scalar_type()), (int)p.b, (int)p.h, (int)p.hk,
+                 (int)p.nk, (int)p.d, scale, p.strided ? p.strides : nullptr, static_cast<const int32_t*>(len->data_ptr()),
+                 ws_bytes ? ws.data_ptr() : nullptr, ws_bytes, stream);
     }
     return rc ? raise_status(rc) : THPVariable_Wrap(std::move(o));
   });
@@ -392,7 +393,10 @@ PyMethodDef methods[] = {
     METHOD(int4_linear, "int4_linear(x, packed, scales, group_size, bias) -> y, or None when the call is not a plain one"),
     METHOD(plain_constant, "plain_constant(t) -> whether t may go into a kernel as a bias"),
     METHOD(flash_attn, "flash_attn(q, k, v, causal, scale, views) -> o, or None when the call is not a plain one"),
-    METHOD(flash_attn_decode, "flash_attn_decode(q, k_cache, v_cache, kv_len, scale) -> o, or None when the call is not a plain one"),
+    {"flash_attn_decode", (PyCFunction)(void*)flash_attn_decode<kfb_flash_attn_decode_kvlen>, METH_FASTCALL,
+     "flash_attn_decode(q, k_cache, v_cache, kv_len, scale) -> o, or None when the call is not a plain one"},
+    {"flash_attn_decode_step", (PyCFunction)(void*)flash_attn_decode<kfb_flash_attn_decode_step>, METH_FASTCALL,
+     "flash_attn_decode_step(q, k_cache, v_cache, kv_len, scale) -> o, or None when the call is not a plain one"},
     METHOD(quantize_pack, "quantize_pack(weight, group_size) -> (packed, scales), or None when the call is not a plain one"),
     METHOD(add_rmsnorm, "add_rmsnorm(x, weight, eps, residual) -> (y, s), or None"),
     METHOD(rope_tokens, "rope_tokens(qkv, cos, sin, k_cache, v_cache, batch, heads, pairs) -> q [B, T, H, D], or None"),

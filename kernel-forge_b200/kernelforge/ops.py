@@ -490,38 +490,32 @@ def flash_attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
     replayed while the cache fills (the reference's graph-mode decode has to use SDPA instead,
     bench/e2e_model.py:91-92).  Returns [B, H, 1, D]."""
     o = _capi.host().flash_attn_decode(q, k_cache, v_cache, kv_len, scale)
-    if o is not None:
-        return o
-    _check_decode(q, k_cache, v_cache, kv_len)
-    scale = _resolve_scale(scale, q.shape[-1])
-    if q.numel() == 0:
-        return torch.empty_like(q)
-    plain = lambda t: t.as_subclass(torch.Tensor)
-    o = _capi.host().flash_attn_decode(plain(q), plain(k_cache), plain(v_cache), plain(kv_len).contiguous(), scale)
-    if o is None:
-        raise ValueError("q, k_cache, v_cache and kv_len must be non-empty and on one CUDA device")
-    return o
+    return o if o is not None else _decode_general(_capi.host().flash_attn_decode, q, k_cache, v_cache, kv_len, scale)
 
 
 def flash_attn_decode_step(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, kv_len: torch.Tensor) -> torch.Tensor:
     """flash_attn_decode for a loop whose kernel in front of this one wrote q and at most the last valid row of each sequence's cache:
     kv_len and all other rows are older, and are read before that kernel has finished (kfb_flash_attn_decode_step).  kv_len has to be
     contiguous: a copy of it would be younger."""
+    o = _capi.host().flash_attn_decode_step(q, k_cache, v_cache, kv_len, None)
+    if o is not None:
+        return o
     _check_decode(q, k_cache, v_cache, kv_len)
     if not kv_len.is_contiguous():
         raise ValueError("flash_attn_decode_step takes a contiguous kv_len")
+    return _decode_general(_capi.host().flash_attn_decode_step, q, k_cache, v_cache, kv_len, None)
+
+
+def _decode_general(call, q, k_cache, v_cache, kv_len, scale) -> torch.Tensor:
+    """A decode call that the native path has declined: the exception that says why, or the call on plain tensors."""
+    _check_decode(q, k_cache, v_cache, kv_len)
+    scale = _resolve_scale(scale, q.shape[-1])
     if q.numel() == 0:
         return torch.empty_like(q)
-    b, h, _, d = q.shape
-    hk, nk = k_cache.shape[1], k_cache.shape[2]
-    lib, o = _capi.lib(), torch.empty_like(q)
-    nbytes = lib.kfb_flash_attn_ws_bytes(b, h, hk, 1, nk, d)
-    ws = torch.empty(nbytes, dtype=torch.uint8, device=q.device) if nbytes else None
-    strides = (ctypes.c_int64 * 3)(*k_cache.stride()[:3])
-    with _capi.on_device(q.device):
-        _capi.check(lib.kfb_flash_attn_decode_step(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), o.data_ptr(), _capi.dtype_code(q.dtype),
-                                                   b, h, hk, nk, d, _resolve_scale(None, d), strides, kv_len.data_ptr(),
-                                                   ws.data_ptr() if nbytes else None, nbytes, _capi.stream_ptr(q.device)))
+    plain = lambda t: t.as_subclass(torch.Tensor)
+    o = call(plain(q), plain(k_cache), plain(v_cache), plain(kv_len).contiguous(), scale)
+    if o is None:
+        raise ValueError("q, k_cache, v_cache and kv_len must be non-empty and on one CUDA device")
     return o
 
 
