@@ -544,6 +544,10 @@ def flash_attn_decode_partial(q: torch.Tensor, k_shard: torch.Tensor, v_shard: t
     b, h, _, d = q.shape
     hk, nk = k_shard.shape[1], k_shard.shape[2]
     if kv_len is not None:
+        if kv_len.dtype != torch.int32 or not kv_len.is_cuda or kv_len.numel() < b:
+            raise TypeError("kv_len must be an int32 CUDA tensor with one entry per batch item")
+        if kv_len.device != q.device:
+            raise ValueError(f"q and kv_len must be on one CUDA device, got {q.device} and {kv_len.device}")
         kv_len = kv_len.contiguous()
     lib = _capi.lib()
     nbytes = lib.kfb_flash_attn_decode_partial_bytes(b, h, hk, nk, d, None)

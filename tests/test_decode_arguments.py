@@ -16,14 +16,14 @@ def operands(b=2):
     return [on(0, torch.zeros(b, 4, n, 64, dtype=torch.float16)) for n in (1, 70, 70)]
 
 
-@pytest.mark.parametrize("call", ["flash_attn_decode", "flash_attn_decode_step"])
+@pytest.mark.parametrize("call", ["flash_attn_decode", "flash_attn_decode_step", "flash_attn_decode_partial"])
 def test_lengths_on_another_gpu(call):
     with pytest.raises(ValueError, match="one CUDA device"):
         getattr(ops, call)(*operands(), on(1, torch.ones(2, dtype=torch.int32)))
 
 
-@pytest.mark.parametrize("call", ["flash_attn_decode", "flash_attn_decode_step"])
-@pytest.mark.parametrize("lengths", [torch.ones(2, dtype=torch.int32), on(0, torch.ones(2, dtype=torch.int64)), on(0, torch.ones(3, dtype=torch.int32))])
+@pytest.mark.parametrize("call", ["flash_attn_decode", "flash_attn_decode_step", "flash_attn_decode_partial"])
+@pytest.mark.parametrize("lengths", [torch.ones(2, dtype=torch.int32), on(0, torch.ones(2, dtype=torch.int64)), on(0, torch.ones(1, dtype=torch.int32))])
 def test_lengths_that_are_none(call, lengths):
     with pytest.raises(TypeError, match="kv_len must be"):
         getattr(ops, call)(*operands(), lengths)
