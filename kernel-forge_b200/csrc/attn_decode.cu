@@ -533,12 +533,19 @@ struct SplitPlan {
 //     of the chip idle, and from 16 tiles of D = 64 per CTA on that costs more than the merge kernel, whose own cost grows with
 //     the splits (4 groups of 16384 keys: eight in a cluster 11.4, 16 to 32 and a merge 9.7; 4096 keys: 6.7 and 6.8; one group
 //     of 131072: 48 splits 16.3, 148 19.6).
-SplitPlan plan_splits(int B, int H, int Hk, int Nk, int D) {
+// Where every split writes a partial (`partials`: one shard of a cache split along the sequence) there is no cluster to merge them:
+// the partials go through an all-gather and a kernel that reads all ranks', so a CTA keeps two tiles and two or three CTAs need longer
+// caches (partials + merge of 1 / of 4 ranks, us, with the lines of clusters and with these: 8 groups of 8 tiles D=128 6.6 / 7.3 and 6.1 /
+// 6.9; 24 of 6 7.6 / 10.4 and 7.3 / 7.3; 40 of 8 7.7 / 11.1 and 7.9 / 8.0; 64 of 16 10.9 / 13.8 and 10.2 / 10.7; 24 of 8 D=64 6.0 / 7.3 and
+// 5.3 / 6.6; but 8 groups of 7 tiles D=128 7.1 / 7.3 and 7.7 / 7.5).
+SplitPlan plan_splits(int B, int H, int Hk, int Nk, int D, bool partials = false) {
   // Clusters of 1..8 CTAs, one per SM, that fit at once: cudaOccupancyMaxActiveClusters gives 148, 74, 45, 33, 26, 22, 15, 15;
   // from three on a little less here, since which SMs a chip has differs.  (With one cluster too many, 16 of eight, 3072 keys
   // took 13 us instead of 9.6.)
   constexpr int kFit[9] = {0, 148, 74, 44, 32, 24, 20, 14, 14};
-  constexpr int kLeastTiles[9] = {0, 6, 16, 8, 6, 6, 6, 6, 6};   // of the capacity, for a cluster of that size
+  // tiles of the capacity, for so many CTAs: as a cluster, and with partials
+  constexpr int kLeast[2][9] = {{0, 6, 16, 8, 6, 6, 6, 6, 6}, {0, 8, 24, 12, 8, 10, 12, 14, 16}};
+  const int(&kLeastTiles)[9] = kLeast[partials];
   SplitPlan p;
   p.chunks = ceil_div(H / Hk, kRows);
   p.splits = 1;
@@ -551,7 +558,7 @@ SplitPlan plan_splits(int B, int H, int Hk, int Nk, int D) {
   else if (D == 64 && groups > kFit[2] && groups <= 88 && tiles >= 128) cluster = 4;
   else if (D == 64 && groups > kFit[1] && groups <= 192 && tiles >= 64) cluster = 2;
   else if (groups <= kFit[2]) {
-    const int wanted = D == 64 && tiles > 8 ? ceil_div(tiles, 2) : tiles;
+    const int wanted = partials ? tiles / 2 : D == 64 && tiles > 8 ? ceil_div(tiles, 2) : tiles;
     cluster = wanted < kMaxCluster ? wanted : kMaxCluster;
     while (cluster > 1 && groups > kFit[cluster]) --cluster;
     if (tiles < kLeastTiles[cluster]) return p;
@@ -643,7 +650,7 @@ size_t decode_ws_bytes(int B, int H, int Hk, int Nk, int D) {
 }
 
 size_t decode_partial_bytes(int B, int H, int Hk, int Nk, int D, int* splits_out) {
-  const SplitPlan plan = plan_splits(B, H, Hk, Nk, D);
+  const SplitPlan plan = plan_splits(B, H, Hk, Nk, D, true);
   if (splits_out) *splits_out = plan.splits;
   return (size_t)B * Hk * plan.chunks * plan.splits * kRows * (D + 2) * sizeof(float);
 }
@@ -662,7 +669,7 @@ int launch_merge(const float* partial, void* o, int dtype, int B, int H, int Hk,
 int launch_decode(const Problem& p, void* ws, size_t ws_bytes, cudaStream_t stream, bool partial_only) {
   if (p.Hk * ceil_div(p.H / p.Hk, kRows) > 65535 || p.B > 65535 || p.H > 65535)
     return fail(KFB_ERR_INVALID, "B, H and Hk * ceil(H/Hk/16) must each be <= 65535");
-  const SplitPlan plan = plan_splits(p.B, p.H, p.Hk, p.Nk, p.D);
+  const SplitPlan plan = plan_splits(p.B, p.H, p.Hk, p.Nk, p.D, partial_only);
   const size_t need = partial_only ? decode_partial_bytes(p.B, p.H, p.Hk, p.Nk, p.D, nullptr) : decode_ws_bytes(p.B, p.H, p.Hk, p.Nk, p.D);
   if (need > 0 && (!ws || ws_bytes < need))
     return fail(KFB_ERR_WORKSPACE, "decode attention needs a %zu-byte workspace, got %zu", need, ws_bytes);

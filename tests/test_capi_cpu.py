@@ -151,6 +151,22 @@ def test_every_decode_plan_fits_the_array_of_the_allocation_free_entry():
     assert lib.kfb_flash_attn_ws_bytes(1, 32, 4, 1, 16384, 64) > 0      # more than eight splits
 
 
+def test_splits_that_write_partials_have_two_tiles_of_keys():
+    """A shard's partials are gathered from all ranks and merged by a kernel: no split of less than two tiles, no pairs below 24 tiles and
+    no threes below 12, unlike clusters.  Host logic."""
+    lib = _capi.lib()
+    split = 0
+    for d in (64, 128):
+        for groups in list(range(1, 76)):
+            for tiles in range(1, 80):
+                n = ctypes.c_int()
+                nbytes = lib.kfb_flash_attn_decode_partial_bytes(groups, 8, 1, tiles * 64, d, ctypes.byref(n))
+                assert nbytes == groups * n.value * 16 * (d + 2) * 4
+                assert n.value == 1 or (n.value * 2 <= tiles and tiles >= {2: 24, 3: 12}.get(n.value, 8)), (d, groups, tiles, n.value)
+                split += n.value > 1
+    assert split > 2000
+
+
 def test_no_kernel_asks_for_non_coherent_loads():
     """Kernels are resident while the one in front still writes (programmatic dependent launch): what they read has to go through
     coherent loads behind pdl_wait.  __ldg and ld.global.nc are taken to be invariant and may be moved above it."""
