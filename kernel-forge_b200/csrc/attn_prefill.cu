@@ -103,8 +103,14 @@ __device__ __forceinline__ TileOrder decode_tile_order(unsigned int block, int n
 // 128, equally the tensor pipe (1024 clocks per tile and step).  Either is reached only if a softmax warp never waits, so
 // its own chain -- scores, maximum, exponentials, P, PV, next QK -- is what counts:
 //   * exponentials do not wait for the maximum of their step: they are taken with the base of the steps before, while the
-//     maxima of the row run under them, and in the rare step whose maximum outgrows the base the first two of four chunks are
-//     taken again (the results are those of looking first).  Only the first step of a CTA looks first;
+//     maxima of the row run under them, and in a step whose maximum outgrows the base they are taken again (the results are those
+//     of looking first).  One row of a warp's 32 is enough for that, so with scores of a standard deviation of 6 (natural units)
+//     every second step is such a step.  The first of four chunks is taken ahead, two chunks only in head dim 128 CTAs of two tiles,
+//     where the baton makes one chunk too short (us, scores of deviation 1 / 3 / 6, looking first - two chunks ahead - one: 2 x 16 x
+//     2048 D=64 56.9 / 58.5 / 61.6 - 53.1 / 58.6 / 72.8 - 52.9 / 55.8 / 64.0; 4 heads x 5806 causal D=64 45.2 / 45.7 / 47.8 - 44.0 / 48.8 /
+//     63.7 - 44.4 / 45.4 / 52.3; 1 x 16 x 2048 causal D=128 33.3 / 33.8 / 35.4 - 27.0 / 28.5 / 33.0 - 27.0 / 28.1 / 31.7; 2 x 16 x 2048 D=128
+//     73.9 / 75.4 / 80.1 - 68.0 / 75.7 / 96.5 - 73.6 / 79.1 / 95.8).  Going back to looking first after two grown steps in a row helps
+//     there (92.5 at 6, 85 at 30 instead of 98) but costs every call (8192 causal 550 us -> 556).  Only the first step looks first;
 //   * the scores are loaded in chunks of 32, one ahead.  Head dim 64 releases the S buffer after the last, and QK(j+1) runs
 //     under step j; P has columns of its own;
 //   * head dim 128: P(j) overwrites half of S(j), so QK(j+1) can only follow PV(j).  P is handed over in two halves, and
@@ -229,6 +235,8 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   constexpr int S = L::kStages, kHalves = L::kHalves;
   constexpr bool kAliasP = L::kAliasP;
   constexpr bool kBaton = NT == 2;               // the two tiles take turns
+  constexpr int kGuess = D == 128 && NT == 2 ? 2 : 1;   // chunks whose exponentials do not wait for the step's maximum
+  constexpr int kOrder = D == 64 && NT == 1 ? 7 : 5;    // pairs of a chunk are taken in the order e * kOrder (see chunk)
   constexpr int kBatonAfter = kAliasP ? 2 : 1;   // the chunk after which the other tile may start
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -513,34 +521,58 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         else p[c][e] = exp_pair<kBf16>(v[c][2 * e], v[c][2 * e + 1], sc2, nb2, sum[e & 1]);
       };
       auto seen = [&](int c, int e) { mx[e & 3] = max3(mx[e & 3], __uint_as_float(v[c][2 * e]), __uint_as_float(v[c][2 * e + 1])); };
-      auto chunk = [&](int c) {   // (the order spreads the polynomials among the others)
+      // The order spreads the polynomials among the others.  (7 instead of 5 in head dim 64 one-tile CTAs: 53.8 us -> 52.9 at 2 x 16 x
+      // 2048, fewer registers spilled; in two-tile CTAs 5 is the better one, 44.5 and 45.6 at 4 heads x 5806 causal.)
+      auto chunk = [&](int c) {
 #pragma unroll
-        for (int e = 0; e < 16; ++e) expo(c, (e * 5) & 15);
+        for (int e = 0; e < 16; ++e) expo(c, (e * kOrder) & 15);
       };
       auto pass_baton = [&]() {   // (the operands keep the exponentials summed so far in front of it)
         asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0]; // %1 %2" ::"r"(smem_u32(&turn[X ^ 1])), "f"(sum[0].x), "f"(sum[1].x) : "memory");
       };
-      // The maxima run under the exponentials of the first two chunks, which are taken with the base of the steps before: it
+      // The maxima run under the exponentials of the first kGuess chunks, which are taken with the base of the steps before: it
       // only moves when a maximum outgrows it by more than the threshold, and then they are taken again.
+      auto land = [&]() {
+        tmem_wait_ld_regs(v[1]);
+        tmem_wait_ld_regs(v[2]);
+        tmem_wait_ld_regs(v[3]);
+        if (i > 0) {
+          mask(1);
+          mask(2);
+          mask(3);
+        }
+      };
+      if constexpr (kGuess == 1) {
 #pragma unroll
-      for (int e = 0; e < 16; ++e) {
-        expo(0, (e * 5) & 15);
-        seen(0, e);
-      }
-      tmem_wait_ld_regs(v[1]);
-      tmem_wait_ld_regs(v[2]);
-      tmem_wait_ld_regs(v[3]);
-      if (i > 0) {
-        mask(1);
-        mask(2);
-        mask(3);
-      }
+        for (int e = 0; e < 8; ++e) {
+          expo(0, (e * kOrder) & 15);
+          seen(0, e);
+        }
+        land();
 #pragma unroll
-      for (int e = 0; e < 16; ++e) {
-        expo(1, (e * 5) & 15);
-        seen(1, e);
-        seen(2, e);
-        seen(3, e);
+        for (int e = 8; e < 16; ++e) {
+          expo(0, (e * kOrder) & 15);
+          seen(0, e);
+#pragma unroll
+          for (int x = 2 * e - 16; x < 2 * e - 14; ++x) {
+            seen(1, x);
+            seen(2, x);
+            seen(3, x);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < 32; ++e) {
+          if (e == 16) land();
+          expo(e / 16, (e * kOrder) & 15);
+          if (e < 16) {
+            seen(0, e);
+          } else {
+            seen(1, e - 16);
+            seen(2, e - 16);
+            seen(3, e - 16);
+          }
+        }
       }
       const float m_step = max_of(mx) * pr.scale_log2;
       // lazy rescale: move the base only when the maximum outgrew it by more than the threshold
@@ -577,15 +609,16 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         base = (m_base == -INFINITY) ? 0.f : m_base;
         nb2 = make_float2(-base, -base);
         sum[0] = sum[1] = make_float2(0.f, 0.f);
-        fetch(i, 0);
-        fetch(i, 1);
-        tmem_wait_ld_regs(v[0]);
-        tmem_wait_ld_regs(v[1]);
-        mask(0);
-        mask(1);
-        chunk(0);
-        chunk(1);
+#pragma unroll
+        for (int c = 0; c < kGuess; ++c) fetch(i, c);
+#pragma unroll
+        for (int c = 0; c < kGuess; ++c) {
+          tmem_wait_ld_regs(v[c]);
+          mask(c);
+          chunk(c);
+        }
       }
+      if (kGuess == 1) chunk(1);
       if constexpr (!kAliasP) {   // the S buffer can take the next product already
         tc_fence_before_sync();
         mbar_arrive(&s_free[X]);

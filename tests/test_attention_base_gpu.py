@@ -41,6 +41,22 @@ def test_a_maximum_that_jumps(b, h, hk, nq, nk, d, causal, tiles, key):
     assert _capi.device_status(torch.device("cuda", 0)) == 0
 
 
+@pytest.mark.parametrize("deviation", [6.0, 30.0])
+@pytest.mark.parametrize("b,h,hk,nq,nk,d,causal,tiles", KINDS)
+def test_maxima_that_keep_growing(b, h, hk, nq, nk, d, causal, tiles, deviation):
+    """Sharp scores: in every second step and more some row of a warp outgrows its base, in any of the four chunks."""
+    assert tiles_per_cta(b, h, hk, nq, nk, d, causal) == tiles
+    q, k, v = qkv_case(b, h, hk, nq, nk, d, torch.float16, seed=nq, scale_q=deviation)
+    got = ops.flash_attn(q.cuda(), k.cuda(), v.cuda(), causal=causal).float().cpu()
+    for i, j in [(0, 0), (b - 1, h - 1)]:
+        ref = torch.from_numpy(attn_oracle(q[i:i + 1, j:j + 1], k[i:i + 1, j:j + 1], v[i:i + 1, j:j + 1], causal))
+        s = (q[i, j].float() @ k[i, j].float().T).abs().max().item() / d ** 0.5
+        # the reference's bound, and the rounding of scores of this size (as above); P is rounded to 11 bits: 2^-11 of the largest |v|
+        vmax = v.abs().max().item()
+        assert (got[i, j] - ref[0, 0]).abs().max().item() <= 2e-3 + (8 * 2.0 ** -24 * s + 2.0 ** -11) * vmax
+    assert _capi.device_status(torch.device("cuda", 0)) == 0
+
+
 @pytest.mark.parametrize("nk", [2, 128, 129, 256, 257, 384, 500, 640, 1100, 2048])
 def test_two_buffers_of_scores(nk):
     """One tile per CTA at head dim 128, from one step to sixteen; with 256 CTAs, which follow one another on an SM; often."""
