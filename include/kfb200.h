@@ -329,7 +329,9 @@ int kfb_flash_attn_decode_kvlen(const void* q, const void* k, const void* v, voi
 
 /* The same inside a decode step, with one more promise by the caller: the kernel in front of this launch in the stream wrote q and at
  * most ONE row of each sequence's cache, the last valid one; kv_len_dev and all other valid rows are older.  The launch may then read
- * those before that kernel has finished (it carries the attribute described at kfb_set_programmatic_launch). */
+ * those before that kernel has finished (it carries the attribute described at kfb_set_programmatic_launch).  "Older" has to mean
+ * complete: the kernel in front either never lets its successor start early, or does so (griddepcontrol.launch_dependents) only after
+ * its own griddepcontrol.wait, so that what ran before it has ended when this launch begins.  All kernels of this library do. */
 int kfb_flash_attn_decode_step(const void* q, const void* k, const void* v, void* o, int dtype,
                                int B, int H, int Hk, int Nk, int D, float scale,
                                const int64_t* kv_strides, const int32_t* kv_len_dev,

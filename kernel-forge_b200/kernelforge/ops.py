@@ -495,8 +495,9 @@ def flash_attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
 
 def flash_attn_decode_step(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, kv_len: torch.Tensor) -> torch.Tensor:
     """flash_attn_decode for a loop whose kernel in front of this one wrote q and at most the last valid row of each sequence's cache:
-    kv_len and all other rows are older, and are read before that kernel has finished (kfb_flash_attn_decode_step).  kv_len has to be
-    contiguous: a copy of it would be younger."""
+    kv_len and all other rows are older, and are read before that kernel has finished (kfb_flash_attn_decode_step).  A kernel of your own
+    in front may let its successor start early only after its own griddepcontrol.wait.  kv_len has to be contiguous: a copy of it would
+    be younger."""
     o = _capi.host().flash_attn_decode_step(q, k_cache, v_cache, kv_len, None)
     if o is not None:
         return o
