@@ -114,6 +114,7 @@ template <int G, int KS, int RB, int MB, bool kBf16, bool kHalves>
 __global__ void __launch_bounds__(KS * 32, min_blocks<KS, RB, MB>())
 int4_small_kernel(const uint16_t* __restrict__ x, const uint32_t* __restrict__ packed, const __half* __restrict__ scales,
                   uint16_t* __restrict__ y, int M, int N, int K, const gemv::Fusion fu) {
+  static_assert(!kHalves || G == 128, "a group of 64 is a block of 64");
   constexpr int U = kHalves ? 64 : G;               // K is walked in scale groups, or in blocks of 64
   constexpr int W = U / 32;                         // packed words per lane, row and unit; and 16-byte pieces of x
   constexpr int kDepth = (KS == 16 && MB == 1 ? 4 : 2) * (128 / U);   // units a warp keeps in flight
@@ -271,14 +272,15 @@ int run(const void* x, const void* packed, const void* scales, void* y, int M, i
   // 1792 4.7 -> 4.1; step of the 22-layer model at batch 32 952 -> 921).  Fewer row blocks (M = 22, 371 x 1792 3.8 and 3.9; M = 29, 512
   // x 2560 4.8 and 4.9) and smaller M (M = 16, 1536 x 8960 6.8 and 7.5; M = 4, 1216 x 2688 3.5 and 4.0) gain nothing from it.
   const bool halves = group == 128 && row_blocks > 48;
-#define KFB_SMALL(G, KS, RB, MB, BF) return launch<G, KS, RB, MB, BF>(x, packed, scales, y, M, N, K, stream, fu)
+#define KFB_SMALL(G, ...) return launch<G, __VA_ARGS__>(x, packed, scales, y, M, N, K, stream, fu)
 #define KFB_SMALL_KS(G, BF)                                                            \
   {                                                                                    \
     if (two_rows) KFB_SMALL(G, 8, 2, 2, BF);                                           \
     if (M <= 8) { if (long_k) KFB_SMALL(G, 16, 1, 1, BF); KFB_SMALL(G, 8, 1, 1, BF); } \
     if (M <= 16) { if (long_k) KFB_SMALL(G, 16, 1, 2, BF); KFB_SMALL(G, 8, 1, 2, BF); } \
-    if (long_k && halves) return launch<G, 16, 1, 4, BF, true>(x, packed, scales, y, M, N, K, stream, fu); \
-    if (halves) return launch<G, 8, 1, 4, BF, true>(x, packed, scales, y, M, N, K, stream, fu);            \
+    constexpr bool kHalves = G == 128;                                                 \
+    if (long_k && halves) KFB_SMALL(G, 16, 1, 4, BF, kHalves);                         \
+    if (halves) KFB_SMALL(G, 8, 1, 4, BF, kHalves);                                    \
     if (long_k) KFB_SMALL(G, 16, 1, 4, BF);                                            \
     KFB_SMALL(G, 8, 1, 4, BF);                                                         \
   }
