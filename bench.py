@@ -898,7 +898,7 @@ def main():
         "roofline": roofline("tensor", fa["tflops"] / world, peaks, kind,
                              # dram__bytes_read.sum + dram__bytes_write.sum of one launch of this workload from an ncu capture
                              # (q, k, v read once = 25.2 MB; o stays in L2 until after the launch)
-                             traffic=25205760, kernel="attn_prefill_kernel<64,fp16,2>"),
+                             traffic=25205760, kernel="attn_prefill_kernel<64,fp16,1>"),
     })
     c1 = also.get("c1_int4_linear_m1_5632x2048")
     if c1:

@@ -123,12 +123,14 @@ __device__ __forceinline__ TileOrder decode_tile_order(unsigned int block, int n
 // the pair of tiles, each 1200 from its last P to its next scores and 1640 of exponentials (1024 at the unit's rate; a single
 // warp per scheduler reaches 86 % of it), which overlap with the other tile's.
 // Measured (us in a graph, before -> after the exponentials stopped waiting, one-tile CTAs with an SM to themselves got two
-// buffers and head dim 64 one-tile CTAs wherever keys are not split): B=2 H=16 N=2048 D=64 58.0 -> 53.9, N=8192 701 -> 651; 32 x 32 heads
+// buffers and head dim 64 one-tile CTAs wherever keys are not split): B=2 H=16 N=2048 D=64 58.0 -> 53.9 (back to back, at the power limit,
+// 58.7 -> 57.8), N=8192 701 -> 651; 32 x 32 heads
 // x 200 tokens D=64 causal 50.6 -> 45.3; N=2048 D=128 75.4 -> 69.8; N=8192 D=128 causal 495 -> 471 (577 -> 549 back to back at the
 // power limit's clock); 1 x 16 x 2048 D=128 causal 34.0 -> 29.5; 509 queries on 4093 keys, 12 heads over 2, D=128 26.5 -> 23.5.
 // Also measured: D=64, N=2048, two tiles per CTA 56.8, without baton 58.1; two pairs of 16 by polynomial 56.7, four 57.2; the last
 // chunk of scores read twice, to save registers, 55.3; the first step on the path that takes exponentials again (registers spill) 73.  D=128, N=2048 (70.0): no baton 86.7, baton after two chunks 83.7, after
-// four 75.1; one polynomial pair in 16 73.7; P handed over in three pieces 70.6.
+// four 75.1; one polynomial pair in 16 73.7; P handed over in three pieces 70.6.  Registers: head dim 64 spills 12 bytes (two tiles 16),
+// head dim 128 28 in CTAs of two tiles, none in the others.
 //
 // Split over keys: a problem with few tiles (short chunks against a long cache) is cut along the keys too; a CTA then
 // writes its unnormalised O and (m, l) per row and attn_prefill_merge_kernel puts the pieces together in order.

@@ -18,12 +18,14 @@ enum class Route { kGemv, kStream, kSmall, kGemm };
 //   M = 1: GEMV / small-batch kernel 5632x2048 4.1/4.7, 1536x8960 5.2/6.2, 2560x2048 3.7/3.7, but 8960x1536 5.0/4.8,
 //     11264x2048 8.0/7.3: the GEMV's four or eight rows per warp leave it too few warps there.
 //   16 < M <= 32: small-batch kernel / GEMM, M = 32, 5632x2048 10.2/10.7, 8960x1536 9.1/10.2, 2048x8192 9.7/11.1, 4096x4096 9.6/11.8,
-//     11264x2048 14.9/12.1, 16384x2048 19.6/12.6 (M = 17 12.2/13.1 and 16.1/13.4); its activation reads grow with M * N, the GEMM's
-//     time hardly with M.  Few rows and a long K leave a warp too many groups one after the other, while the GEMM splits K over the
-//     chip: M = 17 / 24 / 32, 512x8192 8.8/8.3, 9.1/8.4, 10.0/8.5, 512x12288 10.8/9.2, 11.5/9.4, 12.8/9.5, 1280x12288 11.4/10.8,
-//     11.7/11.1, 12.8/11.2 (the widest on that side of the line give a little away: 1536x8960 9.2/9.7, 9.5/10.1, 10.1/10.5); bf16,
-//     whose unpacking costs more: 512x6144 7.6/8.4, 7.8/8.6, 8.5/8.7, 512x8192 9.4/8.7, 9.8/8.9, 10.6/9.0, 2048x8192 8.8/12.0,
-//     9.0/11.9, 9.6/12.1.
+//     11264x2048 14.9/12.1, 16384x2048 19.6/12.6; its activation reads grow with M * N, the GEMM's time hardly with M.  Few rows and a
+//     long K leave a warp too many groups one after the other, while the GEMM splits K over the chip: M = 17 / 24 / 32, 512x8192 8.8/8.3,
+//     9.1/8.4, 10.0/8.5, 512x12288 10.8/9.2, 11.5/9.4, 12.8/9.5, 1280x12288 11.4/10.8, 11.7/11.1, 12.8/11.2; bf16, whose unpacking
+//     costs more: 512x6144 7.6/8.4, 7.8/8.6, 8.5/8.7, 512x8192 9.4/8.7, 9.8/8.9, 10.6/9.0.
+//     Both lines were drawn before K was walked in blocks of 64, which made the small-batch kernel faster, and are too low for it in
+//     places: on the GEMM's side it would be the faster one at M = 17 of 11264x2048 (12.2/13.1; not of 16384x2048, 16.1/13.4), at
+//     M = 24 and 32 of 1536x8960 (9.5/10.1, 10.1/10.5; M = 17, on its own side, 9.2/9.7), and for bf16 probably from some N between
+//     512 and 1536 on (2048x8192, on its own side, 8.8/12.0, 9.0/11.9, 9.6/12.1).
 Route route(int M, int N, int K, int dtype, bool bias) {
   const bool fp16 = dtype == KFB_F16;
   if (fp16 && N >= 75776 && !bias && M <= 16) return M <= 8 ? Route::kGemv : Route::kStream;

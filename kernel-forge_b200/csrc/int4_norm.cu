@@ -15,7 +15,8 @@
 //     561, 141 of five 513).
 //   * with RB > 1 the packed nibbles are multiplied as they are, subnormal fp16 numbers, which takes 10 clocks of unpacking per word
 //     instead of 18 (unpack_tiny; step of 22 layers 484 us -> 477; the error against 64 bits is the same, 4.41e-4 of a SiLU output).
-//     With one row block the product that makes up for the offset costs as much as it saves.
+//     With one row block the product that makes up for the offset costs as much as it saves.  (RB = 5 with groups of 128 takes all
+//     128 registers and spills 16 bytes, with NG = 2 groups of 64 32 bytes.)
 // Weights staged in shared memory with asynchronous copies instead of registers were slower (+2 us per layer), and so was
 // this structure without the norm (o and down projection: int4_small.cu, which has fewer and smaller CTAs there).
 // Step of the 22-layer model at batch 1: 593 us with separate norm kernels and the CUDA-core GEMV -> 503.  At batch 2 the step

@@ -18,9 +18,9 @@
 //     is applied in FP32 once per group, the result is rounded once.  The batch is the N = 8 of the MMA.
 //
 // Measured (graph of L2-cold calls, us; TMA / shared-memory kernels of int4_gemv_mma.cuh or the tcgen05 GEMM, whichever
-// was faster -> this kernel):  5632 x 2048 M = 8 8.6 -> 5.1, M = 16 12.4 -> 6.0, M = 32 14.5 -> 11.7;  2048 x 5632 9.5 ->
-// 5.3, 11.3 -> 5.9, 11.9 -> 8.7;  1536 x 8960 12.1 -> 6.5, 12.2 -> 7.4, 12.8 -> 11.5;  8960 x 1536 7.7 -> 5.1, 11.5 -> 6.2,
-// 16.0 -> 10.7.
+// was faster -> this kernel):  5632 x 2048 M = 8 8.6 -> 5.5, M = 16 12.4 -> 5.9, M = 32 14.5 -> 10.1;  2048 x 5632 9.5 ->
+// 4.8, 11.3 -> 5.6, 11.9 -> 7.4;  1536 x 8960 12.1 -> 6.3, 12.2 -> 7.3, 12.8 -> 10.1;  8960 x 1536 7.7 -> 5.1, 11.5 -> 6.2,
+// 16.0 -> 9.1.
 // Also built: activations staged in shared memory, K split over a cluster of CTAs and added up through distributed shared
 // memory.  It reads fewer activation bytes, but the staging, two cluster barriers and the cluster launch cost 2-3 us:
 // 5632 x 2048 M = 8 6.9 us, 1536 x 8960 M = 16 10.2 us.

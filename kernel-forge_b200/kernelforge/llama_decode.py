@@ -123,10 +123,10 @@ class LlamaInt4Decoder:
         # independently, so this is exact; prefill reads the same matrices and undoes the order with a view.
         # Batch 2 and more: the qkv and gate_up projections run on private fragment-order copies of their weights
         # (ops.prepack_int4; as much memory again), with the same pair epilogues; o and down on the public format
-        # (int4_linear).  Measured, us per step on the TinyLlama-1.1B shape at batch 3 / 8 / 16 / 32: everything on
-        # fragment-order copies 597 / 620 / 764 / 1065, this 534 / 554 / 687 / 991, gate_up by int4_linear too 577 / 610 / 739 /
-        # 994 (so at batch 32 the copy of gate_up saves no time worth its memory).
-        # (Later attention, lm_head and linear kernels, at batch 8 / 16 / 32 on 200 cached tokens: 554 / 689 / 991 -> 528 / 651 / 921.)
+        # (int4_linear).  Measured, us per step on the TinyLlama-1.1B shape on 200 cached tokens, at batch 17 / 24 / 32: this 812 / 845 /
+        # 924, gate_up by int4_linear_silu_pairs 857 / 881 / 922, no copies (RoPE and SiLU as kernels of their own) 932 / 949 / 970.  So
+        # at batch 32 the copy of gate_up saves no time worth its memory.  With earlier kernels, at batch 3 / 8 / 16: everything on
+        # copies 597 / 620 / 764, this 534 / 554 / 687, gate_up by int4_linear 577 / 610 / 739.
         # With tensor parallelism the same holds for the rank's own rows (local heads, local share of the hidden and
         # intermediate features); only the four gathers per layer are added.
         # Batch 1 on one GPU: five kernels per layer (_step_fused), both RMSNorms in the prologue of the projection behind them
