@@ -851,7 +851,10 @@ int launch(const Problem& p, const PrefillPlan& plan, const CUtensorMap& tq, con
            unsigned int* status, cudaStream_t stream) {
   if (plan.per_cta == 2) return launch_tiles<D, kBf16, 2, false>(p, plan, tq, tk, tv, partial, status, stream);
   if constexpr (D == 128) {
-    if (plan.alone) return launch_tiles<D, kBf16, 1, true>(p, plan, tq, tk, tv, partial, status, stream);
+    // A second buffer of scores has a use from two steps of keys on.  One step, us in a graph, two buffers and one: 88 heads of 3 tokens
+    // 5.17 and 4.92, 128 heads of 60 5.54 and 5.34, 32 heads of 128 5.20 and 4.99; two steps, 16 heads of 200 tokens 6.13 and 6.22.
+    const bool one_step = ceil_div(ceil_div(p.Nk, kBlockN), plan.splits) == 1;
+    if (plan.alone && !one_step) return launch_tiles<D, kBf16, 1, true>(p, plan, tq, tk, tv, partial, status, stream);
   }
   return launch_tiles<D, kBf16, 1, false>(p, plan, tq, tk, tv, partial, status, stream);
 }

@@ -27,6 +27,24 @@ def test_tiles_and_splits(b, h, hk, nq, nk, d, causal, dtype):
     assert _capi.device_status(torch.device("cuda", 0)) == 0
 
 
+# One step of keys per CTA (one buffer of scores) next to two (two buffers), grids below and above one CTA per SM, splits of one step
+ONE_STEP = [(1, 1, 1, 2, 2), (11, 8, 8, 3, 3), (2, 4, 1, 32, 127), (1, 32, 32, 128, 128), (1, 4, 4, 128, 129), (18, 8, 8, 50, 50), (19, 8, 8, 50, 50),
+            (1, 1, 1, 2, 1000), (1, 2, 2, 6, 1480)]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("b,h,hk,nq,nk", ONE_STEP)
+def test_one_step_of_keys(b, h, hk, nq, nk, causal, dtype):
+    q, k, v = qkv_case(b, h, hk, nq, nk, 128, dtype, seed=3 * nq + nk)
+    ref = torch.from_numpy(attn_oracle(q, k, v, causal))
+    q, k, v = q.cuda(), k.cuda(), v.cuda()
+    got = [ops.flash_attn(q, k, v, causal=causal) for _ in range(3)]
+    assert (got[0].float().cpu() - ref).abs().max().item() <= ATTN_ATOL[dtype]
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+    assert _capi.device_status(torch.device("cuda", 0)) == 0
+
+
 @pytest.mark.parametrize("d", [64, 128])
 def test_large_scores_and_growing_maxima(d):
     """Rows whose maximum grows by far more than the rescale threshold from step to step, and rows far below zero."""
