@@ -105,11 +105,12 @@ __device__ __forceinline__ TileOrder decode_tile_order(unsigned int block, int n
 //   * exponentials do not wait for the maximum of their step: they are taken with the base of the steps before, while the
 //     maxima of the row run under them, and in a step whose maximum outgrows the base they are taken again (the results are those
 //     of looking first).  One row of a warp's 32 is enough for that, so with scores of a standard deviation of 6 (natural units)
-//     every second step is such a step.  The first of four chunks is taken ahead, two chunks only in head dim 128 CTAs of two tiles,
-//     where the baton makes one chunk too short (us, scores of deviation 1 / 3 / 6, looking first - two chunks ahead - one: 2 x 16 x
-//     2048 D=64 56.9 / 58.5 / 61.6 - 53.1 / 58.6 / 72.8 - 52.9 / 55.8 / 64.0; 4 heads x 5806 causal D=64 45.2 / 45.7 / 47.8 - 44.0 / 48.8 /
-//     63.7 - 44.4 / 45.4 / 52.3; 1 x 16 x 2048 causal D=128 33.3 / 33.8 / 35.4 - 27.0 / 28.5 / 33.0 - 27.0 / 28.1 / 31.7; 2 x 16 x 2048 D=128
-//     73.9 / 75.4 / 80.1 - 68.0 / 75.7 / 96.5 - 73.6 / 79.1 / 95.8).  Going back to looking first after two grown steps in a row helps
+//     every second step is such a step.  The first of four chunks is taken ahead, two in head dim 128 CTAs of two tiles, where the
+//     baton makes one chunk too short, and of two score buffers, where one costs short calls more than it gives (us, scores of
+//     deviation 1 / 3 / 6, looking first - two chunks ahead - one: 2 x 16 x 2048 D=64 56.9 / 58.5 / 61.6 - 53.1 / 58.6 / 72.8 - 52.9 /
+//     55.8 / 64.0; 4 heads x 5806 causal D=64 45.2 / 45.7 / 47.8 - 44.0 / 48.8 / 63.7 - 44.4 / 45.4 / 52.3; 1 x 16 x 2048 causal D=128
+//     33.3 / 33.8 / 35.4 - 27.0 / 28.5 / 33.0 - 27.0 / 28.1 / 31.7; 2 x 16 x 314 causal D=128 8.8 / 8.9 / 9.2 - 7.8 / 8.3 / 9.1 - 8.0 / 8.2 /
+//     8.8; 2 x 16 x 2048 D=128 73.9 / 75.4 / 80.1 - 68.0 / 75.7 / 96.5 - 73.6 / 79.1 / 95.8).  Going back to looking first after two grown steps in a row helps
 //     there (92.5 at 6, 85 at 30 instead of 98) but costs every call (8192 causal 550 us -> 556).  Only the first step looks first;
 //   * the scores are loaded in chunks of 32, one ahead.  Head dim 64 releases the S buffer after the last, and QK(j+1) runs
 //     under step j; P has columns of its own;
@@ -237,7 +238,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   constexpr int S = L::kStages, kHalves = L::kHalves;
   constexpr bool kAliasP = L::kAliasP;
   constexpr bool kBaton = NT == 2;               // the two tiles take turns
-  constexpr int kGuess = D == 128 && NT == 2 ? 2 : 1;   // chunks whose exponentials do not wait for the step's maximum
+  constexpr int kGuess = D == 128 && (NT == 2 || kDouble) ? 2 : 1;   // chunks whose exponentials do not wait for the step's maximum
   constexpr int kOrder = D == 64 && NT == 1 ? 7 : 5;    // pairs of a chunk are taken in the order e * kOrder (see chunk)
   constexpr int kBatonAfter = kAliasP ? 2 : 1;   // the chunk after which the other tile may start
   extern __shared__ uint8_t smem_raw[];
@@ -617,8 +618,9 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         for (int c = 0; c < kGuess; ++c) {
           tmem_wait_ld_regs(v[c]);
           mask(c);
-          chunk(c);
         }
+#pragma unroll
+        for (int c = 0; c < kGuess; ++c) chunk(c);
       }
       if (kGuess == 1) chunk(1);
       if constexpr (!kAliasP) {   // the S buffer can take the next product already
