@@ -815,7 +815,13 @@ PrefillPlan plan_prefill(const Problem& p, int max_splits = 32) {
         const Kind& left = slots > sms && last <= sms ? kinds[1] : k;
         cost = (double)(ctas / slots) * (longest * k.step + k.wave) + (last ? longest * left.step + left.wave : 0.0);
       }
-      if (s > 1) cost += (wide ? 3.2 : 2.4) + s * merge_us;
+      if (s > 1) {
+        double merge = (wide ? 3.2 : 2.4) + s * merge_us;
+        // Pieces of one step have a cheaper kernel, which counts where they are few and short of rows (4 steps, in one piece and in four:
+        // 2 x 32 heads over 4 x 2 queries 7.9 and 7.5, 8 heads x 20 7.6 and 7.4, 32 heads x 4 7.85 and 7.77, but 8 heads x 100 8.4 and 9.0).
+        if (wide && k.alone && longest == 1) merge = std::min(merge, 1.8 + s * (0.43 + 2.5 * (merge_us - 0.30)));
+        cost += merge;
+      }
       if (cost < best) { best = cost; c.per_cta = k.per_cta; c.splits = s; c.alone = k.alone; }
     }
   return c;

@@ -29,7 +29,7 @@ def test_tiles_and_splits(b, h, hk, nq, nk, d, causal, dtype):
 
 # One step of keys per CTA (one buffer of scores) next to two (two buffers), grids below and above one CTA per SM, splits of one step
 ONE_STEP = [(1, 1, 1, 2, 2), (11, 8, 8, 3, 3), (2, 4, 1, 32, 127), (1, 32, 32, 128, 128), (1, 4, 4, 128, 129), (18, 8, 8, 50, 50), (19, 8, 8, 50, 50),
-            (1, 1, 1, 2, 1000), (1, 2, 2, 6, 1480)]
+            (1, 1, 1, 2, 1000), (1, 2, 2, 6, 1480), (2, 32, 4, 2, 422), (1, 8, 8, 20, 385), (1, 8, 8, 100, 512)]
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
