@@ -183,14 +183,14 @@ def prepack_weight_(packed: torch.Tensor) -> torch.Tensor:
 
 def _prepacked_wins(m: int, n: int, k: int) -> bool:
     """Where a weight with a private copy runs on it: from M = 2 on, and at M = 1 unless N is small and K long.  Measured
-    (B200, graph of L2-cold calls, us on the public format / on the copy at M = 1, 2, 8, 16, 32):
-        5632 x 2048   4.0 / 3.8   5.1 / 3.9   5.5 / 4.1    6.0 / 6.0   11.4 / 10.6
-        2560 x 2048   3.5 / 2.9   3.5 / 3.0   3.7 / 3.1    4.4 / 3.9    6.3 / 6.5
-       11264 x 2048   7.4 / 5.7   7.4 / 6.0   8.2 / 6.0   10.6 / 9.2   12.3 / 16.0
-        2048 x 5632   5.8 / 5.7   4.6 / 5.8   4.8 / 6.0    5.7 / 6.8    8.3 / 8.5
-        1536 x 8960   5.0 / 8.0   6.1 / 8.0   6.3 / 8.6    7.3 / 9.6   11.2 / 11.9
+    (B200, graph of L2-cold calls, us on the public format / on the copy at M = 1, 2, 8, 16, 24, 32):
+        5632 x 2048   4.0 / 3.8   5.1 / 3.9   5.4 / 4.1    5.9 / 6.0    8.4 / 9.3   10.1 / 10.3
+        2560 x 2048   3.3 / 2.9   3.4 / 2.9   3.6 / 3.1    4.3 / 3.8    5.2 / 5.8    5.6 / 6.4
+       11264 x 2048   7.3 / 5.9   7.4 / 5.9   8.2 / 6.0   10.4 / 9.1   13.1 / 14.3  12.1 / 16.0
+        2048 x 5632   5.7 / 5.7   4.6 / 5.7   4.7 / 6.0    5.5 / 6.8    7.1 / 7.9    7.4 / 8.4
+        1536 x 8960   5.0 / 8.0   6.1 / 8.1   6.2 / 8.6    7.3 / 9.7   10.0 / 11.2  10.5 / 11.8
     So the copy pays at K = 2048 up to 16 rows; at a longer K with few rows (96 to 128 CTAs, 11 to 18 blocks of K per warp)
-    and for many rows at M = 32 the public kernels have become the faster ones, and a weight of that kind is better left
+    and above 16 rows the public kernels have become the faster ones, and a weight that is used so is better left
     without a copy."""
     return m >= 2 or n * 8 >= k * 5
 
